@@ -39,6 +39,24 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// v[0..V-1] summed over the warp; the lane's result belongs to index lane >> (5 - log2 V) (V <= 32)
+template <int V>
+__device__ __forceinline__ float warp_fold(float (&v)[V], int lane) {
+  int off = 16;
+#pragma unroll
+  for (int n = V; n > 1; n >>= 1, off >>= 1) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int i = 0; i < n / 2; ++i) {
+      const float keep = up ? v[i + n / 2] : v[i], send = up ? v[i] : v[i + n / 2];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+  float s = v[0];
+  for (; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+  return s;
+}
+
 // Block-wide sum with a fixed order (lanes by butterfly, then warps in index order).
 // `red` is shared memory of at least 33 floats. All threads get the result.
 __device__ __forceinline__ float block_sum(float v, float* red) {

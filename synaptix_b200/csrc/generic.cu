@@ -253,6 +253,223 @@ __global__ void __launch_bounds__(128) gemm_rows_kernel(const TA* __restrict__ A
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// The float32 product, rows of whole 16-byte pieces (K % 4 == 0, aligned operands): the same FFMA arithmetic, every sum in
+// 32-bit, in an order fixed by the sizes.
+//
+// Up to 16 rows: gemm_rows_f32_kernel streams W once.  A warp owns four rows of W and every KS-th 128-wide slice of K (the KS
+// warps of a group cover a row, so a narrow matrix still puts some 16 warps on every SM and a row's bytes are all on their way
+// at once); A comes through L1; the 4 x MR sums of a warp fold over its lanes in V - 1 shuffles (each step halves the values a
+// lane keeps) and over the warps in order.  Bound by HBM: N x K x 4 bytes.  Two rows, weights from HBM: 4,096 x 1,024 4.6 us (3.6
+// TB/s), 1,024 x 3,072 4.3 us, 151,936 x 1,024 98 us (6.3 TB/s); a warp per row of W with 4-byte loads, one in flight, took 45 us
+// over a step's products on average where this takes 8.
+// ---------------------------------------------------------------------------------------
+template <int MR, int KS>
+__global__ void __launch_bounds__(256, MR <= 2 ? 4 : (MR == 4 ? 3 : 2)) gemm_rows_f32_kernel(const float* __restrict__ A, const float* __restrict__ W,
+                                                            float* __restrict__ C, int M, int N, int K,
+                                                            const float* __restrict__ bias, float cap) {
+  constexpr int R = 4, GROUPS = 8 / KS, V = MR * R, FV = V < 32 ? V : 32;
+  __shared__ float part[8][V];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, group = warp / KS, ks = warp % KS;
+  const int n0 = (blockIdx.x * GROUPS + group) * R;
+  const float* wr[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) wr[r] = W + (size_t)min(n0 + r, N - 1) * K;
+  float acc[MR][R];
+#pragma unroll
+  for (int i = 0; i < MR; ++i)
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[i][r] = 0.f;
+  pdl_wait();
+  pdl_trigger();
+#pragma unroll (MR <= 2 ? 2 : 1)
+  for (int k = (ks * 32 + lane) * 4; k < K; k += KS * 128) {
+    float4 w[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) w[r] = __ldg(reinterpret_cast<const float4*>(wr[r] + k));
+#pragma unroll
+    for (int i = 0; i < MR; ++i) {
+      const float4 a = *reinterpret_cast<const float4*>(A + (size_t)min(i, M - 1) * K + k);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        acc[i][r] = fmaf(a.w, w[r].w, fmaf(a.z, w[r].z, fmaf(a.y, w[r].y, fmaf(a.x, w[r].x, acc[i][r]))));
+    }
+  }
+#pragma unroll
+  for (int b = 0; b < V / FV; ++b) {
+    float v[FV];
+#pragma unroll
+    for (int i = 0; i < FV; ++i) v[i] = acc[(b * FV + i) / R][i % R];
+    const float s = warp_fold<FV>(v, lane);
+    constexpr int REP = 32 / FV;               // lanes that hold the same sum
+    if (lane % REP == 0) part[warp][b * FV + lane / REP] = s;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < GROUPS * V; i += 256) {
+    const int g = i / V, m = (i % V) / R, n = (blockIdx.x * GROUPS + g) * R + i % R;
+    if (m >= M || n >= N) continue;
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < KS; ++w) s += part[g * KS + w][i % V];
+    C[(size_t)m * N + n] = soft_limit(bias ? s + bias[n] : s, cap);
+  }
+}
+
+// More rows: gemm_tile_f32_kernel, tiles of (8 TM) x 128 by 128 threads, TM x 8 sums a thread, slices of 16 of K through a ring
+// of four stages (cp.async, rows padded to 80 bytes so that eight neighbouring rows' 16-byte pieces fall on different banks).
+// Two products of neighbouring k go through one packed multiply-add (fma.rn.f32x2, each half rounded as fmaf rounds it): the sums
+// over even and odd k are kept apart and added at the end.  Where tiles are few, K is shared by the blocks of a cluster (grid x =
+// column tile * cluster), which lay their partial tiles into shared memory and add them up in block order, each a share of the
+// rows.  Bound by shared-memory reads and the FP32 pipe together: 37 TFLOP/s at 1,024 rows of 6,144 x 1,024 (350 us), 28 at 263
+// rows of 4,096 x 1,024 (78 us); the 64 x 64 tiles of 4 x 4 sums a thread below took 218 us over a 263-row step's products on
+// average where these take 80.
+#define F32_BK 16
+#define F32_STAGES 4
+#define F32_ROW 20                               // floats a staged row takes
+__device__ __forceinline__ void f32_cp16(uint32_t dst, const void* src, bool live) {
+  const int bytes = live ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void f32_fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(d) : "l"(a), "l"(b));
+}
+struct f32_quad { unsigned long long lo, hi; };  // four floats as two pairs
+
+template <int TM>
+__global__ void __launch_bounds__(128, TM == 4 ? 3 : 2) gemm_tile_f32_kernel(const float* __restrict__ A, const float* __restrict__ W,
+                                                            float* __restrict__ C, int M, int N, int K,
+                                                            const float* __restrict__ bias, float cap, int cluster) {
+  constexpr int BM = 8 * TM, BN = 128, ROWS = BM + BN, STAGE = ROWS * F32_ROW;
+  extern __shared__ __align__(16) float f32_smem[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int mi = (warp & 1) * 4 + (lane >> 3), ni = (warp >> 1) * 8 + (lane & 7);
+  const int m0 = blockIdx.y * BM, n0 = (blockIdx.x / cluster) * BN, z = blockIdx.x % cluster;
+  const int nkb_all = (K + F32_BK - 1) / F32_BK, kper = (nkb_all + cluster - 1) / cluster;
+  const int kb0 = z * kper, nkb = max(0, min(nkb_all, kb0 + kper) - kb0);
+  const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(f32_smem);
+  auto load = [&](int kb, int s) {
+#pragma unroll
+    for (int i = 0; i < ROWS * 4 / 128; ++i) {
+      const int idx = tid + i * 128, r = idx >> 2, c = idx & 3, k = (kb0 + kb) * F32_BK + c * 4;
+      const bool is_a = r < BM;
+      const int row = is_a ? m0 + r : n0 + r - BM;
+      const bool live = row < (is_a ? M : N) && k < K;
+      const float* src = is_a ? A : W;
+      f32_cp16(smem0 + (uint32_t)(s * STAGE + r * F32_ROW + c * 4) * 4, live ? src + (size_t)row * K + k : src, live);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  unsigned long long acc[TM][8];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
+  pdl_wait();
+  pdl_trigger();
+#pragma unroll
+  for (int s = 0; s < F32_STAGES - 1; ++s) {
+    if (s < nkb) load(s, s);
+    else asm volatile("cp.async.commit_group;\n" ::: "memory");
+  }
+  for (int kb = 0; kb < nkb; ++kb) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(F32_STAGES - 2) : "memory");
+    __syncthreads();
+    if (kb + F32_STAGES - 1 < nkb) load(kb + F32_STAGES - 1, (kb + F32_STAGES - 1) % F32_STAGES);
+    else asm volatile("cp.async.commit_group;\n" ::: "memory");
+    const float* as = f32_smem + (kb % F32_STAGES) * STAGE + mi * F32_ROW;
+    const float* ws = f32_smem + (kb % F32_STAGES) * STAGE + (BM + ni) * F32_ROW;
+#pragma unroll
+    for (int kk = 0; kk < F32_BK; kk += 4) {
+      f32_quad a[TM];
+#pragma unroll
+      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const f32_quad*>(as + 8 * i * F32_ROW + kk);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const f32_quad w = *reinterpret_cast<const f32_quad*>(ws + 16 * j * F32_ROW + kk);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) f32_fma2(acc[i][j], a[i].lo, w.lo);
+#pragma unroll
+        for (int i = 0; i < TM; ++i) f32_fma2(acc[i][j], a[i].hi, w.hi);
+      }
+    }
+  }
+  float out[TM][8];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float lo, hi;
+      asm("mov.b64 {%0, %1}, %2;\n" : "=f"(lo), "=f"(hi) : "l"(acc[i][j]));
+      out[i][j] = lo + hi;
+    }
+  if (cluster == 1) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+      const int m = m0 + mi + 8 * i;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int n = n0 + ni + 16 * j;
+        if (m < M && n < N) C[(size_t)m * N + n] = soft_limit(bias ? out[i][j] + bias[n] : out[i][j], cap);
+      }
+    }
+    return;
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();                                // the ring has been read: the partial tile goes over it
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f32_smem[(mi + 8 * i) * BN + ni + 16 * j] = out[i][j];
+  cluster_sync_all();
+  const int per = (BM + cluster - 1) / cluster, r1 = min(BM, (z + 1) * per);
+  for (int r = z * per; r < r1; ++r) {
+    const int m = m0 + r, n = n0 + tid;
+    if (m >= M) break;
+    float s = 0.f;
+    for (int c = 0; c < cluster; ++c) s += cluster_load_f32(f32_smem + r * BN + tid, (uint32_t)c);
+    if (n < N) C[(size_t)m * N + n] = soft_limit(bias ? s + bias[n] : s, cap);
+  }
+  cluster_sync_all();                             // nobody's shared memory goes away while it is read
+}
+
+template <int MR>
+static int gemm_rows_f32_launch(const float* A, const float* W, float* C, int M, int N, int K, const float* bias, float cap,
+                                cudaStream_t stream) {
+  const int tiles = (N + 3) / 4;
+  if (K >= 1024) return sx_launch(gemm_rows_f32_kernel<MR, 8>, dim3(tiles), dim3(256), 0, stream, A, W, C, M, N, K, bias, cap);
+  if (K >= 256) return sx_launch(gemm_rows_f32_kernel<MR, 2>, dim3((tiles + 3) / 4), dim3(256), 0, stream, A, W, C, M, N, K, bias, cap);
+  return sx_launch(gemm_rows_f32_kernel<MR, 1>, dim3((tiles + 7) / 8), dim3(256), 0, stream, A, W, C, M, N, K, bias, cap);
+}
+
+template <int TM>
+static int gemm_tile_f32_launch(const float* A, const float* W, float* C, int M, int N, int K, const float* bias, float cap,
+                                cudaStream_t stream) {
+  constexpr int BM = 8 * TM, BN = 128;
+  const long long tiles_n = (N + BN - 1) / BN, tiles_m = (M + BM - 1) / BM, tiles = tiles_n * tiles_m;
+  // About a block an SM is enough (263 x 1,024 x 3,072 in tiles of 32 rows: 72 blocks 127 us, 144 in clusters of two 71, 288 in
+  // clusters of four 82); every block of a cluster keeps at least 128 of K.
+  int cluster = 1;
+  while (cluster < 8 && tiles * cluster < 140 && K >= 256 * cluster) cluster *= 2;
+  const size_t ring = (size_t)F32_STAGES * (BM + BN) * F32_ROW * sizeof(float);
+  cudaError_t e = cudaFuncSetAttribute(gemm_tile_f32_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring);
+  if (e != cudaSuccess) return (int)e;
+  const dim3 grid((unsigned)(tiles_n * cluster), (unsigned)tiles_m);
+  if (cluster == 1) return sx_launch(gemm_tile_f32_kernel<TM>, grid, dim3(128), ring, stream, A, W, C, M, N, K, bias, cap, 1);
+  return sx_launch_cluster(gemm_tile_f32_kernel<TM>, grid, dim3(128), ring, stream, cluster, A, W, C, M, N, K, bias, cap, cluster);
+}
+
+static int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, const float* bias, float cap, cudaStream_t stream) {
+  if (M <= 1) return gemm_rows_f32_launch<1>(A, W, C, M, N, K, bias, cap, stream);
+  if (M <= 2) return gemm_rows_f32_launch<2>(A, W, C, M, N, K, bias, cap, stream);
+  if (M <= 4) return gemm_rows_f32_launch<4>(A, W, C, M, N, K, bias, cap, stream);
+  if (M <= 8) return gemm_rows_f32_launch<8>(A, W, C, M, N, K, bias, cap, stream);
+  if (M <= 16) return gemm_rows_f32_launch<16>(A, W, C, M, N, K, bias, cap, stream);
+  // Tiles of 64 rows only where they come to two a SM (1,024 x 6,144 x 1,024: 350 us; 263 x 4,096 x 1,024: 98 us, 78 in tiles of
+  // 32 rows, which waste less of the last tile and keep more warps an SM).
+  if (((M + 63) / 64) * ((N + 127LL) / 128) < 296) return gemm_tile_f32_launch<4>(A, W, C, M, N, K, bias, cap, stream);
+  return gemm_tile_f32_launch<8>(A, W, C, M, N, K, bias, cap, stream);
+}
+
 template <typename TA, typename TW, typename TC>
 static int gemm_generic_launch(const void* A, const void* W, void* C, int M, int N, int K, const float* bias, float cap,
                                cudaStream_t stream) {
@@ -270,6 +487,9 @@ extern "C" int sx_gemm_generic(const void* A, int a_dt, const void* W, int w_dt,
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return SX_ERR_SIZE;
   if ((size_t)((M + 63) / 64) > 65535) return SX_ERR_SIZE;
+  // (whole, aligned 16-byte pieces of every row, or the kernels that take every size)
+  if (a_dt == SX_F32 && w_dt == SX_F32 && c_dt == SX_F32 && (K & 3) == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0)
+    return gemm_f32((const float*)A, (const float*)W, (float*)C, M, N, K, bias, cap, stream);
   if (a_dt == SX_F32 && w_dt == SX_F32 && c_dt == SX_F32)
     return gemm_generic_launch<float, float, float>(A, W, C, M, N, K, bias, cap, stream);
   if (a_dt == SX_BF16 && w_dt == SX_BF16 && c_dt == SX_BF16)
@@ -751,6 +971,209 @@ __global__ void __launch_bounds__(128) attn_generic_kernel(
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// The float32 form of the kernel above for heads of 64 and 128 (keys and values alike): eight lanes share a key, so that a
+// key's or value's row is read in whole 128-byte lines, and the R query rows of a block (the heads that share a kv head; with
+// fewer heads than R also neighbouring tokens of the same sequence) read it once.  Every group of eight lanes is an online
+// softmax of its own over every 32nd (times the cluster's blocks) key; the groups, warps and blocks are merged at the end,
+// in order.  A few tokens: the keys are shared by the blocks of a cluster too.  Bound by the latency of a few dependent loads in
+// single-token steps: 14 us where the plain kernel, in which a thread walks a whole key alone, 4 bytes a load and each lane on
+// lines of its own, took 55 (steps of 2 and of 263 tokens, 16 heads, up to 158 keys).
+// ---------------------------------------------------------------------------------------
+template <int HD, int R>
+__global__ void __launch_bounds__(256) attn_f32_kernel(
+    const float* __restrict__ q, const float* __restrict__ k_pages, const float* __restrict__ v_pages, float* __restrict__ out,
+    const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ block_table, int maxp,
+    int n_tokens, int nh, int nkv, float scale, int window, float softcap, const float* __restrict__ sinks, int chunk,
+    int out_stride, float out_scale, int tpb, int cluster) {
+  constexpr int C4 = HD / 32;                     // 16-byte pieces a lane holds of a head
+  __shared__ float s_acc[8][R][HD];
+  __shared__ float s_ml[8][R][2], s_blk[R][2];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7, grp = lane >> 3;
+  const int G = nh / nkv, hg = (G + R - 1) / R;   // blocks that share a kv head's query heads (1 when tpb > 1)
+  const int kvh = blockIdx.y / hg, h0 = (blockIdx.y % hg) * R;
+  const int t0 = blockIdx.z * tpb, rank = blockIdx.x;
+  const int stream0 = (rank * 8 + warp) * 4 + grp, streams = cluster * 32;
+  pdl_wait();
+  pdl_trigger();
+  int first = 0;                                  // tokens of one sequence at a time
+  const int n_here = min(tpb, n_tokens - t0);
+  while (first < n_here) {
+    const int seq = seq_of_token[t0 + first];
+    int end = first + 1;
+    while (end < n_here && seq_of_token[t0 + end] == seq) ++end;
+    const int* bt = block_table + (size_t)seq * maxp;
+    int pos[R], lo[R];
+    float4 qv[R][C4], acc[R][C4];
+    float m[R], l[R];
+    int jlo = 0x7fffffff, jhi = -1;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int tok = tpb > 1 ? r / G : 0, head = tpb > 1 ? r % G : h0 + r;
+      const bool live = tok >= first && tok < end && head < G;
+      pos[r] = live ? positions[t0 + tok] : -1;
+      lo[r] = window > 0 ? max(0, pos[r] - window + 1) : 0;
+      if (chunk > 0 && live) lo[r] = max(lo[r], (pos[r] / chunk) * chunk);
+      if (live) { jlo = min(jlo, lo[r]); jhi = max(jhi, pos[r]); }
+      m[r] = -INFINITY; l[r] = 0.f;
+#pragma unroll
+      for (int c = 0; c < C4; ++c) {
+        acc[r][c] = qv[r][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (live) qv[r][c] = *reinterpret_cast<const float4*>(q + ((size_t)(t0 + tok) * nh + kvh * G + head) * HD + (c * 8 + sub) * 4);
+      }
+    }
+    auto row_of = [&](int j) { return (((size_t)bt[j >> 6] * nkv + kvh) * SX_PAGE + (j & 63)) * HD + sub * 4; };
+    float4 kc[C4], vc[C4];
+    auto fetch = [&](int j) {
+      if (j <= jhi) {
+        const size_t at = row_of(j);
+#pragma unroll
+        for (int c = 0; c < C4; ++c) kc[c] = *reinterpret_cast<const float4*>(k_pages + at + c * 32);
+#pragma unroll
+        for (int c = 0; c < C4; ++c) vc[c] = *reinterpret_cast<const float4*>(v_pages + at + c * 32);
+      } else {
+#pragma unroll
+        for (int c = 0; c < C4; ++c) kc[c] = vc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    };
+    // (the warp's groups walk together: the sums over eight lanes are whole-warp shuffles)
+    const int j_warp = jlo + (rank * 8 + warp) * 4;
+    fetch(jlo + stream0);
+    for (int jw = j_warp; jw <= jhi; jw += streams) {
+      const int j = jw + grp;
+      float s[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float d = 0.f;
+#pragma unroll
+        for (int c = 0; c < C4; ++c)
+          d = fmaf(qv[r][c].w, kc[c].w, fmaf(qv[r][c].z, kc[c].z, fmaf(qv[r][c].y, kc[c].y, fmaf(qv[r][c].x, kc[c].x, d))));
+        s[r] = d;
+      }
+      float4 v[C4];
+#pragma unroll
+      for (int c = 0; c < C4; ++c) v[c] = vc[c];
+      fetch(j + streams);                         // the next key is on its way behind the softmax
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
+        s[r] *= scale;
+        if (softcap > 0.f) s[r] = softcap * tanhf(s[r] / softcap);
+        if (j > pos[r] || j < lo[r]) continue;
+        const float m_new = fmaxf(m[r], s[r]);
+        const float corr = m[r] == -INFINITY ? 0.f : expf(m[r] - m_new), p = expf(s[r] - m_new);
+        m[r] = m_new;
+        l[r] = fmaf(l[r], corr, p);
+#pragma unroll
+        for (int c = 0; c < C4; ++c) {
+          acc[r][c].x = fmaf(p, v[c].x, acc[r][c].x * corr); acc[r][c].y = fmaf(p, v[c].y, acc[r][c].y * corr);
+          acc[r][c].z = fmaf(p, v[c].z, acc[r][c].z * corr); acc[r][c].w = fmaf(p, v[c].w, acc[r][c].w * corr);
+        }
+      }
+    }
+    // the four groups of the warp, then its result to shared memory
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+#pragma unroll
+      for (int o = 8; o < 32; o <<= 1) {
+        const float mo = __shfl_xor_sync(0xffffffffu, m[r], o), lo_ = __shfl_xor_sync(0xffffffffu, l[r], o);
+        const float mx = fmaxf(m[r], mo);
+        const float a = m[r] == -INFINITY ? 0.f : expf(m[r] - mx), b = mo == -INFINITY ? 0.f : expf(mo - mx);
+        l[r] = l[r] * a + lo_ * b;
+        m[r] = mx;
+#pragma unroll
+        for (int c = 0; c < C4; ++c) {
+          acc[r][c].x = acc[r][c].x * a + __shfl_xor_sync(0xffffffffu, acc[r][c].x, o) * b;
+          acc[r][c].y = acc[r][c].y * a + __shfl_xor_sync(0xffffffffu, acc[r][c].y, o) * b;
+          acc[r][c].z = acc[r][c].z * a + __shfl_xor_sync(0xffffffffu, acc[r][c].z, o) * b;
+          acc[r][c].w = acc[r][c].w * a + __shfl_xor_sync(0xffffffffu, acc[r][c].w, o) * b;
+        }
+      }
+      if (grp == 0) {
+#pragma unroll
+        for (int c = 0; c < C4; ++c) *reinterpret_cast<float4*>(&s_acc[warp][r][(c * 8 + sub) * 4]) = acc[r][c];
+        if (sub == 0) { s_ml[warp][r][0] = m[r]; s_ml[warp][r][1] = l[r]; }
+      }
+    }
+    __syncthreads();
+    // the block's warps; with a cluster the result stays in shared memory (in the place of warp 0's, which only this thread reads)
+    for (int i = threadIdx.x; i < R * HD; i += 256) {
+      const int r = i / HD, d = i % HD;
+      const int tok = tpb > 1 ? r / G : 0, head = tpb > 1 ? r % G : h0 + r;
+      const bool live = tok >= first && tok < end && head < G;
+      const int h = kvh * G + head;
+      float mx = cluster == 1 && sinks && live ? sinks[h] : -INFINITY;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) mx = fmaxf(mx, s_ml[w][r][0]);
+      float sum = cluster == 1 && sinks && live ? expf(sinks[h] - mx) : 0.f, o = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        const float f = s_ml[w][r][0] == -INFINITY ? 0.f : expf(s_ml[w][r][0] - mx);
+        sum = fmaf(s_ml[w][r][1], f, sum);
+        o = fmaf(s_acc[w][r][d], f, o);
+      }
+      if (cluster == 1) {
+        if (live) out[(size_t)(t0 + tok) * out_stride + (size_t)h * HD + d] = o / sum * out_scale;
+      } else {
+        s_acc[0][r][d] = o;
+        if (d == 0) { s_blk[r][0] = mx; s_blk[r][1] = sum; }
+      }
+    }
+    if (cluster > 1) {
+      cluster_sync_all();
+      // block `rank` finishes every cluster-th piece of 256 elements
+      for (int i = threadIdx.x + rank * 256; i < R * HD; i += 256 * cluster) {
+        const int r = i / HD, d = i % HD, head = h0 + r;
+        if (head >= G) continue;
+        const int h = kvh * G + head;
+        float mb[8], lb[8], ob[8];
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+          const uint32_t from = (uint32_t)min(b, cluster - 1);
+          mb[b] = cluster_load_f32(&s_blk[r][0], from);
+          lb[b] = cluster_load_f32(&s_blk[r][1], from);
+          ob[b] = cluster_load_f32(&s_acc[0][r][d], from);
+        }
+        float mx = sinks ? sinks[h] : -INFINITY;
+#pragma unroll
+        for (int b = 0; b < 8; ++b) mx = fmaxf(mx, mb[b]);
+        float sum = sinks ? expf(sinks[h] - mx) : 0.f, o = 0.f;
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+          const float f = b < cluster && mb[b] != -INFINITY ? expf(mb[b] - mx) : 0.f;
+          sum = fmaf(lb[b], f, sum);
+          o = fmaf(ob[b], f, o);
+        }
+        out[(size_t)t0 * out_stride + (size_t)h * HD + d] = o / sum * out_scale;
+      }
+      cluster_sync_all();                         // nobody's shared memory goes away while it is read
+    } else {
+      __syncthreads();
+    }
+    first = end;
+  }
+}
+
+template <int HD, int R>
+static int attn_f32_launch(const float* q, const float* k, const float* v, float* out, const int* positions, const int* seq_of_token,
+                           const int* block_table, int maxp, int n_tokens, int nh, int nkv, float scale, int window, float softcap,
+                           const float* sinks, int chunk, int out_stride, float out_scale, cudaStream_t stream) {
+  const int G = nh / nkv, hg = (G + R - 1) / R;
+  // Few tokens: one a block, and the keys shared by up to eight blocks.  Tokens enough for every SM: as many neighbours a block as
+  // fit its rows (a cluster's blocks finish ONE token).
+  int tpb = 1, cluster = 1;
+  const long long blocks = (long long)nkv * hg * n_tokens;
+  while (cluster < 8 && blocks * cluster < 148 && maxp >= 2 * cluster) cluster *= 2;
+  if (cluster == 1 && G < R && R % G == 0 && blocks >= 148 * (R / G)) tpb = R / G;
+  const dim3 grid((unsigned)cluster, (unsigned)(nkv * hg), (unsigned)((n_tokens + tpb - 1) / tpb));
+  if (cluster > 1)
+    return sx_launch_cluster(attn_f32_kernel<HD, R>, grid, dim3(256), 0, stream, cluster, q, k, v, out, positions, seq_of_token, block_table,
+                             maxp, n_tokens, nh, nkv, scale, window, softcap, sinks, chunk, out_stride, out_scale, tpb, cluster);
+  return sx_launch(attn_f32_kernel<HD, R>, grid, dim3(256), 0, stream, q, k, v, out, positions, seq_of_token, block_table, maxp,
+                   n_tokens, nh, nkv, scale, window, softcap, sinks, chunk, out_stride, out_scale, tpb, 1);
+}
+
 static int attn_generic_any(const void* q, const void* k_pages, const void* v_pages, void* out,
                             const int* positions, const int* seq_of_token, const int* block_table,
                             int maxp, int n_tokens, int nh, int nkv, int hd, float scale, int window,
@@ -759,6 +1182,15 @@ static int attn_generic_any(const void* q, const void* k_pages, const void* v_pa
   if (n_tokens <= 0) return 0;
   if (hd <= 0 || hd > 512 || vd <= 0 || vd > 512 || nkv <= 0 || nh % nkv != 0 || nh > 65535 || out_stride < nh * vd)
     return SX_ERR_SIZE;
+  if (dt == SX_F32 && hd == vd && (hd == 64 || hd == 128) && n_tokens <= 65535 && nkv <= 8191 &&
+      (((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0) {
+#define ATTN_F32(HD, R) attn_f32_launch<HD, R>((const float*)q, (const float*)k_pages, (const float*)v_pages, (float*)out, positions, \
+                                               seq_of_token, block_table, maxp, n_tokens, nh, nkv, scale, window, softcap, sinks, chunk, \
+                                               out_stride, out_scale, stream)
+    if (nh / nkv <= 2) return hd == 64 ? ATTN_F32(64, 2) : ATTN_F32(128, 2);
+    return hd == 64 ? ATTN_F32(64, 4) : ATTN_F32(128, 4);
+#undef ATTN_F32
+  }
   dim3 grid(n_tokens, nh);
   const size_t smem = (size_t)(hd + 128) * sizeof(float);
   if (dt == SX_F32)
