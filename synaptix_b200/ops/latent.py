@@ -3,7 +3,7 @@
 float32."""
 from __future__ import annotations
 
-from typing import Optional
+from typing import Optional, Tuple
 
 import torch
 
@@ -80,18 +80,38 @@ class WeightedLatents:
 _SMS = {}
 
 
+def _sm_count(device) -> int:
+    idx = device.index or 0
+    if idx not in _SMS:
+        _SMS[idx] = torch.cuda.get_device_properties(device).multi_processor_count
+    return _SMS[idx]
+
+
 def _pick_latent_splits(ctx, heads: int, window: Optional[int], device) -> int:
     """Parts of the window for single-token steps, so that the blocks fill the SMs about twice; prompts take one."""
     if not ctx.all_single:
         return 1
     keys = ctx.max_len if window is None else min(ctx.max_len, int(window))
     tiles = (keys + 31) // 32
-    idx = device.index or 0
-    if idx not in _SMS:
-        _SMS[idx] = torch.cuda.get_device_properties(device).multi_processor_count
     blocks = ctx.n_tokens * ((heads + 7) // 8)
-    want = (2 * _SMS[idx] + blocks - 1) // blocks
+    want = (2 * _sm_count(device) + blocks - 1) // blocks
     return max(1, min(want, tiles // 2, 16))
+
+
+def _pick_latent_shares(ctx, heads: int, window: Optional[int], device) -> Tuple[int, int]:
+    """``(parts, cluster)`` for the tensor-core kernel (16 heads a block): blocks that share a token's window, so that a step of
+    few sequences fills the SMs about once, each with at least one tile of 32 keys.  Up to eight of them are a cluster that
+    merges among itself; more leave parts for the output kernel."""
+    if not ctx.all_single:
+        return 1, 1
+    keys = ctx.max_len if window is None else min(ctx.max_len, int(window))
+    tiles = (keys + 31) // 32
+    blocks = ctx.n_tokens * ((heads + 15) // 16)
+    want = max(1, min((_sm_count(device) + blocks // 2) // blocks, tiles, 64))
+    cluster = 1
+    while cluster < 8 and cluster * 2 <= want:
+        cluster *= 2
+    return max(1, want // cluster), cluster
 
 
 def latent_attention(qa: torch.Tensor, k_pages: torch.Tensor, ctx, block_table: torch.Tensor, heads: int, kv_rank: int,
@@ -104,14 +124,22 @@ def latent_attention(qa: torch.Tensor, k_pages: torch.Tensor, ctx, block_table: 
         raise KernelError("latent_attention: queries are float32 [T, heads, kv_rank + rot_dim]")
     if k_pages.dim() != 4 or tuple(k_pages.shape[1:]) != (1, 64, kv_rank + rot_dim):
         raise KernelError("latent_attention: cache pages must be [n_pages, 1, 64, kv_rank + rot_dim]")
+    cluster = 0                          # the kernel for every size
+    if (k_pages.dtype == torch.bfloat16 and (qa.data_ptr() | k_pages.data_ptr()) % 16 == 0
+            and fn("latent", "sx_latent_mma_fits")(c_int(kv_rank), c_int(rot_dim), c_int(T))):
+        cluster = 1
     if splits is None:
-        splits = _pick_latent_splits(ctx, heads, window, qa.device)
+        if cluster:
+            splits, cluster = _pick_latent_shares(ctx, heads, window, qa.device)
+        else:
+            splits = _pick_latent_splits(ctx, heads, window, qa.device)
     out = torch.empty((T, heads, splits, kv_rank), dtype=torch.float32, device=qa.device)
     ml = torch.empty((T, heads, splits, 2), dtype=torch.float32, device=qa.device)
     check(fn("latent", "sx_latent_attention")(ptr(qa), ptr(k_pages), ptr(ctx.positions), ptr(ctx.seq_of_token), ptr(block_table),
                                               c_int(block_table.shape[1]), c_int(heads), c_int(kv_rank), c_int(rot_dim),
                                               c_float(scale), c_int(0 if window is None else int(window)), ptr(out), ptr(ml),
-                                              c_int(splits), c_int(T), c_int(dt_code(k_pages.dtype)), stream()), "latent_attention")
+                                              c_int(splits), c_int(cluster), c_int(T), c_int(dt_code(k_pages.dtype)), stream()),
+          "latent_attention")
     return WeightedLatents(out, ml, splits)
 
 
