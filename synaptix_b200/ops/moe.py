@@ -30,11 +30,13 @@ def moe_tc_status(reset: bool = False) -> int:
 
 class ExpertPlan(NamedTuple):
     """The step's (token, choice) pairs sorted by expert, all on the device: ``offsets [experts + 1]`` (first sorted place
-    of each expert), ``order [pairs]`` (sorted place -> pair ``token * top + choice``), ``place [pairs]`` (the inverse)."""
+    of each expert), ``order [pairs]`` (sorted place -> pair ``token * top + choice``), ``place [pairs]`` (the inverse).
+    ``most``: the most pairs an expert can have (the step's tokens, whose choices differ; 0: not known)."""
     offsets: torch.Tensor
     order: torch.Tensor
     place: torch.Tensor
     experts: int
+    most: int = 0
 
 
 def moe_route(x: torch.Tensor, router: torch.Tensor, top: int, scale: float, sum_eps: float, *, scoring: str = "softmax",
@@ -73,7 +75,7 @@ def moe_sort(ids: torch.Tensor, experts: int) -> ExpertPlan:
     order = torch.empty(n, dtype=torch.int32, device=ids.device)
     place = torch.empty(n, dtype=torch.int32, device=ids.device)
     check(fn("moe", "sx_moe_sort")(ptr(ids), c_int(n), c_int(experts), ptr(offsets), ptr(order), ptr(place), stream()), "moe_sort")
-    return ExpertPlan(offsets, order, place, experts)
+    return ExpertPlan(offsets, order, place, experts, ids.shape[0] if ids.dim() == 2 else 0)
 
 
 def moe_gate_up(x: torch.Tensor, gate_up: torch.Tensor, plan: ExpertPlan, top: int) -> torch.Tensor:
@@ -96,7 +98,7 @@ def moe_gate_up(x: torch.Tensor, gate_up: torch.Tensor, plan: ExpertPlan, top: i
         return z
     use_gate("moe")
     check(fn("moe", "sx_moe_gemm")(ptr(x), ptr(gate_up), ptr(z), ptr(plan.offsets), ptr(plan.order), c_int(rows), c_int(E),
-                                   c_int(ff2 // 2), c_int(W), c_int(top), c_int(MODE_GATE_UP), c_int(dt_code(x.dtype)),
+                                   c_int(ff2 // 2), c_int(W), c_int(top), c_int(MODE_GATE_UP), c_int(plan.most), c_int(dt_code(x.dtype)),
                                    c_int(dt_code(z.dtype)), stream()), "moe_gate_up")
     return z
 
@@ -121,7 +123,7 @@ def moe_up(x: torch.Tensor, up: torch.Tensor, plan: ExpertPlan, top: int) -> tor
         return z
     use_gate("moe")
     check(fn("moe", "sx_moe_gemm")(ptr(x), ptr(up), ptr(z), ptr(plan.offsets), ptr(plan.order), c_int(rows), c_int(E), c_int(ff),
-                                   c_int(W), c_int(top), c_int(MODE_UP), c_int(dt_code(x.dtype)), c_int(dt_code(z.dtype)),
+                                   c_int(W), c_int(top), c_int(MODE_UP), c_int(plan.most), c_int(dt_code(x.dtype)), c_int(dt_code(z.dtype)),
                                    stream()), "moe_up")
     return z
 
@@ -139,7 +141,7 @@ def moe_down(z: torch.Tensor, down: torch.Tensor, plan: ExpertPlan) -> torch.Ten
                                         c_int(MODE_PLAIN), stream()), "moe_down")
         return y
     check(fn("moe", "sx_moe_gemm")(ptr(z), ptr(down), ptr(y), ptr(plan.offsets), ptr(plan.order), c_int(rows), c_int(E),
-                                   c_int(W), c_int(ff), c_int(1), c_int(MODE_PLAIN), c_int(dt_code(z.dtype)), c_int(dt_code(y.dtype)),
+                                   c_int(W), c_int(ff), c_int(1), c_int(MODE_PLAIN), c_int(plan.most), c_int(dt_code(z.dtype)), c_int(dt_code(y.dtype)),
                                    stream()), "moe_down")
     return y
 

@@ -1,0 +1,145 @@
+"""The kernels of single-token steps for attention over a cached latent and for experts, against 64-bit sums, at the sizes where
+they change form.  A sum of n 32-bit products in any order is off by at most (n + 2) 2^-24 times the sum of their magnitudes."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+ULP = 2.0 ** -24
+BF16 = 2.0 ** -8        # rounding to bfloat16 (8 bits of significand) moves a value by at most this share
+
+
+class Step:
+    """What the kernels' faces read of a step's context: single tokens, one a sequence."""
+
+    def __init__(self, positions, maxp):
+        self.positions = torch.tensor(positions, dtype=torch.int32, device="cuda")
+        self.seq_of_token = torch.arange(len(positions), dtype=torch.int32, device="cuda")
+        self.n_tokens, self.all_single, self.max_len = len(positions), True, maxp * 64
+
+
+def latent_cache(lens, E, seed):
+    """Pages [P, 1, 64, E] in bfloat16 of sequences with random rows, their tables, and the rows in 64-bit.  Every row that no
+    sequence owns is NaN."""
+    g = torch.Generator().manual_seed(seed)
+    maxp = max((n + 63) // 64 for n in lens)
+    ids = torch.randperm(len(lens) * maxp, generator=g) + 1
+    pages = torch.full((len(lens) * maxp + 1, 1, 64, E), float("nan"), dtype=torch.bfloat16)
+    table = torch.zeros((len(lens), maxp), dtype=torch.int32)
+    rows = []
+    for s, n in enumerate(lens):
+        r = torch.randn(n, E, generator=g).to(torch.bfloat16)
+        for p in range((n + 63) // 64):
+            table[s, p] = ids[s * maxp + p]
+            part = r[p * 64:(p + 1) * 64]
+            pages[table[s, p], 0, :part.shape[0]] = part
+        rows.append(r.double())
+    return pages.cuda(), table.cuda(), rows, maxp
+
+
+@pytest.mark.parametrize("H,R,Dr", [(1, 16, 0), (9, 32, 16), (16, 128, 32), (32, 320, 64), (17, 512, 64), (4, 400, 48)])
+@pytest.mark.parametrize("lens,window", [([1], None), ([32, 33, 700], None), ([31, 64, 97, 700, 1100], 130)])
+@pytest.mark.parametrize("parts,cluster", [(None, None), (1, 1), (3, 1), (1, 8), (2, 4), (5, 2), (1, 0)])
+def test_latent_attention(H, R, Dr, lens, window, parts, cluster):
+    from synaptix_b200 import ops
+    from synaptix_b200.ops._lib import c_float, c_int, check, dt_code, fn, ptr, stream
+    from synaptix_b200.ops.latent import WeightedLatents
+    E, T, scale = R + Dr, len(lens), 0.1
+    pages, table, rows, maxp = latent_cache(lens, E, H + R)
+    qa = torch.randn(T, H, E, generator=torch.Generator().manual_seed(1)).cuda()
+    ctx = Step([n - 1 for n in lens], maxp)
+    if parts is None:
+        got = ops.latent_attention(qa, pages, ctx, table, H, R, Dr, scale, window)
+    else:
+        out, ml = torch.full((T, H, parts, R), 7.0, device="cuda"), torch.full((T, H, parts, 2), 7.0, device="cuda")
+        check(fn("latent", "sx_latent_attention")(ptr(qa), ptr(pages), ptr(ctx.positions), ptr(ctx.seq_of_token), ptr(table), c_int(maxp),
+                                                  c_int(H), c_int(R), c_int(Dr), c_float(scale), c_int(window or 0), ptr(out), ptr(ml),
+                                                  c_int(parts), c_int(cluster), c_int(T), c_int(dt_code(torch.bfloat16)), stream()), "latent_attention")
+        got = WeightedLatents(out, ml, parts)
+    got = got.merged().double().cpu()
+    for s, n in enumerate(lens):
+        k = rows[s][max(0, n - (window or n)):]
+        z = qa[s].double().cpu() @ k.T * scale
+        want = torch.softmax(z, -1) @ k[:, :R]
+        # scores off by (E + 8) 2^-24 |q| |k| scale at most, weights by twice that and a few roundings, the mean by (keys + 16) more
+        off = (E + 8) * ULP * float(qa[s].norm(dim=-1).max()) * float(k.norm(dim=-1).max()) * scale
+        assert (got[s] - want).abs().max() <= (2 * off + (n + 32) * ULP) * float(k.abs().max())
+
+
+@pytest.mark.parametrize("T,H,D,Dr,R", [(1, 1, 1, 0, 2), (3, 2, 16, 8, 126), (8, 3, 65, 4, 128), (9, 2, 64, 16, 320), (8, 1, 130, 0, 130)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_latent_query(T, H, D, Dr, R, dtype):
+    from synaptix_b200 import ops
+    g = torch.Generator().manual_seed(T + D)
+    q = torch.randn(T, H * (D + Dr), generator=g).to(dtype)
+    w = torch.randn(H * D, R, generator=g).to(dtype)
+    got = ops.latent_query(q.cuda(), w.cuda(), H, D, Dr, R, None, 0, False, Step(list(range(T)), 1)).double().cpu()
+    qd, wd = q.double().view(T, H, D + Dr), w.double().view(H, D, R)
+    want = torch.einsum("thd,hdr->thr", qd[..., :D], wd)
+    bound = (D + 8) * ULP * torch.einsum("thd,hdr->thr", qd[..., :D].abs(), wd.abs())
+    assert ((got[..., :R] - want).abs() <= bound).all()
+    assert torch.equal(got[..., R:], qd[..., D:])
+
+
+@pytest.mark.parametrize("T,H,Dv,R,parts", [(1, 1, 1, 4, 1), (7, 2, 33, 128, 3), (8, 3, 128, 320, 1), (9, 2, 40, 512, 40), (5, 1, 65, 516, 2)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("gate,sink", [(None, False), ("head", True), ("elements", False)])
+def test_latent_output(T, H, Dv, R, parts, dtype, gate, sink):
+    from synaptix_b200 import ops
+    from synaptix_b200.ops.latent import WeightedLatents
+    g = torch.Generator().manual_seed(T + Dv)
+    ol = torch.randn(T, H, parts, R, generator=g)
+    ml = torch.stack([torch.randn(T, H, parts, generator=g), torch.rand(T, H, parts, generator=g) + 0.5], -1)
+    if parts > 1:
+        ml[:, :, 0, 0], ml[:, :, 0, 1], ol[:, :, 0] = float("-inf"), 0.0, 0.0          # a part without a key
+    w = torch.randn(H * Dv, R, generator=g).to(dtype)
+    proj = torch.randn(T, 3 + H * Dv, generator=g).to(dtype)
+    sinks = torch.randn(H, generator=g) if sink else None
+    got = ops.latent_output(WeightedLatents(ol.cuda(), ml.cuda(), parts), w.cuda(), H, Dv, R, proj.cuda(), -1 if gate is None else 3, dtype,
+                            sinks=None if sinks is None else sinks.cuda(), gate_elements=gate == "elements").double().cpu().view(T, H, Dv)
+    m, l = ml[..., 0].double(), ml[..., 1].double()
+    e = torch.exp(m)
+    total = (e * l).sum(-1) + (0 if sinks is None else torch.exp(sinks.double())[None])
+    o = (ol.double() * e[..., None]).sum(2) / total[..., None]
+    mag = (ol.double().abs() * e[..., None]).sum(2) / total[..., None]
+    wd = w.double().view(H, Dv, R)
+    want, mag = torch.einsum("thr,hjr->thj", o, wd), torch.einsum("thr,hjr->thj", mag, wd.abs())
+    if gate is not None:
+        z = torch.sigmoid(proj.double()[:, 3:])
+        f = z.view(T, H, Dv) if gate == "elements" else z[:, :H, None]
+        want, mag = want * f, mag * f
+    bound = (R + 3 * parts + 24) * ULP * mag + (BF16 if dtype == torch.bfloat16 else ULP) * want.abs()
+    assert ((got - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("T,E,top", [(1, 1, 1), (1, 16, 4), (8, 5, 2), (9, 16, 4), (16, 3, 3)])
+@pytest.mark.parametrize("ff,W", [(8, 32), (24, 96), (41, 1056), (130, 544)])
+@pytest.mark.parametrize("same", [False, True])
+def test_experts(T, E, top, ff, W, same):
+    """Gated and ungated first products and the second one; ``same``: every choice of every token names the last expert."""
+    from synaptix_b200 import ops
+    g = torch.Generator().manual_seed(T * 100 + ff)
+    x = torch.randn(T, W, generator=g).to(torch.bfloat16)
+    gate_up = (torch.randn(E, 2 * ff, W, generator=g) * W ** -0.5).to(torch.bfloat16)
+    ids = torch.full((T, top), E - 1) if same else torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)])
+    plan = ops.moe_sort(ids.to(torch.int32).cuda(), E)
+    order = plan.order.long().cpu()
+    row, ex = order // top, ids.flatten()[order]
+    xd, wd = x.double()[row], gate_up.double()[ex]                                # [pairs, W], [pairs, 2 ff, W]
+    z, mag = torch.einsum("pw,pfw->pf", xd, wd), torch.einsum("pw,pfw->pf", xd.abs(), wd.abs())
+    off = (W + 4) * ULP * mag
+    a, u = z[:, :ff], z[:, ff:]
+    got = ops.moe_gate_up(x.cuda(), gate_up.cuda(), plan, top).double().cpu()
+    want = a * torch.sigmoid(a) * u
+    # |d silu| <= 1.1
+    bound = 1.1 * off[:, :ff] * u.abs() + a.abs() * off[:, ff:] + (BF16 + 1e-6) * want.abs() + 1e-9
+    assert ((got - want).abs() <= bound).all()
+    with ops.gate_activation(form="relu2"):
+        got = ops.moe_up(x.cuda(), gate_up.cuda(), plan, top).double().cpu()
+    want = z.clamp(min=0) ** 2
+    assert ((got - want).abs() <= 2 * z.abs() * off + off ** 2 + (BF16 + 1e-6) * want + 1e-9).all()
+    h = torch.randn(T * top, W, generator=g).to(torch.bfloat16)
+    down = (torch.randn(E, ff, W, generator=g)).to(torch.bfloat16)
+    got = ops.moe_down(h.cuda(), down.cuda(), plan).double().cpu()
+    hd, dd = h.double(), down.double()[ex]
+    want, mag = torch.einsum("pw,pfw->pf", hd, dd), torch.einsum("pw,pfw->pf", hd.abs(), dd.abs())
+    assert ((got - want).abs() <= (W + 4) * ULP * mag).all()
