@@ -21,6 +21,7 @@ from __future__ import annotations
 import ctypes
 import hashlib
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -225,6 +226,24 @@ def build_host_library(name: str, verbose: bool = True) -> str:
             except OSError:
                 pass
     return out
+
+
+_C_TYPES = {"int": ctypes.c_int, "float": ctypes.c_float, "long long": ctypes.c_longlong,
+            "unsigned long long": ctypes.c_ulonglong, "cudaStream_t": ctypes.c_void_p}
+
+
+def signature(name: str, function: str) -> list:
+    """The ctypes types of an exported function's parameters, read from its declaration in the library's source (pointers
+    are ``c_void_p``), so that a caller can hand over plain numbers."""
+    with open(os.path.join(CSRC_DIR, LIBRARIES[name][0])) as f:
+        found = re.search(r'extern "C" int ' + function + r"\(([^)]*)\)\s*\{", f.read())
+    if found is None:
+        raise KernelsUnavailable(f"csrc/{LIBRARIES[name][0]} defines no {function}")
+    types = []
+    for param in found.group(1).split(","):
+        words = param.replace("const", " ").split()
+        types.append(ctypes.c_void_p if "*" in param else _C_TYPES[" ".join(words[:-1])])
+    return types
 
 
 _LOADED: Dict[str, ctypes.CDLL] = {}

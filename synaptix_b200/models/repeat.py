@@ -1,0 +1,135 @@
+"""A prompt step's launches for layers of one form, made again with other pointers.
+
+The layers of a decoder are mostly the same parts with other weights: what differs between two neighbouring layers' launches
+are the pointers of their parameters, of their cache entries and of the branch that travels from one to the next.  A prompt
+step of a few hundred tokens is bound by the host, which walks the parts and makes some twenty arguments for each of two
+hundred launches (17 us a launch at 0.6B sizes, more than the kernels take); so the step walks the first two layers of a
+stretch, records what the second one launched, and makes the same launches for the others with their pointers put in (5 us).
+Nothing of a step outlasts it; between steps only the layers' forms are remembered, never a pointer.
+
+Only parts whose class says ``repeatable`` in its own body are asked (their ``forward`` launches kernels through ``ops.launch``
+and does nothing else on the device, and depends on nothing but their sizes, the step and their inputs), and only a recording
+that holds everything that was launched is used; any other layer is simply walked.
+"""
+from __future__ import annotations
+
+import bisect
+import ctypes
+from typing import List, Optional, Tuple
+
+import torch
+
+from ..parts.base import Part, PendingLinear
+
+MIN_LAYERS = 4                 # a stretch shorter than this is walked
+
+
+class _Unlike(Exception):
+    pass
+
+
+def _walk(value, where, key, form: list, places: list) -> None:
+    """Append what ``value`` is, names aside, to ``form`` and the place of every tensor in it to ``places``."""
+    if isinstance(value, torch.Tensor):
+        form.append((tuple(value.shape), value.dtype, value.device, value.is_contiguous()))
+        places.append((where, key))
+    elif isinstance(value, Part):
+        if not type(value).__dict__.get("repeatable", False):
+            raise _Unlike
+        form.append(type(value))
+        for k, v in vars(value).items():
+            form.append(k)
+            _walk(v, vars(value), k, form, places)
+    elif isinstance(value, str):
+        form.append("")
+    elif value is None or isinstance(value, (bool, int, float, torch.dtype, torch.device)):
+        form.append((type(value), value))
+    elif isinstance(value, (list, tuple)):
+        form.append((type(value), len(value)))
+        for i, v in enumerate(value):
+            _walk(v, value, i, form, places)
+    elif isinstance(value, dict):
+        form.append((dict, len(value)))
+        for k, v in value.items():
+            _walk(v, value, k, form, places)
+    else:
+        raise _Unlike
+
+
+def form_of(layer: Part) -> Optional[Tuple[tuple, list]]:
+    """``(form, places of its tensors)`` of a layer, or ``None`` if it holds anything that is not repeatable."""
+    form, places = [], []
+    try:
+        _walk(layer, None, None, form, places)
+    except _Unlike:
+        return None
+    return tuple(form), places
+
+
+def _tensors(places: list) -> List[torch.Tensor]:
+    return [where[key] for where, key in places]
+
+
+def _at(tensors: List[torch.Tensor], t: Optional[torch.Tensor]) -> Optional[int]:
+    return None if t is None else next((i for i, x in enumerate(tensors) if x is t), -1)
+
+
+def repeat(recording, before, after, places: list, views: list):
+    """Make the launches of ``recording`` again for the layers behind the recorded one.
+
+    ``places[0]`` and ``places[1]`` are the tensors' places of the layer before the recorded one and of the recorded one,
+    ``places[2:]`` those of the layers to come; ``views[1:]`` are the cache views of the recorded and the coming ones.
+    ``before`` and ``after`` are the branches the recorded layer was handed and handed on (``PendingLinear``).  Returns the
+    branch that the last layer hands on, or ``None`` if the recording cannot be used (nothing has been launched then)."""
+    from ..ops._lib import check
+    if not recording.whole or type(before) is not PendingLinear or type(after) is not PendingLinear:
+        return None
+    if before.x.shape != after.x.shape or before.x.dtype != after.x.dtype or (before.bias is None) != (after.bias is None):
+        return None
+    first, second = _tensors(places[0]), _tensors(places[1])
+    weight, bias = _at(second, after.weight), _at(second, after.bias)
+    if weight == -1 or bias == -1 or first[weight] is not before.weight or (bias is not None and first[bias] is not before.bias):
+        return None
+    if any(v.group != views[1].group or v.window != views[1].window for v in views[2:]):
+        return None
+    # where a recorded pointer comes from: (row of the table below, column)
+    source = {}
+    for row, tensors in ((0, first), (1, second)):
+        for i, t in enumerate(tensors):
+            source[t.data_ptr()] = (row, i)
+    n = len(second)
+    for i, t in ((n, views[1].k), (n + 1, views[1].v)):
+        if t is not None:
+            source[t.data_ptr()] = (1, i)
+    source[before.x.data_ptr()] = (0, n)
+    source[after.x.data_ptr()] = (1, n + 2)
+    source.pop(0, None)
+    # (a pointer into the middle of one of these has no place to come from in the next layer)
+    spans = sorted((t.data_ptr(), t.data_ptr() + t.numel() * t.element_size())
+                   for t in first + second + [t for t in (views[1].k, views[1].v) if t is not None])
+    starts = [a for a, _ in spans]
+
+    def inside(a: int) -> bool:
+        i = bisect.bisect_right(starts, a)
+        return i > 0 and a < spans[i - 1][1]
+    calls = []
+    for f, args, what, launches in recording.calls:
+        if any(kind is ctypes.c_void_p and a and a not in source and inside(a) for a, kind in zip(args, f.argtypes)):
+            return None
+        put = [(j,) + source[a] for j, (a, kind) in enumerate(zip(args, f.argtypes))
+               if kind is ctypes.c_void_p and a in source]
+        calls.append((f, list(args), put, what, launches))
+    x_in, x_out = before.x, after.x
+    above = [t.data_ptr() for t in second]
+    for p, view in zip(places[2:], views[2:]):
+        x_in, x_out = x_out, x_in                  # the branch a layer hands on is the next one's
+        mine = [where[key].data_ptr() for where, key in p]
+        table = (above + [x_in.data_ptr()],
+                 mine + [0 if view.k is None else view.k.data_ptr(), 0 if view.v is None else view.v.data_ptr(), x_out.data_ptr()])
+        for f, args, put, what, launches in calls:
+            for j, row, i in put:
+                args[j] = table[row][i]
+            check(f(*args), what, launches)
+        above = mine
+    last = _tensors(places[-1])
+    return PendingLinear(x_out, last[weight], None if bias is None else last[bias])

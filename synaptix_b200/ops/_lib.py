@@ -3,11 +3,12 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import threading
 from typing import Optional
 
 import torch
 
-from ..csrc.build import KernelsUnavailable, load_library
+from ..csrc.build import KernelsUnavailable, load_library, signature
 from .options import OPTIONS as _PDL_OPTION
 
 _DT = {torch.float32: 0, torch.bfloat16: 1}
@@ -44,10 +45,16 @@ def ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
     return ctypes.c_void_p(0 if t is None else t.data_ptr())
 
 
+def good(t: torch.Tensor) -> bool:
+    """What ``require_cuda`` asks of one tensor, for the faces that a prompt step calls hundreds of times."""
+    return t.is_cuda and t.is_contiguous()
+
+
 try:                                    # the raw handle without building a Stream object (an order of magnitude cheaper)
     _raw_stream = torch._C._cuda_getCurrentRawStream
 except AttributeError:                  # pragma: no cover - older torch
     _raw_stream = None
+_get_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
 
 
 def stream() -> ctypes.c_void_p:
@@ -85,7 +92,51 @@ def count_launches(n: int) -> None:
         _COUNTER[0].kernel_launches += n
 
 
+class Recording:
+    """The launches of a stretch of a step as they were made: ``calls`` holds ``(function, arguments, what, launches)`` of
+    everything that went through ``launch``, ``keep`` the tensors made for them.  ``whole`` says whether that is all that was
+    launched, under the options that hold outside too, so that the calls can be made again with other pointers."""
+
+    def __init__(self):
+        self.calls, self.keep = [], []
+        self.checked, self.plain = 0, True
+
+    @property
+    def whole(self) -> bool:
+        return self.plain and self.checked == len(self.calls)
+
+
+class _Local(threading.local):
+    recording: Optional[Recording] = None          # of this thread
+
+
+_TLS = _Local()
+
+
+@contextlib.contextmanager
+def recording():
+    """Record this thread's launches (they are made all the same)."""
+    old, _TLS.recording = _TLS.recording, Recording()
+    try:
+        yield _TLS.recording
+    finally:
+        _TLS.recording = old
+
+
+def launch(f, args: tuple, what: str, launches: int = 1, keep: tuple = ()) -> None:
+    """Call ``f`` (of ``launcher``) and check its code; a recording in progress notes the call."""
+    check(f(*args), what, launches)
+    r = _TLS.recording
+    if r is not None:
+        r.calls.append((f, args, what, launches))
+        r.keep += keep
+        if _LATE[0] or _GATE[0] != _GATE_DEFAULT:
+            r.plain = False
+
+
 def check(code: int, what: str, launches: int = 1) -> None:
+    if _TLS.recording is not None:
+        _TLS.recording.checked += 1
     if code == 0:
         if _COUNTER[0] is not None:
             _COUNTER[0].kernel_launches += launches
@@ -163,6 +214,30 @@ def fn(lib: str, name: str):
     return f
 
 
+_LAUNCHERS = {}
+
+
+def launcher(lib: str, name: str):
+    """``fn`` with the parameters' types set: it takes plain numbers, and ``t.data_ptr()`` or ``None`` for a pointer.  (Making
+    a ctypes object of every argument and converting it again is a third of what a launch costs the host, and a prompt step
+    of a few hundred tokens is bound by that.)"""
+    f = _LAUNCHERS.get(name)
+    if f is None:
+        f = _library(lib)[name]                # an object of its own: ``fn``'s keeps taking ctypes objects
+        f.restype, f.argtypes = ctypes.c_int, signature(lib, name)
+        _LAUNCHERS[name] = f
+    if _LIB_PDL[lib] is not (not _LATE[0] and _PDL_OPTION.pdl):
+        _set_pdl(lib)
+    return f
+
+
+def raw_stream() -> int:
+    """``stream()`` as a plain number."""
+    if _raw_stream is not None:
+        return _raw_stream(_get_device())
+    return torch.cuda.current_stream().cuda_stream
+
+
 c_int = ctypes.c_int
 c_float = ctypes.c_float
 c_longlong = ctypes.c_longlong
@@ -178,7 +253,8 @@ c_ulonglong = ctypes.c_ulonglong
 # experts' products of ONE matrix (``moe_up``): relu(z)^2.
 # ---------------------------------------------------------------------------------------------------------------
 GATE_FORMS = {"sigmoid": 0, "gelu_tanh": 1, "relu2": 2}
-_GATE = [(0.0, 0.0, 0)]
+_GATE_DEFAULT = (0.0, 0.0, 0)
+_GATE = [_GATE_DEFAULT]
 _LIB_GATE = {}
 
 

@@ -7,7 +7,7 @@ import torch
 
 import ctypes
 
-from ._lib import KernelError, c_float, c_int, c_longlong, check, fn, ptr, require_cuda, stream
+from ._lib import KernelError, c_float, c_int, c_longlong, check, fn, launch, launcher, ptr, raw_stream, require_cuda, stream
 from .decode import sm_count
 from .options import OPTIONS
 
@@ -306,12 +306,12 @@ def attn_prefill_tc(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tenso
     if not tc_prefill_supported(q.dtype, nh, nkv, hd) or k_pages.dtype != q.dtype:
         raise KernelError("attn_prefill_tc: bfloat16 and head size 128")
     if out is None:
-        out = torch.empty((T, nh * hd), dtype=q.dtype, device=q.device)
-    check(fn("attn_tc", "sx_attn_prefill_tc")(
-        ptr(q), ptr(k_pages), ptr(v_pages), ptr(out), c_longlong(T), c_longlong(k_pages.shape[0]), ptr(tile_seq),
-        ptr(tile_q0), c_int(tile_seq.numel()), ptr(cu_seqlens), ptr(seq_past), ptr(seq_lens), ptr(block_table),
-        c_int(block_table.shape[1]), c_int(nh), c_int(nkv), c_int(hd), c_float(scale),
-        c_int(0 if window is None else int(window)), ptr(sinks), stream()), "attn_prefill_tc")
+        out = q.new_empty((T, nh * hd))
+    launch(launcher("attn_tc", "sx_attn_prefill_tc"), (
+        q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), out.data_ptr(), T, k_pages.shape[0], tile_seq.data_ptr(),
+        tile_q0.data_ptr(), tile_seq.numel(), cu_seqlens.data_ptr(), seq_past.data_ptr(), seq_lens.data_ptr(), block_table.data_ptr(),
+        block_table.shape[1], nh, nkv, hd, scale, 0 if window is None else int(window), None if sinks is None else sinks.data_ptr(),
+        raw_stream()), "attn_prefill_tc", 1, (out,))
     return out
 
 

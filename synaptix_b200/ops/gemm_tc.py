@@ -6,7 +6,7 @@ from typing import Optional
 
 import torch
 
-from ._lib import KernelError, c_float, c_int, check, check_bias, check_resid_tanh, fn, ptr, require_cuda, stream, use_gate
+from ._lib import KernelError, c_float, c_int, check, check_bias, check_resid_tanh, fn, good, launch, launcher, ptr, raw_stream, require_cuda, stream, use_gate
 from .decode import sm_count
 from .options import OPTIONS
 
@@ -119,7 +119,8 @@ def gemm_tc_resid_tanh(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Te
 
 
 def _gemm_tc(x, w, epilogue, out, splits, cut, bias, cap, h=None, alpha=0.0, gain=None, shift=None) -> torch.Tensor:
-    require_cuda(x, w, out, bias)
+    if not (good(x) and good(w)) or out is not None or bias is not None:
+        require_cuda(x, w, out, bias)
     M, K = x.shape
     N, K2 = w.shape
     if K != K2:
@@ -130,7 +131,7 @@ def _gemm_tc(x, w, epilogue, out, splits, cut, bias, cap, h=None, alpha=0.0, gai
     if epilogue == "silu_mul":
         use_gate("gemm_tc")
     if out is None:
-        out = torch.empty((M, n_out), dtype=torch.float32 if epilogue == "f32" else torch.bfloat16, device=x.device)
+        out = x.new_empty((M, n_out), dtype=torch.float32 if epilogue == "f32" else torch.bfloat16)
     ws = counts = None
     if cut is None:
         cut = OPTIONS.gemm_cut
@@ -152,10 +153,11 @@ def _gemm_tc(x, w, epilogue, out, splits, cut, bias, cap, h=None, alpha=0.0, gai
         ws = _workspace(ws_floats, x.device)
         if splits == 1:
             counts = _counts(x.device)
-    check(fn("gemm_tc", "sx_gemm_tc")(ptr(x), ptr(w), ptr(out), c_int(M), c_int(N), c_int(K), c_int(_EPI[epilogue]),
-                                      c_int(splits), ptr(ws), ctypes.c_ulonglong(0 if ws is None else ws.numel()),
-                                      ptr(counts), ptr(bias), c_float(cap), ptr(h), c_float(alpha), ptr(gain), ptr(shift),
-                                      stream()), "gemm_tc", launches=2 if splits > 1 else 1)
+    launch(launcher("gemm_tc", "sx_gemm_tc"), (
+        x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, _EPI[epilogue], splits, None if ws is None else ws.data_ptr(),
+        0 if ws is None else ws.numel(), None if counts is None else counts.data_ptr(), None if bias is None else bias.data_ptr(), cap,
+        None if h is None else h.data_ptr(), alpha, None if gain is None else gain.data_ptr(), None if shift is None else shift.data_ptr(),
+        raw_stream()), "gemm_tc", 2 if splits > 1 else 1, (out, ws))
     return out
 
 
@@ -202,10 +204,12 @@ def gemm_tc_qkv(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, k_pages: 
     for t in (positions, seq_of_token, block_table):
         if t.dtype != torch.int32:
             raise KernelError("gemm_tc_qkv: index tensors are int32")
-    check(fn("gemm_tc", "sx_gemm_tc_qkv")(
-        ptr(x), ptr(w), ptr(bias), c_int(M), c_int(N), c_int(K), ptr(q_out), ptr(k_pages), ptr(v_pages), ptr(wq), ptr(wk), ptr(cos),
-        ptr(sin), ptr(positions), ptr(seq_of_token), ptr(block_table), c_int(block_table.shape[1]), c_int(nh), c_int(nkv),
-        c_int(n_pages), ctypes.c_float(eps), stream()), "gemm_tc_qkv")
+    launch(launcher("gemm_tc", "sx_gemm_tc_qkv"), (
+        x.data_ptr(), w.data_ptr(), None if bias is None else bias.data_ptr(), M, N, K, q_out.data_ptr(),
+        None if k_pages is None else k_pages.data_ptr(), None if v_pages is None else v_pages.data_ptr(),
+        None if wq is None else wq.data_ptr(), None if wk is None else wk.data_ptr(), None if cos is None else cos.data_ptr(),
+        None if sin is None else sin.data_ptr(), positions.data_ptr(), seq_of_token.data_ptr(), block_table.data_ptr(),
+        block_table.shape[1], nh, nkv, n_pages, eps, raw_stream()), "gemm_tc_qkv", 1, (q_out,))
 
 
 def gemm_tc_status(reset: bool = False) -> int:

@@ -6,7 +6,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from ._lib import KernelError, c_float, c_int, check, check_bias, check_resid_tanh, fn, ptr, require_cuda, stream, use_gate
+from ._lib import KernelError, c_float, c_int, check, check_bias, check_resid_tanh, fn, launch, launcher, ptr, raw_stream, require_cuda, stream, use_gate
 
 _EPI = {None: 0, "f32": 1, "silu_mul": 2, "residual": 3, "resid_tanh": 4}
 MAX_ROWS = 256
@@ -55,9 +55,10 @@ def gemm_ws(x: torch.Tensor, w: torch.Tensor, *, epilogue: Optional[str] = None,
         out = torch.empty((M, n_out), dtype=torch.float32 if epilogue == "f32" else torch.bfloat16, device=x.device)
     if epilogue == "silu_mul":
         use_gate("gemm_ws")
-    check(fn("gemm_ws", "sx_gemm_ws")(ptr(x), ptr(w), ptr(out), c_int(M), c_int(N), c_int(K), c_int(_EPI[epilogue]),
-                                      c_int(splits or 0), c_int(stages or 0), ptr(ssq), c_int(0 if ssq is None else ssq.shape[1]),
-                                      c_float(eps), ptr(None), ptr(None), ptr(None), ptr(bias), c_float(cap), c_float(0.0), ptr(None), stream()), "gemm_ws")
+    launch(launcher("gemm_ws", "sx_gemm_ws"), (
+        x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, _EPI[epilogue], splits or 0, stages or 0, None if ssq is None else ssq.data_ptr(),
+        0 if ssq is None else ssq.shape[1], eps, None, None, None, None if bias is None else bias.data_ptr(), cap, 0.0, None,
+        raw_stream()), "gemm_ws", 1, (out,))
     return out
 
 
@@ -84,9 +85,9 @@ def gemm_ws_residual(x: torch.Tensor, w: torch.Tensor, h: torch.Tensor, gain: to
         splits //= 2
     out = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
     ssq = torch.empty((M, tiles * splits), dtype=torch.float32, device=x.device)
-    check(fn("gemm_ws", "sx_gemm_ws")(ptr(x), ptr(w), ptr(out), c_int(M), c_int(N), c_int(K), c_int(3), c_int(splits),
-                                      c_int(stages or 0), ptr(None), c_int(0), c_float(0.0), ptr(h), ptr(gain), ptr(ssq), ptr(None), c_float(0.0),
-                                      c_float(0.0), ptr(None), stream()), "gemm_ws_residual")
+    launch(launcher("gemm_ws", "sx_gemm_ws"), (
+        x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, 3, splits, stages or 0, None, 0, 0.0, h.data_ptr(), gain.data_ptr(),
+        ssq.data_ptr(), None, 0.0, 0.0, None, raw_stream()), "gemm_ws_residual", 1, (out, ssq))
     return out, ssq
 
 

@@ -5,8 +5,8 @@ from typing import Optional
 
 import torch
 
-from ._lib import (KernelError, c_float, c_int, c_longlong, check, check_bias, dt_code, fn, ptr, require_cuda,
-                   stream)
+from ._lib import (KernelError, c_float, c_int, c_longlong, check, check_bias, dt_code, fn, good, launch, launcher, ptr, raw_stream,
+                   require_cuda, stream)
 
 
 def embed_gather(table: torch.Tensor, ids: torch.Tensor, out: Optional[torch.Tensor] = None,
@@ -40,7 +40,8 @@ def add_rmsnorm(h: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.Te
     Returns ``rmsnorm(h) * weight`` in ``out_dtype``; with ``rows`` (int32 ``[R]``)
     only for those rows, as ``[R, H]``.
     """
-    require_cuda(h, delta, weight, rows, out)
+    if not (good(h) and good(weight) and (delta is None or good(delta))) or rows is not None or out is not None:
+        require_cuda(h, delta, weight, rows, out)
     if h.dtype != torch.float32 or weight.dtype != torch.float32:
         raise KernelError("the residual stream and norm gains are float32")
     T, H = h.shape
@@ -50,10 +51,10 @@ def add_rmsnorm(h: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.Te
         raise KernelError(f"norm gain has {weight.numel()} elements for width {H}")
     R = T if rows is None else rows.numel()
     if out is None:
-        out = torch.empty((R, H), dtype=out_dtype, device=h.device)
-    check(fn("generic", "sx_add_rmsnorm")(ptr(h), ptr(delta), ptr(weight), c_float(eps), ptr(out), ptr(rows),
-                                          c_int(R), c_int(H), c_int(dt_code(out_dtype)),
-                                          c_int(1 if rows is None else 0), stream()), "add_rmsnorm")
+        out = h.new_empty((R, H), dtype=out_dtype)
+    launch(launcher("generic", "sx_add_rmsnorm"), (h.data_ptr(), None if delta is None else delta.data_ptr(), weight.data_ptr(), eps,
+                                                   out.data_ptr(), None if rows is None else rows.data_ptr(), R, H, dt_code(out_dtype),
+                                                   1 if rows is None else 0, raw_stream()), "add_rmsnorm", 1, (out,))
     return out
 
 
@@ -127,11 +128,11 @@ def qkv_prepare(qkv: torch.Tensor, q_out: torch.Tensor, k_pages: Optional[torch.
             c_int(T), c_int(nh), c_int(nkv), c_int(hd), c_int(n_pages), c_int(dt_code(qkv.dtype)),
             c_int(qkv.shape[1]), c_int(vd), stream()), "qkv_prepare")
         return
-    check(fn("generic", "sx_qkv_prepare")(
-        ptr(qkv), ptr(q_out), ptr(k_pages), ptr(v_pages), ptr(wq), ptr(wk), ptr(inv_freq), c_int(rotary_dim),
-        c_float(eps), ptr(positions), ptr(seq_of_token), ptr(block_table), c_int(block_table.shape[1]),
-        c_int(T), c_int(nh), c_int(nkv), c_int(hd), c_int(n_pages), c_int(dt_code(qkv.dtype)),
-        stream()), "qkv_prepare")
+    launch(launcher("generic", "sx_qkv_prepare"), (
+        qkv.data_ptr(), q_out.data_ptr(), None if k_pages is None else k_pages.data_ptr(), None if v_pages is None else v_pages.data_ptr(),
+        None if wq is None else wq.data_ptr(), None if wk is None else wk.data_ptr(), None if inv_freq is None else inv_freq.data_ptr(),
+        rotary_dim, eps, positions.data_ptr(), seq_of_token.data_ptr(), block_table.data_ptr(), block_table.shape[1], T, nh, nkv, hd,
+        n_pages, dt_code(qkv.dtype), raw_stream()), "qkv_prepare", 1, (q_out,))
 
 
 def rope_table(positions: torch.Tensor, inv_freq: torch.Tensor):

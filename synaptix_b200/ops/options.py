@@ -32,6 +32,8 @@ switches in its runtime options (crates/synaptix-config/src/runtime.rs, ``AttnBa
                     the graph), else one after the other; likewise the second of two mixers that run side by side
                     behind norms of their own.  A branch's last product is then launched late (``late_launch``): scheduled
                     early it holds the room that the other branch's kernels need (a Zekalorn step at batch 1: 0.87 -> 0.70 ms)
+``repeat_layers``   prompt steps: the launches of layers of one form are recorded from one of them and made again with the
+                    others' pointers (else every layer's parts are walked)
 """
 from __future__ import annotations
 
@@ -53,6 +55,7 @@ class KernelOptions:
     attn_scored_tc: bool = True
     pdl: bool = True
     branch_streams: bool = True
+    repeat_layers: bool = True
 
 
 OPTIONS = KernelOptions()

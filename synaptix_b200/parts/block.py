@@ -41,6 +41,7 @@ from .base import (FeedForward, Mixer, Norm, NormedDelta, NormedSum, Part, Pendi
 
 class PreNormBlock(Part):
     """``norm2`` and ``ffn`` may both be ``None`` (a layer without a feed-forward)."""
+    repeatable = True
     takes_pending_product = True   # forward's ``pending`` may be a PendingLinear
 
     def __init__(self, norm1: Norm, mixer: Mixer, norm2: Optional[Norm], ffn: Optional[FeedForward]):

@@ -30,6 +30,7 @@ from .linear import Linear
 
 
 class SwiGLU(FeedForward):
+    repeatable = True
     accepts_lazy_input = True      # x goes straight into the fused gate/up product
     can_defer_output = True        # the down projection may be handed on unrun
 

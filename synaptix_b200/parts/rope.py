@@ -38,6 +38,7 @@ class RotaryHalf(PositionEncoding):
     """``scaling`` (a ``FrequencyRamp``): the slow frequencies are stretched and cos and sin both multiplied by
     ``magnitude``; the frequencies are then formed in 64-bit and rounded once.  A kernel that rotates for a part with such
     an encoding multiplies by ``magnitude`` (the parts that take one say so)."""
+    repeatable = True
     pairs = False
 
     def __init__(self, head_dim: int, theta: float, rotary_dim: int = None, scaling: "FrequencyRamp" = None):
@@ -132,3 +133,4 @@ class FrequencyBands(NamedTuple):
 
 class NoPosition(PositionEncoding):
     """Queries and keys are used as they are."""
+    repeatable = True

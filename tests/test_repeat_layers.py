@@ -1,0 +1,117 @@
+"""Launches of layers of one form made again with other pointers: which layers are alike, which pointers are put in, and (on the
+GPU) that a prompt step gives the same bits as one that walks every layer."""
+import ctypes
+import types
+
+import pytest
+import torch
+
+import tiny
+from synaptix_b200.models import model_skeleton
+from synaptix_b200.models.repeat import form_of, repeat
+from synaptix_b200.ops import _lib
+from synaptix_b200.parts import RMSNorm
+from synaptix_b200.parts.base import PendingLinear
+
+QWEN3 = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", num_hidden_layers=7, hidden_size=256, num_attention_heads=4,
+             num_key_value_heads=2, head_dim=128, intermediate_size=320, vocab_size=997, rope_theta=10000.0, rms_norm_eps=1e-6,
+             tie_word_embeddings=True, max_position_embeddings=4096, hidden_act="silu", attention_bias=False, use_sliding_window=False)
+
+
+def skeleton(**more):
+    from synaptix_b200.config import Qwen3Config
+    return model_skeleton(Qwen3Config.from_dict(dict(QWEN3, **more)))
+
+
+def test_forms():
+    layers = skeleton().layers
+    assert len({form_of(x)[0] for x in layers}) == 1
+    windowed = skeleton(use_sliding_window=True, sliding_window=64, max_window_layers=3).layers
+    forms = [form_of(x)[0] for x in windowed]
+    assert len(set(forms[:3])) == 1 and len(set(forms[3:])) == 1 and forms[2] != forms[3]
+
+    class Other(RMSNorm):           # says nothing of itself: never repeated
+        pass
+    layers[0].norm1.__class__ = Other
+    assert form_of(layers[0]) is None and form_of(layers[1]) is not None
+    layers[1].extra = object()
+    assert form_of(layers[1]) is None
+
+
+def test_pointers_are_put_in():
+    n, made = 5, []
+
+    class Launch:
+        argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int]
+
+        def __call__(self, *args):
+            made.append(args)
+            return 0
+    launch = Launch()
+    weights = [[torch.zeros(4, 4), torch.zeros(4)] for _ in range(n)]
+    views = [types.SimpleNamespace(k=torch.zeros(2), v=torch.zeros(2), group=0, window=None) for _ in range(n)]
+    places = [[(w, 0), (w, 1)] for w in weights]
+    z = [torch.zeros(3, 4), torch.zeros(3, 4)]
+    inside = torch.zeros(3, 4)
+
+    def calls(i, read, write):      # what layer i launches
+        return [(read.data_ptr(), weights[i - 1][0].data_ptr(), inside.data_ptr(), 7),
+                (weights[i][1].data_ptr(), views[i].k.data_ptr(), views[i].v.data_ptr(), 8),
+                (inside.data_ptr(), write.data_ptr(), None, 9)]
+
+    def record(whole=True):
+        with _lib.recording() as r:
+            for a in calls(1, z[0], z[1]):
+                _lib.launch(launch, a, "test")
+            if not whole:
+                _lib.check(0, "a launch of another kind")
+        return r
+    before, after = PendingLinear(z[0], weights[0][0]), PendingLinear(z[1], weights[1][0])
+    r = record()
+    made.clear()
+    done = repeat(r, before, after, places, views)
+    want = [a for i in range(2, n) for a in calls(i, z[(i + 1) % 2], z[i % 2])]
+    assert made == want
+    assert done.weight is weights[n - 1][0] and done.bias is None and done.x is z[(n - 1) % 2]
+    made.clear()
+    assert repeat(record(whole=False), before, after, places, views) is None
+    assert repeat(record(), PendingLinear(z[0], torch.zeros(4, 4)), after, places, views) is None
+    with _lib.recording() as r:      # a pointer into the middle of a weight
+        _lib.launch(launch, (weights[1][0].data_ptr() + 16, None, None, 7), "test")
+    assert repeat(r, before, after, places, views) is None
+    views[3].group = 1
+    assert repeat(record(), before, after, places, views) is None
+    with _lib.gate_activation(form="gelu_tanh"):
+        assert not record().whole
+    with _lib.late_launch():
+        assert not record().whole
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("more", [{}, dict(head_dim=64), dict(use_sliding_window=True, sliding_window=64, max_window_layers=2)])
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+def test_same_bits(more, dtype):
+    from synaptix_b200 import ops
+    from synaptix_b200.api import LLM
+    from synaptix_b200.engine import Entry
+    from synaptix_b200.parts import Runtime
+    from synaptix_b200.weights import RandomSource
+    model = skeleton(**more)
+    model.load(RandomSource(model.all_tensor_specs(), seed=1, device="cuda:0"),
+               Runtime(torch.device("cuda:0"), torch.bfloat16 if dtype == "bf16" else torch.float32))
+    engine = LLM.from_model(model, max_tokens=4096, max_batch=8).engine
+
+    def run(on, lens):
+        with ops.options(repeat_layers=on):
+            slots = [engine.open() for _ in lens]
+            before = engine.kernel_launches
+            out = [engine.step([Entry(s, tiny.random_tokens(997, n, n), [0, n - 1]) for s, n in zip(slots, lens)])]
+            launches = engine.kernel_launches - before
+            out.append(engine.step([Entry(s, tiny.random_tokens(997, 3, n), [2]) for s, n in zip(slots, lens)]))   # behind a cache
+            out.append(engine.step([Entry(s, [5], [0]) for s in slots]))
+            for s in slots:
+                engine.close(s)
+        return out, launches
+    for lens in ([2], [17], [100, 33], [161], [300, 5, 260], [1000]):
+        (a, n), (b, m) = run(False, lens), run(True, lens)
+        assert n == m and all(torch.equal(x, y) for x, y in zip(a, b)), lens
