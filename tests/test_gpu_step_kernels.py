@@ -143,3 +143,45 @@ def test_experts(T, E, top, ff, W, same):
     hd, dd = h.double(), down.double()[ex]
     want, mag = torch.einsum("pw,pfw->pf", hd, dd), torch.einsum("pw,pfw->pf", hd.abs(), dd.abs())
     assert ((got - want).abs() <= (W + 4) * ULP * mag).all()
+
+
+@pytest.mark.parametrize("counts", [[512], [0, 1, 127, 128, 129, 0, 300, 2], [3] * 200, [0] * 37 + [600, 0, 0]])
+@pytest.mark.parametrize("ff,W", [(8, 64), (130, 200), (384, 1048)])
+def test_experts_of_a_prompt(counts, ff, W):
+    """From 512 rows on: tiles of 128 rows of one expert, dealt out to the blocks that walk over all of them.  The tensor cores add
+    in 32-bit without rounding to nearest, so a sum is off by at most (n + 4) 2^-23 times the magnitudes."""
+    from synaptix_b200 import ops
+    E, g = len(counts), torch.Generator().manual_seed(ff + len(counts))
+    ids = torch.cat([torch.full((c,), e) for e, c in enumerate(counts)])[torch.randperm(sum(counts), generator=g)]
+    T, top = len(ids), 1
+    x = torch.randn(T, W, generator=g).to(torch.bfloat16)
+    gate_up = (torch.randn(E, 2 * ff, W, generator=g) * W ** -0.5).to(torch.bfloat16)
+    plan = ops.moe_sort(ids.to(torch.int32).view(T, top).cuda(), E)
+    order, ex = plan.order.long().cpu(), ids[plan.order.long().cpu()]
+    z = torch.empty(T, 2 * ff, dtype=torch.float64)
+    mag = torch.empty_like(z)
+    for e in range(E):
+        r = (ex == e).nonzero()[:, 0]
+        z[r], mag[r] = x.double()[order[r]] @ gate_up[e].double().T, x.double()[order[r]].abs() @ gate_up[e].double().abs().T
+    off = (W + 4) * 2 * ULP * mag
+    a, u = z[:, :ff], z[:, ff:]
+    want = a * torch.sigmoid(a) * u
+    got = ops.moe_gate_up(x.cuda(), gate_up.cuda(), plan, top).double().cpu()
+    assert ((got - want).abs() <= 1.1 * off[:, :ff] * u.abs() + a.abs() * off[:, ff:] + (BF16 + 1e-5) * want.abs() + 1e-9).all()
+    got = ops.moe_down(x.cuda()[plan.order.long()], gate_up.cuda(), plan).double().cpu()
+    assert ((got - z).abs() <= off).all()
+
+
+@pytest.mark.parametrize("T,W,top", [(1, 4, 1), (3, 1024, 4), (5, 1028, 3), (2, 6, 2), (300, 260, 5)])
+@pytest.mark.parametrize("y_dtype,out_dtype", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16)])
+def test_weighted_sum_of_experts(T, W, top, y_dtype, out_dtype):
+    from synaptix_b200.ops.moe import moe_combine_rows
+    g = torch.Generator().manual_seed(T + W)
+    y = torch.randn(T * top, W, generator=g).to(y_dtype)
+    place = torch.randperm(T * top, generator=g).to(torch.int32)
+    w = torch.rand(T, top, generator=g)
+    got = moe_combine_rows(y.cuda(), place.cuda(), w.cuda(), out_dtype).double().cpu()
+    rows = y.double()[place.long()].view(T, top, W)
+    want = (rows * w.double()[..., None]).sum(1)
+    bound = (top + 1) * ULP * (rows.abs() * w.double()[..., None]).sum(1) + (BF16 if out_dtype == torch.bfloat16 else 0) * want.abs() + 1e-30
+    assert ((got - want).abs() <= bound).all()
