@@ -280,6 +280,12 @@ __global__ void __launch_bounds__(256, MR <= 2 ? 4 : (MR == 4 ? 3 : 2)) gemm_row
   for (int i = 0; i < MR; ++i)
 #pragma unroll
     for (int r = 0; r < R; ++r) acc[i][r] = 0.f;
+  // the first slice of W is on its way into L2 before the kernel ahead has ended (a hint: whatever it brings is read below;
+  // two prompts and eight steps of a 0.6B model in 32 bits: 21.75 -> 21.5 ms, with the activation launched early as well)
+  if ((lane & 7) == 0 && (ks * 32 + lane) * 4 < K) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(wr[r] + (ks * 32 + lane) * 4));
+  }
   pdl_wait();
   pdl_trigger();
 #pragma unroll (MR <= 2 ? 2 : 1)
@@ -1229,6 +1235,8 @@ extern "C" int sx_attn_generic_ex(const void* q, const void* k_pages, const void
 // ---------------------------------------------------------------------------------------
 template <typename T>
 __global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, int I, size_t n) {
+  pdl_wait();
+  pdl_trigger();
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n) return;
   const size_t t = idx / I;
@@ -1242,10 +1250,9 @@ extern "C" int sx_silu_mul(const void* gu, void* out, int n_tokens, int I, int d
   const size_t n = (size_t)n_tokens * I;
   if (n == 0) return 0;
   const unsigned grid = (unsigned)((n + 255) / 256);
-  if (dt == SX_F32) silu_mul_kernel<float><<<grid, 256, 0, stream>>>((const float*)gu, (float*)out, I, n);
-  else if (dt == SX_BF16) silu_mul_kernel<bf16><<<grid, 256, 0, stream>>>((const bf16*)gu, (bf16*)out, I, n);
-  else return SX_ERR_DTYPE;
-  return sx_launch_status();
+  if (dt == SX_F32) return sx_launch(silu_mul_kernel<float>, dim3(grid), dim3(256), 0, stream, (const float*)gu, (float*)out, I, n);
+  if (dt == SX_BF16) return sx_launch(silu_mul_kernel<bf16>, dim3(grid), dim3(256), 0, stream, (const bf16*)gu, (bf16*)out, I, n);
+  return SX_ERR_DTYPE;
 }
 
 // ---------------------------------------------------------------------------------------
