@@ -12,7 +12,7 @@
 //            W (128 rows x 64 each) into a ring of STAGES stages, signalled through mbarriers
 //   warp 1   allocates 256 columns of tensor memory; one lane issues 4 tcgen05.mma (K = 16
 //            each) per stage, and tcgen05.commit hands the stage back to the producer
-//   warps 2-5 epilogue: each reads its 32 lanes of the accumulator in chunks of 32 columns,
+//   warps 2-5 (2-9 in the persistent form) epilogue: each reads its 32 lanes of the accumulator in chunks of 32 columns,
 //            converts and stores
 // Rows of A beyond M, rows of W beyond N and the tail of K are zero-filled by TMA, so every size
 // with K % 8 == 0 is taken.  Epilogues: bfloat16 store; float32 store; SiLU(gate) * up for a
@@ -26,9 +26,11 @@
 #define TC_BK 64
 #define TC_A_BYTES (TC_BM * TC_BK * 2)            // 16 KB
 #define TC_THREADS 192
-// (Two groups of four epilogue warps, each with half of the tile's columns, where the epilogue has much to do: the ones that
-// prepare heads (a head a group) and the one that ends in the residual stream and its norm, which moves 10 bytes an element.)
-template <int EPI> struct TcThreads { static constexpr int N = (EPI == 4 || EPI == 5 || EPI == 6) ? 320 : TC_THREADS; };
+// The persistent kernel: two groups of four epilogue warps, each with half of the tile's columns (a head a group where heads are
+// prepared).  With one group the epilogue of gate/up, 128 x 128 results in 128 threads, took 11 us: all of a tile's MMAs at
+// K = 1,024, and the end of every product (1,024 -> 2 x 3,072 at 8,191 rows: 120 us, with two groups 74; 2,560 -> 2 x 9,728
+// at 521 rows: 58.5 and 52.3 us).
+#define TC_PERSISTENT_THREADS 320
 #define TC_RED_ROWS 6
 
 enum { TC_EPI_BF16 = 0, TC_EPI_F32 = 1, TC_EPI_SILU_MUL = 2, TC_EPI_PARTIAL = 3, TC_EPI_QKV = 4, TC_EPI_RESID_TANH = 5, TC_EPI_QKV_BIAS = 6 };
@@ -69,7 +71,7 @@ struct TcEp {
 
 // floats a warp of the persistent kernel's epilogue stages of a tile's vectors (see tc_store_chunk)
 template <int EPI> struct TcVec { static constexpr int N = EPI == 4 ? 0 : (EPI == 6 ? 128 : (EPI == 5 ? 384 : 256)); };
-template <int EPI> constexpr int tc_vec_floats() { return TcVec<EPI>::N * ((TcThreads<EPI>::N - 64) / 32); }
+template <int EPI> constexpr int tc_vec_floats() { return TcVec<EPI>::N * ((TC_PERSISTENT_THREADS - 64) / 32); }
 
 // BN: columns of W per block (256, or 128 for the split-K form); stages fill the shared memory
 template <int BN> struct TcShape {
@@ -349,14 +351,24 @@ __device__ __forceinline__ void tc_store_chunk(const uint32_t (&v)[32], const ui
     }
   }
   if (EPI == TC_EPI_SILU_MUL) {
+    float g[32];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (ep.bias) b = *reinterpret_cast<const float4*>(sv + 128 + 4 * i);
-      f[4 * i] = gate_mul(f[4 * i], __uint_as_float(u[4 * i]) + b.x, ep.act);
-      f[4 * i + 1] = gate_mul(f[4 * i + 1], __uint_as_float(u[4 * i + 1]) + b.y, ep.act);
-      f[4 * i + 2] = gate_mul(f[4 * i + 2], __uint_as_float(u[4 * i + 2]) + b.z, ep.act);
-      f[4 * i + 3] = gate_mul(f[4 * i + 3], __uint_as_float(u[4 * i + 3]) + b.w, ep.act);
+    for (int i = 0; i < 32; ++i) g[i] = __uint_as_float(u[i]);
+    if (ep.bias) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 b = *reinterpret_cast<const float4*>(sv + 128 + 4 * i);
+        g[4 * i] += b.x; g[4 * i + 1] += b.y; g[4 * i + 2] += b.z; g[4 * i + 3] += b.w;
+      }
+    }
+    // (the form is asked once a chunk: asked at every value, the values of a row were finished one after the other)
+    if (ep.act.form != SX_GATE_GELU_TANH && !(ep.act.limit > 0.f)) {
+      constexpr GateAct plain = {0.f, 0.f, SX_GATE_SIGMOID};
+#pragma unroll
+      for (int i = 0; i < 32; ++i) f[i] = gate_mul(f[i], g[i], plain);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) f[i] = gate_mul(f[i], g[i], ep.act);
     }
   }
   if (EPI == TC_EPI_F32) {
@@ -448,7 +460,7 @@ __host__ __device__ inline bool tc_piece(const TcPlan& p, int c, int i, TcPiece&
 }
 
 template <int EPI, int BN>
-__global__ void __launch_bounds__(TcThreads<EPI>::N, 1) gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
+__global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                            const __grid_constant__ CUtensorMap map_w,
                                                                            void* __restrict__ out, int M, int N, int K,
                                                                            int n_whole, int zmax, int sp,
@@ -496,7 +508,7 @@ __global__ void __launch_bounds__(TcThreads<EPI>::N, 1) gemm_tc_persistent_kerne
     }
     for (int b = 0; b < 2; ++b) {
       tc_mbar_init(acc_full0 + 8 * b, 1);
-      tc_mbar_init(acc_empty0 + 8 * b, (TcThreads<EPI>::N - 64) / 32);          // one arrival per epilogue warp
+      tc_mbar_init(acc_empty0 + 8 * b, (TC_PERSISTENT_THREADS - 64) / 32);          // one arrival per epilogue warp
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -583,7 +595,7 @@ __global__ void __launch_bounds__(TcThreads<EPI>::N, 1) gemm_tc_persistent_kerne
     }
   } else {
     const int quarter = warp & 3;
-    constexpr int ET = TcThreads<EPI>::N - 64, GROUPS = ET / 128;        // epilogue threads; groups of four warps
+    constexpr int ET = TC_PERSISTENT_THREADS - 64, GROUPS = ET / 128;        // epilogue threads; groups of four warps
     const int group = (warp - 2) >> 2;                                  // which half of the tile's columns (one group: all)
     const int et = threadIdx.x - 64;                                    // among the epilogue threads
     // a partial tile in the workspace: [tile among the cut ones][piece][128 rows][BN columns] float32
@@ -1067,7 +1079,7 @@ static int tc_launch_persistent(const CUtensorMap& ma, const CUtensorMap& mw, vo
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   // with whole tiles after them, the blocks of a cut tile add up inside the kernel; without, a second kernel does
-  int rc = sx_launch(kern, h.G, dim3(TcThreads<EPI>::N), smem, stream, ma, mw, out, M, N, K, h.n_whole, h.zmax, h.sp, ws, counts, status, qk, ep);
+  int rc = sx_launch(kern, h.G, dim3(TC_PERSISTENT_THREADS), smem, stream, ma, mw, out, M, N, K, h.n_whole, h.zmax, h.sp, ws, counts, status, qk, ep);
   if (rc || h.R == 0 || h.sp > 0 || EPI == TC_EPI_QKV || EPI == TC_EPI_QKV_BIAS) return rc;
   const int tile_n = (EPI == TC_EPI_SILU_MUL) ? BN / 2 : BN;
   const long long total = (long long)h.R * TC_BM * (tile_n / 4);
