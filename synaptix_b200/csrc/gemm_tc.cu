@@ -7,12 +7,12 @@
 // (crates/synaptix-kernels-cuda/src/best_cu/gemm/gemm_bf16.cu:37-61,1678-2013); it has no
 // tcgen05 path.
 //
-// One block computes one 128 x 256 tile of C.
+// One block computes one 128 x 256 tile of C (the persistent form below: pairs of blocks and other widths, too).
 //   warp 0   producer: for every 64-wide slice of K, one TMA load of A (128 rows x 64) and two of
 //            W (128 rows x 64 each) into a ring of STAGES stages, signalled through mbarriers
 //   warp 1   allocates 256 columns of tensor memory; one lane issues 4 tcgen05.mma (K = 16
 //            each) per stage, and tcgen05.commit hands the stage back to the producer
-//   warps 2-5 (2-9 in the persistent form) epilogue: each reads its 32 lanes of the accumulator in chunks of 32 columns,
+//   warps 2-5 epilogue: each reads its 32 lanes of the accumulator in chunks of 32 columns,
 //            converts and stores
 // Rows of A beyond M, rows of W beyond N and the tail of K are zero-filled by TMA, so every size
 // with K % 8 == 0 is taken.  Epilogues: bfloat16 store; float32 store; SiLU(gate) * up for a
@@ -27,10 +27,10 @@
 #define TC_A_BYTES (TC_BM * TC_BK * 2)            // 16 KB
 #define TC_THREADS 192
 // The persistent kernel: two groups of four epilogue warps, each with half of the tile's columns (a head a group where heads are
-// prepared).  With one group the epilogue of gate/up, 128 x 128 results in 128 threads, took 11 us: all of a tile's MMAs at
-// K = 1,024, and the end of every product (1,024 -> 2 x 3,072 at 8,191 rows: 120 us, with two groups 74; 2,560 -> 2 x 9,728
-// at 521 rows: 58.5 and 52.3 us).
-#define TC_PERSISTENT_THREADS 320
+// prepared; a 128-wide tile holds one head and has one group there).  With one group the epilogue of gate/up, 128 x 128 results in
+// 128 threads, took 11 us: all of a tile's MMAs at K = 1,024, and the end of every product (1,024 -> 2 x 3,072 at 2,048 rows:
+// 39.0 us, with two groups 23.3; 2,560 -> 2 x 9,728 at 521 rows: 58.5 and 52.3).
+template <int EPI, int BN> struct TcThreads { static constexpr int N = 64 + (BN == 256 ? 2 : ((EPI == 4 || EPI == 6) ? 1 : 2)) * 128; };
 #define TC_RED_ROWS 6
 
 enum { TC_EPI_BF16 = 0, TC_EPI_F32 = 1, TC_EPI_SILU_MUL = 2, TC_EPI_PARTIAL = 3, TC_EPI_QKV = 4, TC_EPI_RESID_TANH = 5, TC_EPI_QKV_BIAS = 6 };
@@ -71,13 +71,14 @@ struct TcEp {
 
 // floats a warp of the persistent kernel's epilogue stages of a tile's vectors (see tc_store_chunk)
 template <int EPI> struct TcVec { static constexpr int N = EPI == 4 ? 0 : (EPI == 6 ? 128 : (EPI == 5 ? 384 : 256)); };
-template <int EPI> constexpr int tc_vec_floats() { return TcVec<EPI>::N * ((TC_PERSISTENT_THREADS - 64) / 32); }
+template <int EPI, int BN> constexpr int tc_vec_floats() { return TcVec<EPI>::N * ((TcThreads<EPI, BN>::N - 64) / 32); }
 
-// BN: columns of W per block (256, or 128 for the split-K form); stages fill the shared memory
-template <int BN> struct TcShape {
-  static constexpr int B_BYTES = BN * TC_BK * 2;
+// BN: rows of W per tile (256 or 128); CG: blocks that compute a tile's instructions together (a pair stages half of W's rows
+// each); stages fill the shared memory
+template <int BN, int CG = 1> struct TcShape {
+  static constexpr int B_BYTES = BN / CG * TC_BK * 2;
   static constexpr int STAGE_BYTES = TC_A_BYTES + B_BYTES;
-  static constexpr int STAGES = BN == 256 ? 4 : 6;
+  static constexpr int STAGES = (192 << 10) / STAGE_BYTES;      // 4, 6 or 8
 };
 
 template <int EPI, int BN>
@@ -223,13 +224,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
 }
 
 // =======================================================================================
-// The persistent form for many rows: one block per SM walks over the 128 x 256 tiles of C
+// The persistent form for many rows: one block per SM (or a pair per two) walks over the tiles of C
 // (tile t -> row tile t % tiles_m, column tile t / tiles_m, so that blocks running at the same
-// time share W tiles through L2).  Tensor memory holds TWO accumulators (2 x 256 columns): while
+// time share W tiles through L2).  Tensor memory holds TWO accumulators (2 x BN columns): while
 // the epilogue warps read tile i out of one, the MMA warp is already filling the other with tile
 // i + 1, and the TMA ring runs ahead across tiles.  Barriers: full/empty per stage, and
 // acc_full/acc_empty per accumulator.  When the tiles do not fill a round of all SMs (a nearly empty last
 // round, or fewer tiles than SMs as in steps of a few dozen rows), those tiles are cut over K (TcPlan below).
+//
+// Tiles come in four forms.  CG == 2: a pair of neighbouring SMs computes 256 rows with one instruction (cta_group::2); each
+// stages its 128 rows of A and HALF of the tile's rows of W, so that a W tile crosses from L2 once for 256 rows and an
+// instruction reads 6 instead of 8 KB of shared memory a 128 x 128 x 16 step.  The first block's barriers count both blocks'
+// copies, its warp 1 issues, and the commits arrive at both blocks' barriers.  BN == 128: half as wide, for few hundred rows,
+// where 256-wide tiles leave SMs idle.  Products of a step of 8,191 rows (2,560 -> 6,144, 4,096 -> 2,560, 2,560 -> 2 x 9,728,
+// 9,728 -> 2,560) take 1,298 us in 256-wide tiles of one block and 1,104 of a pair, at 2,048 rows 338 and 292; at 611 rows
+// 4,096 -> 2,560 takes 27 us in 256-wide tiles of one block, 25.3 of a pair, 21.2 and 18.6 in 128-wide ones of one and of a pair
+// (a 128 x 128 instruction of one block needs all of shared memory's bandwidth: its slices of K take 0.264 instead of 0.21 us).
 // =======================================================================================
 __device__ __forceinline__ void tc_mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
@@ -459,8 +469,8 @@ __host__ __device__ inline bool tc_piece(const TcPlan& p, int c, int i, TcPiece&
   return true;
 }
 
-template <int EPI, int BN>
-__global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
+template <int EPI, int BN, int CG>
+__global__ void __launch_bounds__(TcThreads<EPI, BN>::N, 1) gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                            const __grid_constant__ CUtensorMap map_w,
                                                                            void* __restrict__ out, int M, int N, int K,
                                                                            int n_whole, int zmax, int sp,
@@ -469,7 +479,7 @@ __global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_k
                                                                            int* __restrict__ status, const TcQkv qk,
                                                                            const TcEp ep) {
   constexpr bool QKV = EPI == TC_EPI_QKV || EPI == TC_EPI_QKV_BIAS;
-  constexpr int STAGES = TcShape<BN>::STAGES, B_BYTES = TcShape<BN>::B_BYTES, STAGE_BYTES = TcShape<BN>::STAGE_BYTES;
+  constexpr int STAGES = TcShape<BN, CG>::STAGES, B_BYTES = TcShape<BN, CG>::B_BYTES, STAGE_BYTES = TcShape<BN, CG>::STAGE_BYTES;
   extern __shared__ unsigned char tc_smem_raw[];
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + STAGES * STAGE_BYTES);   // full[S], empty[S], acc_full[2], acc_empty[2]
@@ -482,23 +492,26 @@ __global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_k
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_out = (EPI == TC_EPI_SILU_MUL) ? N / 2 : N;
   const int tile_n = (EPI == TC_EPI_SILU_MUL) ? BN / 2 : BN;
-  const int tiles_m = (M + TC_BM - 1) / TC_BM, tiles_n = (n_out + tile_n - 1) / tile_n;
+  // (rows of tiles are counted in tiles of the block or pair: 128 or 256 rows)
+  const int tiles_m = (M + CG * TC_BM - 1) / (CG * TC_BM), tiles_n = (n_out + tile_n - 1) / tile_n;
   const int nkb = (K + TC_BK - 1) / TC_BK;
+  const int rank = CG == 2 ? (int)(blockIdx.x & 1) : 0, unit = (int)blockIdx.x / CG, units = (int)gridDim.x / CG;
+  auto m_of = [&](int tile) { return ((tile % tiles_m) * CG + rank) * TC_BM; };
   TcPlan plan;
-  plan.n_whole = n_whole; plan.R = tiles_m * tiles_n - n_whole; plan.nkb = nkb; plan.G = (int)gridDim.x;
+  plan.n_whole = n_whole; plan.R = tiles_m * tiles_n - n_whole; plan.nkb = nkb; plan.G = units;
   plan.sp = sp;
   plan.U = (long long)plan.R * nkb;
   const bool coop = sp > 0;            // the blocks of a cut tile add up in this kernel (else a second kernel does)
-  // This block's work in order: its pieces of the cut tiles FIRST (short, so that adding the partial tiles up
-  // hides behind the MMAs of the whole tiles), then whole tiles blockIdx.x, blockIdx.x + G, ...
+  // This block's (or pair's) work in order: its pieces of the cut tiles FIRST (short, so that adding the partial tiles up
+  // hides behind the MMAs of the whole tiles), then whole tiles unit, unit + G, ...
   TcPiece pc[2];
   int n_pc = 0;
-  if (tc_piece(plan, blockIdx.x, 0, pc[0])) { n_pc = 1; if (tc_piece(plan, blockIdx.x, 1, pc[1])) n_pc = 2; }
-  const int n_mine = n_whole > (int)blockIdx.x ? (n_whole - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  if (tc_piece(plan, unit, 0, pc[0])) { n_pc = 1; if (tc_piece(plan, unit, 1, pc[1])) n_pc = 2; }
+  const int n_mine = n_whole > unit ? (n_whole - 1 - unit) / units + 1 : 0;
   const int n_work = n_pc + n_mine;
   auto work_of = [&](int w, int& tile, int& kb_lo, int& kb_hi) {
     if (w < n_pc) { tile = pc[w].tile; kb_lo = pc[w].kb_lo; kb_hi = pc[w].kb_hi; }
-    else { tile = blockIdx.x + (w - n_pc) * gridDim.x; kb_lo = 0; kb_hi = nkb; }
+    else { tile = unit + (w - n_pc) * units; kb_lo = 0; kb_hi = nkb; }
   };
 
   if (threadIdx.x == 0) {
@@ -508,16 +521,22 @@ __global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_k
     }
     for (int b = 0; b < 2; ++b) {
       tc_mbar_init(acc_full0 + 8 * b, 1);
-      tc_mbar_init(acc_empty0 + 8 * b, (TC_PERSISTENT_THREADS - 64) / 32);          // one arrival per epilogue warp
+      tc_mbar_init(acc_empty0 + 8 * b, CG * ((TcThreads<EPI, BN>::N - 64) / 32));   // one arrival per epilogue warp (of both blocks)
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc_smem(tmem_slot)), "r"((uint32_t)(2 * BN)) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    if (CG == 2) {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc_smem(tmem_slot)), "r"((uint32_t)(2 * BN)) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc_smem(tmem_slot)), "r"((uint32_t)(2 * BN)) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-  __syncthreads();
+  __syncwarp();
+  if (CG == 2) cluster_sync_all(); else __syncthreads();      // a pair's barriers are used by both blocks
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();          // barriers and tensor memory are set up; the operands may come from the kernel before
@@ -529,12 +548,16 @@ __global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_k
   if (warp == 0) {
     const bool leader = tc_elect_one();
     const uint32_t tiles_addr = tc_smem(tiles);
+    // a pair's copies are counted by the first block's barriers
+    const uint32_t full_at = CG == 2 ? tc_mapa(full0, 0) : full0;
     uint32_t it = 0;
     bool ok = true;
     for (int w = 0; w < n_work && ok; ++w) {
       int tile, kb_lo, kb_hi;
       work_of(w, tile, kb_lo, kb_hi);
-      const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * tile_n;
+      const int m0 = m_of(tile), n0 = (tile / tiles_m) * tile_n;
+      // W's rows: the second half of a tile's are the next 128, or the up rows; a pair's blocks take a half each
+      const int n1 = (EPI == TC_EPI_SILU_MUL) ? N / 2 + n0 : n0 + BN / 2;
       for (int kb = kb_lo; kb < kb_hi; ++kb, ++it) {
         const uint32_t s = it % STAGES;
         ok = __all_sync(0xffffffffu, tc_mbar_wait(empty0 + 8 * s, ((it / STAGES) & 1) ^ 1));
@@ -542,20 +565,25 @@ __global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_k
           if (leader) sx_set_status(status, 1);
           break;
         }
-        const uint32_t a_dst = tiles_addr + s * STAGE_BYTES, b_dst = a_dst + TC_A_BYTES, bar = full0 + 8 * s;
+        const uint32_t a_dst = tiles_addr + s * STAGE_BYTES, b_dst = a_dst + TC_A_BYTES, bar = full_at + 8 * s;
         if (leader) {
-          tc_mbar_expect_tx(bar, STAGE_BYTES);
-          tc_tma_load_2d(a_dst, &map_a, kb * TC_BK, m0, bar);
-          tc_tma_load_2d(b_dst, &map_w, kb * TC_BK, n0, bar);
-          if (BN == 256)
-            tc_tma_load_2d(b_dst + B_BYTES / 2, &map_w, kb * TC_BK, (EPI == TC_EPI_SILU_MUL) ? N / 2 + n0 : n0 + BN / 2, bar);
+          if (CG == 2) {
+            if (rank == 0) tc_mbar_expect_tx(full0 + 8 * s, 2 * STAGE_BYTES);
+            tc_tma_load_2d_pair(a_dst, &map_a, kb * TC_BK, m0, bar);
+            tc_tma_load_2d_pair(b_dst, &map_w, kb * TC_BK, rank ? n1 : n0, bar);
+          } else {
+            tc_mbar_expect_tx(bar, STAGE_BYTES);
+            tc_tma_load_2d(a_dst, &map_a, kb * TC_BK, m0, bar);
+            tc_tma_load_2d(b_dst, &map_w, kb * TC_BK, n0, bar);
+            tc_tma_load_2d(b_dst + B_BYTES / 2, &map_w, kb * TC_BK, n1, bar);
+          }
         }
         __syncwarp();
       }
     }
     __syncwarp();
-  } else if (warp == 1) {
-    constexpr uint32_t idesc = tc_instr_desc(TC_BM, BN);
+  } else if (warp == 1 && rank == 0) {          // (a pair's instructions are issued by its first block)
+    constexpr uint32_t idesc = tc_instr_desc(CG * TC_BM, BN);
     const bool leader = tc_elect_one();
     const uint32_t tiles_addr = tc_smem(tiles);
     uint32_t it = 0;
@@ -584,26 +612,31 @@ __global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_k
         const uint32_t acc = kb != kb_lo;
         if (leader) {
 #pragma unroll
-          for (int k = 0; k < TC_BK / 16; ++k)          // 32 bytes further along K: 2 in the descriptor's 16-byte units
-            tc_mma(d_tmem, da + 2 * k, db + 2 * k, idesc, acc | (k != 0));
-          tc_commit(empty0 + 8 * s);
+          for (int k = 0; k < TC_BK / 16; ++k) {        // 32 bytes further along K: 2 in the descriptor's 16-byte units
+            if (CG == 2) tc_mma_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, acc | (k != 0));
+            else tc_mma(d_tmem, da + 2 * k, db + 2 * k, idesc, acc | (k != 0));
+          }
+          if (CG == 2) tc_commit_pair(empty0 + 8 * s); else tc_commit(empty0 + 8 * s);
         }
         __syncwarp();
       }
-      if (leader) tc_commit(acc_full0 + 8 * buf);
+      if (leader) { if (CG == 2) tc_commit_pair(acc_full0 + 8 * buf); else tc_commit(acc_full0 + 8 * buf); }
       __syncwarp();
     }
-  } else {
+  } else if (warp >= 2) {
     const int quarter = warp & 3;
-    constexpr int ET = TC_PERSISTENT_THREADS - 64, GROUPS = ET / 128;        // epilogue threads; groups of four warps
+    // an accumulator is handed back to whoever issues the instructions
+    const uint32_t acc_empty_at = CG == 2 ? tc_mapa(acc_empty0, 0) : acc_empty0;
+    auto hand_back = [&](uint32_t buf) { if (CG == 2) tc_mbar_arrive_cluster(acc_empty_at + 8 * buf); else tc_mbar_arrive(acc_empty_at + 8 * buf); };
+    constexpr int ET = TcThreads<EPI, BN>::N - 64, GROUPS = ET / 128;        // epilogue threads; groups of four warps
     const int group = (warp - 2) >> 2;                                  // which half of the tile's columns (one group: all)
     const int et = threadIdx.x - 64;                                    // among the epilogue threads
     // a partial tile in the workspace: [tile among the cut ones][piece][128 rows][BN columns] float32
-    auto ws_of = [&](int tile, int z) { return piece_ws + ((size_t)(tile - n_whole) * zmax + z) * (TC_BM * BN); };
+    auto ws_of = [&](int tile, int z) { return piece_ws + ((size_t)((tile - n_whole) * CG + rank) * zmax + z) * (TC_BM * BN); };
     // a finished accumulator -> out, with the epilogue
     auto finish_tile = [&](int w, int tile) -> bool {
       const uint32_t buf = w & 1, use = w >> 1;
-      const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * tile_n;
+      const int m0 = m_of(tile), n0 = (tile / tiles_m) * tile_n;
       const int row = m0 + quarter * 32 + lane;
       // (head preparation: where this thread's token goes is looked up while the tile's MMAs still run)
       const bool live = row < M;
@@ -677,7 +710,7 @@ __global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_k
           // this warp's part of the accumulator is in registers: hand it back
           asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
           __syncwarp();
-          if (lane == 0) tc_mbar_arrive(acc_empty0 + 8 * buf);
+          if (lane == 0) hand_back(buf);
           const bool is_q = head < qk.nh, is_k = !is_q && head < qk.nh + qk.nkv, is_v = !is_q && !is_k && head < qk.nh + 2 * qk.nkv;
           bf16* dst = nullptr;
           if (live) {
@@ -746,7 +779,7 @@ __global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_k
             // everything of this accumulator is in registers: hand it back before the last stores
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncwarp();
-            if (lane == 0) tc_mbar_arrive(acc_empty0 + 8 * buf);
+            if (lane == 0) hand_back(buf);
           }
           if (row < M && n0 + c0 < n_out) tc_store_chunk<EPI>(v, u, out, row, n0 + c0, n_out, whole_at(c0), sv + (c0 - cb), hv, ep);
           if (RESID) {
@@ -765,7 +798,7 @@ __global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_k
       const int tile = pc[w].tile;
       if (pc[w].nz == 1) { alive = finish_tile(w, tile); continue; }
       const uint32_t buf = w & 1, use = w >> 1;
-      const int m0 = (tile % tiles_m) * TC_BM;
+      const int m0 = m_of(tile);
       const int row = m0 + quarter * 32 + lane;
       if (!tc_mbar_wait(acc_full0 + 8 * buf, use & 1)) {
         if (lane == 0) sx_set_status(status, 3);
@@ -775,21 +808,22 @@ __global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_k
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       const uint32_t t_row = tmem_base + buf * BN + ((uint32_t)(quarter * 32) << 16);
       float* dst = ws_of(tile, pc[w].z) + (size_t)(quarter * 32 + lane) * BN;
-      // (four tcgen05.ld on the way per wait)
+      // (up to four tcgen05.ld on the way per wait)
+      constexpr int CWP = BN / GROUPS < 128 ? BN / GROUPS : 128;
 #pragma unroll 1
-      for (int c0 = group * (BN / GROUPS); c0 < (group + 1) * (BN / GROUPS); c0 += 128) {
-        uint32_t v[4][32];
+      for (int c0 = group * (BN / GROUPS); c0 < (group + 1) * (BN / GROUPS); c0 += CWP) {
+        uint32_t v[CWP / 32][32];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) tc_ld32(t_row + c0 + 32 * j, v[j]);
+        for (int j = 0; j < CWP / 32; ++j) tc_ld32(t_row + c0 + 32 * j, v[j]);
         asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-        if (c0 + 128 >= (group + 1) * (BN / GROUPS)) {
+        if (c0 + CWP >= (group + 1) * (BN / GROUPS)) {
           asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
           __syncwarp();
-          if (lane == 0) tc_mbar_arrive(acc_empty0 + 8 * buf);
+          if (lane == 0) hand_back(buf);
         }
         if (row < M) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
+          for (int j = 0; j < CWP / 32; ++j)
 #pragma unroll
             for (int i = 0; i < 8; ++i)
               reinterpret_cast<float4*>(dst + c0 + 32 * j)[i] = make_float4(__uint_as_float(v[j][4 * i]), __uint_as_float(v[j][4 * i + 1]),
@@ -799,7 +833,7 @@ __global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_k
       if (coop) {
         __threadfence();
         asm volatile("bar.sync 1, %0;\n" ::"n"(ET) : "memory");                 // the epilogue warps
-        if (threadIdx.x == 64) atomicAdd(piece_count + 2 * (tile - n_whole), 1);
+        if (threadIdx.x == 64) atomicAdd(piece_count + 2 * ((tile - n_whole) * CG + rank), 1);
       }
     }
     // 2: the blocks that hold the pieces of one tile add its partial tiles up together: each waits (bounded)
@@ -811,7 +845,7 @@ __global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_k
     for (int w = 0; w < n_pc && alive && coop; ++w) {
       if (pc[w].nz == 1) continue;
       const int tile = pc[w].tile, nz = pc[w].nz, z = pc[w].z;
-      int* cnt = piece_count + 2 * (tile - n_whole);
+      int* cnt = piece_count + 2 * ((tile - n_whole) * CG + rank);
       if (threadIdx.x == 64) {
         bool all = false;
         for (uint32_t i = 0; i < TC_SPIN_LIMIT; ++i) {
@@ -825,18 +859,18 @@ __global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_k
       asm volatile("bar.sync 1, %0;\n" ::"n"(ET) : "memory");
       if (*piece_ok) {
         __threadfence();
-        const int m0 = (tile % tiles_m) * TC_BM, n0 = (tile / tiles_m) * tile_n;
-        const int rows_here = min(TC_BM, M - m0);
+        const int m0 = m_of(tile), n0 = (tile / tiles_m) * tile_n;
+        const int rows_here = max(0, min(TC_BM, M - m0));
         const int per = (rows_here + nz - 1) / nz;
         const int r_lo = m0 + z * per, r_hi = min(m0 + rows_here, r_lo + per);
         const int cols = min(tile_n, n_out - n0);                        // output columns of this tile
-        constexpr int TPR = EPI == TC_EPI_SILU_MUL ? 32 : 64;            // threads a row (four columns a thread)
+        constexpr int TPR = (EPI == TC_EPI_SILU_MUL ? BN / 2 : BN) / 4;  // threads a row (four columns a thread)
         constexpr int RPI = ET / TPR;                                   // rows at a time
         const int c4 = (et % TPR) * 4;
         const float* base = ws_of(tile, 0);
         const size_t plane = (size_t)TC_BM * BN;
         // TC_RED_ROWS of a thread's rows at a time and four pieces unrolled, so that dozens of loads are in flight:
-        // this adding-up runs on 128 threads a block, and with 8 loads in flight it took 40 us for a tile cut
+        // with 128 threads a block and 8 loads in flight this adding-up took 40 us for a tile cut
         // into 13 pieces (longer than the 26 us of MMAs it is meant to hide behind)
         for (int rb = r_lo + et / TPR; rb < r_hi && c4 < cols; rb += TC_RED_ROWS * RPI) {
           float4 a[TC_RED_ROWS], b[TC_RED_ROWS];
@@ -876,15 +910,17 @@ __global__ void __launch_bounds__(TC_PERSISTENT_THREADS, 1) gemm_tc_persistent_k
     }
     // 3: the whole tiles
     for (int w = n_pc; w < n_work && alive; ++w) {
-      alive = finish_tile(w, blockIdx.x + (w - n_pc) * gridDim.x);
+      alive = finish_tile(w, unit + (w - n_pc) * units);
     }
   }
 
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-  __syncthreads();
+  __syncwarp();
+  if (CG == 2) cluster_sync_all(); else __syncthreads();      // neither block leaves while the other may still reach it
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"((uint32_t)(2 * BN)) : "memory");
+    if (CG == 2) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"((uint32_t)(2 * BN)) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"((uint32_t)(2 * BN)) : "memory");
   }
 }
 
@@ -925,6 +961,32 @@ static int tc_sm_count() {
     if (cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n[dev] <= 0) n[dev] = 148;
   }
   return n[dev];
+}
+
+// how many pairs of blocks are on the GPU at once (the pairs of a cut tile wait for one another)
+static int tc_pair_count() {
+  static int n[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (!n[dev]) {
+    using Sh = TcShape<256, 2>;
+    const size_t smem = 1024 + Sh::STAGES * Sh::STAGE_BYTES + (2 * Sh::STAGES + 4) * sizeof(uint64_t) + 32 + tc_vec_floats<TC_EPI_BF16, 256>() * sizeof(float);
+    auto kern = gemm_tc_persistent_kernel<TC_EPI_BF16, 256, 2>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2); cfg.blockDim = dim3(TcThreads<TC_EPI_BF16, 256>::N); cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    int pairs = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&pairs, kern, &cfg) != cudaSuccess || pairs <= 0) {
+      cudaGetLastError();
+      pairs = -1;
+    }
+    n[dev] = pairs;
+  }
+  return n[dev] > 0 ? n[dev] : 0;
 }
 
 // The partial tiles of the cut tiles, added up in piece order, with the epilogue: one thread per (cut tile, row,
@@ -969,31 +1031,39 @@ __global__ void tc_pieces_reduce_kernel(const float* __restrict__ ws, void* __re
 
 // What the persistent kernel does for a product: how many tiles are computed whole, how many are cut, the most
 // pieces a cut tile has, and the grid.
-struct TcHostPlan { int n_whole, R, zmax, G, sp; };
+struct TcHostPlan { int n_whole, R, zmax, G, sp, bn, cg; };    // cg == 2: all of it counted in pairs of blocks and tiles of 256 rows; bn: rows of W a tile
 // Several rows of tiles that are fewer than the SMs (a prompt step of a few hundred rows: 512 x 2,560 has 40
 // tiles) can be cut over K as well.  Whole tiles leave most SMs idle and take 5 + 0.352 us x slices whatever their
 // number (a 128 x 256 tile with K = 4,096: 27.5 us, K = 9,728: 58.5 us), and the uniform split over K in 128-wide
 // tiles (sx_gemm_tc with splits > 1) took 40 us for 512 x 2,560 x 4,096 and 69 us for K = 9,728.  Cut into G
-// shares the same products take about 6.5 + 0.352 x slices / G + 0.07 G us (the last term: G partial tiles written
-// and read again by the second kernel): 23.5 and 37 us for the two products above.
+// shares the same products take about 6.3 + 0.352 x slices / G + 0.07 G us (the last term: G partial tiles written
+// and read again by the second kernel): 23.5 and 37 us for the two products above.  (128-wide tiles of a pair take 18.5 and
+// 36.5 whole: the cut form is left for fewer rows still, 256 x 9,728 -> 2,560 in 128-wide tiles cut in three 23.5 against 33.1.)
 // The figures are measured on a B200 with the weights coming from HBM; a product is cut only when the estimate is
 // a tenth below the whole tiles'.  Not for a handful of tiles (the uniform split is faster up to a dozen).  The
 // pieces of the row tiles over one block of W run at different times, so W is read once per row of tiles, from HBM
 // when L2 cannot keep it (5,120 x 25,600 at 512 rows: 196 us cut, 153 us whole): for a matrix larger than half
 // of L2 the estimate is at least that traffic's time.
+// What a form's work takes, us, measured on a B200 with the weights coming from HBM: launching, filling the ring and the last
+// epilogue; a slice of K (64) of a tile; the partial tiles' trip through memory and their adding up, behind whole tiles (which
+// grows with the pieces of a tile) and by the second kernel (which grows with all pieces).
+static double tc_base_time(int bn, int cg) { return bn == 256 ? (cg == 2 ? 6.1 : 4.8) : (cg == 2 ? 4.9 : 4.3); }
+static double tc_slice_time(int bn, int cg) { return bn == 256 ? (cg == 2 ? 0.315 : 0.352) : (cg == 2 ? 0.21 : 0.264); }
+static double tc_trip_time(int bn, int cg, int pieces) { return (bn == 256 ? (cg == 2 ? 4.8 : 6.5) : 3.5) + 0.2 * pieces; }
+static double tc_second_time(int bn, int pieces) { return 1.5 + 0.07 * (bn / 256.0) * pieces; }
 static int g_tc_cut_few = 1;
 extern "C" void sx_gemm_tc_cut_few(int on) { g_tc_cut_few = on ? 1 : 0; }
-static bool tc_cut_few(int tiles_m, int n_tiles, int nkb, long long U, long long w_bytes, int sms, int* G) {
+static bool tc_cut_few(int tiles_m, int n_tiles, int nkb, int bn, long long w_bytes, int sms, int* G) {
   if (!g_tc_cut_few || tiles_m <= 1 || n_tiles >= sms || n_tiles <= 12) return false;
   // a matrix larger than half of L2 comes from HBM once per row of tiles
   const double t_hbm = w_bytes > (64LL << 20) ? (double)tiles_m * (double)w_bytes / 6.0e6 : 0.0;
   // every tile into the same number of pieces, so that no block's share begins in one tile and ends in the next
   // (a block with two pieces stores two partial tiles: 30 tiles in 97 shares took 24.4 us, in 120 shares 18.4 us)
-  const double t_whole = 5.0 + 0.352 * nkb;
+  const double base = tc_base_time(bn, 1), slice = tc_slice_time(bn, 1), t_whole = base + slice * nkb;
   double best = 0.9 * t_whole;
   int pieces = 0;
   for (int z = 2; z * n_tiles <= sms && z <= nkb; ++z) {
-    double t_cut = 6.5 + 0.352 * (double)nkb / z + 0.07 * z * n_tiles;
+    double t_cut = base + slice * nkb / z + tc_second_time(bn, z * n_tiles);
     if (t_cut < t_hbm + 6.5) t_cut = t_hbm + 6.5;
     if (t_cut < best) { best = t_cut; pieces = z; }
   }
@@ -1002,16 +1072,18 @@ static bool tc_cut_few(int tiles_m, int n_tiles, int nkb, long long U, long long
   return true;
 }
 
-static TcHostPlan tc_plan_stream(int M, int N, int K, int epi, bool allow_cut) {
-  const int tile_n = epi == TC_EPI_SILU_MUL ? 128 : 256;
+static TcHostPlan tc_plan_form(int M, int N, int K, int epi, bool allow_cut, int bn, int cg) {
+  const int tile_n = epi == TC_EPI_SILU_MUL ? bn / 2 : bn;
   const int n_out = epi == TC_EPI_SILU_MUL ? N / 2 : N;
-  const int tiles_m = (M + TC_BM - 1) / TC_BM, tiles_n = (n_out + tile_n - 1) / tile_n;
+  const int tiles_m = (M + cg * TC_BM - 1) / (cg * TC_BM), tiles_n = (n_out + tile_n - 1) / tile_n;
   const long long n_tiles_ll = (long long)tiles_m * tiles_n;
-  const int sms = tc_sm_count();
+  const int sms = cg == 2 ? tc_pair_count() : tc_sm_count();
   const int nkb = (K + TC_BK - 1) / TC_BK;
   TcHostPlan h;
   h.sp = 0;
-  if (n_tiles_ll > 0x3fffffffLL) { h.n_whole = -1; h.R = h.zmax = h.G = 0; return h; }
+  h.bn = bn;
+  h.cg = cg;
+  if (n_tiles_ll > 0x3fffffffLL || sms <= 0) { h.n_whole = -1; h.R = h.zmax = h.G = 0; return h; }
   const int n_tiles = (int)n_tiles_ll;
   const int R0 = n_tiles >= sms ? n_tiles % sms : n_tiles;
   // cut when the round would be at most half full, or for a single row of tiles (few rows: the partial tiles are small)
@@ -1021,23 +1093,21 @@ static TcHostPlan tc_plan_stream(int M, int N, int K, int epi, bool allow_cut) {
   // Fewer tiles than SMs are cut only when they are at least half as many (each then falls into two or three
   // pieces); a handful of tiles would fall into a dozen pieces each, and the older uniform split (sx_gemm_tc with
   // splits > 1: 128-wide tiles, fewer and larger partial tiles) measured faster there.
-  // Behind three or more rounds of whole tiles a short last round costs little, and cutting it did not pay
-  // (gate/up at 2,048 rows: 1,216 tiles, 164 us cut against 155 us whole).
   int G_few = 0;
-  const bool few = tc_cut_few(tiles_m, n_tiles, nkb, U, (long long)N * K * 2, sms, &G_few);
-  // Behind whole tiles a piece costs its share of a tile's slices and about 8.6 us for the partial tiles' trip and the
-  // adding up (by the four epilogue warps, before their whole tile's epilogue); that has to stay well under the
+  const bool few = cg == 1 && tc_cut_few(tiles_m, n_tiles, nkb, bn, (long long)N * K * 2, sms, &G_few);
+  // Behind whole tiles a piece costs its share of a tile's slices and the time of the partial tiles' trip and the
+  // adding up (by the epilogue warps, before their whole tile's epilogue); that has to stay well under the
   // round of whole tiles it saves (1,024 x 6,144 x 2,560, 44 tiles in three pieces each: 40.1 us cut, 34.7 whole;
   // the same rows x 6,144 x 4,096: 48.2 cut, 52.3 whole).
   bool last_round_pays = false;
   if (n_tiles >= sms && R0 > 0) {
     int sp = sms / R0;
     if (sp > nkb) sp = nkb;
-    last_round_pays = 5.0 + 0.352 * nkb / sp + 8.6 < 0.8 * (5.0 + 0.352 * nkb);
+    last_round_pays = tc_slice_time(bn, cg) * nkb / sp + tc_trip_time(bn, cg, sp) + 3.0 < 0.8 * tc_slice_time(bn, cg) * nkb;
   }
   const bool cut = allow_cut && R0 > 0 && nkb >= 2 && R0 < sms &&
-                   (n_tiles >= sms ? (2 * R0 <= sms && U >= sms && n_tiles < 3 * sms && last_round_pays)
-                                   : ((tiles_m == 1 && 2 * R0 >= sms) || few));
+                   (n_tiles >= sms ? (2 * R0 <= sms && U >= sms && last_round_pays)
+                                   : cg == 1 && ((tiles_m == 1 && 2 * R0 >= sms) || few));
   if (!cut) { h.n_whole = n_tiles; h.R = 0; h.zmax = 0; h.G = n_tiles < sms ? n_tiles : sms; return h; }
   h.n_whole = n_tiles - R0; h.R = R0; h.G = U < sms ? (int)U : sms;
   if (few && n_tiles < sms && tiles_m > 1 && G_few < h.G) h.G = G_few;
@@ -1059,32 +1129,66 @@ static TcHostPlan tc_plan_stream(int M, int N, int K, int epi, bool allow_cut) {
   return h;
 }
 
-// n_whole, cut tiles, most pieces a tile, grid: what sx_gemm_tc will do with a workspace (out4[1] * out4[2] * 128 * 256 floats)
-extern "C" int sx_gemm_tc_plan(int M, int N, int K, int epi, int* out4) {
-  if (M <= 0 || N <= 0 || K <= 0) return SX_ERR_SIZE;
-  const TcHostPlan h = tc_plan_stream(M, N, K, epi, true);
+// A plan's time in us by what a tile's slices take (measured), for comparing the forms of the persistent kernel.
+static double tc_plan_time(const TcHostPlan& h, int K) {
+  const int nkb = (K + TC_BK - 1) / TC_BK;
+  const double slice = tc_slice_time(h.bn, h.cg);
+  double t = tc_base_time(h.bn, h.cg);
+  if (h.n_whole > 0) t += slice * nkb * ((h.n_whole + h.G - 1) / h.G);
+  if (h.R > 0) t += slice * nkb / (h.zmax > 0 ? h.zmax : 1) + (h.n_whole > 0 ? tc_trip_time(h.bn, h.cg, h.zmax) : tc_second_time(h.bn, h.G));
+  return t;
+}
+
+// form 0: the one that takes the least time by that estimate (of 48 products of 300 to 8,191 rows that was the fastest measured form,
+// or within 4% of it, in all but one: 24 tiles x 3 pieces of 300 x 2,048 -> 1,024, 10.8 against 10.0 us); 1 and 2: tiles 256 wide, of one block or of a pair; 3 and 4: 128 wide
+static TcHostPlan tc_plan_stream(int M, int N, int K, int epi, bool allow_cut, int form) {
+  if (form) return tc_plan_form(M, N, K, epi, allow_cut, form > 2 ? 128 : 256, 2 - (form & 1));
+  TcHostPlan best = tc_plan_form(M, N, K, epi, allow_cut, 256, 1);
+  for (int f = 2; f <= 4; ++f) {
+    const TcHostPlan h = tc_plan_form(M, N, K, epi, allow_cut, f > 2 ? 128 : 256, 2 - (f & 1));
+    if (h.n_whole >= 0 && (best.n_whole < 0 || tc_plan_time(h, K) < tc_plan_time(best, K))) best = h;
+  }
+  return best;
+}
+
+// n_whole, cut tiles, most pieces a tile, grid, floats of workspace: what sx_gemm_tc will do with a workspace
+extern "C" int sx_gemm_tc_plan(int M, int N, int K, int epi, int form, long long* out5) {
+  if (M <= 0 || N <= 0 || K <= 0 || form < 0 || form > 4) return SX_ERR_SIZE;
+  const TcHostPlan h = tc_plan_stream(M, N, K, epi, true, form);
   if (h.n_whole < 0) return SX_ERR_SIZE;
-  out4[0] = h.n_whole; out4[1] = h.R; out4[2] = h.zmax; out4[3] = h.G;
+  out5[0] = h.n_whole; out5[1] = h.R * h.cg; out5[2] = h.zmax; out5[3] = h.G * h.cg;
+  out5[4] = (long long)h.R * h.cg * h.zmax * TC_BM * h.bn;
   return 0;
 }
 
-template <int EPI, int BN>
+template <int EPI, int BN, int CG>
 static int tc_launch_persistent(const CUtensorMap& ma, const CUtensorMap& mw, void* out, int M, int N, int K,
-                                const TcHostPlan& h, float* ws, int* counts, const TcEp& ep, cudaStream_t stream, const TcQkv& qk = TcQkv()) {
+                                const TcHostPlan& h, float* ws, int* counts, const TcEp& ep, cudaStream_t stream, const TcQkv& qk) {
   int* status = tc_status_word();
   if (!status) return (int)cudaErrorMemoryAllocation;
   if (h.n_whole < 0 || h.G <= 0) return SX_ERR_SIZE;
-  const size_t smem = 1024 + TcShape<BN>::STAGES * TcShape<BN>::STAGE_BYTES + (2 * TcShape<BN>::STAGES + 4) * sizeof(uint64_t) + 32 + tc_vec_floats<EPI>() * sizeof(float);
-  auto kern = gemm_tc_persistent_kernel<EPI, BN>;
+  using Sh = TcShape<BN, CG>;
+  const size_t smem = 1024 + Sh::STAGES * Sh::STAGE_BYTES + (2 * Sh::STAGES + 4) * sizeof(uint64_t) + 32 + tc_vec_floats<EPI, BN>() * sizeof(float);
+  const dim3 threads(TcThreads<EPI, BN>::N);
+  auto kern = gemm_tc_persistent_kernel<EPI, BN, CG>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
+  const int rc = CG == 2 ? sx_launch_cluster(kern, dim3(2 * h.G), threads, smem, stream, 2, ma, mw, out, M, N, K, h.n_whole, h.zmax, h.sp, ws, counts, status, qk, ep)
+                         : sx_launch(kern, dim3(h.G), threads, smem, stream, ma, mw, out, M, N, K, h.n_whole, h.zmax, h.sp, ws, counts, status, qk, ep);
   // with whole tiles after them, the blocks of a cut tile add up inside the kernel; without, a second kernel does
-  int rc = sx_launch(kern, h.G, dim3(TC_PERSISTENT_THREADS), smem, stream, ma, mw, out, M, N, K, h.n_whole, h.zmax, h.sp, ws, counts, status, qk, ep);
   if (rc || h.R == 0 || h.sp > 0 || EPI == TC_EPI_QKV || EPI == TC_EPI_QKV_BIAS) return rc;
   const int tile_n = (EPI == TC_EPI_SILU_MUL) ? BN / 2 : BN;
   const long long total = (long long)h.R * TC_BM * (tile_n / 4);
   return sx_launch(tc_pieces_reduce_kernel<EPI, BN>, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, (const float*)ws, out,
                    M, N, h.n_whole, h.R, (K + TC_BK - 1) / TC_BK, h.G, h.zmax, 0, ep);
+}
+template <int EPI>
+static int tc_launch_form(const CUtensorMap& ma, const CUtensorMap& mw, void* out, int M, int N, int K, const TcHostPlan& h, float* ws,
+                          int* counts, const TcEp& ep, cudaStream_t stream, const TcQkv& qk = TcQkv()) {
+  if (h.bn == 256) return h.cg == 2 ? tc_launch_persistent<EPI, 256, 2>(ma, mw, out, M, N, K, h, ws, counts, ep, stream, qk)
+                                    : tc_launch_persistent<EPI, 256, 1>(ma, mw, out, M, N, K, h, ws, counts, ep, stream, qk);
+  return h.cg == 2 ? tc_launch_persistent<EPI, 128, 2>(ma, mw, out, M, N, K, h, ws, counts, ep, stream, qk)
+                   : tc_launch_persistent<EPI, 128, 1>(ma, mw, out, M, N, K, h, ws, counts, ep, stream, qk);
 }
 
 // sum of the split-K partial tiles ws[splits][M][N] in split order, then the epilogue
@@ -1148,10 +1252,10 @@ static int tc_split_product(const void* A, const void* W, void* out, int M, int 
 
 // A [M, K], W [N, K] bfloat16 row-major, 16-byte aligned, K % 8 == 0.
 // epi 0: out bf16 [M, N]; 1: out f32 [M, N]; 2: W = [gate; up] stacked, out bf16 [M, N/2].
-// splits == 1: the persistent kernel over 128 x 256 tiles, epilogue in the kernel.  With a workspace it cuts the
-//   tiles that would not fill a round of all SMs over K (sx_gemm_tc_plan says how): `workspace` holds
-//   ws_floats >= cut tiles * most pieces a tile * 128 * 256 floats, `counts` 2 * cut tiles ints that are zero
-//   (the kernel leaves them zero).  Without a workspace every tile is computed whole.
+// splits == 1: the persistent kernel, epilogue in the kernel, tiles of the form that tc_plan_stream takes (-1 to -4: of form 1 to
+//   4).  With a workspace it cuts the tiles that would not fill a round of all SMs over K (sx_gemm_tc_plan says how, and how many
+//   floats `workspace` has to hold), `counts`: 2 * cut tiles ints that are zero (the kernel leaves them zero).  Without a
+//   workspace every tile is computed whole.
 // splits > 1: 128 x 128 tiles, K split over `splits` blocks whose float32 partial tiles go to `workspace`
 //   [splits, M, N] and are added, in split order, by a second kernel that applies the epilogue.  Every split
 //   gets a non-empty range of K.
@@ -1165,40 +1269,38 @@ extern "C" int sx_gemm_tc(const void* A, const void* W, void* out, int M, int N,
   if (((uintptr_t)bias | (uintptr_t)h_io | (uintptr_t)gain | (uintptr_t)shift) & 15) return SX_ERR_ALIGN;
   TcEp ep;
   ep.act = g_sx_gate; ep.bias = bias; ep.cap = cap; ep.h = h_io; ep.alpha = alpha; ep.gain = gain; ep.shift = shift;
-  if (K <= 0 || (K & 7) || splits < 1) return SX_ERR_SIZE;
+  if (K <= 0 || (K & 7) || splits == 0 || splits < -4) return SX_ERR_SIZE;
   if (epi == TC_EPI_SILU_MUL && (N & 1)) return SX_ERR_SIZE;
   if (((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return SX_ERR_ALIGN;
   if (splits > 1) {
     if (!workspace || ws_floats < (unsigned long long)splits * M * N) return SX_ERR_SIZE;
     return tc_split_product(A, W, out, M, N, K, epi, splits, workspace, epi == TC_EPI_SILU_MUL ? N / 2 : N, ep, stream);
   }
+  const TcHostPlan h = tc_plan_stream(M, N, K, epi, workspace != nullptr && counts != nullptr, splits < 0 ? -splits : 0);
   CUtensorMap ma, mw;
   int rc = tc_make_map(&ma, A, M, K);
   if (rc) return rc;
-  rc = tc_make_map(&mw, W, N, K);
-  if (rc) return rc;
-  TcHostPlan h = tc_plan_stream(M, N, K, epi, workspace != nullptr && counts != nullptr);
-  if (h.R > 0 && (ws_floats < (unsigned long long)h.R * h.zmax * TC_BM * 256 || ((uintptr_t)workspace & 15))) return SX_ERR_SIZE;
+  if ((rc = tc_make_map_rows(&mw, W, N, K, h.bn / 2))) return rc;
+  if (h.R > 0 && (ws_floats < (unsigned long long)h.R * h.cg * h.zmax * TC_BM * h.bn || ((uintptr_t)workspace & 15))) return SX_ERR_SIZE;
   switch (epi) {
-    // (128-wide tiles were tried for shapes whose last wave is nearly empty: the MMA then waits on
-    //  shared-memory reads of A and the product got slower, 607 against 828 TFLOP/s)
-    case TC_EPI_BF16: return tc_launch_persistent<TC_EPI_BF16, 256>(ma, mw, out, M, N, K, h, workspace, counts, ep, stream);
-    case TC_EPI_F32: return tc_launch_persistent<TC_EPI_F32, 256>(ma, mw, out, M, N, K, h, workspace, counts, ep, stream);
-    case TC_EPI_SILU_MUL: return tc_launch_persistent<TC_EPI_SILU_MUL, 256>(ma, mw, out, M, N, K, h, workspace, counts, ep, stream);
-    case TC_EPI_RESID_TANH: return tc_launch_persistent<TC_EPI_RESID_TANH, 256>(ma, mw, out, M, N, K, h, workspace, counts, ep, stream);
+    case TC_EPI_BF16: return tc_launch_form<TC_EPI_BF16>(ma, mw, out, M, N, K, h, workspace, counts, ep, stream);
+    case TC_EPI_F32: return tc_launch_form<TC_EPI_F32>(ma, mw, out, M, N, K, h, workspace, counts, ep, stream);
+    case TC_EPI_SILU_MUL: return tc_launch_form<TC_EPI_SILU_MUL>(ma, mw, out, M, N, K, h, workspace, counts, ep, stream);
+    case TC_EPI_RESID_TANH: return tc_launch_form<TC_EPI_RESID_TANH>(ma, mw, out, M, N, K, h, workspace, counts, ep, stream);
     default: return SX_ERR_DTYPE;
   }
 }
 
 // The fused q/k/v projection of a prompt step with its head preparation as the epilogue (see TcQkv): A [M, K], W [N, K] with
 // N = (nh + 2 nkv) * 128 (or nh * 128: query heads alone, of a layer that reads another layer's cache) a multiple of 256;
-// bias [N] (null: none); q_out [M, nh * 128]; k_pages / v_pages [n_pages, nkv, 64, 128] (null: nothing is
+// form: as splits of sx_gemm_tc (0: the rule's); bias [N] (null: none); q_out [M, nh * 128]; k_pages / v_pages [n_pages, nkv, 64, 128] (null: nothing is
 // written to the cache); wq / wk [128] (null: no norm); cs / sn [M, 64] (null: no rotation).  All tiles are computed whole.
 extern "C" int sx_gemm_tc_qkv(const void* A, const void* W, const float* bias, int M, int N, int K, void* q_out, void* k_pages, void* v_pages,
                               const float* wq, const float* wk, const float* cs, const float* sn, const int* positions,
                               const int* seq_of_token, const int* block_table, int maxp, int nh, int nkv, int n_pages,
-                              float eps, cudaStream_t stream) {
+                              float eps, int form, cudaStream_t stream) {
   if (M <= 0) return 0;
+  if (form < 0 || form > 4) return SX_ERR_SIZE;
   if (K <= 0 || (K & 7) || nh <= 0 || nkv <= 0 || (N != (nh + 2 * nkv) * 128 && N != nh * 128) || (N & 255) || !q_out || (!cs) != (!sn)) return SX_ERR_SIZE;
   if (((uintptr_t)A & 15) || ((uintptr_t)W & 15) || ((uintptr_t)q_out & 15) || ((uintptr_t)k_pages & 15) || ((uintptr_t)v_pages & 15) ||
       ((uintptr_t)wq & 15) || ((uintptr_t)wk & 15) || ((uintptr_t)cs & 15) || ((uintptr_t)sn & 15) || ((uintptr_t)bias & 15))
@@ -1206,14 +1308,14 @@ extern "C" int sx_gemm_tc_qkv(const void* A, const void* W, const float* bias, i
   CUtensorMap ma, mw;
   int rc = tc_make_map(&ma, A, M, K);
   if (rc) return rc;
-  if ((rc = tc_make_map(&mw, W, N, K))) return rc;
-  const TcHostPlan h = tc_plan_stream(M, N, K, TC_EPI_BF16, false);
+  const TcHostPlan h = tc_plan_stream(M, N, K, TC_EPI_BF16, false, form);
+  if ((rc = tc_make_map_rows(&mw, W, N, K, h.bn / 2))) return rc;
   TcQkv qk;
   qk.q_out = (bf16*)q_out; qk.k_pages = (bf16*)k_pages; qk.v_pages = (bf16*)v_pages; qk.bias = bias; qk.wq = wq; qk.wk = wk; qk.cs = cs; qk.sn = sn;
   qk.positions = positions; qk.seq_of_token = seq_of_token; qk.block_table = block_table;
   qk.maxp = maxp; qk.nh = nh; qk.nkv = nkv; qk.n_pages = n_pages; qk.eps = eps;
-  if (bias) return tc_launch_persistent<TC_EPI_QKV_BIAS, 256>(ma, mw, nullptr, M, N, K, h, nullptr, nullptr, TcEp(), stream, qk);
-  return tc_launch_persistent<TC_EPI_QKV, 256>(ma, mw, nullptr, M, N, K, h, nullptr, nullptr, TcEp(), stream, qk);
+  if (bias) return tc_launch_form<TC_EPI_QKV_BIAS>(ma, mw, nullptr, M, N, K, h, nullptr, nullptr, TcEp(), stream, qk);
+  return tc_launch_form<TC_EPI_QKV>(ma, mw, nullptr, M, N, K, h, nullptr, nullptr, TcEp(), stream, qk);
 }
 
 // 0, or which bounded wait ran out (1 producer, 2 and 4 MMA issuer, 3 epilogue, 5 the blocks of a cut tile waiting for one another)

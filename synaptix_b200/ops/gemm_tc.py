@@ -72,31 +72,41 @@ def _apply_cut_few() -> None:
         _cut_few_applied = OPTIONS.gemm_cut_few
 
 
-def plan_stream(M: int, N: int, K: int, epilogue: Optional[str] = None):
-    """``(whole tiles, cut tiles, most pieces a cut tile has, grid)`` of the persistent kernel on the current
-    device.  Tiles that would not fill a round of all SMs (a last round at most half full: 2,048 x 2,560 has
-    160 tiles for 148 SMs; or all tiles of a step with at most 128 rows) are cut over K: their 64-wide slices
+# tiles of the persistent kernel: 256 or 128 wide, of one block (128 rows) or of a pair of blocks (256 rows)
+FORMS = {None: 0, "one": 1, "pair": 2, "one_128": 3, "pair_128": 4}
+
+
+def _plan(M: int, N: int, K: int, epilogue: Optional[str], form: Optional[str]):
+    _apply_cut_few()
+    out = (ctypes.c_longlong * 5)()
+    check(fn("gemm_tc", "sx_gemm_tc_plan")(c_int(M), c_int(N), c_int(K), c_int(_EPI[epilogue]), c_int(FORMS[form]), out),
+          "gemm_tc_plan", launches=0)
+    return tuple(int(v) for v in out)
+
+
+def plan_stream(M: int, N: int, K: int, epilogue: Optional[str] = None, form: Optional[str] = "one"):
+    """``(whole tiles, cut tiles, most pieces a cut tile has, grid)`` of a form of the persistent kernel on the current
+    device (``None``: of the form it takes for the shape).  Tiles that would not fill a round of all SMs (a last
+    round at most half full: 2,048 x 2,560 has 160 tiles for 148 SMs; or all tiles of a step with at most 128 rows) are cut over K: their 64-wide slices
     of K form one sequence that is dealt out to the blocks in equal contiguous shares, the blocks of a tile
     leave float32 partial tiles in a workspace and add them up together, in a fixed order.  Several rows of tiles
     that are fewer than the SMs (a few hundred rows) are cut when an estimate from measured times says that pays
     (option ``gemm_cut_few``)."""
-    _apply_cut_few()
-    out = (ctypes.c_int * 4)()
-    check(fn("gemm_tc", "sx_gemm_tc_plan")(c_int(M), c_int(N), c_int(K), c_int(_EPI[epilogue]), out), "gemm_tc_plan",
-          launches=0)
-    return tuple(int(v) for v in out)
+    return _plan(M, N, K, epilogue, form)[:4]
 
 
 def gemm_tc(x: torch.Tensor, w: torch.Tensor, *, epilogue: Optional[str] = None,
             out: Optional[torch.Tensor] = None, splits: Optional[int] = None,
-            cut: Optional[bool] = None, bias: Optional[torch.Tensor] = None, cap: float = 0.0) -> torch.Tensor:
+            cut: Optional[bool] = None, bias: Optional[torch.Tensor] = None, cap: float = 0.0,
+            form: Optional[str] = None) -> torch.Tensor:
     """``x[M, K] @ w[N, K].T`` on the tcgen05 tensor cores, 32-bit accumulation in tensor memory.
 
     Default: the persistent kernel, which cuts tiles over K where whole tiles would leave SMs idle (see
     ``plan_stream``; ``cut=False`` turns that off); for a handful of tiles the two-kernel form instead
     (``plan_splits``).  ``splits > 1`` asks for that form: K split over ``splits`` blocks per 128 x 128 tile,
     float32 partial tiles in a workspace of ``splits * M * N`` floats, added in a fixed order by a second kernel;
-    ``splits=1`` for whole tiles (or cut ones) in any case.
+    ``splits=1`` for whole tiles (or cut ones) in any case.  ``form`` asks for one of ``FORMS``; by default an estimate from
+    measured times chooses.
 
     ``epilogue``: ``None`` -> bfloat16 ``[M, N]``; ``"f32"`` -> float32 ``[M, N]``; ``"silu_mul"`` ->
     ``w`` is ``[gate; up]`` stacked and the result is bfloat16 ``[M, N/2]``.  Needs ``K % 8 == 0``.  ``bias`` (float32
@@ -105,20 +115,21 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, *, epilogue: Optional[str] = None,
     if epilogue not in (None, "f32", "silu_mul"):
         raise KernelError(f"gemm_tc: unknown epilogue {epilogue!r}")
     check_bias(bias, w.shape[0])
-    return _gemm_tc(x, w, epilogue, out, splits, cut, bias, cap)
+    return _gemm_tc(x, w, epilogue, out, splits, cut, bias, cap, form=form)
 
 
 def gemm_tc_resid_tanh(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], h: torch.Tensor, alpha: float,
                        gain: torch.Tensor, shift: torch.Tensor, *, splits: Optional[int] = None,
-                       cut: Optional[bool] = None) -> torch.Tensor:
+                       cut: Optional[bool] = None, form: Optional[str] = None) -> torch.Tensor:
     """``h += x @ w.T + bias`` in place (``h`` float32 ``[M, N]``); returns bfloat16 ``tanh(alpha h) * gain + shift``, in the
     product's epilogue."""
     require_cuda(h, gain, shift)
     check_resid_tanh(x, w, bias, h, gain, shift)
-    return _gemm_tc(x, w, "resid_tanh", None, splits, cut, bias, 0.0, h, alpha, gain, shift)
+    return _gemm_tc(x, w, "resid_tanh", None, splits, cut, bias, 0.0, h, alpha, gain, shift, form)
 
 
-def _gemm_tc(x, w, epilogue, out, splits, cut, bias, cap, h=None, alpha=0.0, gain=None, shift=None) -> torch.Tensor:
+def _gemm_tc(x, w, epilogue, out, splits, cut, bias, cap, h=None, alpha=0.0, gain=None, shift=None,
+             form=None) -> torch.Tensor:
     if not (good(x) and good(w)) or out is not None or bias is not None:
         require_cuda(x, w, out, bias)
     M, K = x.shape
@@ -137,21 +148,21 @@ def _gemm_tc(x, w, epilogue, out, splits, cut, bias, cap, h=None, alpha=0.0, gai
         cut = OPTIONS.gemm_cut
     _apply_cut_few()
     # what the library will do with this shape, remembered: a prompt step asks a hundred times for a handful of shapes
-    key = (M, N, K, epilogue, splits, bool(cut), OPTIONS.gemm_cut_few)
+    key = (M, N, K, epilogue, splits, bool(cut), OPTIONS.gemm_cut_few, form)
     plan = _PLANS.get(key)
     if plan is None:
-        n_cut = zmax = 0
+        n_cut = floats = 0
         if splits is None and cut is not False:
-            _, n_cut, zmax, _ = plan_stream(M, N, K, epilogue)
+            _, n_cut, _, _, floats = _plan(M, N, K, epilogue, form)
         sp = splits
         if sp is None:
-            sp = 1 if n_cut else plan_splits(M, N, K, sm_count(x.device))
+            sp = 1 if n_cut or form else plan_splits(M, N, K, sm_count(x.device))
         sp = max(1, min(int(sp), (K + 63) // 64))
-        plan = _PLANS[key] = (sp, n_cut, sp * M * N if sp > 1 else n_cut * zmax * 128 * 256)
+        plan = _PLANS[key] = (-FORMS[form] if sp == 1 and form else sp, n_cut, sp * M * N if sp > 1 else floats)
     splits, n_cut, ws_floats = plan
     if ws_floats:
         ws = _workspace(ws_floats, x.device)
-        if splits == 1:
+        if splits <= 1:
             counts = _counts(x.device)
     launch(launcher("gemm_tc", "sx_gemm_tc"), (
         x.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, _EPI[epilogue], splits, None if ws is None else ws.data_ptr(),
@@ -175,7 +186,7 @@ def gemm_tc_qkv(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, k_pages: 
                 v_pages: Optional[torch.Tensor], wq: Optional[torch.Tensor], wk: Optional[torch.Tensor],
                 cos: Optional[torch.Tensor], sin: Optional[torch.Tensor], eps: float, positions: torch.Tensor,
                 seq_of_token: torch.Tensor, block_table: torch.Tensor, nh: int, nkv: int,
-                bias: Optional[torch.Tensor] = None) -> None:
+                bias: Optional[torch.Tensor] = None, form: Optional[str] = None) -> None:
     """``x @ w.T`` for the stacked q/k/v matrix with heads of 128, and what ``qkv_prepare`` does to the result, in
     the product's epilogue: per-head RMSNorm of q and k (gains ``wq`` / ``wk``, skipped when ``None``), rotate-half
     rotation by the angles whose cosines and sines are ``cos`` / ``sin [M, 64]`` (skipped when ``None``), q to
@@ -209,7 +220,7 @@ def gemm_tc_qkv(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, k_pages: 
         None if k_pages is None else k_pages.data_ptr(), None if v_pages is None else v_pages.data_ptr(),
         None if wq is None else wq.data_ptr(), None if wk is None else wk.data_ptr(), None if cos is None else cos.data_ptr(),
         None if sin is None else sin.data_ptr(), positions.data_ptr(), seq_of_token.data_ptr(), block_table.data_ptr(),
-        block_table.shape[1], nh, nkv, n_pages, eps, raw_stream()), "gemm_tc_qkv", 1, (q_out,))
+        block_table.shape[1], nh, nkv, n_pages, eps, FORMS[form], raw_stream()), "gemm_tc_qkv", 1, (q_out,))
 
 
 def gemm_tc_status(reset: bool = False) -> int:
