@@ -474,6 +474,284 @@ __global__ void __launch_bounds__(FT_THREADS, 1) attn_tc_prefill_kernel(
 }
 
 // ---------------------------------------------------------------------------------------
+// Two query heads of one key/value head at a time: more tiles than SMs.  In the kernel above all softmax warps work on the same
+// scores, so that the special-function unit (16 exponentials a clock: 1,024 clocks for 128 x 128 scores, as long as the two MMAs)
+// idles while they load, compare and store, and the tensor cores idle while they exponentiate.  Here warps 0-7 own the 128 query
+// rows of one head and warps 8-15 those of the next, which reads the same keys and values; while one head's scores go through the
+// softmax the other's products run.  S, P (over S) and O of both heads fill the tensor memory, so Q stays in shared memory (and
+// Q K^T reads 8 KB of it an instruction, all its bandwidth).  K and V tiles pass through one ring (K(j) is its tile 2 j, V(j) its
+// tile 2 j + 1) and serve both heads.  A step of 128 keys takes 2.3 us for both heads; what bounds it is a head's chain, softmax,
+// P V and the next Q K^T (P lies over S, so it cannot run ahead).  With a row a thread (eight softmax warps) a prompt of 8,191
+// tokens took 555 instead of 564 us, eight of 333 tokens 39.2 instead of 36.3.
+// ---------------------------------------------------------------------------------------
+#define FP_MMA_WARP 16
+#define FP_TMA_WARP 17
+#define FP_THREADS 576
+#define FP_TILES 4                      // K and V tiles in flight
+#define FP_SMEM_TILES ((2 + FP_TILES) * FT_TILE)
+enum { FP_B_QFULL = 0, FP_B_FULL = 1, FP_B_EMPTY = FP_B_FULL + FP_TILES, FP_B_SFULL = FP_B_EMPTY + FP_TILES, FP_B_PREADY = FP_B_SFULL + 2,
+       FP_B_ODONE = FP_B_PREADY + 2, FP_B_XCH = FP_B_ODONE + 2, FP_NBARS = FP_B_XCH + 24 };
+
+__global__ void __launch_bounds__(FP_THREADS, 1) attn_tc_prefill_pair_kernel(
+    const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+    const __grid_constant__ CUtensorMap map_v, bf16* __restrict__ out, const int* __restrict__ tile_seq,
+    const int* __restrict__ tile_q0, const int* __restrict__ cu_seqlens, const int* __restrict__ seq_past,
+    const int* __restrict__ seq_lens, const int* __restrict__ block_table, int maxp, int nh, int nkv,
+    float scale_log2, int window, const float* __restrict__ sinks, int* __restrict__ status) {
+  extern __shared__ unsigned char ft_smem_raw[];
+  unsigned char* q_s = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ft_smem_raw) + 1023) & ~(uintptr_t)1023);   // [2 heads]
+  unsigned char* kv_s = q_s + 2 * FT_TILE;                       // [FP_TILES]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(q_s + FP_SMEM_TILES);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + FP_NBARS);
+  float* xch_all = reinterpret_cast<float*>(tmem_slot + 4);      // [2 heads][6][128]: the halves' maxima (two buffers), their sums
+  const uint32_t bar0 = ft_smem(bars);
+  auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tile = gridDim.y - 1 - blockIdx.y, h0 = 2 * blockIdx.x;      // (long tiles first, as above)
+  const int seq = tile_seq[tile], q0 = tile_q0[tile];
+  const int t_begin = cu_seqlens[seq], n_new = cu_seqlens[seq + 1] - t_begin;
+  const int past = seq_past[seq], len = seq_lens[seq];
+  const int rows = min(FT_BM, n_new - q0);
+  const int first_pos = past + q0, last_pos = past + q0 + rows - 1;
+  const int lo_key = window > 0 ? max(0, first_pos - window + 1) : 0;
+  const int kb0 = (lo_key / FT_BN) * FT_BN;
+  const int nb = (last_pos + 1 - kb0 + FT_BN - 1) / FT_BN;       // >= 1
+
+  if (threadIdx.x == 0) {
+    ft_mbar_init(bar(FP_B_QFULL), 1);
+    for (int s = 0; s < FP_TILES; ++s) {
+      ft_mbar_init(bar(FP_B_FULL + s), 1);
+      ft_mbar_init(bar(FP_B_EMPTY + s), 1);
+    }
+    for (int x = 0; x < 2; ++x) {
+      ft_mbar_init(bar(FP_B_SFULL + x), 1);
+      ft_mbar_init(bar(FP_B_PREADY + x), 8);       // one arrival per softmax warp of the head
+      ft_mbar_init(bar(FP_B_ODONE + x), 1);
+    }
+    for (int s = 0; s < 24; ++s) ft_mbar_init(bar(FP_B_XCH + s), 2);      // the exchanges between warps w and w + 4: [2 heads][3][4]
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == FP_MMA_WARP) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(ft_smem(tmem_slot)), "r"((uint32_t)FT_TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  pdl_trigger();
+
+  if (warp == FP_TMA_WARP) {
+    if (lane == 0) {
+      const int kvh = h0 / (nh / nkv);
+      const int* bt = block_table + (size_t)seq * maxp;
+      ft_mbar_expect_tx(bar(FP_B_QFULL), 2 * FT_TILE);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) ft_tma_2d(ft_smem(q_s + c * FT_CHUNK), &map_q, h0 * FT_HD + c * 64, t_begin + q0, bar(FP_B_QFULL));
+      for (int t = 0; t < 2 * nb; ++t) {
+        const int s = t % FP_TILES, u = t / FP_TILES;
+        if (!ft_mbar_wait(bar(FP_B_EMPTY + s), (u & 1) ^ 1)) { sx_set_status(status, 1); break; }
+        ft_mbar_expect_tx(bar(FP_B_FULL + s), FT_TILE);
+        const uint32_t dst = ft_smem(kv_s + s * FT_TILE);
+        const int key0 = kb0 + (t >> 1) * FT_BN;
+        const CUtensorMap* map = (t & 1) ? &map_v : &map_k;
+#pragma unroll
+        for (int hp = 0; hp < 2; ++hp) {
+          const int pi = (key0 >> 6) + hp;
+          // a page beyond the sequence's keys is never looked up: page 0 stands in, its keys are masked
+          const int page = (pi * 64 < len && pi < maxp) ? bt[pi] : 0;
+#pragma unroll
+          for (int c = 0; c < 2; ++c) ft_tma_4d(dst + c * FT_CHUNK + hp * 8192, map, c * 64, 0, kvh, page, bar(FP_B_FULL + s));
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == FP_MMA_WARP) {
+    constexpr uint32_t idesc_qk = ft_idesc(FT_BM, FT_BN, false);
+    constexpr uint32_t idesc_pv = ft_idesc(FT_BM, FT_HD, true);
+    const bool leader = ft_elect_one();
+    const uint32_t q_addr = ft_smem(q_s), kv_addr = ft_smem(kv_s);
+    auto tile_ready = [&](int t) {
+      const bool ok = __all_sync(0xffffffffu, ft_mbar_wait(bar(FP_B_FULL + t % FP_TILES), (t / FP_TILES) & 1));
+      if (!ok && leader) sx_set_status(status, 3);
+      return ok;
+    };
+    auto issue_qk = [&](int j, int x) -> bool {
+      if (!tile_ready(2 * j)) return false;
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const int s = (2 * j) % FP_TILES;
+      const uint64_t dq = ft_desc_kmajor(q_addr + x * FT_TILE), dk = ft_desc_kmajor(kv_addr + s * FT_TILE);
+      if (leader) {
+#pragma unroll
+        for (int k = 0; k < FT_HD / 16; ++k) {
+          const uint64_t at = ((k >> 2) * FT_CHUNK + (k & 3) * 32) >> 4;
+          ft_mma(tmem_base + x * 128, dq + at, dk + at, idesc_qk, k != 0);
+        }
+        ft_commit(bar(FP_B_SFULL + x));
+        if (x == 1) ft_commit(bar(FP_B_EMPTY + s));          // both heads have read K(j)
+      }
+      __syncwarp();
+      return true;
+    };
+    bool ok = __all_sync(0xffffffffu, ft_mbar_wait(bar(FP_B_QFULL), 0));
+    if (!ok && leader) sx_set_status(status, 2);
+    if (ok) ok = issue_qk(0, 0) && issue_qk(0, 1);
+    for (int j = 0; j < nb && ok; ++j) {
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        if (!ok) break;
+        ok = __all_sync(0xffffffffu, ft_mbar_wait(bar(FP_B_PREADY + x), j & 1));
+        if (!ok) {
+          if (leader) sx_set_status(status, 5);
+          break;
+        }
+        if (!(ok = tile_ready(2 * j + 1))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        const int s = (2 * j + 1) % FP_TILES;
+        const uint64_t dv = ft_desc_mnmajor(kv_addr + s * FT_TILE);
+        const uint32_t pa = tmem_base + x * 128, o_acc = tmem_base + 256 + x * 128, acc = j != 0;
+        if (leader) {
+#pragma unroll
+          for (int k = 0; k < FT_BN / 16; ++k) ft_mma_ta(o_acc, pa + k * 8, dv + k * (2048 >> 4), idesc_pv, acc | (k != 0));
+          if (x == 1) ft_commit(bar(FP_B_EMPTY + s));
+          if (j + 1 == nb) ft_commit(bar(FP_B_ODONE + x));
+        }
+        __syncwarp();
+        // (MMAs run in the order they are issued: the next scores do not overtake P V, whose P they overwrite)
+        if (j + 1 < nb) ok = issue_qk(j + 1, x);
+      }
+    }
+    __syncwarp();
+  } else {
+    // ---------------- softmax: threads r and r + 128 of a head's eight warps own query row r, 64 columns each ----------------
+    const int x = warp >> 3, hf = (warp >> 2) & 1, r = threadIdx.x & 127, h = h0 + x;
+    const uint32_t t_row = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t t_s = t_row + x * 128, t_o = t_row + 256 + x * 128 + hf * FT_HALF;
+    float* xch = xch_all + x * 6 * FT_BM;
+    const int xb = FP_B_XCH + x * 12 + (warp & 3);
+    const int pos = r < rows ? past + q0 + r : -1;
+    float m = -INFINITY, l = 0.f;                                 // l: this thread's columns only
+    if (sinks != nullptr) {                // a sink: a term exp(sink) of the denominator without a key, counted by one half
+      m = sinks[h] * 1.4426950408889634f / scale_log2;
+      l = hf == 0 ? 1.f : 0.f;
+    }
+    bool ok = true;
+    for (int j = 0; j < nb && ok; ++j) {
+      const int s = j & 1, u = j >> 1;
+      // (the scores' barrier follows the P V of the block before, too: O may be touched)
+      if (!ft_mbar_wait(bar(FP_B_SFULL + x), j & 1)) { sx_set_status(status, 6); ok = false; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      float sc[FT_HALF];
+#pragma unroll
+      for (int c = 0; c < FT_HALF / 32; ++c) ft_ld32(t_s + hf * FT_HALF + c * 32, sc + c * 32);
+      asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+      const int key0 = kb0 + j * FT_BN;
+      const bool need_mask = key0 + FT_BN - 1 > first_pos || (window > 0 && key0 <= last_pos - window);
+      if (need_mask) {                     // visible: columns lo < i <= hi of this thread's
+        const int hi = pos - key0 - hf * FT_HALF, lo = window > 0 ? hi - window : -1;
+#pragma unroll
+        for (int i = 0; i < FT_HALF; ++i) sc[i] = (i <= hi && i > lo) ? sc[i] : -INFINITY;
+      }
+      float mxs[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) mxs[i] = sc[i];
+#pragma unroll
+      for (int i = 8; i < FT_HALF; ++i) mxs[i & 7] = fmaxf(mxs[i & 7], sc[i]);
+      const float hmax = fmaxf(fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])), fmaxf(fmaxf(mxs[4], mxs[5]), fmaxf(mxs[6], mxs[7])));
+      xch[(s * 2 + hf) * FT_BM + r] = hmax;
+      __syncwarp();
+      if (lane == 0) ft_mbar_arrive(bar(xb + s * 4));
+      if (!ft_mbar_wait(bar(xb + s * 4), u & 1)) { sx_set_status(status, 9); ok = false; break; }
+      const float bmax = fmaxf(hmax, xch[(s * 2 + (hf ^ 1)) * FT_BM + r]);
+      // the reference point moves lazily, as above
+      float corr = 1.f;
+      if (bmax != -INFINITY && (m == -INFINITY || (bmax - m) * scale_log2 > FT_LAZY)) {
+        corr = (m == -INFINITY) ? 0.f : ft_ex2((m - bmax) * scale_log2);
+        m = bmax;
+      }
+      const float ms = (m == -INFINITY) ? 0.f : m * scale_log2;
+      float sums[4] = {0.f, 0.f, 0.f, 0.f};
+      uint32_t pk[FT_HALF / 2];
+#pragma unroll
+      for (int i = 0; i < FT_HALF; i += 2) {
+        const float p0 = ft_ex2(fmaf(sc[i], scale_log2, -ms));
+        const float p1 = ft_ex2(fmaf(sc[i + 1], scale_log2, -ms));
+        sums[(i >> 1) & 3] += p0 + p1;
+        pk[i >> 1] = ft_pack(p0, p1);
+      }
+      // P over the scores (both threads of the row have read theirs: the exchange of the maxima came after the loads)
+      ft_st32u(t_s + hf * 32, pk);
+      l = l * corr + ((sums[0] + sums[1]) + (sums[2] + sums[3]));
+      // rows of V at or beyond the sequence's length (threads r stand for key r of the block, each for
+      // half of the head's values; both heads zero the same bytes)
+      if (key0 + FT_BN > len) {
+        const int vs = (2 * j + 1) % FP_TILES;
+        if (!ft_mbar_wait(bar(FP_B_FULL + vs), ((2 * j + 1) / FP_TILES) & 1)) { sx_set_status(status, 7); ok = false; break; }
+        if (key0 + r >= len) {
+#pragma unroll
+          for (int p = 0; p < 8; ++p)
+            *reinterpret_cast<uint4*>(kv_s + vs * FT_TILE + hf * FT_CHUNK + r * 128 + p * 16) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");    // the zeroed rows, for the tensor cores
+      }
+      // O *= corr, when some row of this warp moved its reference point
+      if (j > 0 && __any_sync(0xffffffffu, corr != 1.f)) {
+#pragma unroll 1
+        for (int c = 0; c < FT_HALF / 32; ++c) {
+          float o[32];
+          ft_ld32(t_o + c * 32, o);
+          asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] *= corr;
+          ft_st32(t_o + c * 32, o);
+        }
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+      __syncwarp();
+      if (lane == 0) ft_mbar_arrive(bar(FP_B_PREADY + x));
+    }
+    xch[(4 + hf) * FT_BM + r] = l;         // the row's sum: both halves
+    __syncwarp();
+    if (lane == 0) ft_mbar_arrive(bar(xb + 8));
+    if (ok && !ft_mbar_wait(bar(xb + 8), 0)) { sx_set_status(status, 9); ok = false; }
+    l += xch[(4 + (hf ^ 1)) * FT_BM + r];
+    if (ok && !ft_mbar_wait(bar(FP_B_ODONE + x), 0)) { sx_set_status(status, 8); ok = false; }
+    if (ok) {
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      bf16* dst = out + ((size_t)(t_begin + q0 + r) * nh + h) * FT_HD + hf * FT_HALF;
+#pragma unroll 1
+      for (int c = 0; c < FT_HALF / 32; ++c) {
+        float o[32];
+        ft_ld32(t_o + c * 32, o);
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+        if (r < rows) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            uint4 v;
+            v.x = ft_pack(o[8 * i] * inv, o[8 * i + 1] * inv);
+            v.y = ft_pack(o[8 * i + 2] * inv, o[8 * i + 3] * inv);
+            v.z = ft_pack(o[8 * i + 4] * inv, o[8 * i + 5] * inv);
+            v.w = ft_pack(o[8 * i + 6] * inv, o[8 * i + 7] * inv);
+            reinterpret_cast<uint4*>(dst + c * 32)[i] = v;
+          }
+        }
+      }
+    }
+  }
+
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  if (warp == FP_MMA_WARP) {
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"((uint32_t)FT_TMEM_COLS) : "memory");
+  }
+}
+
+// ---------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------
 typedef CUresult (*ft_encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -519,6 +797,16 @@ static int ft_map_pages(CUtensorMap* map, const void* pages, long long n_pages, 
   return r == CUDA_SUCCESS ? 0 : 20000 + (int)r;
 }
 
+static int ft_sm_count() {
+  static int n[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  if (!n[dev]) {
+    if (cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n[dev] <= 0) n[dev] = 148;
+  }
+  return n[dev];
+}
+
 static int* ft_status_word() {
   static int* p = nullptr;
   if (!p) p = sx_status_word_alloc();
@@ -542,6 +830,17 @@ extern "C" int sx_attn_prefill_tc(const void* q, const void* k_pages, const void
   if (rc) return rc;
   if ((rc = ft_map_pages(&mk, k_pages, n_pages, nkv))) return rc;
   if ((rc = ft_map_pages(&mv, v_pages, n_pages, nkv))) return rc;
+  // Two heads a block where their blocks fill the SMs well beyond once.  Us, one head a block and two: 8,191 new tokens, 32 heads
+  // 597 and 564; 2,048 tokens 57.6 and 51.6; eight prompts of 333 tokens 45.5 and 36.3; 1,500 tokens (192 pairs) 37.9 and 36.4;
+  // but 1,024 tokens (128 pairs) 21.0 and 26.4: fewer blocks than SMs, and a pair's step takes 2.3 us for two tiles, not 1.27.
+  if ((nh / nkv) % 2 == 0 && 4LL * (nh / 2) * n_tiles >= 5LL * ft_sm_count()) {
+    const size_t smem = 1024 + FP_SMEM_TILES + FP_NBARS * sizeof(uint64_t) + 16 + 12 * FT_BM * sizeof(float);
+    auto kern = attn_tc_prefill_pair_kernel;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    return sx_launch(kern, dim3(nh / 2, n_tiles), dim3(FP_THREADS), smem, stream, mq, mk, mv, (bf16*)out, tile_seq, tile_q0,
+                     cu_seqlens, seq_past, seq_lens, block_table, maxp, nh, nkv, scale * 1.4426950408889634f, window, sinks, status);
+  }
   const size_t smem = 1024 + FT_SMEM_TILES + FT_NBARS * sizeof(uint64_t) + 16 + 6 * FT_BM * sizeof(float);
   auto kern = attn_tc_prefill_kernel;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
