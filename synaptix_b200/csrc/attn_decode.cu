@@ -227,6 +227,15 @@ __device__ __forceinline__ void ad_attend_page(const uint32_t (&qf)[HD / 16][4],
   }
 }
 
+#define AD_MAX_CLUSTER 16
+__device__ __forceinline__ float4 ad_cluster_load4(const float* local, uint32_t rank) {
+  uint32_t r;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(ad_smem(local)), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(r) : "memory");
+  return v;
+}
+
 template <int HD, bool PREP, bool CLUSTER>
 __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_tma_kernel(
     const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -459,51 +468,90 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_tma_kernel(
     wml[(warp * 16 + g + 8) * 2 + 1] = l[1];
   }
   asm volatile("bar.sync 1, %0;\n" ::"n"(AD_COMPUTE_WARPS * 32) : "memory");
-  // this block's result: O [G][HD], then (M, L) [G][2], behind the warps' results in the ring
+  // this block's result: O [G][HD], then (M, L) [G][2], behind the warps' results in the ring; four values a thread
   float* res = wml + AD_COMPUTE_WARPS * 16 * 2;
   float* res_ml = res + 16 * HD;
-  for (int idx = threadIdx.x; idx < G * HD; idx += AD_COMPUTE_WARPS * 32) {
-    const int r = idx / HD, d = idx % HD;
+  const bool out8 = ((uintptr_t)out & 7) == 0;
+  auto put = [&](int r, int d, float4 O, float Lsum) {
+    const bool some = Lsum > 0.f;
+    const float v[4] = {some ? O.x / Lsum : 0.f, some ? O.y / Lsum : 0.f, some ? O.z / Lsum : 0.f, some ? O.w / Lsum : 0.f};
+    bf16* dst = out + ((size_t)seq * nh + kvh * G + r) * HD + d;
+    if (out8) {
+      uint2 pk;
+      pk.x = ad_pack(v[0], v[1]); pk.y = ad_pack(v[2], v[3]);
+      *reinterpret_cast<uint2*>(dst) = pk;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dst[i] = __float2bfloat16_rn(v[i]);
+    }
+  };
+  for (int idx = threadIdx.x; idx < G * HD / 4; idx += AD_COMPUTE_WARPS * 32) {
+    const int r = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
     float M = -INFINITY;
 #pragma unroll
     for (int w = 0; w < AD_COMPUTE_WARPS; ++w) M = fmaxf(M, wml[(w * 16 + r) * 2]);
-    float Lsum = 0.f, O = 0.f;
+    float Lsum = 0.f;
+    float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int w = 0; w < AD_COMPUTE_WARPS; ++w) {
       const float mw = wml[(w * 16 + r) * 2];
       const float f = (mw == -INFINITY) ? 0.f : exp2f(mw - M);
       Lsum += wml[(w * 16 + r) * 2 + 1] * f;
-      O += wo[(w * 16 + r) * HD + d] * f;
+      const float4 x = *reinterpret_cast<const float4*>(wo + (w * 16 + r) * HD + d);
+      O.x += x.x * f; O.y += x.y * f; O.z += x.z * f; O.w += x.w * f;
     }
-    const int head = kvh * G + r;
     if (n_splits == 1) {
-      out[((size_t)seq * nh + head) * HD + d] = __float2bfloat16_rn(Lsum > 0.f ? O / Lsum : 0.f);
+      put(r, d, O, Lsum);
     } else if (CLUSTER) {
-      res[r * HD + d] = O;
+      *reinterpret_cast<float4*>(res + r * HD + d) = O;
       if (d == 0) { res_ml[r * 2] = M; res_ml[r * 2 + 1] = Lsum; }
     } else {
-      const size_t pi = ((size_t)seq * nh + head) * n_splits + split;
-      part_o[pi * HD + d] = O;
+      const size_t pi = ((size_t)seq * nh + kvh * G + r) * n_splits + split;
+      if (((uintptr_t)part_o & 15) == 0) {
+        *reinterpret_cast<float4*>(part_o + pi * HD + d) = O;
+      } else {
+        part_o[pi * HD + d] = O.x; part_o[pi * HD + d + 1] = O.y; part_o[pi * HD + d + 2] = O.z; part_o[pi * HD + d + 3] = O.w;
+      }
       if (d == 0) { part_ml[pi * 2] = M; part_ml[pi * 2 + 1] = Lsum; }
     }
   }
   if (CLUSTER && n_splits > 1) {
     // The cluster is the n_splits blocks of this (sequence, kv head); its rank is the split.  After the barrier
-    // every block's result lies in its shared memory; block k merges outputs k, k + n_splits, ... of the G * HD
-    // (head, value) pairs, in rank order, reading the others' results from afar.
+    // every block's result lies in its shared memory; block k merges the k-th share of the G * HD (head, value) pairs, in
+    // rank order, reading the others' results from afar.  All maxima and sums are fetched at once, then all blocks' values of
+    // a thread's four places: two trips through the cluster, where one remote load followed the other, three a block (with four
+    // values a thread in the merge of the warps: 18.9 -> 18.4 us at 48 sequences of 100 to 230 keys, 7.65 -> 7.15 at one of 1,500).
+    float* far_m = res_ml + 32;                               // [G][n_splits]
+    float* far_l = far_m + 16 * AD_MAX_CLUSTER;
     cluster_sync_all();
-    for (int idx = split + n_splits * (int)threadIdx.x; idx < G * HD; idx += n_splits * AD_COMPUTE_WARPS * 32) {
-      const int r = idx / HD, d = idx % HD;
+    for (int i = threadIdx.x; i < G * n_splits; i += AD_COMPUTE_WARPS * 32) {
+      const int r = i / n_splits, k = i - r * n_splits;
+      far_m[i] = cluster_load_f32(res_ml + r * 2, k);
+      far_l[i] = cluster_load_f32(res_ml + r * 2 + 1, k);
+    }
+    asm volatile("bar.sync 1, %0;\n" ::"n"(AD_COMPUTE_WARPS * 32) : "memory");
+    const int quads = G * HD / 4, per_block = (quads + n_splits - 1) / n_splits, q1 = min(quads, (split + 1) * per_block);
+    for (int idx = split * per_block + threadIdx.x; idx < q1; idx += AD_COMPUTE_WARPS * 32) {
+      const int r = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
+      float4 x[AD_MAX_CLUSTER];
+#pragma unroll
+      for (int k = 0; k < AD_MAX_CLUSTER; ++k)
+        if (k < n_splits) x[k] = ad_cluster_load4(res + r * HD + d, (uint32_t)k);
       float M = -INFINITY;
-      for (int k = 0; k < n_splits; ++k) M = fmaxf(M, cluster_load_f32(res_ml + r * 2, k));
-      float Lsum = 0.f, O = 0.f;
-      for (int k = 0; k < n_splits; ++k) {
-        const float mk = cluster_load_f32(res_ml + r * 2, k);
-        const float f = (mk == -INFINITY) ? 0.f : exp2f(mk - M);
-        Lsum += cluster_load_f32(res_ml + r * 2 + 1, k) * f;
-        if (f != 0.f) O += cluster_load_f32(res + r * HD + d, k) * f;
-      }
-      out[((size_t)seq * nh + kvh * G + r) * HD + d] = __float2bfloat16_rn(Lsum > 0.f ? O / Lsum : 0.f);
+#pragma unroll
+      for (int k = 0; k < AD_MAX_CLUSTER; ++k)
+        if (k < n_splits) M = fmaxf(M, far_m[r * n_splits + k]);
+      float Lsum = 0.f;
+      float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < AD_MAX_CLUSTER; ++k)
+        if (k < n_splits) {
+          const float mk = far_m[r * n_splits + k];
+          const float f = (mk == -INFINITY) ? 0.f : exp2f(mk - M);
+          Lsum += far_l[r * n_splits + k] * f;
+          if (f != 0.f) { O.x += x[k].x * f; O.y += x[k].y * f; O.z += x[k].z * f; O.w += x[k].w * f; }
+        }
+      put(r, d, O, Lsum);
     }
     cluster_sync_all();             // nobody leaves while its shared memory may still be read
   }
@@ -553,8 +601,8 @@ static int ad_launch(const CUtensorMap& mk, const CUtensorMap& mv, const bf16* q
                      int window, int n_splits, const AdPrep& prep, const float* sinks, int* status, cudaStream_t stream) {
   using L = AdLayout<HD>;
   static_assert(AD_STAGES == AD_COMPUTE_WARPS, "a stage has one consumer");
-  static_assert(AD_STAGES * L::STAGE >= (AD_COMPUTE_WARPS + 1) * (16 * HD + 16 * 2) * (int)sizeof(float),
-                "the ring holds the warps' results and the block's");
+  static_assert(AD_STAGES * L::STAGE >= ((AD_COMPUTE_WARPS + 1) * (16 * HD + 16 * 2) + 2 * 16 * AD_MAX_CLUSTER) * (int)sizeof(float),
+                "the ring holds the warps' results, the block's and the cluster's maxima and sums");
   // 2, 4, 8 or 16 splits: the splits of a (sequence, kv head) are a cluster and merge among themselves
   if (part_o == nullptr && n_splits > 1) {
     auto kern = attn_decode_tma_kernel<HD, PREP, true>;

@@ -141,9 +141,11 @@ class LatentAttention(Mixer):
         c, kr = ops.latent_gather(cache_view.k, ctx, bt, self.kv_rank, Dr)
         kv = ops.linear(c, self.ukv)
         table, n_pages = self._step_pages(ctx, x.device)
-        # zeros: the rows behind a sequence's end are masked, but a tensor-core product still multiplies them
-        kp = torch.zeros((n_pages, H, 64, D + Dr), dtype=x.dtype, device=x.device)
-        vp = torch.zeros((n_pages, H, 64, Dv), dtype=x.dtype, device=x.device)
+        # the rows behind a sequence's end are masked, but a tensor-core product still multiplies them: the tcgen05 kernel puts
+        # zeros in their place itself, for the other one they are zeros here
+        make = torch.empty if ops.tc_prefill_supported(x.dtype, H, H, D + Dr) else torch.zeros
+        kp = make((n_pages, H, 64, D + Dr), dtype=x.dtype, device=x.device)
+        vp = make((n_pages, H, 64, Dv), dtype=x.dtype, device=x.device)
         ops.latent_expand(kv, kr, ctx, table, H, D, Dr, Dv, kp, vp)
         q = ops.latent_rotate_q(q, H, D, Dr, inv_freq, rot_dims, pairs, ctx, mag)
         y = ops.attention(q, kp, vp, ctx, table, H, H, D + Dr, self.scale, self.window, sinks=self.sinks)
