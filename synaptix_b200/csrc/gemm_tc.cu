@@ -70,7 +70,7 @@ struct TcEp {
 };
 
 // floats a warp of the persistent kernel's epilogue stages of a tile's vectors (see tc_store_chunk)
-template <int EPI> struct TcVec { static constexpr int N = EPI == 4 ? 0 : (EPI == 6 ? 128 : (EPI == 5 ? 384 : 256)); };
+template <int EPI> struct TcVec { static constexpr int N = (EPI == 4 || EPI == 6) ? 1024 : (EPI == 5 ? 384 : 256); };
 template <int EPI, int BN> constexpr int tc_vec_floats() { return TcVec<EPI>::N * ((TcThreads<EPI, BN>::N - 64) / 32); }
 
 // BN: rows of W per tile (256 or 128); CG: blocks that compute a tile's instructions together (a pair stages half of W's rows
@@ -323,6 +323,15 @@ __device__ __forceinline__ void tc_ldg8(const float* p, float* v) {
 __device__ __forceinline__ void tc_stg8(float* p, const float* v) {
   asm volatile("st.global.v8.f32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};\n"
                ::"f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "l"(p) : "memory");
+}
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&x)[16]) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr));
+#pragma unroll
+  for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(r[i]);
 }
 __device__ __forceinline__ float tc_pack_bf16(float a, float b) {
   __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
@@ -676,12 +685,24 @@ __global__ void __launch_bounds__(TcThreads<EPI, BN>::N, 1) gemm_tc_persistent_k
         }
         __syncwarp();
       }
-      if (EPI == TC_EPI_QKV_BIAS) {                    // (a warp's columns are one head's)
-        __syncwarp();
-        *reinterpret_cast<float4*>(sv + lane * 4) = __ldg(reinterpret_cast<const float4*>(qk.bias + n0 + cb) + lane);
-        __syncwarp();
-      }
       if (RESID) load_h(cb, hv);
+      // Head preparation: this warp's 32 rows of cosines and sines pass through shared memory, 16 pairs of columns at a time (16
+      // bytes of place p of row r at p ^ r: neighbouring rows on different banks); the first are asked for while the tile's MMAs run.
+      const bool rot = QKV && qk.cs != nullptr && (n0 + cb) / 128 < qk.nh + qk.nkv;
+      auto place = [&](int r, int p) { return sv + (r * 8 + (p ^ (r & 7))) * 4; };
+      auto ask_rot = [&](int c) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int r = k * 4 + (lane >> 3), p = lane & 7;                    // places 0-3 cosines, 4-7 sines
+          const float* src = (p < 4 ? qk.cs : qk.sn) + (size_t)min(m0 + quarter * 32 + r, M - 1) * 64 + c * 16 + (p & 3) * 4;
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(tc_smem(place(r, p))), "l"(src) : "memory");
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+      };
+      if (rot) {
+        __syncwarp();                                  // (the tile before has been read)
+        ask_rot(0);
+      }
       if (!tc_mbar_wait(acc_full0 + 8 * buf, use & 1)) {
         if (lane == 0) sx_set_status(status, 3);
         return false;
@@ -689,81 +710,120 @@ __global__ void __launch_bounds__(TcThreads<EPI, BN>::N, 1) gemm_tc_persistent_k
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
       const uint32_t t_row = tmem_base + buf * BN + ((uint32_t)(quarter * 32) << 16);
       if (QKV) {
-        // head preparation: this thread's token, the tile's two heads one after the other
+        // Head preparation: this thread's token of this group's head (warps 2-5 the tile's first, 6-9 its second), read from the
+        // accumulator twice, for the norm's sum and 16 pairs of columns at a time for the rotation.  (Held in registers whole, a
+        // head left none for loads on the way, each thread read its own row of the tables, 32 lines a load, and the unrolled code
+        // was long enough that fetching it cost microseconds a launch.  2,560 -> 6,144 at 2,048 rows 58.3 -> 52.1 us, at 8,191 rows
+        // 187.9 -> 173.5, the plain product 46.0 and 162.8; 2,048 -> 4,096 at 611 rows 24.5 -> 21.9, in a prompt step 27.8 -> 23.2.)
         const bool page_ok = page >= 0 && page < qk.n_pages;
-        {
-          const int hh = (warp - 2) >> 2;                 // warps 2-5 take the tile's first head, warps 6-9 its second
-          const int head = n0 / 128 + hh;
-          float x[128];
+        const int head = (n0 + cb) / 128;
+        const uint32_t t_head = t_row + cb;
+        const bool is_q = head < qk.nh, is_k = !is_q && head < qk.nh + qk.nkv, is_v = !is_q && !is_k && head < qk.nh + 2 * qk.nkv;
+        const float* bias = EPI == TC_EPI_QKV_BIAS ? qk.bias + n0 + cb : nullptr;
+        // the projection's own output: bias added, rounded to bfloat16
+        auto projected = [&](float (&x)[16], int c) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) tc_ld32(t_row + hh * 128 + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&x[c * 32]));
-          asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
+          for (int i = 0; i < 4; ++i) {
             if (EPI == TC_EPI_QKV_BIAS) {
-              const float4 b = *reinterpret_cast<const float4*>(sv + 4 * i);
+              const float4 b = __ldg(reinterpret_cast<const float4*>(bias + c) + i);
               x[4 * i] += b.x; x[4 * i + 1] += b.y; x[4 * i + 2] += b.z; x[4 * i + 3] += b.w;
             }
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj) x[4 * i + jj] = __bfloat162float(__float2bfloat16_rn(x[4 * i + jj]));
+            for (int j = 0; j < 4; ++j) x[4 * i + j] = __bfloat162float(__float2bfloat16_rn(x[4 * i + j]));
           }
-          // this warp's part of the accumulator is in registers: hand it back
-          asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-          __syncwarp();
-          if (lane == 0) hand_back(buf);
-          const bool is_q = head < qk.nh, is_k = !is_q && head < qk.nh + qk.nkv, is_v = !is_q && !is_k && head < qk.nh + 2 * qk.nkv;
-          bf16* dst = nullptr;
-          if (live) {
-            if (is_q) {
-              dst = qk.q_out + ((size_t)row * qk.nh + head) * 128;
-            } else if (is_k || is_v) {
-              bf16* base = is_k ? qk.k_pages : qk.v_pages;
-              const int kvh = is_k ? head - qk.nh : head - qk.nh - qk.nkv;
-              if (base && page_ok) dst = base + (((size_t)page * qk.nkv + kvh) * SX_PAGE + (pos & 63)) * 128;
-            }
+        };
+        bf16* dst = nullptr;
+        if (live) {
+          if (is_q) {
+            dst = qk.q_out + ((size_t)row * qk.nh + head) * 128;
+          } else if (is_k || is_v) {
+            bf16* base = is_k ? qk.k_pages : qk.v_pages;
+            const int kvh = is_k ? head - qk.nh : head - qk.nh - qk.nkv;
+            if (base && page_ok) dst = base + (((size_t)page * qk.nkv + kvh) * SX_PAGE + (pos & 63)) * 128;
           }
-          if (!dst) return true;
-          if (is_q || is_k) {
-            // (four sums side by side: this thread has no other warp to hide behind; every index a constant, so that
-            //  the head stays in registers)
-            const float* w = is_q ? qk.wq : qk.wk;
-            float inv = 1.f;
-            if (w) {
-              float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+        }
+        const bool dst32 = (reinterpret_cast<uintptr_t>(dst) & 31) == 0;
+        const float* w = is_q ? qk.wq : (is_k ? qk.wk : nullptr);
+        float inv = 1.f;
+        if (w) {
+          float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll 1
+          for (int c = 0; c < 128; c += 32) {
+            float x[2][16];
+            tc_ld16(t_head + c, x[0]);
+            tc_ld16(t_head + c + 16, x[1]);
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
-              for (int i = 0; i < 128; i += 4) {
-                s0 += x[i] * x[i]; s1 += x[i + 1] * x[i + 1]; s2 += x[i + 2] * x[i + 2]; s3 += x[i + 3] * x[i + 3];
+            for (int k = 0; k < 2; ++k) {
+              projected(x[k], c + 16 * k);
+#pragma unroll
+              for (int i = 0; i < 16; i += 4) {
+                s0 += x[k][i] * x[k][i]; s1 += x[k][i + 1] * x[k][i + 1]; s2 += x[k][i + 2] * x[k][i + 2]; s3 += x[k][i + 3] * x[k][i + 3];
               }
-              inv = rsqrtf(((s0 + s1) + (s2 + s3)) / 128.f + qk.eps);
             }
-            const float4* cs4 = qk.cs ? reinterpret_cast<const float4*>(qk.cs + (size_t)row * 64) : nullptr;
-            const float4* sn4 = qk.cs ? reinterpret_cast<const float4*>(qk.sn + (size_t)row * 64) : nullptr;
+          }
+          inv = rsqrtf(((s0 + s1) + (s2 + s3)) / 128.f + qk.eps);
+        }
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          float lo[16], hi[16];
+          tc_ld16(t_head + 16 * c, lo);
+          tc_ld16(t_head + 64 + 16 * c, hi);
+          asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+          if (c == 3) {                                  // this warp's part of the accumulator has been read: hand it back
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) hand_back(buf);
+          }
+          projected(lo, 16 * c);
+          projected(hi, 64 + 16 * c);
+          if (rot) {
+            asm volatile("cp.async.wait_all;\n" ::: "memory");
+            __syncwarp();
+          }
+          if (is_q || is_k) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
+            for (int p = 0; p < 4; ++p) {
               float4 glo = make_float4(1.f, 1.f, 1.f, 1.f), ghi = glo, c4 = glo, s4 = make_float4(0.f, 0.f, 0.f, 0.f);
               if (w) {
-                glo = *reinterpret_cast<const float4*>(w + 4 * i);
-                ghi = *reinterpret_cast<const float4*>(w + 64 + 4 * i);
+                glo = *reinterpret_cast<const float4*>(w + 16 * c + 4 * p);
+                ghi = *reinterpret_cast<const float4*>(w + 64 + 16 * c + 4 * p);
               }
-              if (cs4) { c4 = cs4[i]; s4 = sn4[i]; }
+              if (rot) {
+                c4 = *reinterpret_cast<const float4*>(place(lane, p));
+                s4 = *reinterpret_cast<const float4*>(place(lane, 4 + p));
+              }
               const float gl[4] = {glo.x, glo.y, glo.z, glo.w}, gh[4] = {ghi.x, ghi.y, ghi.z, ghi.w};
-              const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, sv[4] = {s4.x, s4.y, s4.z, s4.w};
+              const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                const float a = x[4 * i + j] * inv * gl[j], bb = x[64 + 4 * i + j] * inv * gh[j];
-                x[4 * i + j] = a * cc[j] - bb * sv[j];
-                x[64 + 4 * i + j] = a * sv[j] + bb * cc[j];
+                const float a = lo[4 * p + j] * inv * gl[j], bb = hi[4 * p + j] * inv * gh[j];
+                lo[4 * p + j] = a * cc[j] - bb * ss[j];
+                hi[4 * p + j] = a * ss[j] + bb * cc[j];
               }
             }
           }
+          if (rot && c < 3) {
+            __syncwarp();
+            ask_rot(c + 1);
+          }
+          if (dst) {
+            float pl[8], ph[8];
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            uint4 pk;
-            __nv_bfloat162 t0 = __floats2bfloat162_rn(x[8 * i], x[8 * i + 1]), t1 = __floats2bfloat162_rn(x[8 * i + 2], x[8 * i + 3]);
-            __nv_bfloat162 t2 = __floats2bfloat162_rn(x[8 * i + 4], x[8 * i + 5]), t3 = __floats2bfloat162_rn(x[8 * i + 6], x[8 * i + 7]);
-            pk.x = *reinterpret_cast<uint32_t*>(&t0); pk.y = *reinterpret_cast<uint32_t*>(&t1);
-            pk.z = *reinterpret_cast<uint32_t*>(&t2); pk.w = *reinterpret_cast<uint32_t*>(&t3);
-            reinterpret_cast<uint4*>(dst)[i] = pk;
+            for (int j = 0; j < 8; ++j) {
+              pl[j] = tc_pack_bf16(lo[2 * j], lo[2 * j + 1]);
+              ph[j] = tc_pack_bf16(hi[2 * j], hi[2 * j + 1]);
+            }
+            if (dst32) {
+              tc_stg8(reinterpret_cast<float*>(dst + 16 * c), pl);
+              tc_stg8(reinterpret_cast<float*>(dst + 64 + 16 * c), ph);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 2; ++j) {
+                *reinterpret_cast<float4*>(dst + 16 * c + 8 * j) = make_float4(pl[4 * j], pl[4 * j + 1], pl[4 * j + 2], pl[4 * j + 3]);
+                *reinterpret_cast<float4*>(dst + 64 + 16 * c + 8 * j) = make_float4(ph[4 * j], ph[4 * j + 1], ph[4 * j + 2], ph[4 * j + 3]);
+              }
+            }
           }
         }
       } else {

@@ -114,3 +114,26 @@ def test_rule():
             chosen |= {f for f in FORMS if plan_stream(M, N, K, None, f) == plan}
             assert any(plan_stream(M, N, K, None, f) == plan for f in FORMS)
     assert chosen == set(FORMS)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bias", [False, True])
+def test_head_preparation_at_16_byte_places(bias):
+    """Outputs that begin 16 bytes behind a 32-byte boundary are written in 16-byte pieces: the same bits, and nothing beside."""
+    from synaptix_b200 import ops
+    from synaptix_b200.ops.gemm_tc import gemm_tc_qkv, gemm_tc_status
+    M, nh, nkv, K = 161, 4, 2, 264
+    x, w, b, _ = operands(M, (nh + 2 * nkv) * 128, K, 3)
+    i32 = lambda t: t.to(torch.int32).cuda()
+    cos, sin = ops.rope_table(i32(torch.arange(M)), (torch.arange(64) / 100).cuda())
+    got = []
+    for off in (0, 8):
+        bufs = [torch.full((n + 16,), float("nan"), dtype=BF, device="cuda") for n in (M * nh * 128, 3 * nkv * 64 * 128, 3 * nkv * 64 * 128)]
+        q, k, v = (t[off:off + t.numel() - 16] for t in bufs)
+        gemm_tc_qkv(x.cuda(), w.cuda(), q.view(M, nh * 128), k.view(3, nkv, 64, 128), v.view(3, nkv, 64, 128), None, None, cos, sin, 1e-6,
+                    i32(torch.arange(M)), i32(torch.zeros(M)), i32(torch.tensor([[2, 0, 1]])), nh, nkv, b.cuda() if bias else None)
+        got.append([t.clone() for t in (q, k, v)])
+        assert all(torch.isnan(t[:off].float()).all() and torch.isnan(t[off + t.numel() - 16:].float()).all() for t in bufs)
+    for a, c in zip(*got):
+        assert torch.equal(torch.isnan(a), torch.isnan(c)) and torch.equal(torch.nan_to_num(a), torch.nan_to_num(c))
+    assert not torch.isnan(got[0][0].float()).any() and gemm_tc_status() == 0
