@@ -93,7 +93,6 @@ class DecoderModel(Part):
             if owners[r.cache_entry] is None:
                 raise ValueError(f"cache entry {r.cache_entry} is read but never written")
         self._entry_owner = owners
-        self._forms: Optional[list] = None       # per layer: its form and where its tensors lie (see repeat.py)
         # an embedding with a state of its own (the token before) gets the cache entry behind the layers' entries
         self._embedding_entry = n_entries if getattr(embedding, "cache_request", None) is not None else None
         if self._embedding_entry is not None and self._keeps_embedding:
@@ -126,30 +125,21 @@ class DecoderModel(Part):
     def load(self, source: WeightSource, rt: Runtime, where: str = "weights") -> "DecoderModel":
         tensors = bind_tensors(self.all_tensor_specs(), source, where=where)
         self.bind_all(tensors, rt)
-        self._forms = None
         self.runtime = rt
         return self
 
-    def _same_until(self, first: int) -> int:
-        """The end of the stretch of runs from ``first`` on whose layers have one form and keys of their own; ``first``
-        itself if there is none, or if the run before it belongs to the same stretch (it began earlier)."""
-        if self._forms is None:
-            numbers: dict = {}             # equal forms get one number
-            self._forms = [f if f is None else (numbers.setdefault(f[0], len(numbers)), f[1])
-                           for f in (form_of(layer) for layer in self.layers)]
-
-        def form(k):
-            run = self.steps[k] if 0 <= k < len(self.steps) else None
-            if not isinstance(run, LayerRun) or not run.write_cache or self._forms[run.layer] is None:
-                return None
-            return self._forms[run.layer][0]
-        mine = form(first)
-        if mine is None or form(first - 1) == mine:
-            return first
-        end = first + 1
-        while form(end) == mine and self.steps[end].layer != self.steps[end - 1].layer:
-            end += 1
-        return end
+    def _same_as_before(self, k: int, forms: dict) -> bool:
+        """Whether run ``k`` is the one before it again, on another layer of the same form; both with keys of their own.
+        ``forms``: those of the step's layers that were asked for."""
+        if not 0 < k < len(self.steps):
+            return False
+        a, b = self.steps[k - 1], self.steps[k]
+        if not (isinstance(a, LayerRun) and isinstance(b, LayerRun) and a.write_cache and b.write_cache) or a.layer == b.layer:
+            return False
+        for n in (a.layer, b.layer):
+            if n not in forms:
+                forms[n] = form_of(self.layers[n])
+        return forms[a.layer] is not None and forms[b.layer] is not None and forms[a.layer][0] == forms[b.layer][0]
 
     # -- one step ------------------------------------------------------------
     def forward(self, ctx: StepContext, cache) -> torch.Tensor:
@@ -160,6 +150,7 @@ class DecoderModel(Part):
         observe = getattr(ctx, "observe", None)
         n_run = 0
         may_repeat = observe is None and not ctx.all_single and ctx.host is not None and ops.OPTIONS.repeat_layers
+        forms: dict = {}                         # layer: its form and where its tensors lie (see repeat.py)
         i = 0
         while i < len(self.steps):
             run = self.steps[i]
@@ -176,18 +167,22 @@ class DecoderModel(Part):
                 continue
             if isinstance(pending, PendingLinear) and not getattr(self.layers[run.layer], "takes_pending_product", False):
                 pending = pending.materialize()
-            end = self._same_until(i - 2) if may_repeat else 0          # a stretch that began with the layer before this one
-            if end - (i - 2) >= MIN_LAYERS:
+            if may_repeat and type(pending) is PendingLinear and self._same_as_before(i - 1, forms):
                 before, h_before = pending, h
                 with ops.recording() as launched:
                     h, pending = self.layers[run.layer].forward(h, before, ctx, cache.view(run.cache_entry), run.write_cache)
-                runs = self.steps[i - 2:end]
-                done = None
-                if h is h_before:
-                    done = repeat(launched, before, pending, [self._forms[r.layer][1] for r in runs],
+                may_repeat = launched.whole and h is h_before          # (else the layers like it are no different)
+                del forms[run.layer]             # a part may have made something of its own when it ran
+                end = i - 1
+                while may_repeat and self._same_as_before(end, forms):
+                    end += 1
+                if end - (i - 2) >= MIN_LAYERS:
+                    runs = self.steps[i - 2:end]
+                    done = repeat(launched, before, pending, [forms[r.layer][1] for r in runs],
                                   [cache.view(r.cache_entry) for r in runs])
-                if done is not None:
-                    pending, i = done, end
+                    may_repeat = done is not None
+                    if may_repeat:
+                        pending, i = done, end
                 continue
             h, pending = self.layers[run.layer].forward(h, pending, ctx, cache.view(run.cache_entry), run.write_cache)
             if observe is not None:              # the stream after this run: h with the branch not yet added

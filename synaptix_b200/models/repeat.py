@@ -5,7 +5,8 @@ are the pointers of their parameters, of their cache entries and of the branch t
 step of a few hundred tokens is bound by the host, which walks the parts and makes some twenty arguments for each of two
 hundred launches (17 us a launch at 0.6B sizes, more than the kernels take); so the step walks the first two layers of a
 stretch, records what the second one launched, and makes the same launches for the others with their pointers put in (5 us).
-Nothing of a step outlasts it; between steps only the layers' forms are remembered, never a pointer.
+Nothing of a step outlasts it: the layers' forms are taken anew in every step (20 us a layer), so that a layer that was put in, a
+number that was changed or a ``forward`` that was wrapped since the last one counts as it does where every layer is walked.
 
 Only parts whose class says ``repeatable`` in its own body are asked (their ``forward`` launches kernels through ``ops.launch``
 and does nothing else on the device, and depends on nothing but their sizes, the step and their inputs), and only a recording
@@ -28,28 +29,41 @@ class _Unlike(Exception):
     pass
 
 
+_VALUES = frozenset((type(None), bool, int, float, torch.dtype, torch.device))
+
+
+def _walk_part(part: Part, form: list, places: list) -> None:
+    """Append what ``part`` is, names aside, to ``form`` and the place of every tensor in it to ``places``."""
+    cls = type(part)
+    if not cls.__dict__.get("repeatable", False):
+        raise _Unlike
+    held = vars(part)
+    form.append(cls)
+    form.append(tuple(held))
+    for key, value in held.items():
+        _walk(value, held, key, form, places)
+
+
 def _walk(value, where, key, form: list, places: list) -> None:
-    """Append what ``value`` is, names aside, to ``form`` and the place of every tensor in it to ``places``."""
-    if isinstance(value, torch.Tensor):
-        form.append((tuple(value.shape), value.dtype, value.device, value.is_contiguous()))
+    kind = type(value)
+    if kind in _VALUES:
+        form.append(kind)
+        form.append(value)
+    elif isinstance(value, torch.Tensor):
+        form.append((value.shape, value.dtype, value.device, value.is_contiguous()))
         places.append((where, key))
     elif isinstance(value, Part):
-        if not type(value).__dict__.get("repeatable", False):
-            raise _Unlike
-        form.append(type(value))
-        for k, v in vars(value).items():
-            form.append(k)
-            _walk(v, vars(value), k, form, places)
-    elif isinstance(value, str):
+        _walk_part(value, form, places)
+    elif kind is str:
         form.append("")
-    elif value is None or isinstance(value, (bool, int, float, torch.dtype, torch.device)):
-        form.append((type(value), value))
-    elif isinstance(value, (list, tuple)):
-        form.append((type(value), len(value)))
+    elif kind is list or isinstance(value, tuple):
+        form.append(kind)
+        form.append(len(value))
         for i, v in enumerate(value):
             _walk(v, value, i, form, places)
-    elif isinstance(value, dict):
-        form.append((dict, len(value)))
+    elif kind is dict:
+        form.append(kind)
+        form.append(len(value))
         for k, v in value.items():
             _walk(v, value, k, form, places)
     else:
@@ -60,7 +74,7 @@ def form_of(layer: Part) -> Optional[Tuple[tuple, list]]:
     """``(form, places of its tensors)`` of a layer, or ``None`` if it holds anything that is not repeatable."""
     form, places = [], []
     try:
-        _walk(layer, None, None, form, places)
+        _walk_part(layer, form, places)
     except _Unlike:
         return None
     return tuple(form), places

@@ -11,7 +11,7 @@ from synaptix_b200.models import model_skeleton
 from synaptix_b200.models.repeat import form_of, repeat
 from synaptix_b200.ops import _lib
 from synaptix_b200.parts import RMSNorm
-from synaptix_b200.parts.base import PendingLinear
+from synaptix_b200.parts.base import Part, PendingLinear
 
 QWEN3 = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", num_hidden_layers=7, hidden_size=256, num_attention_heads=4,
              num_key_value_heads=2, head_dim=128, intermediate_size=320, vocab_size=997, rope_theta=10000.0, rms_norm_eps=1e-6,
@@ -85,6 +85,95 @@ def test_pointers_are_put_in():
         assert not record().whole
     with _lib.late_launch():
         assert not record().whole
+
+
+# ---- a decoder of layers that launch nothing real: what a prompt step launches, walked and repeated ----
+
+class Launches:
+    """Stands for a library's function: notes what it is called with."""
+    argtypes = [ctypes.c_void_p] * 6 + [ctypes.c_int]
+
+    def __init__(self):
+        self.made = []
+
+    def __call__(self, *args):
+        self.made.append(args)
+        return 0
+
+
+class Toy(Part):
+    """One launch a layer: the branch before, its weight, this layer's vector and cache, the branch handed on, a number."""
+    repeatable = True
+    takes_pending_product = True
+
+    def __init__(self, window=7):
+        self.weight, self.vector, self.window = torch.zeros(4, 4), torch.zeros(4), window
+
+    def forward(self, h, pending, ctx, view, write_cache=True):
+        z = torch.zeros(3, 4)
+        x, w = (None, None) if pending is None else (pending.x.data_ptr(), pending.weight.data_ptr())
+        _lib.launch(ctx.f, (x, w, self.vector.data_ptr(), view.k.data_ptr(), view.v.data_ptr(), z.data_ptr(), self.window), "toy", 1, (z,))
+        return h, PendingLinear(z, self.weight)
+
+
+def toy_model(layers):
+    from synaptix_b200.models.decoder import DecoderModel
+    embedding = types.SimpleNamespace(forward_step=lambda ctx, view=None: torch.zeros(3, 4))
+    norm = types.SimpleNamespace(takes_pending_product=True, add_forward=lambda h, pending, rows=None: pending.weight)
+    return DecoderModel(None, embedding, layers, norm, types.SimpleNamespace(forward=lambda x: x))
+
+
+def toy_step(model, views, on=True):
+    """What the step launched, without the branches' places, and the weight of the branch it ended with."""
+    from synaptix_b200 import ops
+    f = Launches()
+    ctx = types.SimpleNamespace(all_single=False, host={}, want_rows=None, observe=None, want_all=False, f=f)
+    with ops.options(repeat_layers=on):
+        last = model.forward(ctx, types.SimpleNamespace(view=lambda i: views[i]))
+    assert [a[0] for a in f.made[1:]] == [a[5] for a in f.made[:-1]]          # each reads what the one before wrote
+    return [a[1:5] + a[6:] for a in f.made], last.data_ptr()
+
+
+def toy_views(n):
+    return [types.SimpleNamespace(k=torch.zeros(2), v=torch.zeros(2), group=0, window=None) for _ in range(n)]
+
+
+def toy(n=8):
+    views = toy_views(n)
+    model = toy_model([Toy() for _ in range(n)])
+    walked = [0]
+    forward = Toy.forward
+
+    def counted(self, *args):
+        walked[0] += 1
+        return forward(self, *args)
+    return model, views, walked, counted
+
+
+def test_steps_after_a_change(monkeypatch):
+    """A layer put in, a number changed, a ``forward`` wrapped or a model loaded anew between two prompt steps count in the next."""
+    model, views, walked, counted = toy()
+    monkeypatch.setattr(Toy, "forward", counted)
+
+    def same(expected):
+        want, walked[0] = toy_step(model, views, on=False), 0
+        assert toy_step(model, views) == want
+        assert walked[0] == expected
+    same(2)                                       # the first two layers; the other six are repeated
+    model.layers[5] = Toy()
+    same(2)
+    model.layers[6].window = 64
+    same(4)                                       # ... the seventh is another, and the last is too short a stretch
+    model.layers[6].window = 7
+    same(2)
+    seen, inner = [], model.layers[7].forward
+    model.layers[7].forward = lambda *args: seen.append(1) or inner(*args)
+    same(3)
+    assert len(seen) == 2
+    del model.layers[7].forward
+    for layer in model.layers:
+        layer.weight, layer.vector = torch.zeros(4, 4), torch.zeros(4)
+    same(2)
 
 
 @pytest.mark.gpu
