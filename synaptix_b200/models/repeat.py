@@ -9,8 +9,9 @@ Nothing of a step outlasts it: the layers' forms are taken anew in every step (2
 number that was changed or a ``forward`` that was wrapped since the last one counts as it does where every layer is walked.
 
 Only parts whose class says ``repeatable`` in its own body are asked (their ``forward`` launches kernels through ``ops.launch``
-and does nothing else on the device, and depends on nothing but their sizes, the step and their inputs), and only a recording
-that holds everything that was launched is used; any other layer is simply walked.
+and does nothing else on the device, and depends on nothing but their sizes, the step and their inputs; strings other than the
+tensors' names, ``name_attributes``, belong to the form), and only a recording that holds everything that was launched is used;
+any other layer is simply walked.
 """
 from __future__ import annotations
 
@@ -33,41 +34,40 @@ _VALUES = frozenset((type(None), bool, int, float, torch.dtype, torch.device))
 
 
 def _walk_part(part: Part, form: list, places: list) -> None:
-    """Append what ``part`` is, names aside, to ``form`` and the place of every tensor in it to ``places``."""
+    """Append what ``part`` is, its tensors' names aside, to ``form`` and the place of every tensor in it to ``places``."""
     cls = type(part)
     if not cls.__dict__.get("repeatable", False):
         raise _Unlike
     held = vars(part)
-    form.append(cls)
-    form.append(tuple(held))
-    for key, value in held.items():
-        _walk(value, held, key, form, places)
+    form += (cls, tuple(held))
+    _walk(held, held.items(), form, places, cls.name_attributes)
 
 
-def _walk(value, where, key, form: list, places: list) -> None:
-    kind = type(value)
-    if kind in _VALUES:
-        form.append(kind)
-        form.append(value)
-    elif isinstance(value, torch.Tensor):
-        form.append((value.shape, value.dtype, value.device, value.is_contiguous()))
-        places.append((where, key))
-    elif isinstance(value, Part):
-        _walk_part(value, form, places)
-    elif kind is str:
-        form.append("")
-    elif kind is list or isinstance(value, tuple):
-        form.append(kind)
-        form.append(len(value))
-        for i, v in enumerate(value):
-            _walk(v, value, i, form, places)
-    elif kind is dict:
-        form.append(kind)
-        form.append(len(value))
-        for k, v in value.items():
-            _walk(v, value, k, form, places)
-    else:
-        raise _Unlike
+def _walk(where, items, form: list, places: list, names) -> None:
+    """The values of ``where``.  ``names``: the keys whose strings are names of tensors (``True``: all)."""
+    put = form.append
+    for key, value in items:
+        kind = type(value)
+        put(kind)
+        if kind in _VALUES:
+            put(value)
+        elif kind is str:
+            if names is not True and key not in names:
+                put(value)
+        elif kind is torch.Tensor or kind is torch.nn.Parameter:
+            put((value.shape, value.dtype, value.device, value.is_contiguous()))
+            places.append((where, key))
+        elif issubclass(kind, Part):
+            _walk_part(value, form, places)
+        elif kind is dict:
+            named = names is True or key in names
+            put(len(value) if named else tuple(value))
+            _walk(value, value.items(), form, places, named or ())
+        elif kind is list or issubclass(kind, tuple):
+            put(len(value))
+            _walk(value, enumerate(value), form, places, names is True or key in names or ())
+        else:
+            raise _Unlike
 
 
 def form_of(layer: Part) -> Optional[Tuple[tuple, list]]:

@@ -289,6 +289,7 @@ class Part:
     """Anything that owns tensors."""
 
     graph_safe = True      # False: forward depends on host values of the step (no CUDA graph)
+    name_attributes = ()   # of a repeatable part: attributes that hold names of tensors (strings, or lists or dicts with them)
 
     def tensor_specs(self) -> Dict[str, TensorSpec]:
         return {}

@@ -24,6 +24,8 @@ from .base import Part, PendingLinear, PendingNorm, Runtime, ScaledRows, to_devi
 
 class Linear(Part):
     repeatable = True
+    name_attributes = ("weight_names", "row_order")
+
     def __init__(self, weight_names: Sequence[str], in_features: int, out_features: Sequence[int],
                  kind: str = "matrix", bias_suffix: Optional[str] = None,
                  row_order: Optional[Mapping[str, torch.Tensor]] = None):

@@ -21,6 +21,7 @@ class RMSNorm(Norm):
     """``offset``: the stored tensor ``w`` lies around zero and the gain is ``offset + w`` (formed once, in 32-bit,
     when the weights are bound); 0 is the plain gain."""
     repeatable = True
+    name_attributes = ("weight_name",)
 
     def __init__(self, weight_name: str, width: int, eps: float, offset: float = 0.0):
         self.weight_name = weight_name

@@ -10,7 +10,7 @@ import tiny
 from synaptix_b200.models import model_skeleton
 from synaptix_b200.models.repeat import form_of, repeat
 from synaptix_b200.ops import _lib
-from synaptix_b200.parts import RMSNorm
+from synaptix_b200.parts import Linear, RMSNorm
 from synaptix_b200.parts.base import Part, PendingLinear
 
 QWEN3 = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", num_hidden_layers=7, hidden_size=256, num_attention_heads=4,
@@ -36,6 +36,26 @@ def test_forms():
     assert form_of(layers[0]) is None and form_of(layers[1]) is not None
     layers[1].extra = object()
     assert form_of(layers[1]) is None
+
+
+def test_strings_of_a_form():
+    """Names of tensors differ between like layers; any other string may decide what a part does."""
+    forms = [form_of(x)[0] for x in skeleton().layers]
+    assert len(set(forms)) == 1
+
+    class Scored(RMSNorm):
+        repeatable = True
+
+        def __init__(self, name, scoring):
+            super().__init__(name, 8, 1e-6)
+            self.scoring, self.by_kind = scoring, {scoring: 1}
+    a, b, c = form_of(Scored("a", "softmax"))[0], form_of(Scored("b", "softmax"))[0], form_of(Scored("a", "sigmoid"))[0]
+    assert a == b and a != c
+    d = Scored("a", "softmax")
+    d.by_kind = {"sigmoid": 1}
+    assert form_of(d)[0] != a
+    a, b = (form_of(Linear(n, 4, 4, kind=k))[0] for n, k in (("a", "matrix"), ("b", "embedding")))
+    assert a != b
 
 
 def test_pointers_are_put_in():
