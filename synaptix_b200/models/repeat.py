@@ -106,18 +106,27 @@ def repeat(recording, before, after, places: list, views: list):
         return None
     if any(v.group != views[1].group or v.window != views[1].window for v in views[2:]):
         return None
-    # where a recorded pointer comes from: (row of the table below, column)
+    # What a recorded pointer can be, as (row, column) of the table that a layer makes of its own: (the layer before, the branch
+    # that comes in) and (the layer, its cache, the branch that goes out).
+    def table(above, mine, view, x_in, x_out):
+        k, v = (0 if t is None else t.data_ptr() for t in (view.k, view.v))
+        return above + [x_in.data_ptr()], mine + [k, v, x_out.data_ptr()]
+    x_in, x_out = before.x, after.x
+    above, mine = [t.data_ptr() for t in first], [t.data_ptr() for t in second]
     source = {}
-    for row, tensors in ((0, first), (1, second)):
-        for i, t in enumerate(tensors):
-            source[t.data_ptr()] = (row, i)
-    n = len(second)
-    for i, t in ((n, views[1].k), (n + 1, views[1].v)):
-        if t is not None:
-            source[t.data_ptr()] = (1, i)
-    source[before.x.data_ptr()] = (0, n)
-    source[after.x.data_ptr()] = (1, n + 2)
+    for row, pointers in enumerate(table(above, mine, views[1], x_in, x_out)):
+        for i, a in enumerate(pointers):
+            source.setdefault(a, []).append((row, i))
     source.pop(0, None)
+    tables = []
+    for p, view in zip(places[2:], views[2:]):
+        x_in, x_out = x_out, x_in                  # the branch a layer hands on is the next one's
+        above, mine = mine, [where[key].data_ptr() for where, key in p]
+        tables.append(table(above, mine, view, x_in, x_out))
+    # one pointer for several things (tied weights): they have to be one in every layer
+    for at in source.values():
+        if len(at) > 1 and any(t[row][i] != t[at[0][0]][at[0][1]] for t in tables for row, i in at[1:]):
+            return None
     # (a pointer into the middle of one of these has no place to come from in the next layer)
     spans = sorted((t.data_ptr(), t.data_ptr() + t.numel() * t.element_size())
                    for t in first + second + [t for t in (views[1].k, views[1].v) if t is not None])
@@ -130,20 +139,13 @@ def repeat(recording, before, after, places: list, views: list):
     for f, args, what, launches in recording.calls:
         if any(kind is ctypes.c_void_p and a and a not in source and inside(a) for a, kind in zip(args, f.argtypes)):
             return None
-        put = [(j,) + source[a] for j, (a, kind) in enumerate(zip(args, f.argtypes))
+        put = [(j,) + source[a][0] for j, (a, kind) in enumerate(zip(args, f.argtypes))
                if kind is ctypes.c_void_p and a in source]
         calls.append((f, list(args), put, what, launches))
-    x_in, x_out = before.x, after.x
-    above = [t.data_ptr() for t in second]
-    for p, view in zip(places[2:], views[2:]):
-        x_in, x_out = x_out, x_in                  # the branch a layer hands on is the next one's
-        mine = [where[key].data_ptr() for where, key in p]
-        table = (above + [x_in.data_ptr()],
-                 mine + [0 if view.k is None else view.k.data_ptr(), 0 if view.v is None else view.v.data_ptr(), x_out.data_ptr()])
+    for t in tables:
         for f, args, put, what, launches in calls:
             for j, row, i in put:
-                args[j] = table[row][i]
+                args[j] = t[row][i]
             check(f(*args), what, launches)
-        above = mine
     last = _tensors(places[-1])
     return PendingLinear(x_out, last[weight], None if bias is None else last[bias])

@@ -196,6 +196,32 @@ def test_steps_after_a_change(monkeypatch):
     same(2)
 
 
+
+def test_one_tensor_in_two_places(monkeypatch):
+    """Where a pointer of the recorded layer stands for two of its tensors, or for one of the layer before, too, and the other
+    layers' do not, the launches are not made again with it."""
+    model, views, walked, counted = toy()
+    monkeypatch.setattr(Toy, "forward", counted)
+    plain = [(x.weight, x.vector) for x in model.layers]
+
+    def same(expected):
+        want, walked[0] = toy_step(model, views, on=False), 0
+        assert toy_step(model, views) == want and walked[0] == expected
+        for x, (w, v) in zip(model.layers, plain):
+            x.weight, x.vector = w, v
+    same(2)
+    model.layers[1].weight = model.layers[0].weight
+    same(8)
+    model.layers[1].vector = model.layers[1].weight.view(-1)[:4]
+    same(8)
+    for x in model.layers:                        # in every layer: one pointer for both
+        x.vector = x.weight.view(-1)[:4]
+    same(2)
+    for x in model.layers:                        # one tensor for all layers
+        x.vector = plain[0][1]
+    same(2)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("more", [{}, dict(head_dim=64), dict(use_sliding_window=True, sliding_window=64, max_window_layers=2)])
 @pytest.mark.parametrize("dtype", ["bf16", "f32"])
