@@ -17,6 +17,7 @@ from __future__ import annotations
 
 import bisect
 import ctypes
+import itertools
 from typing import List, Optional, Tuple
 
 import torch
@@ -129,12 +130,12 @@ def repeat(recording, before, after, places: list, views: list):
             return None
     # (a pointer into the middle of one of these has no place to come from in the next layer)
     spans = sorted((t.data_ptr(), t.data_ptr() + t.numel() * t.element_size())
-                   for t in first + second + [t for t in (views[1].k, views[1].v) if t is not None])
-    starts = [a for a, _ in spans]
+                   for t in first + second + [before.x, after.x] + [t for t in (views[1].k, views[1].v) if t is not None])
+    starts, ends = [a for a, _ in spans], list(itertools.accumulate((b for _, b in spans), max))
 
     def inside(a: int) -> bool:
         i = bisect.bisect_right(starts, a)
-        return i > 0 and a < spans[i - 1][1]
+        return i > 0 and a < ends[i - 1]
     calls = []
     for f, args, what, launches in recording.calls:
         if any(kind is ctypes.c_void_p and a and a not in source and inside(a) for a, kind in zip(args, f.argtypes)):

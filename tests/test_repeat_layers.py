@@ -222,6 +222,17 @@ def test_one_tensor_in_two_places(monkeypatch):
     same(2)
 
 
+def test_pointers_into_the_middle():
+    """A pointer into the middle of the branch that comes in or goes out, or of a weight behind a tensor that lies in it, has
+    another one in its place in the next layer."""
+    z = [torch.zeros(3, 4), torch.zeros(3, 4)]
+    w = [[x, x[0], torch.zeros(4)] for x in (torch.zeros(4, 4) for _ in range(5))]
+    for a in (z[0], z[1], w[1][0]):
+        with _lib.recording() as r:
+            _lib.launch(Launches(), (a.data_ptr() + 32, w[1][2].data_ptr(), None, None, None, None, 0), "test")
+        assert repeat(r, PendingLinear(z[0], w[0][0]), PendingLinear(z[1], w[1][0]), [[(x, i) for i in range(3)] for x in w], toy_views(5)) is None
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("more", [{}, dict(head_dim=64), dict(use_sliding_window=True, sliding_window=64, max_window_layers=2)])
 @pytest.mark.parametrize("dtype", ["bf16", "f32"])
