@@ -41,6 +41,9 @@ def _walk_part(part: Part, form: list, places: list) -> None:
         raise _Unlike
     held = vars(part)
     form += (cls, tuple(held))
+    for key in cls.shared_attributes:              # (what a step makes of such a tensor has a place of its own in the launches)
+        t = held[key]
+        form.append(None if t is None else t.data_ptr())
     _walk(held, held.items(), form, places, cls.name_attributes)
 
 

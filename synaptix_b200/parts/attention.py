@@ -56,6 +56,7 @@ _FOLDED = {}
 class Attention(Mixer):
     repeatable = True
     name_attributes = ("prefix", "names")
+    shared_attributes = ("_inv_freq",)
     accepts_lazy_input = True      # x goes straight into the fused q/k/v product
     can_defer_output = True        # the output projection may be handed on unrun
 

@@ -39,6 +39,7 @@ class RotaryHalf(PositionEncoding):
     ``magnitude``; the frequencies are then formed in 64-bit and rounded once.  A kernel that rotates for a part with such
     an encoding multiplies by ``magnitude`` (the parts that take one say so)."""
     repeatable = True
+    shared_attributes = ("inv_freq",)
     pairs = False
 
     def __init__(self, head_dim: int, theta: float, rotary_dim: int = None, scaling: "FrequencyRamp" = None):

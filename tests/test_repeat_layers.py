@@ -58,6 +58,19 @@ def test_strings_of_a_form():
     assert a != b
 
 
+def test_tensors_that_a_step_makes_something_of():
+    """Layers that rotate by another tensor of frequencies are not alike, whatever its sizes: a step's tables of cosines and sines
+    belong to the tensor they were made of."""
+    for part, key in ((lambda x: x.mixer.position, "inv_freq"), (lambda x: x.mixer, "_inv_freq")):
+        layers, one = skeleton().layers, torch.ones(64)
+        for x in layers:
+            setattr(part(x), key, one)
+        assert len({form_of(x)[0] for x in layers}) == 1
+        setattr(part(layers[4]), key, torch.ones(64))
+        forms = [form_of(x)[0] for x in layers]
+        assert forms[4] != forms[0] and len(set(forms)) == 2
+
+
 def test_pointers_are_put_in():
     n, made = 5, []
 
