@@ -99,7 +99,7 @@ def repeat(recording, before, after, places: list, views: list):
     ``places[2:]`` those of the layers to come; ``views[1:]`` are the cache views of the recorded and the coming ones.
     ``before`` and ``after`` are the branches the recorded layer was handed and handed on (``PendingLinear``).  Returns the
     branch that the last layer hands on, or ``None`` if the recording cannot be used (nothing has been launched then)."""
-    from ..ops._lib import check
+    from ..ops._lib import check, use_gate
     if not recording.whole or type(before) is not PendingLinear or type(after) is not PendingLinear:
         return None
     if before.x.shape != after.x.shape or before.x.dtype != after.x.dtype or (before.bias is None) != (after.bias is None):
@@ -140,16 +140,18 @@ def repeat(recording, before, after, places: list, views: list):
         i = bisect.bisect_right(starts, a)
         return i > 0 and a < ends[i - 1]
     calls = []
-    for f, args, what, launches in recording.calls:
+    for f, args, what, launches, gated in recording.calls:
         if any(kind is ctypes.c_void_p and a and a not in source and inside(a) for a, kind in zip(args, f.argtypes)):
             return None
         put = [(j,) + source[a][0] for j, (a, kind) in enumerate(zip(args, f.argtypes))
                if kind is ctypes.c_void_p and a in source]
-        calls.append((f, list(args), put, what, launches))
+        calls.append((f, list(args), put, what, launches, gated))
     for t in tables:
-        for f, args, put, what, launches in calls:
+        for f, args, put, what, launches, gated in calls:
             for j, row, i in put:
                 args[j] = t[row][i]
+            if gated is not None:                  # (a library's activation may be another thread's since)
+                use_gate(gated)
             check(f(*args), what, launches)
     last = _tensors(places[-1])
     return PendingLinear(x_out, last[weight], None if bias is None else last[bias])

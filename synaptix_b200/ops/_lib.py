@@ -93,12 +93,14 @@ def count_launches(n: int) -> None:
 
 
 class Recording:
-    """The launches of a stretch of a step as they were made: ``calls`` holds ``(function, arguments, what, launches)`` of
-    everything that went through ``launch``, ``keep`` the tensors made for them.  ``whole`` says whether that is all that was
-    launched, under the options that hold outside too, so that the calls can be made again with other pointers."""
+    """The launches of a stretch of a step as they were made: ``calls`` holds ``(function, arguments, what, launches, library)``
+    of everything that went through ``launch`` (``library``: the one that was told the gated activation for it, or ``None``),
+    ``keep`` the tensors made for them.  ``whole`` says whether that is all that was launched, under the options that hold outside
+    too, so that the calls can be made again with other pointers."""
 
     def __init__(self):
         self.calls, self.keep = [], []
+        self.gated: Optional[str] = None
         self.checked, self.plain = 0, True
 
     @property
@@ -128,8 +130,9 @@ def launch(f, args: tuple, what: str, launches: int = 1, keep: tuple = ()) -> No
     check(f(*args), what, launches)
     r = _TLS.recording
     if r is not None:
-        r.calls.append((f, args, what, launches))
+        r.calls.append((f, args, what, launches, r.gated))
         r.keep += keep
+        r.gated = None
         if _LATE[0] or _GATE[0] != _GATE_DEFAULT:
             r.plain = False
 
@@ -274,6 +277,8 @@ def current_gate():
 
 
 def use_gate(lib: str) -> None:
+    if _TLS.recording is not None:
+        _TLS.recording.gated = lib
     want = _GATE[0]
     if _LIB_GATE.get(lib) != want:
         f = getattr(_library(lib), "sx_set_gate_act")

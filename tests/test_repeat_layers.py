@@ -1,6 +1,8 @@
 """Launches of layers of one form made again with other pointers: which layers are alike, which pointers are put in, and (on the
 GPU) that a prompt step gives the same bits as one that walks every layer."""
 import ctypes
+import sys
+import threading
 import types
 
 import pytest
@@ -244,6 +246,37 @@ def test_pointers_into_the_middle():
         with _lib.recording() as r:
             _lib.launch(Launches(), (a.data_ptr() + 32, w[1][2].data_ptr(), None, None, None, None, 0), "test")
         assert repeat(r, PendingLinear(z[0], w[0][0]), PendingLinear(z[1], w[1][0]), [[(x, i) for i in range(3)] for x in w], toy_views(5)) is None
+
+
+
+def test_activation_is_told_again(monkeypatch):
+    """Between two of the launches that are made again, another thread may tell the library another activation."""
+    told = []
+    lib = types.SimpleNamespace(sx_set_gate_act=lambda alpha, limit, form: told.append(form.value))
+    monkeypatch.setitem(_lib._LIBS, "toy", lib)
+    monkeypatch.setitem(_lib._LIB_GATE, "toy", None)
+    seen = []
+
+    def others():
+        with _lib.gate_activation(form="gelu_tanh"):
+            _lib.use_gate("toy")
+
+    class Shared(Launches):
+        def __call__(self, *args):
+            seen.append(told[-1])
+            t = threading.Thread(target=others)
+            t.start()
+            t.join()
+            return super().__call__(*args)
+    n, forward = 8, Toy.forward
+
+    def gated(self, h, pending, ctx, view, write_cache=True):
+        _lib.use_gate("toy")
+        return forward(self, h, pending, ctx, view, write_cache)
+    monkeypatch.setattr(Toy, "forward", gated)
+    monkeypatch.setattr(sys.modules[__name__], "Launches", Shared)
+    toy_step(toy_model([Toy() for _ in range(n)]), toy_views(n))
+    assert seen == [0] * n
 
 
 @pytest.mark.gpu
