@@ -540,19 +540,50 @@ static int moe_mma_launch(const void* A, const void* Wt, void* C, const int* off
 // order.  Blocks are small (82 KB of weights at K = 2,560) and several share an SM, so the last round costs little; the blocks of
 // 128 matrix rows of the kernel above came two to an SM in 2.05 rounds for 16 experts of 2,432 outputs.  Bound by HBM: 8 tokens,
 // 14 of 16 experts chosen, width 2,560, inside a decode step: gate/up 80 -> 68 us (360 MB), down 52 -> 39 (180 MB).
+// The grid's y axis has a place for every expert, or, when the step has fewer rows than there are experts, for every row: block y
+// then takes the y-th expert that has rows (of `find_of`; the count over the experts takes a load and two barriers for 256 of them).
+// One token, width 2,048: 8 of 128 experts of 768 outputs 24.6 us with a place for every expert, 20.5 for every row (30.7 with the
+// kernel above), down 25.4 and 15.2 (21.3); 8 of 1,024 experts of 256 outputs 43.0 and 14.3 (94.2), down 141 and 12.3 (79.8).
 // ---------------------------------------------------------------------------------------------------------------
 #define MS_DEPTH 4
 #define MS_MAX_TOKENS 16
+// the place among the E experts of the `want`-th one that has rows, or -1; all 256 threads get it
+__device__ __forceinline__ int moe_chosen_expert(const int* __restrict__ offsets, int E, int want) {
+  __shared__ int n_warp[8], found;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) found = -1;
+  for (int e0 = 0; e0 < E; e0 += 256) {
+    const int e = e0 + tid;
+    const bool some = e < E && offsets[e + 1] > offsets[e];
+    const unsigned m = __ballot_sync(0xffffffffu, some);
+    if (lane == 0) n_warp[warp] = __popc(m);
+    __syncthreads();
+    int before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      if (w < warp) before += n_warp[w];
+      all += n_warp[w];
+    }
+    if (some && before + __popc(m & ((1u << lane) - 1)) == want) found = e;
+    __syncthreads();
+    if (want < all) break;
+    want -= all;
+  }
+  return found;
+}
+
 template <typename TC, int MODE, int NT>
 __global__ void __launch_bounds__(256) moe_stream_kernel(const bf16* __restrict__ A, const bf16* __restrict__ Wt, TC* __restrict__ C,
-                                                         const int* __restrict__ offsets, const int* __restrict__ order, int N,
+                                                         const int* __restrict__ offsets, const int* __restrict__ order, int find_of, int N,
                                                          int K, int top, const GateAct act) {
   constexpr bool GATE_UP = MODE == MOE_GATE_UP, GATHER = MODE != MOE_PLAIN;
   __shared__ __align__(16) uint4 ring[MS_DEPTH][2][256];
   __shared__ float red[8][NT][4][32];
   pdl_wait();
   pdl_trigger();
-  const int e = blockIdx.y, r_end = offsets[e + 1];
+  const int e = find_of > 0 ? moe_chosen_expert(offsets, find_of, blockIdx.y) : (int)blockIdx.y;
+  if (e < 0) return;                       // (fewer experts than rows were chosen)
+  const int r_end = offsets[e + 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int tile = blockIdx.x;
   int row_lo, row_hi;
@@ -654,6 +685,15 @@ __global__ void __launch_bounds__(256) moe_stream_kernel(const bf16* __restrict_
 // up to this many (token, choice) rows a step, blocks of 16 rows with the deeper ring
 #define MM_FEW_ROWS 64
 
+// the grid of the kernel above: column tiles x experts, or rows where they are fewer
+static dim3 moe_stream_grid(int rows, int E, int N, int mode) {
+  return dim3(mode == MOE_GATE_UP ? (N + 7) / 8 : (N + 15) / 16, E < rows ? E : rows);
+}
+extern "C" long long sx_moe_stream_blocks(int rows, int E, int N, int mode) {
+  const dim3 g = moe_stream_grid(rows, E, N, mode);
+  return (long long)g.x * g.y;
+}
+
 // rows: T * top; the grid's y axis has room for every expert's last, partly filled tile; mode: MOE_PLAIN, MOE_GATE_UP, MOE_UP;
 // most: the most rows one expert can have (the step's tokens; 0: not known)
 extern "C" int sx_moe_gemm(const void* A, const void* Wt, void* C, const int* offsets, const int* order, int rows, int E, int N,
@@ -664,12 +704,13 @@ extern "C" int sx_moe_gemm(const void* A, const void* Wt, void* C, const int* of
   if (tiles > 65535) return SX_ERR_SIZE;
   if (a_dt == SX_BF16 && K % 8 == 0 && ((uintptr_t)A | (uintptr_t)Wt) % 16 == 0) {       // the tensor cores
     // Whole steps of 32 k and at most 16 rows an expert: streamed (figures at the kernel); more rows would read the weights again.
-    const bool stream_it = K % 32 == 0 && most > 0 && most <= MS_MAX_TOKENS && E <= 65535;
-    const dim3 sgrid(mode == MOE_GATE_UP ? (N + 7) / 8 : (N + 15) / 16, E);
+    const bool stream_it = K % 32 == 0 && most > 0 && most <= MS_MAX_TOKENS;
+    const dim3 sgrid = moe_stream_grid(rows, E, N, mode);
+    const int find_of = rows < E ? E : 0;
 #define MM_GO(TC, M)                                                                                              \
   if (stream_it)                                                                                                  \
-    return most <= 8 ? sx_launch(moe_stream_kernel<TC, M, 1>, sgrid, dim3(256), 0, stream, (const bf16*)A, (const bf16*)Wt, (TC*)C, offsets, order, N, K, top, g_sx_gate) \
-                     : sx_launch(moe_stream_kernel<TC, M, 2>, sgrid, dim3(256), 0, stream, (const bf16*)A, (const bf16*)Wt, (TC*)C, offsets, order, N, K, top, g_sx_gate); \
+    return most <= 8 ? sx_launch(moe_stream_kernel<TC, M, 1>, sgrid, dim3(256), 0, stream, (const bf16*)A, (const bf16*)Wt, (TC*)C, offsets, order, find_of, N, K, top, g_sx_gate) \
+                     : sx_launch(moe_stream_kernel<TC, M, 2>, sgrid, dim3(256), 0, stream, (const bf16*)A, (const bf16*)Wt, (TC*)C, offsets, order, find_of, N, K, top, g_sx_gate); \
   return rows <= MM_FEW_ROWS ? moe_mma_launch<TC, M, 16>(A, Wt, C, offsets, order, rows, E, N, K, top, stream)    \
                              : moe_mma_launch<TC, M, 64>(A, Wt, C, offsets, order, rows, E, N, K, top, stream)
     if (mode == MOE_GATE_UP && c_dt == SX_BF16) { MM_GO(bf16, MOE_GATE_UP); }

@@ -145,6 +145,13 @@ def test_experts(T, E, top, ff, W, same):
     assert ((got - want).abs() <= (W + 4) * ULP * mag).all()
 
 
+@pytest.mark.parametrize("T,E,top", [(1, 128, 8), (3, 257, 3), (1, 512, 1), (9, 1024, 2)])
+@pytest.mark.parametrize("same", [False, True])
+def test_fewer_pairs_than_experts(T, E, top, same):
+    """The blocks look for the experts that were chosen, 256 of them at a time."""
+    test_experts(T, E, top, 24, 96, same)
+
+
 @pytest.mark.parametrize("counts", [[512], [0, 1, 127, 128, 129, 0, 300, 2], [3] * 200, [0] * 37 + [600, 0, 0]])
 @pytest.mark.parametrize("ff,W", [(8, 64), (130, 200), (384, 1048)])
 def test_experts_of_a_prompt(counts, ff, W):
