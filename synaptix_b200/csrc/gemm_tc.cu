@@ -324,15 +324,6 @@ __device__ __forceinline__ void tc_stg8(float* p, const float* v) {
   asm volatile("st.global.v8.f32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};\n"
                ::"f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "l"(p) : "memory");
 }
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&x)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(taddr));
-#pragma unroll
-  for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(r[i]);
-}
 __device__ __forceinline__ float tc_pack_bf16(float a, float b) {
   __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<float*>(&t);
@@ -720,8 +711,10 @@ __global__ void __launch_bounds__(TcThreads<EPI, BN>::N, 1) gemm_tc_persistent_k
         const uint32_t t_head = t_row + cb;
         const bool is_q = head < qk.nh, is_k = !is_q && head < qk.nh + qk.nkv, is_v = !is_q && !is_k && head < qk.nh + 2 * qk.nkv;
         const float* bias = EPI == TC_EPI_QKV_BIAS ? qk.bias + n0 + cb : nullptr;
-        // the projection's own output: bias added, rounded to bfloat16
-        auto projected = [&](float (&x)[16], int c) {
+        // the projection's own output out of the accumulator (after the wait for it): bias added, rounded to bfloat16
+        auto projected = [&](const uint32_t (&r)[16], float (&x)[16], int c) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) x[i] = __uint_as_float(r[i]);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             if (EPI == TC_EPI_QKV_BIAS) {
@@ -749,13 +742,14 @@ __global__ void __launch_bounds__(TcThreads<EPI, BN>::N, 1) gemm_tc_persistent_k
           float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll 1
           for (int c = 0; c < 128; c += 32) {
+            uint32_t r[2][16];
             float x[2][16];
-            tc_ld16(t_head + c, x[0]);
-            tc_ld16(t_head + c + 16, x[1]);
+            tc_ld16(t_head + c, r[0]);
+            tc_ld16(t_head + c + 16, r[1]);
             asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-              projected(x[k], c + 16 * k);
+              projected(r[k], x[k], c + 16 * k);
 #pragma unroll
               for (int i = 0; i < 16; i += 4) {
                 s0 += x[k][i] * x[k][i]; s1 += x[k][i + 1] * x[k][i + 1]; s2 += x[k][i + 2] * x[k][i + 2]; s3 += x[k][i + 3] * x[k][i + 3];
@@ -766,17 +760,18 @@ __global__ void __launch_bounds__(TcThreads<EPI, BN>::N, 1) gemm_tc_persistent_k
         }
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
+          uint32_t rlo[16], rhi[16];
           float lo[16], hi[16];
-          tc_ld16(t_head + 16 * c, lo);
-          tc_ld16(t_head + 64 + 16 * c, hi);
+          tc_ld16(t_head + 16 * c, rlo);
+          tc_ld16(t_head + 64 + 16 * c, rhi);
           asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
           if (c == 3) {                                  // this warp's part of the accumulator has been read: hand it back
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncwarp();
             if (lane == 0) hand_back(buf);
           }
-          projected(lo, 16 * c);
-          projected(hi, 64 + 16 * c);
+          projected(rlo, lo, 16 * c);
+          projected(rhi, hi, 64 + 16 * c);
           if (rot) {
             asm volatile("cp.async.wait_all;\n" ::: "memory");
             __syncwarp();
