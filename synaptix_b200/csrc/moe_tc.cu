@@ -67,6 +67,8 @@ __global__ void __launch_bounds__(MT_THREADS, 1) moe_tc_kernel(const __grid_cons
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc_smem(tmem_slot)), "r"((uint32_t)(2 * MT_BN)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
+  // (the next kernel is let in by any warp's trigger, and may ask for tensor memory itself: this block has its own by then)
+  __syncthreads();
   pdl_wait();          // the offsets come from a kernel before
   pdl_trigger();
   if (warp == 0) {     // running sums over the experts, 32 at a time

@@ -29,3 +29,17 @@ def test_loads_from_tensor_memory_end_their_helper():
             assert re.fullmatch(r"\s*\}", rest[rest.index(");") + 2:]), (name, body[:80])
             found += 1
     assert found >= 3
+
+
+def test_tensor_memory_is_taken_before_the_next_kernel_is_let_in():
+    """A block that lets the next kernel in (any warp's trigger does) while it still waits for tensor memory could wait for a
+    block that waits for it."""
+    found = 0
+    for name, text in SOURCES.items():
+        for m in re.finditer(r'"tcgen05\.alloc\.', text):
+            body = body_around(text, m.start())
+            rest = body[body.index("tcgen05.alloc."):]
+            between = rest[:rest.index("pdl_trigger()")]
+            assert "__syncthreads()" in between or "cluster_sync_all()" in between, (name, body[:80])
+            found += 1
+    assert found >= 5
