@@ -84,11 +84,11 @@ def _plan(M: int, N: int, K: int, epilogue: Optional[str], form: Optional[str]):
     return tuple(int(v) for v in out)
 
 
-def plan_stream(M: int, N: int, K: int, epilogue: Optional[str] = None, form: Optional[str] = "one"):
-    """``(whole tiles, cut tiles, most pieces a cut tile has, grid)`` of a form of the persistent kernel on the current
-    device (``None``: of the form it takes for the shape).  Tiles that would not fill a round of all SMs (a last
-    round at most half full: 2,048 x 2,560 has 160 tiles for 148 SMs; or all tiles of a step with at most 128 rows) are cut over K: their 64-wide slices
-    of K form one sequence that is dealt out to the blocks in equal contiguous shares, the blocks of a tile
+def plan_stream(M: int, N: int, K: int, epilogue: Optional[str] = None, form: Optional[str] = None):
+    """``(whole tiles, cut tiles, most pieces a cut tile has, grid)`` of the persistent kernel on the current device, in the form
+    it takes for the shape (or in ``form``, one of ``FORMS``).  Tiles that would not fill a round of all SMs (a last
+    round at most half full: 2,048 x 2,560 has 160 tiles of one block for 148 SMs; or all tiles of a step with at most 128
+    rows) are cut over K: their 64-wide slices of K form one sequence that is dealt out to the blocks in equal contiguous shares, the blocks of a tile
     leave float32 partial tiles in a workspace and add them up together, in a fixed order.  Several rows of tiles
     that are fewer than the SMs (a few hundred rows) are cut when an estimate from measured times says that pays
     (option ``gemm_cut_few``)."""

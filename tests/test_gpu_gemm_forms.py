@@ -55,6 +55,32 @@ def test_products(form, M, N, K, cut):
     assert gemm_tc_status() == 0
 
 
+# a last round of few tiles; several rows of tiles in equal pieces; one row of tiles whose shares end in one tile and begin in the
+# next (of a row's tiles at least half as many as SMs, with ragged columns)
+CUT = [("one", 2048, 2560, 4096), ("pair", 2048, 2560, 4096), ("one_128", 2048, 2560, 4096), ("pair_128", 2048, 2560, 4096),
+       ("pair", 1300, 3484, 3656), ("one_128", 1024, 2560, 9728), ("pair", 8191, 520, 4096), ("one", 385, 1000, 3080), ("one_128", 385, 1000, 3080),
+       ("one", 33, 30000, 264), ("one", 17, 25000, 200), ("one_128", 33, 15000, 264), ("one_128", 17, 12544, 200)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form,M,N,K", CUT)
+def test_cut_products(form, M, N, K):
+    """These sizes are cut over K in these forms, on a GPU of 148 SMs."""
+    from synaptix_b200.ops.gemm_tc import plan_stream
+    assert plan_stream(M, N, K, "f32", form)[1] > 0 and plan_stream(M, N, K, "silu_mul", form)[1] > 0
+    test_products(form, M, N, K, True)
+
+
+@pytest.mark.gpu
+def test_plan_is_of_the_form_that_runs():
+    """Asked for no form, the plan is that of the rule's."""
+    from synaptix_b200.ops.gemm_tc import plan_stream
+    for M, N, K in ((512, 2560, 4096), (2048, 2560, 4096), (385, 1000, 3080), (100, 30000, 264), (64, 19456, 2560)):
+        for e in (None, "silu_mul"):
+            assert plan_stream(M, N, K, e) == plan_stream(M, N, K, e, None) and plan_stream(M, N, K, e) in [plan_stream(M, N, K, e, f) for f in FORMS]
+    assert plan_stream(512, 2560, 4096) == plan_stream(512, 2560, 4096, None, "pair_128") != plan_stream(512, 2560, 4096, None, "one")
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("form", FORMS)
 @pytest.mark.parametrize("M,N,K", [(130, 264, 72), (257, 520, 1032), (2048, 2560, 4096)])

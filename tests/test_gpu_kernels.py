@@ -688,7 +688,7 @@ def test_gemm_tc_tiles_cut_over_k(M, N, K, epilogue, is_cut):
     of a tile add their partial tiles up.  The result must be the product everywhere, for ragged M, N and K,
     and the same bits twice (the order of addition is fixed)."""
     from synaptix_b200.ops.gemm_tc import gemm_tc, gemm_tc_status, plan_stream
-    n_whole, n_cut, zmax, grid = plan_stream(M, N, K, epilogue)
+    n_whole, n_cut, zmax, grid = plan_stream(M, N, K, epilogue, "one")
     assert (n_cut > 0) == is_cut, "what this GPU's SM count makes of the shape"
     g = torch.Generator().manual_seed(M + N + K)
     x = torch.randn(M, K, generator=g).to(torch.bfloat16)
@@ -702,6 +702,11 @@ def test_gemm_tc_tiles_cut_over_k(M, N, K, epilogue, is_cut):
     assert torch.allclose(out.float().cpu().double(), ref, **tol)
     again = gemm_tc(x.cuda(), w.cuda(), epilogue=epilogue)
     assert torch.equal(again, out)
+    if is_cut:             # the shape may run in another form by itself: in 256-wide tiles of one block it is cut
+        one = torch.full_like(out, float("nan"))
+        gemm_tc(x.cuda(), w.cuda(), epilogue=epilogue, out=one, form="one")
+        assert torch.allclose(one.float().cpu().double(), ref, **tol)
+        assert torch.equal(gemm_tc(x.cuda(), w.cuda(), epilogue=epilogue, form="one"), one)
     whole = gemm_tc(x.cuda(), w.cuda(), epilogue=epilogue, cut=False, splits=1)
     assert torch.allclose(whole.float().cpu().double(), ref, **tol)
     assert gemm_tc_status() == 0
