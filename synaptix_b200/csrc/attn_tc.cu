@@ -794,16 +794,6 @@ static int ft_map_pages(CUtensorMap* map, const void* pages, long long n_pages, 
   return r == CUDA_SUCCESS ? 0 : 20000 + (int)r;
 }
 
-static int ft_sm_count() {
-  static int n[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (!n[dev]) {
-    if (cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n[dev] <= 0) n[dev] = 148;
-  }
-  return n[dev];
-}
-
 static int* ft_status_word() {
   static int* p = nullptr;
   if (!p) p = sx_status_word_alloc();
@@ -830,7 +820,7 @@ extern "C" int sx_attn_prefill_tc(const void* q, const void* k_pages, const void
   // Two heads a block where their blocks fill the SMs well beyond once.  Us, one head a block and two: 8,191 new tokens, 32 heads
   // 597 and 564; 2,048 tokens 57.6 and 51.6; eight prompts of 333 tokens 45.5 and 36.3; 1,500 tokens (192 pairs) 37.9 and 36.4;
   // but 1,024 tokens (128 pairs) 21.0 and 26.4: fewer blocks than SMs, and a pair's step takes 2.3 us for two tiles, not 1.27.
-  if ((nh / nkv) % 2 == 0 && 4LL * (nh / 2) * n_tiles >= 5LL * ft_sm_count()) {
+  if ((nh / nkv) % 2 == 0 && 4LL * (nh / 2) * n_tiles >= 5LL * sx_sm_count()) {
     const size_t smem = 1024 + FP_SMEM_TILES + FP_NBARS * sizeof(uint64_t) + 16 + 12 * FT_BM * sizeof(float);
     auto kern = attn_tc_prefill_pair_kernel;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

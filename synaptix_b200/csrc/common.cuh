@@ -125,6 +125,18 @@ static int g_sx_pdl = 1;
 extern "C" void sx_set_pdl(int on) { g_sx_pdl = on ? 1 : 0; }
 static inline bool sx_pdl_enabled() { return g_sx_pdl != 0; }
 
+// SMs of the current device (148 where it cannot be asked)
+static inline int sx_sm_count() {
+  static int n[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  if (!n[dev]) {
+    int v = 0;
+    n[dev] = cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0 ? v : 148;
+  }
+  return n[dev];
+}
+
 template <typename... KArgs, typename... Args>
 static inline int sx_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg = {};

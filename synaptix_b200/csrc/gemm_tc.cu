@@ -1008,16 +1008,6 @@ static int tc_launch(const CUtensorMap& ma, const CUtensorMap& mw, void* out, in
   return sx_launch(kern, grid, dim3(TC_THREADS), smem, stream, ma, mw, out, M, N, K, status, g_sx_gate);
 }
 
-static int tc_sm_count() {
-  static int n[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (!n[dev]) {
-    if (cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n[dev] <= 0) n[dev] = 148;
-  }
-  return n[dev];
-}
-
 // how many pairs of blocks are on the GPU at once (the pairs of a cut tile wait for one another)
 static int tc_pair_count() {
   static int n[64] = {0};
@@ -1132,7 +1122,7 @@ static TcHostPlan tc_plan_form(int M, int N, int K, int epi, bool allow_cut, int
   const int n_out = epi == TC_EPI_SILU_MUL ? N / 2 : N;
   const int tiles_m = (M + cg * TC_BM - 1) / (cg * TC_BM), tiles_n = (n_out + tile_n - 1) / tile_n;
   const long long n_tiles_ll = (long long)tiles_m * tiles_n;
-  const int sms = cg == 2 ? tc_pair_count() : tc_sm_count();
+  const int sms = cg == 2 ? tc_pair_count() : sx_sm_count();
   const int nkb = (K + TC_BK - 1) / TC_BK;
   TcHostPlan h;
   h.sp = 0;

@@ -421,16 +421,6 @@ static int* ws_status_word() {
   return p;
 }
 
-static int ws_sm_count() {
-  static int n[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (!n[dev]) {
-    if (cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n[dev] <= 0) n[dev] = 148;
-  }
-  return n[dev];
-}
-
 // Shared memory a block takes with a ring of `stages` (the partial tile lies over the ring), and how many blocks of
 // that size an SM holds (228 KB an SM, 1 KB of it per resident block).
 // With few rows the blocks of a cluster SEND their partial results to the block that adds a column up (a buffer of
@@ -449,7 +439,7 @@ static int ws_blocks_per_sm(int M, int nmma, int stages) {
 // The deepest ring (up to what lets two blocks share an SM) with which all `blocks` blocks are on the GPU at once;
 // 0 if there is none of at least 2 stages.  A block that has to wait for a place runs behind all the others.
 static int ws_pick_stages(int M, int nmma, long long blocks) {
-  const int sms = ws_sm_count();
+  const int sms = sx_sm_count();
   // (a partial tile of more than 100 KB leaves room for one block an SM whatever the ring: the ring may be as large)
   const size_t room = (size_t)M * 128 * 4 > 100 * 1024 ? 200 * 1024 : 100 * 1024;
   int stages = (int)(room / (WS_W_BYTES + nmma * WS_BK * 2));
@@ -466,7 +456,7 @@ static int ws_pick_stages(int M, int nmma, long long blocks) {
 // are all on the GPU at once and keep 16 slices each: most SMs would otherwise hold ONE block, whose ring of 3 or
 // 4 stages is too few bytes on the way for a loaded HBM (27.5 us with 1 block a tile and 4 stages, 23.9 with 2 and 3).
 static int ws_pick_splits(int M, int tiles, int nkb) {
-  const int sms = ws_sm_count(), want = sms * 7 / 8;
+  const int sms = sx_sm_count(), want = sms * 7 / 8;
   const int nmma = (M + 15) / 16 * 16;
   int s = 1;
   while (s < 8 && tiles * s < want && nkb / (2 * s) >= 2) s *= 2;

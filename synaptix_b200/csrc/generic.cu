@@ -447,15 +447,31 @@ static int gemm_rows_f32_launch(const float* A, const float* W, float* C, int M,
   return sx_launch(gemm_rows_f32_kernel<MR, 1>, dim3((tiles + 7) / 8), dim3(256), 0, stream, A, W, C, M, N, K, bias, cap);
 }
 
+// The tiles of more rows: rows of a tile, and blocks that share a tile's K.
+// Tiles of 64 rows only where they come to two a SM (1,024 x 6,144 x 1,024: 350 us; 263 x 4,096 x 1,024: 98 us, 78 in tiles of
+// 32 rows, which waste less of the last tile and keep more warps an SM).  About a block an SM is enough (263 x 1,024 x 3,072 in tiles
+// of 32 rows on 148 SMs: 72 blocks 127 us, 144 in clusters of two 71, 288 in clusters of four 82); every block of a cluster keeps at
+// least 128 of K.
+struct F32Plan { int rows, cluster; };
+static F32Plan gemm_f32_plan(int M, int N, int K, int sms) {
+  const long long tiles_n = (N + 127LL) / 128;
+  F32Plan p;
+  p.rows = (M + 63) / 64 * tiles_n < 2LL * sms ? 32 : 64;
+  const long long tiles = (M + p.rows - 1) / p.rows * tiles_n;
+  p.cluster = 1;
+  while (p.cluster < 8 && tiles * p.cluster < sms - sms / 18 && K >= 256 * p.cluster) p.cluster *= 2;
+  return p;
+}
+extern "C" void sx_gemm_f32_plan(int M, int N, int K, int sms, int* out2) {
+  const F32Plan p = gemm_f32_plan(M, N, K, sms);
+  out2[0] = p.rows; out2[1] = p.cluster;
+}
+
 template <int TM>
 static int gemm_tile_f32_launch(const float* A, const float* W, float* C, int M, int N, int K, const float* bias, float cap,
-                                cudaStream_t stream) {
+                                int cluster, cudaStream_t stream) {
   constexpr int BM = 8 * TM, BN = 128;
-  const long long tiles_n = (N + BN - 1) / BN, tiles_m = (M + BM - 1) / BM, tiles = tiles_n * tiles_m;
-  // About a block an SM is enough (263 x 1,024 x 3,072 in tiles of 32 rows: 72 blocks 127 us, 144 in clusters of two 71, 288 in
-  // clusters of four 82); every block of a cluster keeps at least 128 of K.
-  int cluster = 1;
-  while (cluster < 8 && tiles * cluster < 140 && K >= 256 * cluster) cluster *= 2;
+  const long long tiles_n = (N + BN - 1) / BN, tiles_m = (M + BM - 1) / BM;
   const size_t ring = (size_t)F32_STAGES * (BM + BN) * F32_ROW * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(gemm_tile_f32_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring);
   if (e != cudaSuccess) return (int)e;
@@ -470,10 +486,9 @@ static int gemm_f32(const float* A, const float* W, float* C, int M, int N, int 
   if (M <= 4) return gemm_rows_f32_launch<4>(A, W, C, M, N, K, bias, cap, stream);
   if (M <= 8) return gemm_rows_f32_launch<8>(A, W, C, M, N, K, bias, cap, stream);
   if (M <= 16) return gemm_rows_f32_launch<16>(A, W, C, M, N, K, bias, cap, stream);
-  // Tiles of 64 rows only where they come to two a SM (1,024 x 6,144 x 1,024: 350 us; 263 x 4,096 x 1,024: 98 us, 78 in tiles of
-  // 32 rows, which waste less of the last tile and keep more warps an SM).
-  if (((M + 63) / 64) * ((N + 127LL) / 128) < 296) return gemm_tile_f32_launch<4>(A, W, C, M, N, K, bias, cap, stream);
-  return gemm_tile_f32_launch<8>(A, W, C, M, N, K, bias, cap, stream);
+  const F32Plan p = gemm_f32_plan(M, N, K, sx_sm_count());
+  return p.rows == 32 ? gemm_tile_f32_launch<4>(A, W, C, M, N, K, bias, cap, p.cluster, stream)
+                      : gemm_tile_f32_launch<8>(A, W, C, M, N, K, bias, cap, p.cluster, stream);
 }
 
 template <typename TA, typename TW, typename TC>
@@ -1161,17 +1176,31 @@ __global__ void __launch_bounds__(256) attn_f32_kernel(
   }
 }
 
+// How many neighbouring tokens a block takes, and how many blocks share the keys.  Few tokens: one a block, and the keys shared by up
+// to eight blocks.  Tokens enough for every SM: as many neighbours a block as fit its rows (a cluster's blocks finish ONE token).
+struct AttnF32Plan { int tpb, cluster; };
+static AttnF32Plan attn_f32_plan(int R, int n_tokens, int nh, int nkv, int maxp, int sms) {
+  const int G = nh / nkv, hg = (G + R - 1) / R;
+  AttnF32Plan p = {1, 1};
+  const long long blocks = (long long)nkv * hg * n_tokens;
+  while (p.cluster < 8 && blocks * p.cluster < sms && maxp >= 2 * p.cluster) p.cluster *= 2;
+  if (p.cluster == 1 && G < R && R % G == 0 && blocks >= (long long)sms * (R / G)) p.tpb = R / G;
+  return p;
+}
+// (rows a block: two query heads a kv head or fewer, two; else four)
+static int attn_f32_rows(int nh, int nkv) { return nh / nkv <= 2 ? 2 : 4; }
+extern "C" void sx_attn_f32_plan(int n_tokens, int nh, int nkv, int maxp, int sms, int* out2) {
+  const AttnF32Plan p = attn_f32_plan(attn_f32_rows(nh, nkv), n_tokens, nh, nkv, maxp, sms);
+  out2[0] = p.tpb; out2[1] = p.cluster;
+}
+
 template <int HD, int R>
 static int attn_f32_launch(const float* q, const float* k, const float* v, float* out, const int* positions, const int* seq_of_token,
                            const int* block_table, int maxp, int n_tokens, int nh, int nkv, float scale, int window, float softcap,
                            const float* sinks, int chunk, int out_stride, float out_scale, cudaStream_t stream) {
   const int G = nh / nkv, hg = (G + R - 1) / R;
-  // Few tokens: one a block, and the keys shared by up to eight blocks.  Tokens enough for every SM: as many neighbours a block as
-  // fit its rows (a cluster's blocks finish ONE token).
-  int tpb = 1, cluster = 1;
-  const long long blocks = (long long)nkv * hg * n_tokens;
-  while (cluster < 8 && blocks * cluster < 148 && maxp >= 2 * cluster) cluster *= 2;
-  if (cluster == 1 && G < R && R % G == 0 && blocks >= 148 * (R / G)) tpb = R / G;
+  const AttnF32Plan plan = attn_f32_plan(R, n_tokens, nh, nkv, maxp, sx_sm_count());
+  const int tpb = plan.tpb, cluster = plan.cluster;
   const dim3 grid((unsigned)cluster, (unsigned)(nkv * hg), (unsigned)((n_tokens + tpb - 1) / tpb));
   if (cluster > 1)
     return sx_launch_cluster(attn_f32_kernel<HD, R>, grid, dim3(256), 0, stream, cluster, q, k, v, out, positions, seq_of_token, block_table,
@@ -1193,7 +1222,7 @@ static int attn_generic_any(const void* q, const void* k_pages, const void* v_pa
 #define ATTN_F32(HD, R) attn_f32_launch<HD, R>((const float*)q, (const float*)k_pages, (const float*)v_pages, (float*)out, positions, \
                                                seq_of_token, block_table, maxp, n_tokens, nh, nkv, scale, window, softcap, sinks, chunk, \
                                                out_stride, out_scale, stream)
-    if (nh / nkv <= 2) return hd == 64 ? ATTN_F32(64, 2) : ATTN_F32(128, 2);
+    if (attn_f32_rows(nh, nkv) == 2) return hd == 64 ? ATTN_F32(64, 2) : ATTN_F32(128, 2);
     return hd == 64 ? ATTN_F32(64, 4) : ATTN_F32(128, 4);
 #undef ATTN_F32
   }

@@ -259,16 +259,6 @@ extern "C" int sx_moe_gather(const void* x, const int* order, void* xs, int rows
   return sx_launch(moe_gather_kernel, dim3(rows), dim3(128), 0, stream, (const bf16*)x, order, (bf16*)xs, K, top);
 }
 
-static int mt_sm_count() {
-  static int n[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (!n[dev]) {
-    if (cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n[dev] <= 0) n[dev] = 148;
-  }
-  return n[dev];
-}
-
 static int* mt_status_word() {
   static int* w = nullptr;
   if (!w) w = sx_status_word_alloc();
@@ -306,7 +296,7 @@ extern "C" int sx_moe_tc(const void* A, const void* Wt, void* out, const int* of
     if (err != cudaSuccess) return (int)err;                                                                                      \
     const long long all = tiles * ((N + COLS - 1) / COLS);                                                                        \
     if (all > 0x3fffffffLL) return SX_ERR_SIZE;                                                                                   \
-    return sx_launch(moe_tc_kernel<M>, dim3((unsigned)(all < mt_sm_count() ? all : mt_sm_count())), dim3(MT_THREADS), smem,       \
+    return sx_launch(moe_tc_kernel<M>, dim3((unsigned)(all < sx_sm_count() ? all : sx_sm_count())), dim3(MT_THREADS), smem,       \
                      stream, ma, mw, out, offsets, E, N, K, status, g_sx_gate);                                                   \
   } while (0)
   if (mode == MT_GATE_UP) MT_GO(MT_GATE_UP, (MT_BN / 2));

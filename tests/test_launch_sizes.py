@@ -22,3 +22,32 @@ def test_streamed_experts(rows, E, N):
     blocks.restype = ctypes.c_longlong
     for mode, tile in ((MODE_GATE_UP, 8), (MODE_PLAIN, 16)):
         assert blocks(rows, E, N, mode) == min(E, rows) * ((N + tile - 1) // tile)
+
+
+def plan(lib, name, *args):
+    out = (ctypes.c_int * 2)()
+    f = getattr(library(lib), name)
+    f.restype = None
+    f(*args, out)
+    return tuple(out)
+
+
+@pytest.mark.parametrize("sms", [74, 108, 148, 160, 296])
+def test_float32_launches_follow_the_sms(sms):
+    """Float32 products: 64-row tiles from two a SM on; else blocks that share a tile's K until there is about one a SM.  Float32
+    attention: blocks that share a token's keys until there is one a SM."""
+    for M, N, K in ((17, 1024, 4096), (263, 1024, 3072), (263, 4096, 1024), (1024, 6144, 1024), (600, 2048, 300), (9000, 2048, 64)):
+        rows, cluster = plan("generic", "sx_gemm_f32_plan", M, N, K, sms)
+        columns = -(-N // 128)
+        assert rows == (64 if -(-M // 64) * columns >= 2 * sms else 32)
+        tiles, few = -(-M // rows) * columns, sms - sms // 18
+        assert cluster in (1, 2, 4, 8) and (cluster == 1 or (tiles * cluster // 2 < few and K >= 128 * cluster))
+        assert cluster == 8 or tiles * cluster >= few or K < 256 * cluster
+    for n, nh, nkv, pages in ((1, 16, 8, 40), (2, 16, 8, 3), (20, 16, 8, 64), (263, 16, 8, 5), (40, 4, 4, 9), (9, 32, 4, 64), (400, 8, 8, 8)):
+        tokens, cluster = plan("generic", "sx_attn_f32_plan", n, nh, nkv, pages, sms)
+        heads = nh // nkv
+        rows = 2 if heads <= 2 else 4
+        blocks = nkv * -(-heads // rows) * n
+        assert cluster == 8 or blocks * cluster >= sms or pages < 2 * cluster
+        assert cluster == 1 or (blocks * cluster // 2 < sms and tokens == 1)
+        assert tokens == (rows // heads if cluster == 1 and heads < rows and blocks >= sms * (rows // heads) else 1)
