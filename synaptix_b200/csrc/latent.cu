@@ -438,13 +438,15 @@ static int latent_attn_any(const float* qa, const void* k_pages, const int* posi
 #define LM_SP (LM_KEYS + 4)        // floats between two heads' partial scores
 #define LM_PP (LM_KEYS + 8)        // elements between two heads' weights
 
+// the upper halves of x and y, of what is left of them, and of what is left then: eight bits of the significand each time, cut and
+// not rounded, so that the largest floats stay finite
 __device__ __forceinline__ void lm_split3(float x, float y, uint32_t (&p)[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const __nv_bfloat162 b = __floats2bfloat162_rn(x, y);
-    p[i] = *reinterpret_cast<const uint32_t*>(&b);
-    x -= __low2float(b);
-    y -= __high2float(b);
+    const uint32_t bx = __float_as_uint(x), by = __float_as_uint(y);
+    p[i] = __byte_perm(bx, by, 0x7632);
+    x -= __uint_as_float(bx & 0xffff0000u);
+    y -= __uint_as_float(by & 0xffff0000u);
   }
 }
 __device__ __forceinline__ void lm_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {

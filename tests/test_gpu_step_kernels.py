@@ -65,6 +65,25 @@ def test_latent_attention(H, R, Dr, lens, window, parts, cluster):
         assert (got[s] - want).abs().max() <= (2 * off + (n + 32) * ULP) * float(k.abs().max())
 
 
+def test_latent_attention_of_the_largest_floats():
+    """Queries between the largest bfloat16 and the largest float32, against cache elements so small that the scores are ordinary."""
+    from synaptix_b200 import ops
+    H, R, Dr, n, scale = 3, 32, 16, 100, 0.25
+    E, g = R + Dr, torch.Generator().manual_seed(0)
+    pages, table, rows, maxp = latent_cache([n], E, 0)
+    small = ((0.5 + torch.rand(n, generator=g)) * torch.randn(n, generator=g).sign() * 2.0 ** -124).to(torch.bfloat16)
+    rows[0][:, 5] = small.double()
+    for p in range(maxp):
+        part = small[p * 64:(p + 1) * 64]
+        pages[table[0, p], 0, :len(part), 5] = part.cuda()
+    qa = torch.zeros(1, H, E)
+    qa[0, :, 5] = torch.tensor([3.4e38, -3.4028234e38, 3.3961e38])
+    got = ops.latent_attention(qa.cuda(), pages, Step([n - 1], maxp), table, H, R, Dr, scale, None).merged().double().cpu()[0]
+    z = qa[0].double() @ rows[0].T * scale                  # one product a score
+    want = torch.softmax(z, -1) @ rows[0][:, :R]
+    assert ((got - want).abs() <= (4 * float(z.abs().max()) + n + 32) * ULP * float(rows[0].abs().max())).all()
+
+
 @pytest.mark.parametrize("T,H,D,Dr,R", [(1, 1, 1, 0, 2), (3, 2, 16, 8, 126), (8, 3, 65, 4, 128), (9, 2, 64, 16, 320), (8, 1, 130, 0, 130)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_latent_query(T, H, D, Dr, R, dtype):
