@@ -28,7 +28,7 @@ from .. import ops
 from ..parts.base import Norm, NormedDelta, Part, PendingLinear, Runtime, StepContext, plain, to_device_f32
 from ..parts.embedding import Embedding, OutputHead
 from ..weights.loader import TensorSpec, WeightSource, bind_tensors
-from .repeat import MIN_LAYERS, form_of, repeat
+from .repeat import form_of, places_of_like, repeat
 
 
 @dataclasses.dataclass(frozen=True)
@@ -128,18 +128,10 @@ class DecoderModel(Part):
         self.runtime = rt
         return self
 
-    def _same_as_before(self, k: int, forms: dict) -> bool:
-        """Whether run ``k`` is the one before it again, on another layer of the same form; both with keys of their own.
-        ``forms``: those of the step's layers that were asked for."""
-        if not 0 < k < len(self.steps):
-            return False
-        a, b = self.steps[k - 1], self.steps[k]
-        if not (isinstance(a, LayerRun) and isinstance(b, LayerRun) and a.write_cache and b.write_cache) or a.layer == b.layer:
-            return False
-        for n in (a.layer, b.layer):
-            if n not in forms:
-                forms[n] = form_of(self.layers[n])
-        return forms[a.layer] is not None and forms[b.layer] is not None and forms[a.layer][0] == forms[b.layer][0]
+    def _may_be_like(self, k: int) -> bool:
+        """Whether run ``k`` may be the one before it again: other layers, both with keys of their own."""
+        a, b = (self.steps[j] if 0 <= j < len(self.steps) else None for j in (k - 1, k))
+        return isinstance(a, LayerRun) and isinstance(b, LayerRun) and a.write_cache and b.write_cache and a.layer != b.layer
 
     # -- one step ------------------------------------------------------------
     def forward(self, ctx: StepContext, cache) -> torch.Tensor:
@@ -150,7 +142,6 @@ class DecoderModel(Part):
         observe = getattr(ctx, "observe", None)
         n_run = 0
         may_repeat = observe is None and not ctx.all_single and ctx.host is not None and ops.OPTIONS.repeat_layers
-        forms: dict = {}                         # layer: its form and where its tensors lie (see repeat.py)
         i = 0
         while i < len(self.steps):
             run = self.steps[i]
@@ -167,22 +158,22 @@ class DecoderModel(Part):
                 continue
             if isinstance(pending, PendingLinear) and not getattr(self.layers[run.layer], "takes_pending_product", False):
                 pending = pending.materialize()
-            if may_repeat and type(pending) is PendingLinear and self._same_as_before(i - 1, forms):
+            if may_repeat and type(pending) is PendingLinear and self._may_be_like(i - 1):
                 before, h_before = pending, h
                 with ops.recording() as launched:
                     h, pending = self.layers[run.layer].forward(h, before, ctx, cache.view(run.cache_entry), run.write_cache)
-                may_repeat = launched.whole and h is h_before          # (else the layers like it are no different)
-                del forms[run.layer]             # a part may have made something of its own when it ran
-                end = i - 1
-                while may_repeat and self._same_as_before(end, forms):
-                    end += 1
-                if end - (i - 2) >= MIN_LAYERS:
-                    runs = self.steps[i - 2:end]
-                    done = repeat(launched, before, pending, [forms[r.layer][1] for r in runs],
-                                  [cache.view(r.cache_entry) for r in runs])
-                    may_repeat = done is not None
-                    if may_repeat:
-                        pending, i = done, end
+                if launched.whole and h is h_before and self._may_be_like(i):
+                    views = [cache.view(self.steps[i - 2].cache_entry), cache.view(run.cache_entry)]
+                    while self._may_be_like(i - 2 + len(views)):
+                        view = cache.view(self.steps[i - 2 + len(views)].cache_entry)
+                        if view.group != views[1].group or view.window != views[1].window:
+                            break
+                        views.append(view)
+                    form = form_of(self.layers[run.layer])
+                    layers = (self.layers[r.layer] for r in self.steps[i - 2:i - 2 + len(views)])
+                    done = None if form is None else repeat(launched, before, pending, places_of_like(layers, form[0]), views)
+                    if done is not None:
+                        pending, i = done, i + launched.repeats
                 continue
             h, pending = self.layers[run.layer].forward(h, pending, ctx, cache.view(run.cache_entry), run.write_cache)
             if observe is not None:              # the stream after this run: h with the branch not yet added

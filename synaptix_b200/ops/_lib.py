@@ -102,6 +102,7 @@ class Recording:
         self.calls, self.keep = [], []
         self.gated: Optional[str] = None
         self.checked, self.plain = 0, True
+        self.repeats = 0                   # how often all of it was launched again
 
     @property
     def whole(self) -> bool:

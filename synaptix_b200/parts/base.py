@@ -289,7 +289,7 @@ class Part:
     """Anything that owns tensors."""
 
     graph_safe = True      # False: forward depends on host values of the step (no CUDA graph)
-    name_attributes = ()   # of a repeatable part: attributes that hold names of tensors (strings, or lists or dicts with them)
+    name_attributes = ()   # of a repeatable part: attributes with names of tensors, and what else counts only while tensors are bound
     shared_attributes = () # of a repeatable part: attributes with tensors that a step makes something of (once for all layers with that tensor)
 
     def tensor_specs(self) -> Dict[str, TensorSpec]:
