@@ -211,3 +211,37 @@ def test_weighted_sum_of_experts(T, W, top, y_dtype, out_dtype):
     want = (rows * w.double()[..., None]).sum(1)
     bound = (top + 1) * ULP * (rows.abs() * w.double()[..., None]).sum(1) + (BF16 if out_dtype == torch.bfloat16 else 0) * want.abs() + 1e-30
     assert ((got - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("dim,rot,vdim", [(96, 32, 128), (48, 16, 64), (24, 8, 32)])
+@pytest.mark.parametrize("window", [None, 70])
+@pytest.mark.parametrize("lens", [[300], [1, 64, 65, 127, 129], [256]])
+def test_prompts_whose_pages_held_anything(dim, rot, vdim, window, lens, monkeypatch):
+    """Whole prompts through keys and values a head, whose pages are made for the step: what the memory held before (NaN, and every
+    other tensor that is made begins so, too) makes no difference to what zeros give."""
+    from synaptix_b200.cache.store import KVView
+    from synaptix_b200.parts import LatentAttention, RotaryPairs, Runtime
+    from test_gpu_vemedra import step_ctx
+    g, bf = torch.Generator().manual_seed(dim), torch.bfloat16
+    W, H, rq, rk, p = 64, 3, 32, 40, "m."
+    sizes = {"dq": (rq, W), "uq": (H * (dim + rot), rq), "dkv": (rk + rot, W), "uk": (H * dim, rk), "uv": (H * vdim, rk), "o": (W, H * vdim)}
+    w = {p + n: (torch.randn(*s, generator=g) * s[1] ** -0.5).to(bf) for n, s in sizes.items()}
+    w[p + "dq.norm"], w[p + "dkv.norm"] = torch.ones(rq), torch.ones(rk)
+    part = LatentAttention(p, W, H, dim, rot, vdim, rq, rk, scale=0.3, norm_eps=1e-5, window=window, position=RotaryPairs(rot, 800.0), gated=False)
+    part.bind_all(w, Runtime(torch.device("cuda:0"), bf))
+    x = torch.randn(sum(lens), W, generator=g).to(bf).cuda()
+    maxp = max((n + 63) // 64 for n in lens)
+    table = (torch.arange(len(lens) * maxp, dtype=torch.int32) + 1).view(len(lens), maxp).cuda()
+    ctx = step_ctx([0] * len(lens), lens, list(range(len(lens))), [table], bf)
+    assert part._whole_prompts(ctx)
+    real, got = torch.empty, []
+    for value in (0.0, float("nan")):
+        def filled(*args, **kw):
+            t = real(*args, **kw)
+            return t.fill_(value) if t.is_floating_point() else t
+        monkeypatch.setattr(torch, "empty", filled)
+        ctx.scratch.clear()
+        pages = torch.full((len(lens) * maxp + 1, 1, 64, rk + rot), value, dtype=bf, device="cuda")
+        got.append(part.forward(x, ctx, KVView(pages, None, 0, window)))
+        monkeypatch.setattr(torch, "empty", real)
+    assert torch.isfinite(got[0]).all() and torch.equal(got[0], got[1])

@@ -307,3 +307,63 @@ def test_same_bits(more, dtype):
     for lens in ([2], [17], [100, 33], [161], [300, 5, 260], [1000]):
         (a, n), (b, m) = run(False, lens), run(True, lens)
         assert n == m and all(torch.equal(x, y) for x, y in zip(a, b)), lens
+
+
+def attention_with_everything(old, i):
+    """A layer's attention again, with biases, sinks and a rotation of a quarter of each head."""
+    from synaptix_b200.parts import Attention, RotaryHalf
+    return Attention(old.prefix, old.width, old.nh, old.nkv, old.hd, position=RotaryHalf(old.hd, 10000.0, old.hd // 4),
+                     qk_norm_eps=old.qk_norm_eps, window=old.window, bias_suffix=".b", sinks=True)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,dtype,repeats", [("plain", "bf16", True), ("windows", "bf16", True), ("everything", "bf16", True),
+                                                ("heads of 64", "bf16", False), ("plain", "f32", False)])
+def test_which_steps_repeat(kind, dtype, repeats, monkeypatch):
+    """Prompt steps of bfloat16 layers with heads of 128 make the launches again (and give the bits of a walk); where an operation
+    does not note its launches every layer is walked.  A model that is loaded anew runs with its new weights."""
+    from synaptix_b200 import ops
+    from synaptix_b200.api import LLM
+    from synaptix_b200.engine import Entry
+    from synaptix_b200.models import decoder
+    from synaptix_b200.parts import Runtime, SwiGLU
+    from synaptix_b200.weights import RandomSource
+    model = skeleton(**{"heads of 64": dict(head_dim=64), "windows": dict(use_sliding_window=True, sliding_window=64, max_window_layers=0)}.get(kind, {}))
+    if kind == "everything":
+        for i, layer in enumerate(model.layers):
+            layer.mixer = attention_with_everything(layer.mixer, i)
+            layer.ffn = SwiGLU("model.layers.%d.mlp." % i, 256, 320, bias_suffix=".b")
+    made = []
+
+    def noted(*args):
+        done = repeat(*args)
+        made.append(done is not None)
+        return done
+    monkeypatch.setattr(decoder, "repeat", noted)
+
+    def load(seed):
+        model.load(RandomSource(model.all_tensor_specs(), seed=seed, device="cuda:0"),
+                   Runtime(torch.device("cuda:0"), torch.bfloat16 if dtype == "bf16" else torch.float32))
+    load(1)
+    engine = LLM.from_model(model, max_tokens=4096, max_batch=8).engine
+
+    def run(on, lens):
+        del made[:]
+        with ops.options(repeat_layers=on):
+            slots = [engine.open() for _ in lens]
+            out = [engine.step([Entry(s, tiny.random_tokens(997, n, n), [0, n - 1]) for s, n in zip(slots, lens)]) for _ in range(1)]
+            for s in slots:
+                engine.close(s)
+        return out, sum(made)
+    run(True, [300])                  # what a part makes of its own when it first runs is made
+    first = None
+    for seed in (1, 2):
+        if seed == 2:
+            load(2)
+            run(True, [300])
+        for lens in ([161], [300, 5, 260], [1000]):
+            (a, none), (b, n) = run(False, lens), run(True, lens)
+            assert none == 0 and n == (1 if repeats else 0), lens
+            assert all(torch.equal(x, y) for x, y in zip(a, b)) and all(torch.isfinite(x).all() for x in a), lens
+        assert first is None or not torch.equal(first, a[0])
+        first = a[0]
