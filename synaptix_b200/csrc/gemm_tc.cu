@@ -1184,8 +1184,11 @@ static double tc_plan_time(const TcHostPlan& h, int K) {
   return t;
 }
 
-// form 0: the one that takes the least time by that estimate (of 48 products of 300 to 8,191 rows that was the fastest measured form,
-// or within 4% of it, in all but one: 24 tiles x 3 pieces of 300 x 2,048 -> 1,024, 10.8 against 10.0 us); 1 and 2: tiles 256 wide, of one block or of a pair; 3 and 4: 128 wide
+// form 0: the one that takes the least time by that estimate (of 48 plain products of 300 to 8,191 rows that was the fastest measured
+// form, or within 4% of it, in all but one: 24 tiles x 3 pieces of 300 x 2,048 -> 1,024, 10.8 against 10.0 us); 1 and 2: tiles 256
+// wide, of one block or of a pair; 3 and 4: 128 wide.  The q/k/v products' head preparation is a longer epilogue than the estimate
+// knows: of 24 of them (161 to 8,191 rows; 2,560 -> 6,144, 2,048 -> 4,096, 1,024 -> 4,096) the choice was the fastest form or
+// within 5% of it in 20, and 8 to 12% off in four of 161 to 611 rows (2,048 -> 4,096 at 611 rows 28.7 us, 26.6 in 128-wide tiles).
 static TcHostPlan tc_plan_stream(int M, int N, int K, int epi, bool allow_cut, int form) {
   if (form) return tc_plan_form(M, N, K, epi, allow_cut, form > 2 ? 128 : 256, 2 - (form & 1));
   TcHostPlan best = tc_plan_form(M, N, K, epi, allow_cut, 256, 1);
@@ -1338,7 +1341,7 @@ extern "C" int sx_gemm_tc(const void* A, const void* W, void* out, int M, int N,
 
 // The fused q/k/v projection of a prompt step with its head preparation as the epilogue (see TcQkv): A [M, K], W [N, K] with
 // N = (nh + 2 nkv) * 128 (or nh * 128: query heads alone, of a layer that reads another layer's cache) a multiple of 256;
-// form: as splits of sx_gemm_tc (0: the rule's); bias [N] (null: none); q_out [M, nh * 128]; k_pages / v_pages [n_pages, nkv, 64, 128] (null: nothing is
+// form: 0 for the rule's, 1 to 4 as tc_plan_stream has them; bias [N] (null: none); q_out [M, nh * 128]; k_pages / v_pages [n_pages, nkv, 64, 128] (null: nothing is
 // written to the cache); wq / wk [128] (null: no norm); cs / sn [M, 64] (null: no rotation).  All tiles are computed whole.
 extern "C" int sx_gemm_tc_qkv(const void* A, const void* W, const float* bias, int M, int N, int K, void* q_out, void* k_pages, void* v_pages,
                               const float* wq, const float* wk, const float* cs, const float* sn, const int* positions,
