@@ -1083,7 +1083,8 @@ __global__ void __launch_bounds__(256) attn_f32_kernel(
         if (softcap > 0.f) s[r] = softcap * tanhf(s[r] / softcap);
         if (j > pos[r] || j < lo[r]) continue;
         const float m_new = fmaxf(m[r], s[r]);
-        const float corr = m[r] == -INFINITY ? 0.f : expf(m[r] - m_new), p = expf(s[r] - m_new);
+        // (a score of minus infinity has no weight, also where a group has seen no other yet)
+        const float corr = m[r] == -INFINITY ? 0.f : expf(m[r] - m_new), p = s[r] == -INFINITY ? 0.f : expf(s[r] - m_new);
         m[r] = m_new;
         l[r] = fmaf(l[r], corr, p);
 #pragma unroll

@@ -86,3 +86,37 @@ def test_attention(nh, nkv, hd, past, new, options):
     bound = (2 * off + (max(p + n for p, n in zip(past, new)) + 16) * ULP) * max(float(v.abs().max()) for v in vs)
     assert (out[:, 4:4 + nh * hd].double().cpu() - want).abs().max() <= bound
     assert (out[:, :4] == 3.0).all() and (out[:, 4 + nh * hd:] == 3.0).all()
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 64), (8, 2, 128)])
+@pytest.mark.parametrize("new", [[1], [1, 1], [200]])
+@pytest.mark.parametrize("far", ["first", "most"])
+def test_attention_with_scores_of_minus_infinity(nh, nkv, hd, new, far):
+    """Keys whose scores overflow to minus infinity have no weight: what the others give is what there would be without them."""
+    from synaptix_b200 import ops
+    torch.manual_seed(nh)
+    n = 300
+    ks, vs = [torch.randn(n, nkv, hd) for _ in new], [torch.randn(n, nkv, hd) for _ in new]
+    gone = [j for j in range(n) if (j < 40 if far == "first" else j % 33 != 0)]
+    q = torch.randn(sum(new), nh, hd)
+    q[..., 3] = 1e20
+    for k in ks:
+        k[:, :, 3] = 0.0
+        k[gone, :, 3] = -1e20
+    kp, vp, bt = make_paged(ks, vs, nkv, hd, torch.float32, seed=2)
+    pos = torch.cat([torch.arange(n - m, n) for m in new]).to(torch.int32)
+    sot = torch.cat([torch.full((m,), i) for i, m in enumerate(new)]).to(torch.int32)
+    scale = 1 / math.sqrt(hd)
+    out = torch.empty(sum(new), nh * hd, device="cuda")
+    ops.attn_generic(dev(q.view(-1, nh * hd)), kp, vp, dev(pos), dev(sot), bt, nh, nkv, hd, scale, None, out)
+    kept = [j for j in range(n) if j not in gone]
+    q[..., 3] = 0.0                                  # (as the kept keys' element)
+    want = torch.empty(sum(new), nh, hd, dtype=torch.float64)
+    for t in range(sum(new)):
+        seen = [j for j in kept if j <= int(pos[t])]
+        k, v = ks[int(sot[t])][seen].double(), vs[int(sot[t])][seen].double()
+        for h in range(nh):
+            want[t, h] = torch.softmax(k[:, h // (nh // nkv)] @ q[t, h].double() * scale, 0) @ v[:, h // (nh // nkv)]
+    off = (hd + 4) * ULP * float(q.norm(dim=-1).max()) * max(float(k[kept].norm(dim=-1).max()) for k in ks) * scale
+    bound = (2 * off + (n + 16) * ULP) * max(float(v.abs().max()) for v in vs)
+    assert (out.double().cpu() - want.view(-1, nh * hd)).abs().max() <= bound
