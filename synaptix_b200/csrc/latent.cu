@@ -575,13 +575,26 @@ __global__ void __launch_bounds__(256) latent_attn_mma_kernel(
       }
       const int j = tile * LM_KEYS + kq * 2;
       const bool ok0 = j >= lo && j <= pos, ok1 = j + 1 >= lo && j + 1 <= pos;
+      // An infinite cache element times a piece that is zero is no number, and one piece's products may overflow to the other sign
+      // before the largest piece's are added: a score that is not finite is formed again as one sum of whole products.
+      if (!(fabsf(s0) < INFINITY && fabsf(s1) < INFINITY) && h0 + row < H) {
+        const float* qr = qa + ((size_t)t * H + h0 + row) * E;
+        const bf16* kr = kt + kq * 2 * LD;
+        s0 = s1 = 0.f;
+#pragma unroll 1
+        for (int e = 0; e < E; ++e) {
+          s0 = fmaf(qr[e], __bfloat162float(kr[e]), s0);
+          s1 = fmaf(qr[e], __bfloat162float(kr[LD + e]), s1);
+        }
+      }
       s0 = ok0 ? s0 * scale : -INFINITY;
       s1 = ok1 ? s1 * scale : -INFINITY;
       float mx = fmaxf(s0, s1);
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
       const float m_new = fmaxf(m, mx);
-      const float p0 = ok0 ? expf(s0 - m_new) : 0.f, p1 = ok1 ? expf(s1 - m_new) : 0.f;
+      // (a score of minus infinity has no weight, also where there has been no other yet)
+      const float p0 = s0 == -INFINITY ? 0.f : expf(s0 - m_new), p1 = s1 == -INFINITY ? 0.f : expf(s1 - m_new);
       const float corr = m == -INFINITY ? 0.f : expf(m - m_new);
       float sum = p0 + p1;
 #pragma unroll

@@ -84,6 +84,29 @@ def test_latent_attention_of_the_largest_floats():
     assert ((got - want).abs() <= (4 * float(z.abs().max()) + n + 32) * ULP * float(rows[0].abs().max())).all()
 
 
+@pytest.mark.parametrize("n,window", [(100, None), (100, 69), (1000, None), (1000, 650)])
+@pytest.mark.parametrize("far,q", [(-float("inf"), [1.0, 0.3, 7.0]), (-2.0 ** 127, [3.3e38, 1e38, 2.9e38])])
+def test_latent_scores_of_minus_infinity(n, window, far, q):
+    """Keys whose scores are minus infinity, by an infinite rotated element or by overflow, have no weight."""
+    from synaptix_b200 import ops
+    H, R, Dr, scale = 3, 32, 16, 0.25
+    pages, table, rows, maxp = latent_cache([n], R + Dr, n)
+    gone = torch.zeros(n, dtype=torch.bool)
+    gone[n - (window or n):][:9], gone[::3] = True, True
+    k, at = rows[0], torch.where(gone, far, 0.0)
+    k[:, R + 5] = 0.0
+    for p in range(maxp):
+        pages[table[0, p], 0, :len(at[p * 64:(p + 1) * 64]), R + 5] = at[p * 64:(p + 1) * 64].to(torch.bfloat16).cuda()
+    qa = torch.randn(1, H, R + Dr, generator=torch.Generator().manual_seed(2))
+    z = qa[0].double()
+    qa[0, :, R + 5] = torch.tensor(q)
+    got = ops.latent_attention(qa.cuda(), pages, Step([n - 1], maxp), table, H, R, Dr, scale, window).merged().double().cpu()[0]
+    k = k[n - (window or n):][~gone[n - (window or n):]]
+    want = torch.softmax(z @ k.T * scale, -1) @ k[:, :R]
+    off = (R + Dr + 8) * ULP * float(z.norm(dim=-1).max()) * float(k.norm(dim=-1).max()) * scale
+    assert (got - want).abs().max() <= (2 * off + (n + 32) * ULP) * float(k.abs().max())
+
+
 @pytest.mark.parametrize("T,H,D,Dr,R", [(1, 1, 1, 0, 2), (3, 2, 16, 8, 126), (8, 3, 65, 4, 128), (9, 2, 64, 16, 320), (8, 1, 130, 0, 130)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_latent_query(T, H, D, Dr, R, dtype):
