@@ -58,6 +58,7 @@ LIBRARIES: Dict[str, tuple] = {
     "attn_tc": ("attn_tc.cu", []),
     "gemm_tc": ("gemm_tc.cu", []),
     "gemm_ws": ("gemm_ws.cu", []),
+    "layers": ("layers.cu", []),
 }
 
 

@@ -29,6 +29,7 @@ from ..parts.base import Norm, NormedDelta, Part, PendingLinear, Runtime, StepCo
 from ..parts.embedding import Embedding, OutputHead
 from ..weights.loader import TensorSpec, WeightSource, bind_tensors
 from .repeat import form_of, places_of_like, repeat
+from .whole import run_layers
 
 
 @dataclasses.dataclass(frozen=True)
@@ -133,6 +134,12 @@ class DecoderModel(Part):
         a, b = (self.steps[j] if 0 <= j < len(self.steps) else None for j in (k - 1, k))
         return isinstance(a, LayerRun) and isinstance(b, LayerRun) and a.write_cache and b.write_cache and a.layer != b.layer
 
+    @property
+    def runs_each_layer_once(self) -> bool:
+        """Whether a step is nothing but its layers, each once, each on keys of its own."""
+        return (all(isinstance(r, LayerRun) and r.write_cache for r in self.steps) and self._embedding_entry is None
+                and len({r.layer for r in self.steps}) == len(self.steps) > 0)
+
     # -- one step ------------------------------------------------------------
     def forward(self, ctx: StepContext, cache) -> torch.Tensor:
         """Logits float32 ``[n_want, vocab]`` for ``ctx.want_rows``."""
@@ -143,6 +150,8 @@ class DecoderModel(Part):
         n_run = 0
         may_repeat = observe is None and not ctx.all_single and ctx.host is not None and ops.OPTIONS.repeat_layers
         i = 0
+        if observe is None and ctx.all_single and run_layers(self, h, ctx, cache):
+            i = len(self.steps)
         while i < len(self.steps):
             run = self.steps[i]
             i += 1

@@ -19,6 +19,7 @@ from .attention import (TC_TILE_ROWS, attn_decode, attn_decode_ex, attn_decode_p
 from .decode import MAX_ROWS as SKINNY_MAX_ROWS, skinny_gemm, skinny_gemm_resid_tanh, skinny_gemm_residual, skinny_gemm_scaled, skinny_supported
 from .gemm_tc import gemm_tc, gemm_tc_qkv, gemm_tc_resid_tanh, qkv_epilogue_supported, tc_supported
 from .gemm_ws import gemm_ws, gemm_ws_resid_tanh, gemm_ws_residual, ws_supported
+from .layers import MAX_ROWS as DECODE_LAYERS_MAX_ROWS, decode_layers, decode_layers_words
 from .options import OPTIONS, KernelOptions, options, set_options
 from .generic import (add_rmsnorm, attn_generic, decode_advance, decode_begin, embed_gather, gemm_generic, qkv_prepare,
                       residual_add, rope_table, silu_mul)
@@ -42,14 +43,15 @@ __all__ = ["OPTIONS", "KernelOptions", "options", "set_options", "KernelsUnavail
            "add_rmsnorm_conv", "capped_glu", "mingru", "retention", "stream_add", "gate_activation",
            "add_normed", "WeightedRows", "embed_bigram", "convqk_prepare", "sigmoid_gate", "add_scaled", "add_scaled_rmsnorm", "scale_rows", "add_layernorm", "attn_scored", "heads_prepare", "latent_attention", "latent_output", "latent_prepare",
            "latent_query", "latent_gather", "latent_expand", "latent_rotate_q", "head_gate", "mlstm", "ExpertPlan", "moe_combine", "moe_down", "moe_gate_up", "moe_route", "moe_sort", "moe_up",
-           "add_dyn_tanh", "linear_into_dyn_tanh", "late_launch", "recording", "side_gate", "DeltaWeights", "delta_rule", "delta_step_fits"]
+           "add_dyn_tanh", "linear_into_dyn_tanh", "late_launch", "recording", "side_gate", "decode_layers", "decode_layers_words", "DECODE_LAYERS_MAX_ROWS", "DeltaWeights", "delta_rule", "delta_step_fits"]
 
 
 _STATUS_READERS = {"gemm_tc": ("the tcgen05 matrix product (gemm_tc)", "gemm_tc_status"),
                    "attn_tc": ("the tcgen05 prompt attention (attn_tc)", "attn_tc_status"),
                    "attn_decode": ("the TMA-fed decode attention (attn_decode)", "attn_decode_status"),
                    "gemm_ws": ("the weight-streaming tcgen05 product (gemm_ws)", "gemm_ws_status"),
-                   "moe_tc": ("the experts' grouped tcgen05 product (moe_tc)", "moe_tc_status")}
+                   "moe_tc": ("the experts' grouped tcgen05 product (moe_tc)", "moe_tc_status"),
+                   "layers": ("the layers of a single-token step in one kernel (layers)", "decode_layers_status")}
 
 
 def check_status(readers=None) -> None:
@@ -64,9 +66,10 @@ def check_status(readers=None) -> None:
         from .attention import attn_decode_status, attn_tc_status
         from .gemm_tc import gemm_tc_status
         from .gemm_ws import gemm_ws_status
+        from .layers import decode_layers_status
         from .moe import moe_tc_status
         fns = {"moe_tc_status": moe_tc_status, "gemm_tc_status": gemm_tc_status, "attn_tc_status": attn_tc_status, "attn_decode_status": attn_decode_status,
-               "gemm_ws_status": gemm_ws_status}
+               "gemm_ws_status": gemm_ws_status, "decode_layers_status": decode_layers_status}
         readers = {}
         for lib, (what, fname) in _STATUS_READERS.items():
             if loaded(lib):

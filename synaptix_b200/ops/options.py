@@ -34,6 +34,8 @@ switches in its runtime options (crates/synaptix-config/src/runtime.rs, ``AttnBa
                     early it holds the room that the other branch's kernels need (a Zekalorn step at batch 1: 0.87 -> 0.70 ms)
 ``repeat_layers``   prompt steps: the launches of layers of one form are recorded from one of them and made again with the
                     others' pointers (else every layer's parts are walked)
+``decode_layers``   single-token steps of one or two rows of a dense decoder in bfloat16: all layers in one kernel (else five
+                    kernels a layer)
 """
 from __future__ import annotations
 
@@ -56,6 +58,7 @@ class KernelOptions:
     pdl: bool = True
     branch_streams: bool = True
     repeat_layers: bool = True
+    decode_layers: bool = True
 
 
 OPTIONS = KernelOptions()
