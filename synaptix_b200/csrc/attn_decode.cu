@@ -9,7 +9,7 @@
 //   * one elected lane of a producer warp (the whole warp walks the pages) brings a page with 2 (head size 64) or 4 (128) TMA copies
 //     (cp.async.bulk.tensor.4d over the cache [pages, kv heads, 64, head size], 128-byte swizzle)
 //     into 3 stages; full/empty mbarriers per stage, no block-wide barrier in the loop;
-//   * each of the 3 compute warps takes WHOLE pages (page i of the block's range goes to warp i % 3, through
+//   * each of the 3 (or 2) compute warps takes WHOLE pages (page i of the block's range goes to warp i % 3, through
 //     stage i % 3: a stage has one consumer, so the parities of its barriers are counted by one warp and the
 //     producer alone, and a wait can never be for a phase further than one ahead):
 //     scores of 64 keys as 8 key tiles x (head size / 16) mma.sync.m16n8k16, one softmax update and one
@@ -42,9 +42,11 @@
 
 #include "attn_merge.cuh"
 
-#define AD_COMPUTE_WARPS 3
-#define AD_THREADS 128                  // 3 compute warps + the producer warp
-#define AD_STAGES 3                     // = AD_COMPUTE_WARPS: stage w belongs to compute warp w (see the kernel)
+// A block has NW compute warps, a producer warp and NW stages (stage w belongs to compute warp w): 3, and two blocks an SM; or 2,
+// and three blocks an SM, where that lets all blocks run at once instead of in two rounds of which the second is nearly empty (many
+// sequences, one share each).  Measured, us in a replayed graph, 32 heads over 8: 48 sequences (384 blocks on 148 SMs) of 20 to
+// 40 keys 9.2 -> 6.5, of 100 to 230 13.6 -> 10.3 (bytes alone 4.7), of 900 to 1,100 42.0 -> 37.2; 38 sequences 9.3 -> 8.8.
+// Beyond three blocks an SM the smaller blocks lose: 56 sequences 13.9 -> 15.3, 64 of 4,096 keys 153 -> 207.
 #define AD_SPIN_LIMIT (1u << 26)
 #define AD_CHUNK (64 * 128)             // bytes of [64 keys][64 values]: one swizzled column half of a page
 
@@ -52,7 +54,7 @@ template <int HD> struct AdLayout {
   static constexpr int HALVES = HD / 64;
   static constexpr int TILE = HALVES * AD_CHUNK;       // K (or V) of one page
   static constexpr int STAGE = 2 * TILE;               // K then V
-  static constexpr int SMEM = AD_STAGES * STAGE + 1024;  // + room to align the ring to 1,024 bytes (the swizzle's period)
+  static constexpr int smem(int stages) { return stages * STAGE + 1024; }  // + room to align the ring to 1,024 bytes (the swizzle's period)
 };
 
 struct AdPrep {
@@ -236,8 +238,8 @@ __device__ __forceinline__ float4 ad_cluster_load4(const float* local, uint32_t 
   return v;
 }
 
-template <int HD, bool PREP, bool CLUSTER>
-__global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_tma_kernel(
+template <int HD, bool PREP, bool CLUSTER, int NW>
+__global__ void __launch_bounds__((NW + 1) * 32, NW == 2 ? 3 : 2) attn_decode_tma_kernel(
     const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
     const bf16* __restrict__ q, bf16* __restrict__ k_pages, bf16* __restrict__ v_pages, bf16* __restrict__ out,
     float* __restrict__ part_o, float* __restrict__ part_ml, const int* __restrict__ seq_lens,
@@ -247,17 +249,17 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_tma_kernel(
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(16) bf16 q_s[PREP ? 16 * HD : 8];       // the group's prepared query heads
   __shared__ __align__(16) bf16 kv_new[PREP ? 2 * HD : 8];     // the token's prepared key and value
-  __shared__ __align__(8) uint64_t bars[2 * AD_STAGES];         // full[stage], empty[stage]
+  __shared__ __align__(8) uint64_t bars[2 * NW];         // full[stage], empty[stage]
   unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const uint32_t ring_a = ad_smem(ring);
   const int split = blockIdx.x, kvh = blockIdx.y, seq = blockIdx.z;
   const int G = nh / nkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   auto full = [&](int s) { return ad_smem(&bars[s]); };
-  auto empty = [&](int s) { return ad_smem(&bars[AD_STAGES + s]); };
+  auto empty = [&](int s) { return ad_smem(&bars[NW + s]); };
   if (threadIdx.x == 0) {
 #pragma unroll
-    for (int s = 0; s < AD_STAGES; ++s) {
+    for (int s = 0; s < NW; ++s) {
       ad_mbar_init(full(s), 1);
       ad_mbar_init(empty(s), 1);
     }
@@ -281,7 +283,7 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_tma_kernel(
   const bool has_last = p0 <= p_last && p_last < p1;
   const bool writes = PREP && prep.write;
 
-  if (warp == AD_COMPUTE_WARPS) {
+  if (warp == NW) {
     // ------------------------------------------------------------------ producer
     // The first pages are asked for while the product before this kernel still runs: what they hold (every row
     // but the token's own, which this kernel makes) and the lengths and block tables were written at least two
@@ -291,7 +293,7 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_tma_kernel(
     // stay in uniform registers, which the copy instruction takes its operands from.)
     const bool leader = ad_elect_one();
     for (int i = 0; i < npages; ++i) {
-      const int st = i % AD_STAGES, use = i / AD_STAGES;
+      const int st = i % NW, use = i / NW;
       if (use > 0 && !__all_sync(0xffffffffu, ad_mbar_wait(empty(st), (use - 1) & 1))) {
         if (leader) sx_set_status(status, 1);
         break;
@@ -345,7 +347,7 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_tma_kernel(
     pdl_trigger();
     // jobs: the G query heads of the group, then (the block with the token's page) the key head and the value head
     const int jobs = G + (writes && has_last ? 2 : 0);
-    for (int j = warp; j < jobs; j += AD_COMPUTE_WARPS) {
+    for (int j = warp; j < jobs; j += NW) {
       const bool is_q = j < G, is_k = j == G;
       const bf16* src = tok + (size_t)(is_q ? kvh * G + j : (is_k ? nh + kvh : nh + nkv + kvh)) * HD;
       if (!is_q && !is_k) {                                   // value: copy
@@ -378,7 +380,7 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_tma_kernel(
         }
       }
     }
-    asm volatile("bar.sync 1, %0;\n" ::"n"(AD_COMPUTE_WARPS * 32) : "memory");       // the compute warps only
+    asm volatile("bar.sync 1, %0;\n" ::"n"(NW * 32) : "memory");       // the compute warps only
   }
 
   // query fragments: row r of the fragment is query head kvh * G + r (rows >= G are zero)
@@ -405,9 +407,9 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_tma_kernel(
   for (int n = 0; n < HD / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
 
   bool ok = true;
-  for (int i = warp; i < npages; i += AD_COMPUTE_WARPS) {
-    const int st = warp;                                      // i % AD_STAGES: this warp's own stage
-    if (!ad_mbar_wait(full(st), (i / AD_STAGES) & 1)) { if (lane == 0) sx_set_status(status, 2); ok = false; break; }
+  for (int i = warp; i < npages; i += NW) {
+    const int st = warp;                                      // i % NW: this warp's own stage
+    if (!ad_mbar_wait(full(st), (i / NW) & 1)) { if (lane == 0) sx_set_status(status, 2); ok = false; break; }
     unsigned char* stage = ring + st * L::STAGE;
     const uint32_t kt = ring_a + st * L::STAGE, vt = kt + L::TILE;
     const int pg = p0 + i, jb = pg * 64;
@@ -441,7 +443,7 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_tma_kernel(
     }
   }
   // every page that was asked for has been consumed by some warp once all compute warps are here
-  asm volatile("bar.sync 1, %0;\n" ::"n"(AD_COMPUTE_WARPS * 32) : "memory");
+  asm volatile("bar.sync 1, %0;\n" ::"n"(NW * 32) : "memory");
   (void)ok;
 
   // the running maxima are of raw scores; the merges below work in the scaled (log2) domain
@@ -454,7 +456,7 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_tma_kernel(
   }
   // merge the compute warps through shared memory (the ring is free now)
   float* wo = reinterpret_cast<float*>(ring);                 // [warps][16][HD]
-  float* wml = wo + AD_COMPUTE_WARPS * 16 * HD;               // [warps][16][2]
+  float* wml = wo + NW * 16 * HD;               // [warps][16][2]
 #pragma unroll
   for (int n = 0; n < HD / 8; ++n) {
     const int c = n * 8 + 2 * t;
@@ -467,9 +469,9 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_tma_kernel(
     wml[(warp * 16 + g + 8) * 2] = m[1];
     wml[(warp * 16 + g + 8) * 2 + 1] = l[1];
   }
-  asm volatile("bar.sync 1, %0;\n" ::"n"(AD_COMPUTE_WARPS * 32) : "memory");
+  asm volatile("bar.sync 1, %0;\n" ::"n"(NW * 32) : "memory");
   // this block's result: O [G][HD], then (M, L) [G][2], behind the warps' results in the ring; four values a thread
-  float* res = wml + AD_COMPUTE_WARPS * 16 * 2;
+  float* res = wml + NW * 16 * 2;
   float* res_ml = res + 16 * HD;
   const bool out8 = ((uintptr_t)out & 7) == 0;
   auto put = [&](int r, int d, float4 O, float Lsum) {
@@ -485,15 +487,15 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_tma_kernel(
       for (int i = 0; i < 4; ++i) dst[i] = __float2bfloat16_rn(v[i]);
     }
   };
-  for (int idx = threadIdx.x; idx < G * HD / 4; idx += AD_COMPUTE_WARPS * 32) {
+  for (int idx = threadIdx.x; idx < G * HD / 4; idx += NW * 32) {
     const int r = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
     float M = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < AD_COMPUTE_WARPS; ++w) M = fmaxf(M, wml[(w * 16 + r) * 2]);
+    for (int w = 0; w < NW; ++w) M = fmaxf(M, wml[(w * 16 + r) * 2]);
     float Lsum = 0.f;
     float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int w = 0; w < AD_COMPUTE_WARPS; ++w) {
+    for (int w = 0; w < NW; ++w) {
       const float mw = wml[(w * 16 + r) * 2];
       const float f = (mw == -INFINITY) ? 0.f : exp2f(mw - M);
       Lsum += wml[(w * 16 + r) * 2 + 1] * f;
@@ -524,14 +526,14 @@ __global__ void __launch_bounds__(AD_THREADS, 2) attn_decode_tma_kernel(
     float* far_m = res_ml + 32;                               // [G][n_splits]
     float* far_l = far_m + 16 * AD_MAX_CLUSTER;
     cluster_sync_all();
-    for (int i = threadIdx.x; i < G * n_splits; i += AD_COMPUTE_WARPS * 32) {
+    for (int i = threadIdx.x; i < G * n_splits; i += NW * 32) {
       const int r = i / n_splits, k = i - r * n_splits;
       far_m[i] = cluster_load_f32(res_ml + r * 2, k);
       far_l[i] = cluster_load_f32(res_ml + r * 2 + 1, k);
     }
-    asm volatile("bar.sync 1, %0;\n" ::"n"(AD_COMPUTE_WARPS * 32) : "memory");
+    asm volatile("bar.sync 1, %0;\n" ::"n"(NW * 32) : "memory");
     const int quads = G * HD / 4, per_block = (quads + n_splits - 1) / n_splits, q1 = min(quads, (split + 1) * per_block);
-    for (int idx = split * per_block + threadIdx.x; idx < q1; idx += AD_COMPUTE_WARPS * 32) {
+    for (int idx = split * per_block + threadIdx.x; idx < q1; idx += NW * 32) {
       const int r = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
       float4 x[AD_MAX_CLUSTER];
 #pragma unroll
@@ -595,28 +597,39 @@ static int* ad_status_word() {
   return p;
 }
 
+template <int HD, bool PREP, bool CLUSTER, int NW>
+static int ad_start(int n_splits, const CUtensorMap& mk, const CUtensorMap& mv, const bf16* q, bf16* k, bf16* v, bf16* out, float* part_o,
+                    float* part_ml, const int* seq_lens, const int* bt, int maxp, int S, int nh, int nkv, float scale_log2,
+                    int window, const AdPrep& prep, const float* sinks, int* status, cudaStream_t stream) {
+  using L = AdLayout<HD>;
+  static_assert(NW * L::STAGE >= ((NW + 1) * (16 * HD + 16 * 2) + 2 * 16 * AD_MAX_CLUSTER) * (int)sizeof(float),
+                "the ring holds the warps' results, the block's and the cluster's maxima and sums");
+  auto kern = attn_decode_tma_kernel<HD, PREP, CLUSTER, NW>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::smem(NW));
+  if (e != cudaSuccess) return (int)e;
+  const dim3 grid(n_splits, nkv, S), block((NW + 1) * 32);
+  if (CLUSTER)
+    return sx_launch_cluster(kern, grid, block, (size_t)L::smem(NW), stream, n_splits, mk, mv, q, k, v, out, part_o, part_ml, seq_lens, bt,
+                             maxp, nh, nkv, scale_log2, window, n_splits, prep, sinks, status);
+  return sx_launch(kern, grid, block, (size_t)L::smem(NW), stream, mk, mv, q, k, v, out, part_o, part_ml, seq_lens, bt, maxp, nh, nkv,
+                   scale_log2, window, n_splits, prep, sinks, status);
+}
+
 template <int HD, bool PREP>
 static int ad_launch(const CUtensorMap& mk, const CUtensorMap& mv, const bf16* q, bf16* k, bf16* v, bf16* out, float* part_o,
                      float* part_ml, const int* seq_lens, const int* bt, int maxp, int S, int nh, int nkv, float scale_log2,
                      int window, int n_splits, const AdPrep& prep, const float* sinks, int* status, cudaStream_t stream) {
-  using L = AdLayout<HD>;
-  static_assert(AD_STAGES == AD_COMPUTE_WARPS, "a stage has one consumer");
-  static_assert(AD_STAGES * L::STAGE >= ((AD_COMPUTE_WARPS + 1) * (16 * HD + 16 * 2) + 2 * 16 * AD_MAX_CLUSTER) * (int)sizeof(float),
-                "the ring holds the warps' results, the block's and the cluster's maxima and sums");
+#define AD_START(CLUSTER, NW) ad_start<HD, PREP, CLUSTER, NW>(n_splits, mk, mv, q, k, v, out, part_o, part_ml, seq_lens, bt, maxp, S, nh, nkv, \
+                                                              scale_log2, window, prep, sinks, status, stream)
   // 2, 4, 8 or 16 splits: the splits of a (sequence, kv head) are a cluster and merge among themselves
-  if (part_o == nullptr && n_splits > 1) {
-    auto kern = attn_decode_tma_kernel<HD, PREP, true>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM);
-    if (e != cudaSuccess) return (int)e;
-    return sx_launch_cluster(kern, dim3(n_splits, nkv, S), dim3(AD_THREADS), (size_t)L::SMEM, stream, n_splits, mk, mv, q, k,
-                             v, out, part_o, part_ml, seq_lens, bt, maxp, nh, nkv, scale_log2, window, n_splits, prep, sinks, status);
+  if (part_o == nullptr && n_splits > 1) return AD_START(true, 3);
+  if (n_splits == 1) {
+    const long long blocks = (long long)S * nkv, sms = sx_sm_count();
+    return blocks > 2 * sms && blocks <= 3 * sms ? AD_START(false, 2) : AD_START(false, 3);
   }
-  auto kern = attn_decode_tma_kernel<HD, PREP, false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM);
-  if (e != cudaSuccess) return (int)e;
-  int rc = sx_launch(kern, dim3(n_splits, nkv, S), dim3(AD_THREADS), (size_t)L::SMEM, stream, mk, mv, q, k, v, out, part_o,
-                     part_ml, seq_lens, bt, maxp, nh, nkv, scale_log2, window, n_splits, prep, sinks, status);
-  if (rc || n_splits == 1) return rc;
+  const int rc = AD_START(false, 3);
+#undef AD_START
+  if (rc) return rc;
   return sx_launch(attn_merge_kernel<HD>, dim3(S * nh), dim3(HD), 2 * n_splits * sizeof(float), stream,
                    (const float*)part_o, (const float*)part_ml, out, n_splits);
 }
