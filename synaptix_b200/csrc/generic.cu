@@ -263,23 +263,42 @@ __global__ void __launch_bounds__(128) gemm_rows_kernel(const TA* __restrict__ A
 // lane keeps) and over the warps in order.  Bound by HBM: N x K x 4 bytes.  Two rows, weights from HBM: 4,096 x 1,024 4.6 us (3.6
 // TB/s), 1,024 x 3,072 4.3 us, 151,936 x 1,024 98 us (6.3 TB/s); a warp per row of W with 4-byte loads, one in flight, took 45 us
 // over a step's products on average where this takes 8.
-// ---------------------------------------------------------------------------------------
-template <int MR, int KS>
+//
+// What stands around a product of a few rows is done by the product (kernels of 3 to 4 us each, that did nothing but wait and copy;
+// two rows, 28 layers of a 0.6B model and its head 1.24 -> 1.13 ms a step): with NORM, A is the residual stream and the rows' RMS norm is formed as they are read (the sum
+// of squares beside the products, gain on the way, the factor on the results); F32_ROWS_SILU reads a stacked [gate; up] and stores
+// silu(gate) * up; F32_ROWS_ADD adds into C, the residual stream.
+enum { F32_ROWS_STORE = 0, F32_ROWS_SILU = 1, F32_ROWS_ADD = 2 };
+struct F32RowsEnd {
+  const float* bias;     // [N] or null
+  float cap;             // F32_ROWS_STORE: soft_limit of the results
+  int epi;
+  const float* gain;     // [K] (NORM)
+  float eps;
+};
+template <int MR, int KS, bool NORM>
 __global__ void __launch_bounds__(256, MR <= 2 ? 4 : (MR == 4 ? 3 : 2)) gemm_rows_f32_kernel(const float* __restrict__ A, const float* __restrict__ W,
-                                                            float* __restrict__ C, int M, int N, int K,
-                                                            const float* __restrict__ bias, float cap) {
+                                                            float* __restrict__ C, int M, int N, int K, const F32RowsEnd end) {
   constexpr int R = 4, GROUPS = 8 / KS, V = MR * R, FV = V < 32 ? V : 32;
   __shared__ float part[8][V];
+  __shared__ float squares[8][MR];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, group = warp / KS, ks = warp % KS;
-  const int n0 = (blockIdx.x * GROUPS + group) * R;
+  const bool silu = end.epi == F32_ROWS_SILU;
+  const int n_out = silu ? N / 2 : N, cols = silu ? R / 2 : R;           // outputs in all, and of a warp's four rows
+  const int n0 = (blockIdx.x * GROUPS + group) * cols;
   const float* wr[R];
 #pragma unroll
-  for (int r = 0; r < R; ++r) wr[r] = W + (size_t)min(n0 + r, N - 1) * K;
-  float acc[MR][R];
+  for (int r = 0; r < R; ++r) {
+    const int row = silu ? min(n0 + (r & 1), n_out - 1) + (r >> 1) * n_out : min(n0 + r, N - 1);      // (two gate rows, two up rows)
+    wr[r] = W + (size_t)row * K;
+  }
+  float acc[MR][R], sq[MR];
 #pragma unroll
-  for (int i = 0; i < MR; ++i)
+  for (int i = 0; i < MR; ++i) {
+    sq[i] = 0.f;
 #pragma unroll
     for (int r = 0; r < R; ++r) acc[i][r] = 0.f;
+  }
   // the first slice of W is on its way into L2 before the kernel ahead has ended (a hint: whatever it brings is read below;
   // two prompts and eight steps of a 0.6B model in 32 bits: 21.75 -> 21.5 ms, with the activation launched early as well)
   if ((lane & 7) == 0 && (ks * 32 + lane) * 4 < K) {
@@ -290,12 +309,17 @@ __global__ void __launch_bounds__(256, MR <= 2 ? 4 : (MR == 4 ? 3 : 2)) gemm_row
   pdl_trigger();
 #pragma unroll (MR <= 2 ? 2 : 1)
   for (int k = (ks * 32 + lane) * 4; k < K; k += KS * 128) {
-    float4 w[R];
+    float4 w[R], gn;
 #pragma unroll
     for (int r = 0; r < R; ++r) w[r] = __ldg(reinterpret_cast<const float4*>(wr[r] + k));
+    if (NORM) gn = __ldg(reinterpret_cast<const float4*>(end.gain + k));
 #pragma unroll
     for (int i = 0; i < MR; ++i) {
-      const float4 a = *reinterpret_cast<const float4*>(A + (size_t)min(i, M - 1) * K + k);
+      float4 a = *reinterpret_cast<const float4*>(A + (size_t)min(i, M - 1) * K + k);
+      if (NORM) {
+        sq[i] = fmaf(a.w, a.w, fmaf(a.z, a.z, fmaf(a.y, a.y, fmaf(a.x, a.x, sq[i]))));
+        a.x *= gn.x; a.y *= gn.y; a.z *= gn.z; a.w *= gn.w;
+      }
 #pragma unroll
       for (int r = 0; r < R; ++r)
         acc[i][r] = fmaf(a.w, w[r].w, fmaf(a.z, w[r].z, fmaf(a.y, w[r].y, fmaf(a.x, w[r].x, acc[i][r]))));
@@ -310,14 +334,37 @@ __global__ void __launch_bounds__(256, MR <= 2 ? 4 : (MR == 4 ? 3 : 2)) gemm_row
     constexpr int REP = 32 / FV;               // lanes that hold the same sum
     if (lane % REP == 0) part[warp][b * FV + lane / REP] = s;
   }
+  if (NORM) {
+    const float s = warp_fold<MR>(sq, lane);
+    constexpr int REP = 32 / MR;
+    if (lane % REP == 0) squares[warp][lane / REP] = s;
+  }
   __syncthreads();
   for (int i = threadIdx.x; i < GROUPS * V; i += 256) {
-    const int g = i / V, m = (i % V) / R, n = (blockIdx.x * GROUPS + g) * R + i % R;
-    if (m >= M || n >= N) continue;
-    float s = 0.f;
+    const int g = i / V, m = (i % V) / R, r = i % R, n = (blockIdx.x * GROUPS + g) * cols + r;
+    if (m >= M || n >= n_out || r >= cols) continue;
+    float s = 0.f, u = 0.f, f = 1.f;
 #pragma unroll
     for (int w = 0; w < KS; ++w) s += part[g * KS + w][i % V];
-    C[(size_t)m * N + n] = soft_limit(bias ? s + bias[n] : s, cap);
+    if (silu)
+#pragma unroll
+      for (int w = 0; w < KS; ++w) u += part[g * KS + w][i % V + 2];
+    if (NORM) {
+      float q = 0.f;
+#pragma unroll
+      for (int w = 0; w < KS; ++w) q += squares[g * KS + w][m];
+      f = rsqrtf(q / (float)K + end.eps);
+    }
+    float* c = C + (size_t)m * n_out + n;
+    s = s * f + (end.bias ? end.bias[n] : 0.f);
+    if (silu) {
+      u = u * f + (end.bias ? end.bias[n_out + n] : 0.f);
+      *c = s / (1.f + expf(-s)) * u;
+    } else if (end.epi == F32_ROWS_ADD) {
+      *c += s;
+    } else {
+      *c = soft_limit(s, end.cap);
+    }
   }
 }
 
@@ -493,13 +540,20 @@ __global__ void __launch_bounds__(128, 3) gemm_tile_f32_kernel(const float* __re
   cluster_sync_all();                             // nobody's shared memory goes away while it is read
 }
 
-template <int MR>
-static int gemm_rows_f32_launch(const float* A, const float* W, float* C, int M, int N, int K, const float* bias, float cap,
-                                cudaStream_t stream) {
-  const int tiles = (N + 3) / 4;
-  if (K >= 1024) return sx_launch(gemm_rows_f32_kernel<MR, 8>, dim3(tiles), dim3(256), 0, stream, A, W, C, M, N, K, bias, cap);
-  if (K >= 256) return sx_launch(gemm_rows_f32_kernel<MR, 2>, dim3((tiles + 3) / 4), dim3(256), 0, stream, A, W, C, M, N, K, bias, cap);
-  return sx_launch(gemm_rows_f32_kernel<MR, 1>, dim3((tiles + 7) / 8), dim3(256), 0, stream, A, W, C, M, N, K, bias, cap);
+template <int MR, bool NORM>
+static int gemm_rows_f32_launch(const float* A, const float* W, float* C, int M, int N, int K, const F32RowsEnd& end, cudaStream_t stream) {
+  const int n_out = end.epi == F32_ROWS_SILU ? N / 2 : N, cols = end.epi == F32_ROWS_SILU ? 2 : 4, tiles = (n_out + cols - 1) / cols;
+  if (K >= 1024) return sx_launch(gemm_rows_f32_kernel<MR, 8, NORM>, dim3(tiles), dim3(256), 0, stream, A, W, C, M, N, K, end);
+  if (K >= 256) return sx_launch(gemm_rows_f32_kernel<MR, 2, NORM>, dim3((tiles + 3) / 4), dim3(256), 0, stream, A, W, C, M, N, K, end);
+  return sx_launch(gemm_rows_f32_kernel<MR, 1, NORM>, dim3((tiles + 7) / 8), dim3(256), 0, stream, A, W, C, M, N, K, end);
+}
+template <bool NORM>
+static int gemm_rows_f32(const float* A, const float* W, float* C, int M, int N, int K, const F32RowsEnd& end, cudaStream_t stream) {
+  if (M <= 1) return gemm_rows_f32_launch<1, NORM>(A, W, C, M, N, K, end, stream);
+  if (M <= 2) return gemm_rows_f32_launch<2, NORM>(A, W, C, M, N, K, end, stream);
+  if (M <= 4) return gemm_rows_f32_launch<4, NORM>(A, W, C, M, N, K, end, stream);
+  if (M <= 8) return gemm_rows_f32_launch<8, NORM>(A, W, C, M, N, K, end, stream);
+  return gemm_rows_f32_launch<16, NORM>(A, W, C, M, N, K, end, stream);
 }
 
 // The tiles of more rows: rows of a tile, and blocks that share a tile's K.
@@ -549,11 +603,11 @@ static int gemm_tile_f32_launch(const float* A, const float* W, float* C, int M,
 }
 
 static int gemm_f32(const float* A, const float* W, float* C, int M, int N, int K, const float* bias, float cap, cudaStream_t stream) {
-  if (M <= 1) return gemm_rows_f32_launch<1>(A, W, C, M, N, K, bias, cap, stream);
-  if (M <= 2) return gemm_rows_f32_launch<2>(A, W, C, M, N, K, bias, cap, stream);
-  if (M <= 4) return gemm_rows_f32_launch<4>(A, W, C, M, N, K, bias, cap, stream);
-  if (M <= 8) return gemm_rows_f32_launch<8>(A, W, C, M, N, K, bias, cap, stream);
-  if (M <= 16) return gemm_rows_f32_launch<16>(A, W, C, M, N, K, bias, cap, stream);
+  if (M <= 16) {
+    F32RowsEnd end = {};
+    end.bias = bias; end.cap = cap;
+    return gemm_rows_f32<false>(A, W, C, M, N, K, end, stream);
+  }
   const F32Plan p = gemm_f32_plan(M, N, K, sx_sm_count());
   return p.rows == 32 ? gemm_tile_f32_launch<32>(A, W, C, M, N, K, bias, cap, p.cluster, stream)
                       : gemm_tile_f32_launch<64>(A, W, C, M, N, K, bias, cap, p.cluster, stream);
@@ -588,6 +642,17 @@ extern "C" int sx_gemm_generic(const void* A, int a_dt, const void* W, int w_dt,
   if (a_dt == SX_F32 && w_dt == SX_BF16 && c_dt == SX_F32)
     return gemm_generic_launch<float, bf16, float>(A, W, C, M, N, K, bias, cap, stream);
   return SX_ERR_DTYPE;
+}
+
+// Up to 16 float32 rows of whole, aligned 16-byte pieces.  gain (or null): A is normed on the way, rows of A * rsqrt(mean(A^2) + eps) * gain.
+// epi 0: C [M, N] = the product (+ bias); 1: W = [gate; up] stacked, C [M, N/2] = silu(gate) * up; 2: C [M, N] += the product (+ bias).
+extern "C" int sx_gemm_rows_f32(const float* A, const float* W, float* C, int M, int N, int K, const float* bias, int epi,
+                                const float* gain, float eps, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (M > 16 || K <= 0 || (K & 3) || epi < 0 || epi > 2 || (epi == F32_ROWS_SILU && (N & 1))) return SX_ERR_SIZE;
+  if (((uintptr_t)A | (uintptr_t)W | (uintptr_t)gain) & 15) return SX_ERR_ALIGN;
+  F32RowsEnd end = {bias, 0.f, epi, gain, eps};
+  return gain ? gemm_rows_f32<true>(A, W, C, M, N, K, end, stream) : gemm_rows_f32<false>(A, W, C, M, N, K, end, stream);
 }
 
 // ---------------------------------------------------------------------------------------

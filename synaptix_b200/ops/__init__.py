@@ -21,8 +21,8 @@ from .gemm_tc import gemm_tc, gemm_tc_qkv, gemm_tc_resid_tanh, qkv_epilogue_supp
 from .gemm_ws import gemm_ws, gemm_ws_resid_tanh, gemm_ws_residual, ws_supported
 from .layers import MAX_ROWS as DECODE_LAYERS_MAX_ROWS, decode_layers, decode_layers_words
 from .options import OPTIONS, KernelOptions, options, set_options
-from .generic import (add_rmsnorm, attn_generic, decode_advance, decode_begin, embed_gather, gemm_generic, qkv_prepare,
-                      residual_add, rope_table, silu_mul)
+from .generic import (F32_ROWS, add_rmsnorm, attn_generic, decode_advance, decode_begin, embed_gather, gemm_generic, gemm_rows_f32,
+                      qkv_prepare, residual_add, rope_table, rows_f32_supported, silu_mul)
 from .sequence import add_rmsnorm_conv, capped_glu, mingru, retention, stream_add
 from .block import add_scaled, add_scaled_rmsnorm, scale_rows, side_gate
 from .delta import DeltaWeights, delta_rule, delta_step_fits
@@ -37,7 +37,7 @@ from .mlstm import mlstm
 from .moe import ExpertPlan, moe_combine, moe_down, moe_gate_up, moe_route, moe_sort, moe_up
 
 __all__ = ["OPTIONS", "KernelOptions", "options", "set_options", "KernelsUnavailable", "KernelError", "set_launch_counter", "decode_advance", "decode_begin", "check_status", "add_rmsnorm", "attn_generic", "embed_gather",
-           "gemm_generic", "qkv_prepare", "residual_add", "silu_mul", "linear", "linear_normed", "norm_fusable", "attention",
+           "gemm_generic", "gemm_rows_f32", "qkv_prepare", "residual_add", "silu_mul", "linear", "linear_normed", "norm_fusable", "attention",
            "attention_from_projection", "decode_attention_takes_projection", "residual_product_fusable",
            "linear_into_residual", "linear_scaled", "projection_prepares_heads", "project_and_prepare", "rope_table",
            "add_rmsnorm_conv", "capped_glu", "mingru", "retention", "stream_add", "gate_activation",
@@ -166,16 +166,21 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
                 return gemm_tc(x, w, epilogue="silu_mul", bias=bias)
         else:
             return gemm_tc(x, w, epilogue="f32" if out_dtype == torch.float32 else None, bias=bias, cap=cap)
+    alpha, limit, form = current_gate()          # which gated activation the epilogue stands for (see gate_activation)
+    if epilogue == "silu_mul" and not (limit > 0 or form != 0) and out_dtype == torch.float32 and rows_f32_supported(x, w):
+        return gemm_rows_f32(x, w, epilogue="silu_mul", bias=bias)
     y = gemm_generic(x, w, out_dtype=out_dtype if epilogue is None else x.dtype, bias=bias, cap=cap)
     if epilogue == "silu_mul":
-        alpha, limit, form = current_gate()      # which gated activation the epilogue stands for (see gate_activation)
         y = capped_glu(y, alpha, limit, form) if (limit > 0 or form != 0) else silu_mul(y)
     return y
 
 
 def norm_fusable(M: int, K: int, dtype) -> bool:
     """Can ``rmsnorm(h + delta)`` of ``M`` rows of width ``K`` run inside the next product's prologue?"""
-    # every block repeats the norm, so it pays only while the rows are few
+    # every block repeats the norm, so it pays only while the rows are few; the 32-bit product forms the sum of squares as it
+    # reads the rows
+    if dtype == torch.float32:
+        return 0 < M <= F32_ROWS and K > 0 and K % 4 == 0
     return dtype == torch.bfloat16 and 0 < M <= PROLOGUE_NORM_MAX_ROWS and K % 32 == 0 and K <= 4096
 
 
@@ -185,6 +190,14 @@ def linear_normed(pn, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
     M, K = pn.h.shape
     if out_dtype is None:
         out_dtype = pn.dtype
+    if pn.dtype == torch.float32:
+        alpha, limit, form = current_gate()
+        if (pn.delta is not None or out_dtype != torch.float32 or not norm_fusable(M, K, pn.dtype) or w.shape[0] > SCALED_MAX_OUT
+                or w.shape[1] != K or not rows_f32_supported(pn.h, w) or pn.gain.data_ptr() % 16
+                or (epilogue is not None and (epilogue != "silu_mul" or limit > 0 or form != 0))):
+            return None
+        pn.h_out()
+        return gemm_rows_f32(pn.h, w, epilogue=epilogue, gain=pn.gain, eps=pn.eps)
     if not (norm_fusable(M, K, pn.dtype) and w.dtype == torch.bfloat16 and w.shape[1] == K):
         return None
     if epilogue == "silu_mul":
@@ -206,6 +219,16 @@ def residual_product_fusable(M: int, N: int, K: int, dtype) -> bool:
     if dtype != torch.bfloat16 or not OPTIONS.fused_residual or K <= 0 or M <= PROLOGUE_NORM_MAX_ROWS:
         return False
     return _weight_stream_kernel(M, N, K, dtype, dtype) is not None
+
+
+def linear_adds_itself(x: torch.Tensor, w: torch.Tensor, h: torch.Tensor) -> bool:
+    """``h += x @ w.T`` by a float32 product of a few rows itself (option ``fused_residual``); ``False``, and nothing done, if no
+    kernel does that."""
+    if (not OPTIONS.fused_residual or h.dtype != torch.float32 or tuple(h.shape) != (x.shape[0], w.shape[0]) or not h.is_contiguous()
+            or not rows_f32_supported(x, w)):
+        return False
+    gemm_rows_f32(x, w, into=h)
+    return True
 
 
 def linear_into_residual(x: torch.Tensor, w: torch.Tensor, h: torch.Tensor, gain: torch.Tensor):

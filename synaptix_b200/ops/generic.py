@@ -87,6 +87,39 @@ def gemm_generic(a: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dty
     return out
 
 
+F32_ROWS = 16
+
+
+def rows_f32_supported(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Can ``gemm_rows_f32`` multiply these: float32, up to 16 rows of whole, aligned 16-byte pieces?"""
+    return (x.dtype == torch.float32 and w.dtype == torch.float32 and 0 < x.shape[0] <= F32_ROWS and w.shape[1] > 0
+            and w.shape[1] % 4 == 0 and w.shape[0] > 0 and x.is_contiguous() and (x.data_ptr() | w.data_ptr()) % 16 == 0)
+
+
+def gemm_rows_f32(x: torch.Tensor, w: torch.Tensor, *, epilogue: Optional[str] = None, bias: Optional[torch.Tensor] = None,
+                  gain: Optional[torch.Tensor] = None, eps: float = 0.0, into: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``x[M, K] @ w[N, K].T + bias`` of up to 16 float32 rows with what stands around it in one kernel.  ``gain`` (float32
+    ``[K]``): of ``rmsnorm(x) * gain``; ``epilogue="silu_mul"``: ``w`` is ``[gate; up]`` stacked, the result ``silu(gate) * up``;
+    ``into`` (float32 ``[M, N]``): added to that, in place."""
+    require_cuda(x, w, bias, gain, into)
+    (M, K), (N, K2) = x.shape, w.shape
+    if K != K2 or epilogue not in (None, "silu_mul") or (epilogue is not None and into is not None):
+        raise KernelError("gemm_rows_f32: inner sizes differ, or an unknown epilogue")
+    if not rows_f32_supported(x, w):
+        raise KernelError("gemm_rows_f32: up to 16 contiguous float32 rows, K a multiple of 4, 16-byte aligned")
+    check_bias(bias, N)
+    if gain is not None and (gain.dtype != torch.float32 or gain.numel() != K):
+        raise KernelError("gemm_rows_f32: gain must be float32 [K]")
+    if into is not None and (tuple(into.shape) != (M, N) or into.dtype != torch.float32):
+        raise KernelError("gemm_rows_f32: the sum must be contiguous float32 [M, N]")
+    n_out = N // 2 if epilogue else N
+    out = into if into is not None else torch.empty((M, n_out), dtype=torch.float32, device=x.device)
+    check(fn("generic", "sx_gemm_rows_f32")(ptr(x), ptr(w), ptr(out), c_int(M), c_int(N), c_int(K), ptr(bias),
+                                            c_int(1 if epilogue else 2 if into is not None else 0), ptr(gain), c_float(eps),
+                                            stream()), "gemm_rows_f32")
+    return out
+
+
 def qkv_prepare(qkv: torch.Tensor, q_out: torch.Tensor, k_pages: Optional[torch.Tensor],
                 v_pages: Optional[torch.Tensor], wq: Optional[torch.Tensor], wk: Optional[torch.Tensor],
                 inv_freq: Optional[torch.Tensor], rotary_dim: int, eps: float, positions: torch.Tensor,

@@ -65,7 +65,10 @@ class RMSNorm(Norm):
                 # the product adds itself into h and leaves the rows of this norm without their factor
                 x, ssq = ops.linear_into_residual(delta.x, delta.weight, h, self.weight)
                 return ScaledRows(x, ssq, self.eps, h, self.weight, self._dtype)
-            delta = delta.materialize()
+            if lazy and delta.bias is None and rows is None and ops.linear_adds_itself(delta.x, delta.weight, h):
+                delta = None                                 # (the sum is in h; what is left is the norm of it)
+            else:
+                delta = delta.materialize()
         if lazy and rows is None and ops.norm_fusable(h.shape[0], h.shape[1], self._dtype):
             return PendingNorm(h, delta, self.weight, self.eps, self._dtype)
         return ops.add_rmsnorm(h, delta, self.weight, self.eps, self._dtype, rows=rows)

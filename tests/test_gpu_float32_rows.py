@@ -1,0 +1,81 @@
+"""The float32 products of up to 16 rows that do what stands around them (the norm of their rows, the gated activation, the sum
+into the residual stream) against 64-bit sums.  Bounds: a sum of n products in any order is off by at most (n + 2) 2^-24 times the
+sum of the products' magnitudes; the gain, the factor (a sum of K squares, a root and a reciprocal of at most 4 ulp) and the sum
+of a row's two parts add a few roundings of the result."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+ULP = 2.0 ** -24
+SIZES = [(2, 4), (6, 252), (130, 256), (30, 1020), (514, 1024), (1022, 2052), (96, 3072)]
+
+
+def operands(M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(M * 1000003 + N * 1009 + K)
+    x, w, bias, gain = (torch.randn(*s, generator=g, device="cuda") for s in ((M, K), (N, K), (N,), (K,)))
+    return x * 3, w / K ** 0.5, bias, gain
+
+
+def product(x, w, gain, eps):
+    """The product in 64 bits and the bound on a 32-bit one."""
+    K = x.shape[1]
+    x64 = x.double()
+    if gain is not None:
+        x64 = x64 * (x64.pow(2).mean(1, keepdim=True) + eps).rsqrt() * gain.double()
+    return x64 @ w.double().T, (K + 3 + (K / 2 + 8 if gain is not None else 0)) * ULP * (x64.abs() @ w.double().abs().T)
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("N,K", SIZES)
+@pytest.mark.parametrize("normed", [False, True])
+def test_rows(M, N, K, normed):
+    from synaptix_b200 import ops
+    x, w, bias, gain = operands(M, N, K)
+    gain = gain if normed else None
+    want, bound = product(x, w, gain, 1e-3)
+    got = ops.gemm_rows_f32(x, w, gain=gain, eps=1e-3, bias=bias).double()
+    assert ((got - want - bias.double()).abs() <= bound + 2 * ULP * (want.abs() + bias.double().abs())).all()
+    h = torch.randn(M, N, device="cuda")
+    before = h.double()
+    assert ops.gemm_rows_f32(x, w, gain=gain, eps=1e-3, into=h) is h
+    assert ((h.double() - before - want).abs() <= bound + 2 * ULP * (want.abs() + before.abs())).all()
+    # silu(g) u: |silu'| < 1.1, |silu(g)| <= |g|; the exponential and the quotient a few ulp of the result
+    g, u = want[:, :N // 2] + bias[:N // 2].double(), want[:, N // 2:] + bias[N // 2:].double()
+    dg, du = (b + 2 * ULP * (z.abs() + c.double().abs()) for b, z, c in
+              ((bound[:, :N // 2], g, bias[:N // 2]), (bound[:, N // 2:], u, bias[N // 2:])))
+    y = ops.gemm_rows_f32(x, w, gain=gain, eps=1e-3, bias=bias, epilogue="silu_mul").double()
+    z = torch.nn.functional.silu(g)
+    assert ((y - z * u).abs() <= 1.1 * dg * (u.abs() + du) + z.abs() * du + 8 * ULP * (z * u).abs() + 1e-37).all()
+
+
+def test_what_it_refuses():
+    from synaptix_b200 import ops
+    x, w, bias, gain = operands(4, 16, 64)
+    for bad in (dict(x=x.bfloat16()), dict(w=w[:, :62].contiguous(), x=x[:, :62].contiguous()), dict(x=torch.randn(17, 64, device="cuda")),
+                dict(x=x.reshape(-1)[1:193].view(3, 64)), dict(gain=gain[:63]), dict(into=torch.zeros(4, 15, device="cuda")),
+                dict(into=torch.zeros(4, 16, device="cuda"), epilogue="silu_mul"), dict(epilogue="f32")):
+        with pytest.raises(ops.KernelError):
+            ops.gemm_rows_f32(**{"x": x, "w": w, **bad})
+
+
+@pytest.mark.parametrize("M", [2, 16])
+def test_dispatch_agrees_with_the_parts_one_by_one(M):
+    """A norm, a stacked product and a sum through the functions that choose, against the kernels they replace."""
+    from synaptix_b200 import ops
+    from synaptix_b200.parts import PendingLinear, PendingNorm
+    from synaptix_b200.parts.base import Runtime
+    from synaptix_b200.parts.norm import RMSNorm
+    x, w, _, gain = operands(M, 512, 256)
+    h = torch.randn(M, 512, device="cuda")
+    norm = RMSNorm("g", 512, 1e-6)
+    norm.weight, norm._dtype = torch.rand(512, device="cuda") + 0.5, torch.float32
+    wide = torch.randn(768, 512, device="cuda") / 20
+    want_h = h + ops.gemm_generic(x, w)
+    want_x = ops.add_rmsnorm(want_h.clone(), None, norm.weight, 1e-6, torch.float32)
+    want = ops.silu_mul(ops.gemm_generic(want_x, wide))
+    pn = norm.add_forward(h, PendingLinear(x, w), lazy=True)
+    assert type(pn) is PendingNorm and pn.delta is None
+    got = ops.linear_normed(pn, wide, epilogue="silu_mul")
+    assert pn.h_after() is h and (h - want_h).abs().max() <= 4 * ULP * float(want_h.abs().max())
+    # two orders of the same sums, each within the bound of test_rows
+    assert (got - want).abs().max() <= 2 * (256 + 512 * 2) * ULP * float((want_x.abs() @ wide.abs().T).max()) ** 2
