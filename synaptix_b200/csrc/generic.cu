@@ -265,9 +265,9 @@ __global__ void __launch_bounds__(128) gemm_rows_kernel(const TA* __restrict__ A
 // over a step's products on average where this takes 8.
 //
 // What stands around a product of a few rows is done by the product (kernels of 3 to 4 us each, that did nothing but wait and copy;
-// two rows, 28 layers of a 0.6B model and its head 1.24 -> 1.13 ms a step): with NORM, A is the residual stream and the rows' RMS norm is formed as they are read (the sum
-// of squares beside the products, gain on the way, the factor on the results); F32_ROWS_SILU reads a stacked [gate; up] and stores
-// silu(gate) * up; F32_ROWS_ADD adds into C, the residual stream.
+// two rows, 28 layers of a 0.6B model and its head 1.24 -> 1.13 ms a step): with NORM, A is the residual stream and the rows' RMS
+// norm is formed as they are read (the sum of squares beside the products, gain on the way, the factor on the results);
+// F32_ROWS_SILU reads a stacked [gate; up] and stores silu(gate) * up; F32_ROWS_ADD adds into C, the residual stream.
 enum { F32_ROWS_STORE = 0, F32_ROWS_SILU = 1, F32_ROWS_ADD = 2 };
 struct F32RowsEnd {
   const float* bias;     // [N] or null
@@ -407,6 +407,21 @@ __device__ __forceinline__ void f32_split3(float x, float y, uint32_t& p0, uint3
     y -= __uint_as_float(p[i] & 0xffff0000u);
   }
   p0 = p[0]; p1 = p[1]; p2 = p[2];
+}
+// slices of 16 of N products, in two sums: of the leading pieces (their products have 16 bits, so little is rounded), and of the
+// other five products of pieces, 2^-8 of the whole
+template <int N>
+__device__ __forceinline__ void f32_products(float (&c)[N][4], float (&d)[N][4], const uint32_t (&a)[3][4], const uint32_t (&b)[N][3][2]) {
+  constexpr int PA[5] = {2, 0, 1, 1, 0}, PB[5] = {0, 2, 1, 0, 1};
+#pragma unroll
+  for (int n = 0; n < N; ++n) f32_mma0(c[n], a[0], b[n][0]);
+#pragma unroll
+  for (int p = 0; p < 5; ++p)
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      if (p == 0) f32_mma0(d[n], a[PA[p]], b[n][PB[p]]);
+      else f32_mma(d[n], a[PA[p]], b[n][PB[p]]);
+    }
 }
 // one element of the product from whole numbers
 __device__ __noinline__ float f32_whole(const float* __restrict__ a, const float* __restrict__ w, int K) {
@@ -1310,6 +1325,280 @@ __global__ void __launch_bounds__(256) attn_f32_kernel(
   }
 }
 
+// ---------------------------------------------------------------------------------------
+// Prompt portions: 32 query rows of a head a block on the tensor cores, with operands in three bfloat16 pieces as in
+// gemm_tile_f32_kernel (six products of pieces, each slice of 16 summed from zero and added in 32 bits; here the leading product on
+// its own, f32_products, which keeps the error below that of the kernel above: 1.2e-7 against 1.3e-7 with 300 keys, 1.9e-7 against 2.0e-7
+// with 1,000).  Eight warps: 16 rows and every fourth 16 of a page's 64 keys each; the four parts of the keys are added up at the end.
+// A row's query pieces lie in shared memory as the instructions take them; keys and values come through two stages (cp.async), rows
+// padded so that 16-byte reads meet no bank twice.  Within an instruction the order of the 16 elements of a head (scores) and of
+// the 32 columns of four instructions (values) is the one in which a thread's numbers are neighbours in memory.  A row with a
+// score or result that is not finite, or with results so small that pieces of the values may have been lost, is done again in 32
+// bits by a warp (attn_f32_row).  Two prompts of 150 tokens, 16 heads of 128: 70 -> 30 us, what is left is the latency of a page
+// (3.5 us: 192 products of pieces and 1,000 other instructions a warp); with four warps and 32 keys a turn 37 us (2,048 tokens 930
+// against 1,059), with the results scaled and divided by the threads that hold them, 64 divisions one after the other, 44.
+// ---------------------------------------------------------------------------------------
+template <int HD>
+__device__ __noinline__ void attn_f32_row(const float* __restrict__ q, const float* __restrict__ k_pages, const float* __restrict__ v_pages,
+                                          float* __restrict__ out, const int* __restrict__ bt, int nkv, int kvh, int lo, int pos,
+                                          float scale, float softcap, const float* sink, float out_scale, int lane) {
+  constexpr int C = HD / 32;
+  float qv[C], acc[C], m = -INFINITY, l = 0.f;
+#pragma unroll
+  for (int c = 0; c < C; ++c) { qv[c] = q[c * 32 + lane]; acc[c] = 0.f; }
+  for (int j = lo; j <= pos; ++j) {
+    const size_t at = (((size_t)bt[j >> 6] * nkv + kvh) * SX_PAGE + (j & 63)) * HD + lane;
+    float d = 0.f;
+#pragma unroll
+    for (int c = 0; c < C; ++c) d = fmaf(qv[c], k_pages[at + c * 32], d);
+    float s = warp_sum(d) * scale;
+    if (softcap > 0.f) s = softcap * tanhf(s / softcap);
+    const float m_new = fmaxf(m, s);
+    const float corr = m == -INFINITY ? 0.f : expf(m - m_new), p = s == -INFINITY ? 0.f : expf(s - m_new);
+    m = m_new;
+    l = fmaf(l, corr, p);
+#pragma unroll
+    for (int c = 0; c < C; ++c) acc[c] = fmaf(p, v_pages[at + c * 32], acc[c] * corr);
+  }
+  const float mx = sink ? fmaxf(m, *sink) : m, f = m == -INFINITY ? 0.f : expf(m - mx);
+  const float sum = l * f + (sink ? expf(*sink - mx) : 0.f);
+#pragma unroll
+  for (int c = 0; c < C; ++c) out[c * 32 + lane] = acc[c] * f / sum * out_scale;
+}
+
+__device__ __noinline__ float f32_capped(float s, float cap) { return cap * tanhf(s / cap); }
+
+template <int HD, int KW>
+__global__ void __launch_bounds__(64 * KW, 4 / KW) attn_f32_tile_kernel(
+    const float* __restrict__ q, const float* __restrict__ k_pages, const float* __restrict__ v_pages, float* __restrict__ out,
+    const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ block_table, int maxp,
+    int n_tokens, int nh, int nkv, float scale, int window, float softcap, const float* __restrict__ sinks, int chunk,
+    int out_stride, float out_scale) {
+  constexpr int KS = HD / 16, NB = HD / 32, SK = HD + 16, SV = HD + 4, KEYS = 16 * KW, THREADS = 64 * KW, STAGE = KEYS * (SK + SV);
+  extern __shared__ __align__(16) float f32_smem[];
+  uint4* s_q = reinterpret_cast<uint4*>(f32_smem + 2 * STAGE);             // [row warp][slice][piece][lane]
+  __shared__ float s_m[KW][32], s_l[KW][32];
+  __shared__ int s_bad[KW][32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, wr = warp & 1, wk = warp >> 1;
+  const int h = blockIdx.x, kvh = h / (nh / nkv), t0 = (gridDim.y - 1 - blockIdx.y) * 32;      // (rows with many keys first)
+  const int n_here = min(32, n_tokens - t0);
+  const uint32_t smem0 = (uint32_t)__cvta_generic_to_shared(f32_smem);
+  pdl_wait();
+  pdl_trigger();
+  int first = 0;                                  // tokens of one sequence at a time
+  while (first < n_here) {
+    const int seq = seq_of_token[t0 + first];
+    int end = first + 1;
+    while (end < n_here && seq_of_token[t0 + end] == seq) ++end;
+    const int* bt = block_table + (size_t)seq * maxp;
+    auto low = [&](int p) {
+      const int a = window > 0 ? max(0, p - window + 1) : 0;
+      return chunk > 0 ? max(a, p / chunk * chunk) : a;
+    };
+    const bool mine = lane >= first && lane < end;
+    const int p_lane = mine ? positions[t0 + lane] : -1;
+    const int jhi = __reduce_max_sync(0xffffffffu, p_lane), jlo = __reduce_min_sync(0xffffffffu, mine ? low(p_lane) : 0x7fffffff);
+    // (keys outside jlo .. jhi are zeros: their pages may hold anything)
+    auto load = [&](int jb, int s) {
+      const size_t at = (((size_t)bt[jb >> 6] * nkv + kvh) * SX_PAGE + (jb & 63)) * HD;
+#pragma unroll 4
+      for (int i = 0; i < KEYS * HD / 4 / THREADS; ++i) {
+        const int idx = tid + i * THREADS, r = idx / (HD / 4), c = idx % (HD / 4) * 4;
+        const bool live = jb + r >= jlo && jb + r <= jhi;
+        const uint32_t dst = smem0 + (uint32_t)(s * STAGE + r * SK + c) * 4, dst_v = smem0 + (uint32_t)(s * STAGE + KEYS * SK + r * SV + c) * 4;
+        f32_cp16(dst, live ? k_pages + at + r * HD + c : k_pages, live);
+        f32_cp16(dst_v, live ? v_pages + at + r * HD + c : v_pages, live);
+      }
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    const int jb0 = jlo & ~(KEYS - 1);
+    load(jb0, 0);
+    int pos[2], lo[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int row = wr * 16 + g + i * 8;
+      const bool live = row >= first && row < end;
+      pos[i] = live ? positions[t0 + row] : -1;
+      lo[i] = live ? low(pos[i]) : 0;
+    }
+    for (int ks = wk; ks < KS; ks += KW) {         // the row's pieces, as the instructions take them
+      uint32_t a[3][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const float4 v = pos[i] >= 0 ? *reinterpret_cast<const float4*>(q + ((size_t)(t0 + wr * 16 + g + i * 8) * nh + h) * HD + ks * 16 + t * 4)
+                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+        f32_split3(v.x, v.y, a[0][i], a[1][i], a[2][i]);
+        f32_split3(v.z, v.w, a[0][i + 2], a[1][i + 2], a[2][i + 2]);
+      }
+#pragma unroll
+      for (int p = 0; p < 3; ++p) s_q[((wr * KS + ks) * 3 + p) * 32 + lane] = make_uint4(a[p][0], a[p][1], a[p][2], a[p][3]);
+    }
+    float acc[NB][4][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+    bool bad[2] = {false, false};
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[b][j][0] = acc[b][j][1] = acc[b][j][2] = acc[b][j][3] = 0.f;
+    int stage = 0;
+    for (int jb = jb0; jb <= jhi; jb += KEYS, stage ^= 1) {
+      if (jb + KEYS <= jhi) load(jb + KEYS, stage ^ 1);
+      else asm volatile("cp.async.commit_group;\n" ::: "memory");
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+      __syncthreads();
+      const float* ks_ = f32_smem + stage * STAGE + (wk * 16 + g) * SK + t * 4;
+      const float* vs_ = f32_smem + stage * STAGE + KEYS * SK + (wk * 16 + 2 * t) * SV + g * 4;
+      float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll 2
+      for (int ks = 0; ks < KS; ++ks) {
+        uint32_t a[3][4], b[2][3][2];
+        float c[2][4], d[2][4];
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+          const uint4 v = s_q[((wr * KS + ks) * 3 + p) * 32 + lane];
+          a[p][0] = v.x; a[p][1] = v.y; a[p][2] = v.z; a[p][3] = v.w;
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          const float4 v = *reinterpret_cast<const float4*>(ks_ + n * 8 * SK + ks * 16);
+          f32_split3(v.x, v.y, b[n][0][0], b[n][1][0], b[n][2][0]);
+          f32_split3(v.z, v.w, b[n][0][1], b[n][1][1], b[n][2][1]);
+        }
+        f32_products<2>(c, d, a, b);
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+          for (int x = 0; x < 4; ++x) s[n][x] += c[n][x] + d[n][x];
+      }
+      float corr[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        float mx = -INFINITY;
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int j = jb + wk * 16 + n * 8 + 2 * t + e;
+            float v = s[n][i * 2 + e] * scale;
+            const bool valid = j <= pos[i] && j >= lo[i];
+            if (valid && !isfinite(v)) bad[i] = true;
+            if (softcap > 0.f) v = f32_capped(v, softcap);
+            v = valid && isfinite(v) ? v : -INFINITY;
+            s[n][i * 2 + e] = v;
+            mx = fmaxf(mx, v);
+          }
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        const float m_new = fmaxf(m[i], mx);
+        corr[i] = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
+        m[i] = m_new;
+        l[i] *= corr[i];
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float v = s[n][i * 2 + e], p = v == -INFINITY ? 0.f : expf(v - m_new);
+            s[n][i * 2 + e] = p;
+            l[i] += p;
+          }
+      }
+      uint32_t pa[3][4];
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) f32_split3(s[n][i * 2], s[n][i * 2 + 1], pa[0][n * 2 + i], pa[1][n * 2 + i], pa[2][n * 2 + i]);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        float4 v[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) v[r] = *reinterpret_cast<const float4*>(vs_ + ((r & 1) + (r >> 1) * 8) * SV + b * 32);
+        uint32_t w[4][3][2];
+        float c[4][4], d[4][4];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const float4 x = v[2 * r], y = v[2 * r + 1];
+          f32_split3(x.x, y.x, w[0][0][r], w[0][1][r], w[0][2][r]);
+          f32_split3(x.y, y.y, w[1][0][r], w[1][1][r], w[1][2][r]);
+          f32_split3(x.z, y.z, w[2][0][r], w[2][1][r], w[2][2][r]);
+          f32_split3(x.w, y.w, w[3][0][r], w[3][1][r], w[3][2][r]);
+        }
+        f32_products<4>(c, d, pa, w);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int x = 0; x < 4; ++x) acc[b][j][x] = fmaf(acc[b][j][x], corr[x >> 1], c[j][x] + d[j][x]);
+      }
+      __syncthreads();                            // the stage has been read
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");      // (a run of rows that see no key has one on its way)
+    __syncthreads();
+    // the parts of the keys: every warp's results to shared memory, then all threads add them up
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int row = wr * 16 + g + i * 8;
+      l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
+      l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
+      const unsigned any = __ballot_sync(0xffffffffu, bad[i]);
+      if (t == 0) { s_m[wk][row] = m[i]; s_l[wk][row] = l[i]; s_bad[wk][row] = (any >> (g * 4)) & 15u; }
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          *reinterpret_cast<float4*>(f32_smem + (wk * 32 + row) * SV + b * 32 + t * 8 + e * 4) =
+              make_float4(acc[b][0][i * 2 + e], acc[b][1][i * 2 + e], acc[b][2][i * 2 + e], acc[b][3][i * 2 + e]);
+    }
+    __syncthreads();
+    const float* sink = sinks ? sinks + h : nullptr;
+    if (tid < 32) {                               // what each part counts
+      float mx = sink ? *sink : -INFINITY, f[KW], sum = 0.f;
+#pragma unroll
+      for (int w = 0; w < KW; ++w) mx = fmaxf(mx, s_m[w][tid]);
+#pragma unroll
+      for (int w = 0; w < KW; ++w) {
+        f[w] = s_m[w][tid] == -INFINITY ? 0.f : expf(s_m[w][tid] - mx);
+        sum = fmaf(s_l[w][tid], f[w], sum);
+        if (w > 0) s_bad[0][tid] |= s_bad[w][tid];
+      }
+      if (sink) sum += expf(*sink - mx);
+#pragma unroll
+      for (int w = 0; w < KW; ++w) s_m[w][tid] = f[w];
+      s_l[0][tid] = sum;
+    }
+    __syncthreads();
+    constexpr int RT = HD / 4;                    // threads a row
+    for (int idx = tid; idx < 32 * RT; idx += THREADS) {
+      const int r = idx / RT, c = idx % RT * 4;
+      const float* src = f32_smem + r * SV + c;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int w = 0; w < KW; ++w) {
+        const float4 x = *reinterpret_cast<const float4*>(src + w * 32 * SV);
+        const float f = s_m[w][r];
+        v.x = fmaf(x.x, f, v.x); v.y = fmaf(x.y, f, v.y); v.z = fmaf(x.z, f, v.z); v.w = fmaf(x.w, f, v.w);
+      }
+      const float sum = s_l[0][r];
+      v.x /= sum; v.y /= sum; v.z /= sum; v.w /= sum;
+      float big = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+      if (!(isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w))) big = INFINITY;
+#pragma unroll
+      for (int o = RT / 2; o > 0; o >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
+      if (c == 0 && (big == INFINITY || (big < 0x1p-90f && big != 0.f))) s_bad[0][r] = 1;
+      if (r >= first && r < end) {
+        float* o = out + (size_t)(t0 + r) * out_stride + (size_t)h * HD + c;
+        o[0] = v.x * out_scale; o[1] = v.y * out_scale; o[2] = v.z * out_scale; o[3] = v.w * out_scale;
+      }
+    }
+    __syncthreads();
+    for (int r = warp; r < 32; r += THREADS / 32)
+      if (r >= first && r < end && s_bad[0][r]) {
+        const int p_r = positions[t0 + r];
+        attn_f32_row<HD>(q + ((size_t)(t0 + r) * nh + h) * HD, k_pages, v_pages, out + (size_t)(t0 + r) * out_stride + (size_t)h * HD, bt, nkv, kvh,
+                         low(p_r), p_r, scale, softcap, sink, out_scale, lane);
+      }
+    __syncthreads();                              // the parts have been read, before the next sequence's keys
+    first = end;
+  }
+}
+
 // How many neighbouring tokens a block takes, and how many blocks share the keys.  Few tokens: one a block, and the keys shared by up
 // to eight blocks.  Tokens enough for every SM: as many neighbours a block as fit its rows (a cluster's blocks finish ONE token).
 struct AttnF32Plan { int tpb, cluster; };
@@ -1326,6 +1615,27 @@ static int attn_f32_rows(int nh, int nkv) { return nh / nkv <= 2 ? 2 : 4; }
 extern "C" void sx_attn_f32_plan(int n_tokens, int nh, int nkv, int maxp, int sms, int* out2) {
   const AttnF32Plan p = attn_f32_plan(attn_f32_rows(nh, nkv), n_tokens, nh, nkv, maxp, sms);
   out2[0] = p.tpb; out2[1] = p.cluster;
+}
+
+// Tiles of 32 rows where a sequence brings 16 tokens and more on average and there are tiles for a third of the SMs, more where a tile
+// has several sequences, which it walks through one after the other (us, the kernel of eight lanes a key first; 16 heads of 128: 33
+// tokens 7.6 and 11.4, 65 14.9 and 14.5, 129 30.5 and 18.5, 300 95 and 29, 4 x 16 12.4 and 20.3, 16 x 16 41 and 21; 16 of 64: 65 8.5
+// and 9.1, 96 12.7 and 10.7; 32 of 64: 4 x 16 behind 500 47 and 54; 32 of 128: 64 23 and 12, 8 x 16 34 and 21, 2,048 4,246 and 1,059).
+static bool attn_f32_tiles(int n_tokens, int n_seqs, int nh, int sms) {
+  const long long per_seq = n_seqs > 0 ? n_tokens / n_seqs : 0, blocks = (n_tokens + 31LL) / 32 * nh;
+  return per_seq >= 16 && blocks * (per_seq < 32 ? per_seq : 32) >= 32LL * sms / 3;
+}
+
+template <int HD>
+static int attn_f32_tile_launch(const float* q, const float* k, const float* v, float* out, const int* positions, const int* seq_of_token,
+                                const int* block_table, int maxp, int n_tokens, int nh, int nkv, float scale, int window, float softcap,
+                                const float* sinks, int chunk, int out_stride, float out_scale, cudaStream_t stream) {
+  constexpr int KW = 4;
+  const size_t smem = (size_t)2 * 16 * KW * (2 * HD + 20) * 4 + (size_t)2 * (HD / 16) * 3 * 32 * 16;
+  cudaError_t e = cudaFuncSetAttribute(attn_f32_tile_kernel<HD, KW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  return sx_launch(attn_f32_tile_kernel<HD, KW>, dim3((unsigned)nh, (unsigned)((n_tokens + 31) / 32)), dim3(64 * KW), smem, stream, q, k, v, out, positions,
+                   seq_of_token, block_table, maxp, n_tokens, nh, nkv, scale, window, softcap, sinks, chunk, out_stride, out_scale);
 }
 
 template <int HD, int R>
@@ -1347,12 +1657,17 @@ static int attn_generic_any(const void* q, const void* k_pages, const void* v_pa
                             const int* positions, const int* seq_of_token, const int* block_table,
                             int maxp, int n_tokens, int nh, int nkv, int hd, float scale, int window,
                             int dt, int vd, float softcap, const float* sinks, int chunk, int out_stride, float out_scale,
-                            cudaStream_t stream) {
+                            int n_seqs, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
   if (hd <= 0 || hd > 512 || vd <= 0 || vd > 512 || nkv <= 0 || nh % nkv != 0 || nh > 65535 || out_stride < nh * vd)
     return SX_ERR_SIZE;
   if (dt == SX_F32 && hd == vd && (hd == 64 || hd == 128) && n_tokens <= 65535 && nkv <= 8191 &&
       (((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0) {
+#define ATTN_F32_TILES(HD) attn_f32_tile_launch<HD>((const float*)q, (const float*)k_pages, (const float*)v_pages, (float*)out, positions, \
+                                                    seq_of_token, block_table, maxp, n_tokens, nh, nkv, scale, window, softcap, sinks,  \
+                                                    chunk, out_stride, out_scale, stream)
+    if (attn_f32_tiles(n_tokens, n_seqs, nh, sx_sm_count())) return hd == 64 ? ATTN_F32_TILES(64) : ATTN_F32_TILES(128);
+#undef ATTN_F32_TILES
 #define ATTN_F32(HD, R) attn_f32_launch<HD, R>((const float*)q, (const float*)k_pages, (const float*)v_pages, (float*)out, positions, \
                                                seq_of_token, block_table, maxp, n_tokens, nh, nkv, scale, window, softcap, sinks, chunk, \
                                                out_stride, out_scale, stream)
@@ -1380,17 +1695,18 @@ extern "C" int sx_attn_generic(const void* q, const void* k_pages, const void* v
                                int maxp, int n_tokens, int nh, int nkv, int hd, float scale, int window,
                                int dt, cudaStream_t stream) {
   return attn_generic_any(q, k_pages, v_pages, out, positions, seq_of_token, block_table, maxp, n_tokens, nh, nkv, hd, scale,
-                          window, dt, hd, 0.f, nullptr, 0, nh * hd, 1.f, stream);
+                          window, dt, hd, 0.f, nullptr, 0, nh * hd, 1.f, n_tokens, stream);
 }
 
-// with the options the plain entry point leaves out (see the kernel's comment)
+// with the options the plain entry point leaves out (see the kernel's comment), and how many sequences the tokens are of
+// (at most: rows of the block table)
 extern "C" int sx_attn_generic_ex(const void* q, const void* k_pages, const void* v_pages, void* out,
                                   const int* positions, const int* seq_of_token, const int* block_table,
                                   int maxp, int n_tokens, int nh, int nkv, int hd, float scale, int window,
                                   int dt, int vd, float softcap, const float* sinks, int chunk, int out_stride,
-                                  float out_scale, cudaStream_t stream) {
+                                  float out_scale, int n_seqs, cudaStream_t stream) {
   return attn_generic_any(q, k_pages, v_pages, out, positions, seq_of_token, block_table, maxp, n_tokens, nh, nkv, hd, scale,
-                          window, dt, vd, softcap, sinks, chunk, out_stride, out_scale, stream);
+                          window, dt, vd, softcap, sinks, chunk, out_stride, out_scale, n_seqs, stream);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -205,7 +205,7 @@ def attn_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, 
         c_int(block_table.shape[1]), c_int(T), c_int(nh), c_int(nkv), c_int(hd), c_float(scale),
         c_int(0 if window is None else int(window)), c_int(dt_code(q.dtype)), c_int(vd),
         c_float(0.0 if softcap is None else float(softcap)), ptr(sinks), c_int(0 if chunk is None else int(chunk)),
-        c_int(out.shape[1]), c_float(out_scale), stream()), "attn_generic")
+        c_int(out.shape[1]), c_float(out_scale), c_int(block_table.shape[0]), stream()), "attn_generic")
     return out
 
 
