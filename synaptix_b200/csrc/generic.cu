@@ -373,11 +373,12 @@ __global__ void __launch_bounds__(256, MR <= 2 ? 4 : (MR == 4 ? 3 : 2)) gemm_row
 // operand is cut into three bfloat16 pieces (8 bits each, rounded, what is left goes to the next), and of the nine products of pieces
 // the six that reach 2^-24 of the whole are taken, the smallest first.  The six of a slice are summed on their own from zero and
 // the slice's sum is added in 32 bits, rounded to nearest, so nothing depends on how the tensor cores round a long sum: one such
-// addition for 16 products, where a chain of multiply-adds had eight.  263 rows of 4,096 x 1,024 99 -> 71 us, 1,024 of 6,144 x 1,024
-// 353 -> 257 (50 TFLOP/s, 300 in bfloat16 instructions, which is what bounds it), 8,192 of 2,560 x 9,728 9.6 -> 7.1 ms; error
+// addition for 16 products, where a chain of multiply-adds had eight.  263 rows of 4,096 x 1,024 98 -> 53 us, 1,024 of 6,144 x 1,024
+// 353 -> 262 (49 TFLOP/s, 295 in bfloat16 instructions, which is what bounds it), 2,048 of 2,560 x 9,728 2.73 -> 2.00 ms; error
 // against 64 bits (2-norm, N(0, 1) operands) 4.1e-7 -> 1.5e-7 at K = 1,024, 1.3e-6 -> 4.5e-7 at 9,728.
-// Where a sum is not finite (a piece of an infinity is no number, and the largest numbers have pieces that overflow) or so small
-// that pieces of its operands may have fallen below 2^-133, the least bfloat16, it is formed again from whole products.
+// The pieces are those of 2^16 times a number (f32_split3_up), so that none of its bits lies below the least bfloat16, and sums are
+// taken back by 2^-32 at the end.  Where one is not finite (a piece of an infinity is no number; operands from 2^112 on and sums from
+// 2^96 on are too large) it is formed again from whole products.
 // A thread's four values of a row are neighbours (16 bytes; their order within the instruction's 16 does not matter), so rows need no
 // padding: eight lanes read two rows of 64 bytes.  Where tiles are few, K is shared by the blocks of a cluster (grid x =
 // column tile * cluster), which lay their partial tiles into shared memory and add them up in block order, each a share of the rows.
@@ -407,6 +408,14 @@ __device__ __forceinline__ void f32_split3(float x, float y, uint32_t& p0, uint3
     y -= __uint_as_float(p[i] & 0xffff0000u);
   }
   p0 = p[0]; p1 = p[1]; p2 = p[2];
+}
+// The same of 2^16 x and 2^16 y: every 32-bit number is a multiple of 2^-149, so 2^16 of it one of 2^-133, the least bfloat16, and its
+// three pieces are all of it whatever its size.  (From 2^112 on the first piece is infinite, and so no sum with it is finite.)  The two
+// multiplications cost the products 2 to 3.5 % (300 rows of 4,096 x 1,024 75.0 -> 76.8 us, 2,048 of 2,560 x 9,728 1,967 -> 2,004).
+#define F32_UP 0x1p16f
+#define F32_DOWN 0x1p-32f             // a product of two such
+__device__ __forceinline__ void f32_split3_up(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+  f32_split3(x * F32_UP, y * F32_UP, p0, p1, p2);
 }
 // slices of 16 of N products, in two sums: of the leading pieces (their products have 16 bits, so little is rounded), and of the
 // other five products of pieces, 2^-8 of the whole
@@ -486,8 +495,8 @@ __global__ void __launch_bounds__(128, 3) gemm_tile_f32_kernel(const float* __re
 #pragma unroll
       for (int h = 0; h < 2; ++h) {               // rows g and g + 8
         const float4 v = *reinterpret_cast<const float4*>(as + (i * 16 + h * 8) * F32_BK);
-        f32_split3(v.x, v.y, a[i][0][h], a[i][1][h], a[i][2][h]);
-        f32_split3(v.z, v.w, a[i][0][h + 2], a[i][1][h + 2], a[i][2][h + 2]);
+        f32_split3_up(v.x, v.y, a[i][0][h], a[i][1][h], a[i][2][h]);
+        f32_split3_up(v.z, v.w, a[i][0][h + 2], a[i][1][h + 2], a[i][2][h + 2]);
       }
 #pragma unroll
     for (int j0 = 0; j0 < NT; j0 += 4) {
@@ -495,8 +504,8 @@ __global__ void __launch_bounds__(128, 3) gemm_tile_f32_kernel(const float* __re
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float4 v = *reinterpret_cast<const float4*>(ws + (j0 + j) * 8 * F32_BK);
-        f32_split3(v.x, v.y, b[j][0][0], b[j][1][0], b[j][2][0]);
-        f32_split3(v.z, v.w, b[j][0][1], b[j][1][1], b[j][2][1]);
+        f32_split3_up(v.x, v.y, b[j][0][0], b[j][1][0], b[j][2][0]);
+        f32_split3_up(v.z, v.w, b[j][0][1], b[j][1][1], b[j][2][1]);
       }
       float c[2][4][4];
       constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
@@ -517,9 +526,14 @@ __global__ void __launch_bounds__(128, 3) gemm_tile_f32_kernel(const float* __re
           for (int x = 0; x < 4; ++x) acc[i][j0 + j][x] += c[i][j][x];
     }
   }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) acc[i][j][x] *= F32_DOWN;
   auto store = [&](int m, int n, float v) {
-    const float mag = fabsf(v);
-    if (!(mag <= 3.4028234e38f) || (mag < 0x1p-90f && mag != 0.f)) v = f32_whole(A + (size_t)m * K, W + (size_t)n * K, K);
+    if (!(fabsf(v) <= 3.4028234e38f)) v = f32_whole(A + (size_t)m * K, W + (size_t)n * K, K);
     C[(size_t)m * N + n] = soft_limit(bias ? v + bias[n] : v, cap);
   };
   if (cluster == 1) {

@@ -1,6 +1,6 @@
 """Float32 products of more than 16 rows, whose operands go to the tensor cores in pieces, over the range of 32-bit numbers against
-64-bit sums.  Bounds: a product of pieces is off by 2^-23 of the whole at most (three products of pieces are left out, each below
-2^-24 / 2^8 of it, and two roundings), a sum of 16 in the tensor cores by 16 * 2^-23 of its magnitudes (whatever way they round),
+64-bit sums: numbers near the least and near the largest, on either side and against each other.  Bounds: a product of pieces is off
+by 2^-23 of the whole at most (three products of pieces are left out, each below 2^-24 / 2^8 of it, and two roundings), a sum of 16 in the tensor cores by 16 * 2^-23 of its magnitudes (whatever way they round),
 and the K / 16 sums of slices by 2^-24 each: below (K + 3) 2^-24, what the same sum of whole products is given, from K = 64 on."""
 import pytest
 import torch
@@ -17,7 +17,8 @@ def operands(M, N, K, seed=0):
 # tiles of 32 and of 64 rows with their remainders, one block a tile and clusters of all sizes, slices of 16 with remainders
 @pytest.mark.parametrize("M,N,K", [(17, 389, 64), (32, 128, 1020), (33, 129, 84), (64, 4100, 260), (65, 7, 4096), (263, 1024, 3072),
                                    (700, 2600, 132)])
-@pytest.mark.parametrize("up,down", [(0, 0), (-60, 0), (0, -118), (-70, -30), (60, 55), (100, -100)])
+@pytest.mark.parametrize("up,down", [(0, 0), (-60, 0), (0, -118), (-70, -30), (60, 55), (100, -100), (60, -120), (110, -125), (100, -126), (100, -140),
+                                     (-140, 100), (0, -140), (-70, -70)])
 def test_products_over_the_range(M, N, K, up, down):
     from synaptix_b200 import ops
     a, w = operands(M, N, K)
