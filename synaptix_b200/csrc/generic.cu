@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(256, MR <= 2 ? 4 : (MR == 4 ? 3 : 2)) gemm_row
 // addition for 16 products, where a chain of multiply-adds had eight.  263 rows of 4,096 x 1,024 98 -> 53 us, 1,024 of 6,144 x 1,024
 // 353 -> 262 (49 TFLOP/s, 295 in bfloat16 instructions, which is what bounds it), 2,048 of 2,560 x 9,728 2.73 -> 2.00 ms; error
 // against 64 bits (2-norm, N(0, 1) operands) 4.1e-7 -> 1.5e-7 at K = 1,024, 1.3e-6 -> 4.5e-7 at 9,728.
-// The pieces are those of 2^16 times a number (f32_split3_up), so that none of its bits lies below the least bfloat16, and sums are
+// The pieces are those of 2^16 times a number, so that none of its bits lies below the least bfloat16, and sums are
 // taken back by 2^-32 at the end.  Where one is not finite (a piece of an infinity is no number; operands from 2^112 on and sums from
 // 2^96 on are too large) it is formed again from whole products.
 // A thread's four values of a row are neighbours (16 bytes; their order within the instruction's 16 does not matter), so rows need no
@@ -397,6 +397,18 @@ __device__ __forceinline__ void f32_mma(float (&c)[4], const uint32_t (&a)[4], c
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
+// What is cut into pieces is 2^16 times a number: every 32-bit number is a multiple of 2^-149, so 2^16 of it one of 2^-133, the least
+// bfloat16, and its three pieces are all of it whatever its size.  (From 2^112 on the first piece is infinite, and so no sum with it
+// is finite.)
+#define F32_UP 0x1p16f
+#define F32_DOWN 0x1p-32f             // a product of two such
+// (Two numbers an instruction.  Against pieces of the numbers themselves, which lose bits below 2^-109: products 0 to 2 %, 300 rows of
+// 4,096 x 1,024 75.0 -> 75.6 us; attention of 2,048 tokens, 16 heads of 128, 530 -> 549, of 64 322 -> 316.  One at a time 2 to 3.5 and 5.5 %.)
+__device__ __forceinline__ float4 f32_up(float4 v) {
+  asm("{\n .reg .b64 a, b, u;\n mov.b64 u, {%4, %4};\n mov.b64 a, {%0, %1};\n mov.b64 b, {%2, %3};\n mul.rn.f32x2 a, a, u;\n mul.rn.f32x2 b, b, u;\n"
+      " mov.b64 {%0, %1}, a;\n mov.b64 {%2, %3}, b;\n}\n" : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w) : "f"(F32_UP));
+  return v;
+}
 // two numbers in three pieces each: p[i] holds piece i of x (low half) and of y
 __device__ __forceinline__ void f32_split3(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
   uint32_t p[3];
@@ -408,14 +420,6 @@ __device__ __forceinline__ void f32_split3(float x, float y, uint32_t& p0, uint3
     y -= __uint_as_float(p[i] & 0xffff0000u);
   }
   p0 = p[0]; p1 = p[1]; p2 = p[2];
-}
-// The same of 2^16 x and 2^16 y: every 32-bit number is a multiple of 2^-149, so 2^16 of it one of 2^-133, the least bfloat16, and its
-// three pieces are all of it whatever its size.  (From 2^112 on the first piece is infinite, and so no sum with it is finite.)  The two
-// multiplications cost the products 2 to 3.5 % (300 rows of 4,096 x 1,024 75.0 -> 76.8 us, 2,048 of 2,560 x 9,728 1,967 -> 2,004).
-#define F32_UP 0x1p16f
-#define F32_DOWN 0x1p-32f             // a product of two such
-__device__ __forceinline__ void f32_split3_up(float x, float y, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
-  f32_split3(x * F32_UP, y * F32_UP, p0, p1, p2);
 }
 // slices of 16 of N products, in two sums: of the leading pieces (their products have 16 bits, so little is rounded), and of the
 // other five products of pieces, 2^-8 of the whole
@@ -494,18 +498,18 @@ __global__ void __launch_bounds__(128, 3) gemm_tile_f32_kernel(const float* __re
     for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {               // rows g and g + 8
-        const float4 v = *reinterpret_cast<const float4*>(as + (i * 16 + h * 8) * F32_BK);
-        f32_split3_up(v.x, v.y, a[i][0][h], a[i][1][h], a[i][2][h]);
-        f32_split3_up(v.z, v.w, a[i][0][h + 2], a[i][1][h + 2], a[i][2][h + 2]);
+        const float4 v = f32_up(*reinterpret_cast<const float4*>(as + (i * 16 + h * 8) * F32_BK));
+        f32_split3(v.x, v.y, a[i][0][h], a[i][1][h], a[i][2][h]);
+        f32_split3(v.z, v.w, a[i][0][h + 2], a[i][1][h + 2], a[i][2][h + 2]);
       }
 #pragma unroll
     for (int j0 = 0; j0 < NT; j0 += 4) {
       uint32_t b[4][3][2];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float4 v = *reinterpret_cast<const float4*>(ws + (j0 + j) * 8 * F32_BK);
-        f32_split3_up(v.x, v.y, b[j][0][0], b[j][1][0], b[j][2][0]);
-        f32_split3_up(v.z, v.w, b[j][0][1], b[j][1][1], b[j][2][1]);
+        const float4 v = f32_up(*reinterpret_cast<const float4*>(ws + (j0 + j) * 8 * F32_BK));
+        f32_split3(v.x, v.y, b[j][0][0], b[j][1][0], b[j][2][0]);
+        f32_split3(v.z, v.w, b[j][0][1], b[j][1][1], b[j][2][1]);
       }
       float c[2][4][4];
       constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0};
@@ -1347,8 +1351,7 @@ __global__ void __launch_bounds__(256) attn_f32_kernel(
 // A row's query pieces lie in shared memory as the instructions take them; keys and values come through two stages (cp.async), rows
 // padded so that 16-byte reads meet no bank twice.  Within an instruction the order of the 16 elements of a head (scores) and of
 // the 32 columns of four instructions (values) is the one in which a thread's numbers are neighbours in memory.  A row with a
-// score or result that is not finite, or with results so small that pieces of the values may have been lost, is done again in 32
-// bits by a warp (attn_f32_row).  Two prompts of 150 tokens, 16 heads of 128: 70 -> 30 us, what is left is the latency of a page
+// score or result that is not finite is done again in 32 bits by a warp (attn_f32_row).  Two prompts of 150 tokens, 16 heads of 128: 70 -> 30 us, what is left is the latency of a page
 // (3.5 us: 192 products of pieces and 1,000 other instructions a warp); with four warps and 32 keys a turn 37 us (2,048 tokens 930
 // against 1,059), with the results scaled and divided by the threads that hold them, 64 divisions one after the other, 44.
 // ---------------------------------------------------------------------------------------
@@ -1439,8 +1442,8 @@ __global__ void __launch_bounds__(64 * KW, 4 / KW) attn_f32_tile_kernel(
       uint32_t a[3][4];
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const float4 v = pos[i] >= 0 ? *reinterpret_cast<const float4*>(q + ((size_t)(t0 + wr * 16 + g + i * 8) * nh + h) * HD + ks * 16 + t * 4)
-                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 v = f32_up(pos[i] >= 0 ? *reinterpret_cast<const float4*>(q + ((size_t)(t0 + wr * 16 + g + i * 8) * nh + h) * HD + ks * 16 + t * 4)
+                                            : make_float4(0.f, 0.f, 0.f, 0.f));
         f32_split3(v.x, v.y, a[0][i], a[1][i], a[2][i]);
         f32_split3(v.z, v.w, a[0][i + 2], a[1][i + 2], a[2][i + 2]);
       }
@@ -1473,7 +1476,7 @@ __global__ void __launch_bounds__(64 * KW, 4 / KW) attn_f32_tile_kernel(
         }
 #pragma unroll
         for (int n = 0; n < 2; ++n) {
-          const float4 v = *reinterpret_cast<const float4*>(ks_ + n * 8 * SK + ks * 16);
+          const float4 v = f32_up(*reinterpret_cast<const float4*>(ks_ + n * 8 * SK + ks * 16));
           f32_split3(v.x, v.y, b[n][0][0], b[n][1][0], b[n][2][0]);
           f32_split3(v.z, v.w, b[n][0][1], b[n][1][1], b[n][2][1]);
         }
@@ -1492,7 +1495,7 @@ __global__ void __launch_bounds__(64 * KW, 4 / KW) attn_f32_tile_kernel(
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int j = jb + wk * 16 + n * 8 + 2 * t + e;
-            float v = s[n][i * 2 + e] * scale;
+            float v = s[n][i * 2 + e] * F32_DOWN * scale;
             const bool valid = j <= pos[i] && j >= lo[i];
             if (valid && !isfinite(v)) bad[i] = true;
             if (softcap > 0.f) v = f32_capped(v, softcap);
@@ -1519,12 +1522,12 @@ __global__ void __launch_bounds__(64 * KW, 4 / KW) attn_f32_tile_kernel(
 #pragma unroll
       for (int n = 0; n < 2; ++n)
 #pragma unroll
-        for (int i = 0; i < 2; ++i) f32_split3(s[n][i * 2], s[n][i * 2 + 1], pa[0][n * 2 + i], pa[1][n * 2 + i], pa[2][n * 2 + i]);
+        for (int i = 0; i < 2; ++i) f32_split3(s[n][i * 2] * F32_UP, s[n][i * 2 + 1] * F32_UP, pa[0][n * 2 + i], pa[1][n * 2 + i], pa[2][n * 2 + i]);
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         float4 v[4];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) v[r] = *reinterpret_cast<const float4*>(vs_ + ((r & 1) + (r >> 1) * 8) * SV + b * 32);
+        for (int r = 0; r < 4; ++r) v[r] = f32_up(*reinterpret_cast<const float4*>(vs_ + ((r & 1) + (r >> 1) * 8) * SV + b * 32));
         uint32_t w[4][3][2];
         float c[4][4], d[4][4];
 #pragma unroll
@@ -1590,12 +1593,8 @@ __global__ void __launch_bounds__(64 * KW, 4 / KW) attn_f32_tile_kernel(
         v.x = fmaf(x.x, f, v.x); v.y = fmaf(x.y, f, v.y); v.z = fmaf(x.z, f, v.z); v.w = fmaf(x.w, f, v.w);
       }
       const float sum = s_l[0][r];
-      v.x /= sum; v.y /= sum; v.z /= sum; v.w /= sum;
-      float big = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-      if (!(isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w))) big = INFINITY;
-#pragma unroll
-      for (int o = RT / 2; o > 0; o >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
-      if (c == 0 && (big == INFINITY || (big < 0x1p-90f && big != 0.f))) s_bad[0][r] = 1;
+      v.x = v.x / sum * F32_DOWN; v.y = v.y / sum * F32_DOWN; v.z = v.z / sum * F32_DOWN; v.w = v.w / sum * F32_DOWN;
+      if (!(isfinite(v.x) && isfinite(v.y) && isfinite(v.z) && isfinite(v.w))) s_bad[0][r] = 1;
       if (r >= first && r < end) {
         float* o = out + (size_t)(t0 + r) * out_stride + (size_t)h * HD + c;
         o[0] = v.x * out_scale; o[1] = v.y * out_scale; o[2] = v.z * out_scale; o[3] = v.w * out_scale;

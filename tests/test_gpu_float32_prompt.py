@@ -91,3 +91,30 @@ def test_numbers_at_the_ends_of_the_range():
     off = (hd + 4) * ULP * float(q.norm(dim=-1).max()) * float(ks[0][kept].nan_to_num().norm(dim=-1).max()) * scale
     finite = vs[0][vs[0].isfinite()].abs().max()
     assert (got - clean).abs().max() <= (2 * off + (n + 16) * ULP) * float(finite)
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("case", ["scores", "columns", "weights"])
+def test_small_numbers_against_large_ones(hd, case):
+    """Keys below the least numbers whose pieces are whole against large queries; columns of values of different sizes; a weight
+    that small against large values.  Every result within the bound of its own magnitudes, a weight's own last bit (2^-149) among them."""
+    nh, nkv, n = 40, 8, 140
+    q, ks, vs, pos, sot = setup(nh, nkv, hd, [0], [n], 3)
+    scale = 1 / math.sqrt(hd)
+    if case == "scores":
+        q, ks[0], scale = q * 2.0 ** 104, ks[0] * 2.0 ** -122, scale * 2.0 ** 18
+    elif case == "columns":
+        vs[0] *= torch.tensor([2.0 ** -(41 * (d % 4)) for d in range(hd)])
+    else:                                            # of neighbouring keys one has the weight 2^-130 and values of 2^106
+        q[..., 3], ks[0][:, :, 3] = 1.0, 0.0
+        ks[0][1::2, :, 3] = -90 / scale
+        vs[0][1::2] *= 2.0 ** 106
+        vs[0][::2] *= 2.0 ** -40
+    out = run(q, ks, vs, pos, sot, [0], [n], nkv, hd, scale).cpu().view(n, nh, hd).double()
+    for h in range(nh):
+        k, v = ks[0][:, h // 5].double(), vs[0][:, h // 5].double()
+        z = (q[:, h].double() @ k.T) * scale
+        w = torch.softmax(z.masked_fill(torch.ones(n, n, dtype=torch.bool).triu(1), -math.inf), -1)
+        off = (hd + 4) * ULP * float((q[:, h].double().abs() @ k.abs().T).max()) * scale
+        bound = (2 * off + (n + 16) * ULP) * (w @ v.abs()) + 2.0 ** -149 * v.abs().sum(0) + n * 2.0 ** -149
+        assert ((out[:, h] - w @ v).abs() <= bound).all(), h
