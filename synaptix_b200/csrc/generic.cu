@@ -373,12 +373,13 @@ __global__ void __launch_bounds__(256, MR <= 2 ? 4 : (MR == 4 ? 3 : 2)) gemm_row
 // operand is cut into three bfloat16 pieces (8 bits each, rounded, what is left goes to the next), and of the nine products of pieces
 // the six that reach 2^-24 of the whole are taken, the smallest first.  The six of a slice are summed on their own from zero and
 // the slice's sum is added in 32 bits, rounded to nearest, so nothing depends on how the tensor cores round a long sum: one such
-// addition for 16 products, where a chain of multiply-adds had eight.  263 rows of 4,096 x 1,024 98 -> 53 us, 1,024 of 6,144 x 1,024
-// 353 -> 262 (49 TFLOP/s, 295 in bfloat16 instructions, which is what bounds it), 2,048 of 2,560 x 9,728 2.73 -> 2.00 ms; error
+// addition for 16 products, where a chain of multiply-adds had eight.  263 rows of 4,096 x 1,024 98 -> 49 us, 1,024 of 6,144 x 1,024
+// 353 -> 258 (50 TFLOP/s, 300 in bfloat16 instructions, which is what bounds it), 2,048 of 2,560 x 9,728 2.73 -> 2.00 ms; error
 // against 64 bits (2-norm, N(0, 1) operands) 4.1e-7 -> 1.5e-7 at K = 1,024, 1.3e-6 -> 4.5e-7 at 9,728.
 // The pieces are those of 2^16 times a number, so that none of its bits lies below the least bfloat16, and sums are
 // taken back by 2^-32 at the end.  Where one is not finite (a piece of an infinity is no number; operands from 2^112 on and sums from
-// 2^96 on are too large) it is formed again from whole products.
+// 2^96 on are too large) its block forms the tile again in multiply-adds of whole numbers and takes those of it
+// (2,048 of 2,560 x 9,728 2.00 ms, with a row of NaN 2.01, all of them NaN 4.8).
 // A thread's four values of a row are neighbours (16 bytes; their order within the instruction's 16 does not matter), so rows need no
 // padding: eight lanes read two rows of 64 bytes.  Where tiles are few, K is shared by the blocks of a cluster (grid x =
 // column tile * cluster), which lay their partial tiles into shared memory and add them up in block order, each a share of the rows.
@@ -436,15 +437,8 @@ __device__ __forceinline__ void f32_products(float (&c)[N][4], float (&d)[N][4],
       else f32_mma(d[n], a[PA[p]], b[n][PB[p]]);
     }
 }
-// one element of the product from whole numbers
-__device__ __noinline__ float f32_whole(const float* __restrict__ a, const float* __restrict__ w, int K) {
-  float s = 0.f;
-  for (int k = 0; k < K; ++k) s = fmaf(a[k], w[k], s);
-  return s;
-}
-
 template <int BM>
-__global__ void __launch_bounds__(128, 3) gemm_tile_f32_kernel(const float* __restrict__ A, const float* __restrict__ W,
+__global__ void __launch_bounds__(128, BM == 32 ? 4 : 3) gemm_tile_f32_kernel(const float* __restrict__ A, const float* __restrict__ W,
                                                             float* __restrict__ C, int M, int N, int K,
                                                             const float* __restrict__ bias, float cap, int cluster) {
   constexpr int BN = 128, ROWS = BM + BN, STAGE = ROWS * F32_BK, WM = BM / 32, WN = 4 / WM, NT = BN / WN / 8;   // a warp: 32 rows x NT tiles of 8 columns
@@ -530,44 +524,78 @@ __global__ void __launch_bounds__(128, 3) gemm_tile_f32_kernel(const float* __re
           for (int x = 0; x < 4; ++x) acc[i][j0 + j][x] += c[i][j][x];
     }
   }
+  float* part = f32_smem + F32_STAGES * STAGE;    // (a cluster's: the block's partial tile)
+  auto store = [&](int m, int n, float v) { C[(size_t)m * N + n] = soft_limit(bias ? v + bias[n] : v, cap); };
+  auto put = [&](int i, int j, int x, float v) {
+    const int r = wm + i * 16 + g + (x >> 1) * 8, c = wn + j * 8 + 2 * t + (x & 1);
+    if (cluster > 1) part[r * BN + c] = v;
+    else if (m0 + r < M && n0 + c < N) store(m0 + r, n0 + c, v);
+  };
+  uint32_t odd[2] = {0u, 0u};                     // of a thread's sums, those that are not finite
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
-      for (int x = 0; x < 4; ++x) acc[i][j][x] *= F32_DOWN;
-  auto store = [&](int m, int n, float v) {
-    if (!(fabsf(v) <= 3.4028234e38f)) v = f32_whole(A + (size_t)m * K, W + (size_t)n * K, K);
-    C[(size_t)m * N + n] = soft_limit(bias ? v + bias[n] : v, cap);
-  };
-  if (cluster == 1) {
+      for (int x = 0; x < 4; ++x) {
+        const float v = acc[i][j][x] * F32_DOWN;
+        odd[i] |= isfinite(v) ? 0u : 1u << (j * 4 + x);
+        put(i, j, x, v);
+      }
+  // (every copy has landed and been read: the groups behind the last slice are empty)
+  if (__syncthreads_or(odd[0] | odd[1])) {        // the tile once more, in whole numbers, for those sums
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
+#pragma unroll 1
+    for (int s = 0; s < F32_STAGES - 1; ++s) {
+      if (s < nkb) load(s, s);
+      else asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+#pragma unroll 1
+    for (int kb = 0; kb < nkb; ++kb) {
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(F32_STAGES - 2) : "memory");
+      __syncthreads();
+      if (kb + F32_STAGES - 1 < nkb) load(kb + F32_STAGES - 1, (kb + F32_STAGES - 1) % F32_STAGES);
+      else asm volatile("cp.async.commit_group;\n" ::: "memory");
+      const float* as = f32_smem + (kb % F32_STAGES) * STAGE + (wm + g) * F32_BK;
+      const float* ws = f32_smem + (kb % F32_STAGES) * STAGE + (BM + wn + 2 * t) * F32_BK;
+#pragma unroll 1
+      for (int q = 0; q < 4; ++q) {
+        const int k = ((q + t) & 3) * 4;          // (lanes with other columns at other places of a row: other banks)
+        float4 v[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) v[r] = *reinterpret_cast<const float4*>(as + r * 8 * F32_BK + k);
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float4 w = *reinterpret_cast<const float4*>(ws + (j * 8 + e) * F32_BK + k);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+              float& c = acc[r >> 1][j][(r & 1) * 2 + e];
+              c = fmaf(v[r].w, w.w, fmaf(v[r].z, w.z, fmaf(v[r].y, w.y, fmaf(v[r].x, w.x, c))));
+            }
+          }
+      }
+    }
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int j = 0; j < NT; ++j)
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          const int m = m0 + wm + i * 16 + g + (x >> 1) * 8, n = n0 + wn + j * 8 + 2 * t + (x & 1);
-          if (m < M && n < N) store(m, n, acc[i][j][x]);
-        }
-    return;
+        for (int x = 0; x < 4; ++x)
+          if (odd[i] >> (j * 4 + x) & 1u) put(i, j, x, acc[i][j][x]);
   }
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  __syncthreads();                                // the ring has been read: the partial tile goes over it
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-      for (int x = 0; x < 4; x += 2)
-        *reinterpret_cast<float2*>(f32_smem + (wm + i * 16 + g + (x >> 1) * 8) * BN + wn + j * 8 + 2 * t) = make_float2(acc[i][j][x], acc[i][j][x + 1]);
+  if (cluster == 1) return;
   cluster_sync_all();
   const int per = (BM + cluster - 1) / cluster, r1 = min(BM, (z + 1) * per);
   for (int r = z * per; r < r1; ++r) {
     const int m = m0 + r, n = n0 + tid;
     if (m >= M) break;
     float s = 0.f;
-    for (int c = 0; c < cluster; ++c) s += cluster_load_f32(f32_smem + r * BN + tid, (uint32_t)c);
+    for (int c = 0; c < cluster; ++c) s += cluster_load_f32(part + r * BN + tid, (uint32_t)c);
     if (n < N) store(m, n, s);
   }
   cluster_sync_all();                             // nobody's shared memory goes away while it is read
@@ -614,8 +642,7 @@ static int gemm_tile_f32_launch(const float* A, const float* W, float* C, int M,
                                 int cluster, cudaStream_t stream) {
   constexpr int BN = 128;
   const long long tiles_n = (N + BN - 1) / BN, tiles_m = (M + BM - 1) / BM;
-  static_assert(F32_STAGES * (BM + BN) * F32_BK >= BM * BN, "the ring holds a partial tile");
-  const size_t ring = (size_t)F32_STAGES * (BM + BN) * F32_BK * sizeof(float);
+  const size_t ring = ((size_t)F32_STAGES * (BM + BN) * F32_BK + (cluster > 1 ? BM * BN : 0)) * sizeof(float);
   cudaError_t e = cudaFuncSetAttribute(gemm_tile_f32_kernel<BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ring);
   if (e != cudaSuccess) return (int)e;
   const dim3 grid((unsigned)(tiles_n * cluster), (unsigned)tiles_m);

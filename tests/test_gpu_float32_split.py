@@ -53,3 +53,43 @@ def test_numbers_at_the_ends_of_the_range(M):
     assert torch.isinf(y[1, :11]).all() and (y[1, :11] < 0).all() and y[1, 11].isnan() and y[2].isnan().all()
     assert (y[4, :9] == 2.0 ** 126).all() and y[4, 9] == float("inf") and (y[5:] == 0).all()
     assert torch.allclose(y[3], torch.full_like(y[3], 2.0 ** -127 * 1.5), rtol=0, atol=2.0 ** -149)
+
+
+@pytest.mark.parametrize("M,N,K", [(32, 260, 1024), (300, 1024, 3072), (2048, 2560, 260)])
+def test_sums_that_are_not_finite(M, N, K):
+    """Rows and columns with a NaN, an infinity or numbers too large for pieces, also where K is shared by a cluster: they are what
+    the numbers give, and the other sums are what they are without them, bit by bit."""
+    from synaptix_b200 import ops
+    a, w = operands(M, N, K, 9)
+    plain = ops.gemm_generic(a, w)
+    a[3, K - 1], a[17, 5], w[130, 0] = float("nan"), float("inf"), float("-inf")
+    a[M - 2] = a[M - 2].abs() * 2.0 ** 115
+    w[N - 1] = w[N - 1].abs() * 2.0 ** 113           # (row M - 2 with column N - 1 overflows, in any order of the sum)
+    got, want = ops.gemm_generic(a, w), a.double() @ w.double().T
+    want = want.float().double()                     # (to infinity where it overflows)
+    other = want.isfinite()
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf()) and (got[got.isinf()] == want[want.isinf()]).all()
+    bound = (K + 3) * ULP * (a.double().abs() @ w.double().abs().T)
+    assert ((got.double() - want).abs() <= bound)[other].all()
+    kept = torch.ones(M, N, dtype=torch.bool, device="cuda")
+    kept[[3, 17, M - 2]], kept[:, [130, N - 1]] = False, False
+    assert torch.equal(got[kept], plain[kept])
+
+
+def test_time_of_sums_that_are_not_finite():
+    """Half of all sums NaN: the tiles once in pieces and once in whole numbers, not a multiple of that."""
+    from synaptix_b200 import ops
+    a, w = operands(1024, 2048, 2048)
+    b = a.clone()
+    b[::2, 7] = float("nan")
+
+    def ms(x):
+        ops.gemm_generic(x, w)
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        for _ in range(5):
+            ops.gemm_generic(x, w)
+        end.record()
+        end.synchronize()
+        return start.elapsed_time(end)
+    assert ms(b) <= 8 * ms(a)
