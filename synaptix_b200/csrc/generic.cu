@@ -1378,31 +1378,50 @@ __global__ void __launch_bounds__(256) attn_f32_kernel(
 // A row's query pieces lie in shared memory as the instructions take them; keys and values come through two stages (cp.async), rows
 // padded so that 16-byte reads meet no bank twice.  Within an instruction the order of the 16 elements of a head (scores) and of
 // the 32 columns of four instructions (values) is the one in which a thread's numbers are neighbours in memory.  A row with a
-// score or result that is not finite is done again in 32 bits by a warp (attn_f32_row).  Two prompts of 150 tokens, 16 heads of 128: 70 -> 30 us, what is left is the latency of a page
+// score or result that is not finite is done again in 32 bits by a warp (attn_f32_row; two prompts of 150 tokens, all rows so, 32 -> 76 us,
+// 2,048 tokens 0.55 -> 3.07 ms, where the kernel above takes 2.5).  Two prompts of 150 tokens, 16 heads of 128: 70 -> 30 us, what is left is the latency of a page
 // (3.5 us: 192 products of pieces and 1,000 other instructions a warp); with four warps and 32 keys a turn 37 us (2,048 tokens 930
 // against 1,059), with the results scaled and divided by the threads that hold them, 64 divisions one after the other, 44.
 // ---------------------------------------------------------------------------------------
+// one query row by one warp, 16 keys at a time: their keys and values are on the way together
 template <int HD>
 __device__ __noinline__ void attn_f32_row(const float* __restrict__ q, const float* __restrict__ k_pages, const float* __restrict__ v_pages,
                                           float* __restrict__ out, const int* __restrict__ bt, int nkv, int kvh, int lo, int pos,
                                           float scale, float softcap, const float* sink, float out_scale, int lane) {
-  constexpr int C = HD / 32;
+  constexpr int C = HD / 32, B = 16;
   float qv[C], acc[C], m = -INFINITY, l = 0.f;
 #pragma unroll
   for (int c = 0; c < C; ++c) { qv[c] = q[c * 32 + lane]; acc[c] = 0.f; }
-  for (int j = lo; j <= pos; ++j) {
-    const size_t at = (((size_t)bt[j >> 6] * nkv + kvh) * SX_PAGE + (j & 63)) * HD + lane;
-    float d = 0.f;
+#pragma unroll 1
+  for (int j0 = lo & ~(B - 1); j0 <= pos; j0 += B) {
+    const size_t at = (((size_t)bt[j0 >> 6] * nkv + kvh) * SX_PAGE + (j0 & 63)) * HD + lane;
+    float d[B], v[B][C];
 #pragma unroll
-    for (int c = 0; c < C; ++c) d = fmaf(qv[c], k_pages[at + c * 32], d);
-    float s = warp_sum(d) * scale;
+    for (int b = 0; b < B; ++b) {
+      const bool seen = j0 + b >= lo && j0 + b <= pos;           // (what lies beside them may be anything)
+      d[b] = 0.f;
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        d[b] = fmaf(qv[c], seen ? k_pages[at + b * HD + c * 32] : 0.f, d[b]);
+        v[b][c] = seen ? v_pages[at + b * HD + c * 32] : 0.f;
+      }
+    }
+    float s = warp_fold<B>(d, lane) * scale;                     // of key lane / 2
     if (softcap > 0.f) s = softcap * tanhf(s / softcap);
-    const float m_new = fmaxf(m, s);
+    const int j = j0 + lane / 2;
+    if (j < lo || j > pos) s = -INFINITY;
+    const float m_new = fmaxf(m, warp_max(s));
     const float corr = m == -INFINITY ? 0.f : expf(m - m_new), p = s == -INFINITY ? 0.f : expf(s - m_new);
     m = m_new;
-    l = fmaf(l, corr, p);
+    l = fmaf(l, corr, warp_sum(lane & 1 ? 0.f : p));
 #pragma unroll
-    for (int c = 0; c < C; ++c) acc[c] = fmaf(p, v_pages[at + c * 32], acc[c] * corr);
+    for (int c = 0; c < C; ++c) acc[c] *= corr;
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      const float pb = __shfl_sync(0xffffffffu, p, 2 * b);
+#pragma unroll
+      for (int c = 0; c < C; ++c) acc[c] = fmaf(pb, v[b][c], acc[c]);
+    }
   }
   const float mx = sink ? fmaxf(m, *sink) : m, f = m == -INFINITY ? 0.f : expf(m - mx);
   const float sum = l * f + (sink ? expf(*sink - mx) : 0.f);

@@ -118,3 +118,30 @@ def test_small_numbers_against_large_ones(hd, case):
         off = (hd + 4) * ULP * float((q[:, h].double().abs() @ k.abs().T).max()) * scale
         bound = (2 * off + (n + 16) * ULP) * (w @ v.abs()) + 2.0 ** -149 * v.abs().sum(0) + n * 2.0 ** -149
         assert ((out[:, h] - w @ v).abs() <= bound).all(), h
+
+
+def test_time_of_rows_that_are_not_finite():
+    """A key whose scores overflow, seen by all rows behind it: the rows once in pieces and once in 32 bits, 16 keys at a time."""
+    from synaptix_b200 import ops
+    nh, nkv, hd, n = 16, 8, 128, 1024
+    q, ks, vs, pos, sot = setup(nh, nkv, hd, [0], [n], 7)
+    ks[0][:, :, 0] = 0.0
+    kp, vp, bt = make_paged(ks, vs, nkv, hd, torch.float32, seed=2)
+    big = q.clone()
+    big[..., 0] = 1e20
+    far = kp.clone()
+    far[int(bt[0, 0]), :, 7, 0] = -1e20
+
+    def ms(q, k):
+        q, p, s = dev(q.view(n, -1)), dev(pos), dev(sot)
+        one = lambda: ops.attn_generic(q, k, vp, p, s, bt, nh, nkv, hd, hd ** -0.5)  # noqa: E731
+        one()
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        for _ in range(5):
+            y = one()
+        end.record()
+        end.synchronize()
+        assert y.isfinite().all()
+        return start.elapsed_time(end)
+    assert ms(big, far) <= 10 * ms(q, kp)
