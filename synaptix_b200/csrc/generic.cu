@@ -1194,19 +1194,31 @@ __global__ void __launch_bounds__(128) attn_generic_kernel(
 // single-token steps: 14 us where the plain kernel, in which a thread walks a whole key alone, 4 bytes a load and each lane on
 // lines of its own, took 55 (steps of 2 and of 263 tokens, 16 heads, up to 158 keys).
 // ---------------------------------------------------------------------------------------
+// Whether the sequence whose neighbouring tokens [from, to) these are brings fewer than `few` (up to 33) in all, going by the tokens
+// beside them (a whole warp asks).
+__device__ __forceinline__ bool attn_f32_few(const int* __restrict__ seq_of_token, int n_tokens, int from, int to, int seq, int few) {
+  if (to - from >= few) return false;
+  const int lane = threadIdx.x & 31, a = from - 1 - lane, b = to + lane;
+  const unsigned ahead = __ballot_sync(0xffffffffu, a >= 0 && seq_of_token[a] == seq);
+  const unsigned behind = __ballot_sync(0xffffffffu, b < n_tokens && seq_of_token[b] == seq);
+  const int n = (ahead == 0xffffffffu ? 32 : __ffs(~ahead) - 1) + (behind == 0xffffffffu ? 32 : __ffs(~behind) - 1);
+  return to - from + n < few;
+}
+
+// (tokens `begin` .. `n_tokens` - 1; few > 0: only those of sequences that bring fewer)
 template <int HD, int R>
 __global__ void __launch_bounds__(256) attn_f32_kernel(
     const float* __restrict__ q, const float* __restrict__ k_pages, const float* __restrict__ v_pages, float* __restrict__ out,
     const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ block_table, int maxp,
     int n_tokens, int nh, int nkv, float scale, int window, float softcap, const float* __restrict__ sinks, int chunk,
-    int out_stride, float out_scale, int tpb, int cluster) {
+    int out_stride, float out_scale, int tpb, int cluster, int begin, int few) {
   constexpr int C4 = HD / 32;                     // 16-byte pieces a lane holds of a head
   __shared__ float s_acc[8][R][HD];
   __shared__ float s_ml[8][R][2], s_blk[R][2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7, grp = lane >> 3;
   const int G = nh / nkv, hg = (G + R - 1) / R;   // blocks that share a kv head's query heads (1 when tpb > 1)
   const int kvh = blockIdx.y / hg, h0 = (blockIdx.y % hg) * R;
-  const int t0 = blockIdx.z * tpb, rank = blockIdx.x;
+  const int t0 = begin + blockIdx.z * tpb, rank = blockIdx.x;
   const int stream0 = (rank * 8 + warp) * 4 + grp, streams = cluster * 32;
   pdl_wait();
   pdl_trigger();
@@ -1216,6 +1228,10 @@ __global__ void __launch_bounds__(256) attn_f32_kernel(
     const int seq = seq_of_token[t0 + first];
     int end = first + 1;
     while (end < n_here && seq_of_token[t0 + end] == seq) ++end;
+    if (few > 0 && !attn_f32_few(seq_of_token, n_tokens, t0 + first, t0 + end, seq, few)) {      // (all blocks of a cluster alike)
+      first = end;
+      continue;
+    }
     const int* bt = block_table + (size_t)seq * maxp;
     int pos[R], lo[R];
     float4 qv[R][C4], acc[R][C4];
@@ -1436,7 +1452,7 @@ __global__ void __launch_bounds__(64 * KW, 4 / KW) attn_f32_tile_kernel(
     const float* __restrict__ q, const float* __restrict__ k_pages, const float* __restrict__ v_pages, float* __restrict__ out,
     const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ block_table, int maxp,
     int n_tokens, int nh, int nkv, float scale, int window, float softcap, const float* __restrict__ sinks, int chunk,
-    int out_stride, float out_scale) {
+    int out_stride, float out_scale, int few) {
   constexpr int KS = HD / 16, NB = HD / 32, SK = HD + 16, SV = HD + 4, KEYS = 16 * KW, THREADS = 64 * KW, STAGE = KEYS * (SK + SV);
   extern __shared__ __align__(16) float f32_smem[];
   uint4* s_q = reinterpret_cast<uint4*>(f32_smem + 2 * STAGE);             // [row warp][slice][piece][lane]
@@ -1453,6 +1469,10 @@ __global__ void __launch_bounds__(64 * KW, 4 / KW) attn_f32_tile_kernel(
     const int seq = seq_of_token[t0 + first];
     int end = first + 1;
     while (end < n_here && seq_of_token[t0 + end] == seq) ++end;
+    if (few > 0 && attn_f32_few(seq_of_token, n_tokens, t0 + first, t0 + end, seq, few)) {
+      first = end;
+      continue;
+    }
     const int* bt = block_table + (size_t)seq * maxp;
     auto low = [&](int p) {
       const int a = window > 0 ? max(0, p - window + 1) : 0;
@@ -1685,51 +1705,115 @@ static bool attn_f32_tiles(int n_tokens, int n_seqs, int nh, int sms) {
   return per_seq >= 16 && blocks * (per_seq < 32 ? per_seq : 32) >= 32LL * sms / 3;
 }
 
+// How a step of several sequences is dealt out.  A tile costs a sequence's pages, for one row as for 32, so sequences of fewer than
+// `few` tokens go to the kernel of eight lanes a key, whatever the others bring; `from` .. `to`: the tokens among which they are.
+// Where the sequences' lengths are known (`cu`: first tokens and the number of all, `past`: keys held before; host memory, or null),
+// `few` is the one of 6, 17 and 33 that is the fastest by what the kernels take, us: a tile 3 + 4.4 a page of each of its sequences, a
+// block an SM; a block of R rows of the other kernel 1.6 + 0.0098 R a key, by all SMs; 4 for the second launch.  Else it is 6.  Measured
+// (16 heads of 128 over 8, us; kernel of eight lanes for all, tiles for all, this): 500 tokens and 20 of one behind 1,000 262, 898, 111;
+// 500 and 8 behind 8,000 373, 589, 151; 300 and 8 x 8 behind 4,000 430, 1,353, 374; 512 and 32 x 8 behind 500 408, 185, 189.  A
+// call that does not know the lengths pays the second launch where it has several sequences: 4 x 64 tokens 48, 12, 24.
+struct AttnF32Mix { int tiles, few, from, to; };
+static AttnF32Mix attn_f32_mix(const int* cu, const int* past, int n_tokens, int n_seqs, int nh, int nkv, int R, int sms) {
+  AttnF32Mix best = {attn_f32_tiles(n_tokens, n_seqs, nh, sms), n_seqs > 1 ? 6 : 0, 0, n_seqs > 1 ? n_tokens : 0};
+  if (n_seqs <= 1 || !cu || !past || cu[0] != 0 || cu[n_seqs] != n_tokens) return best;
+  for (int i = 0; i < n_seqs; ++i)
+    if (cu[i + 1] < cu[i]) return best;
+  const double row_blocks = (double)nkv * ((nh / nkv + R - 1) / R);
+  const int choices[3] = {6, 17, 33};
+  double best_us = -1.0;
+  for (int few : choices) {
+    AttnF32Mix m = {0, few, 0, 0};
+    int tokens = n_tokens, seqs = n_seqs, tile = -1;
+    double here = 0.0, longest = 0.0, all = 0.0, row = 0.0, rows = 0.0;
+    for (int i = 0; i < n_seqs; ++i) {
+      const int n = cu[i + 1] - cu[i];
+      if (n < few) {
+        if (m.to == 0) m.from = cu[i];
+        m.to = cu[i + 1];
+        tokens -= n;
+        --seqs;
+        const double us = 1.6 + 0.0098 * R * (past[i] + n);
+        row = us > row ? us : row;
+        rows += n * row_blocks * us;
+        continue;
+      }
+      for (int at = cu[i]; at < cu[i + 1]; at = (at / 32 + 1) * 32) {
+        const int end = cu[i + 1] < (at / 32 + 1) * 32 ? cu[i + 1] : (at / 32 + 1) * 32;
+        const double us = 3.0 + 4.4 * ((past[i] + end - cu[i] + 63) / 64);
+        here = at / 32 == tile ? here + us : us;
+        tile = at / 32;
+        longest = here > longest ? here : longest;
+        all += us * nh;
+      }
+    }
+    m.tiles = attn_f32_tiles(tokens, seqs, nh, sms);
+    if (!m.tiles) continue;                        // (then the one kernel takes all, or fewer go to it)
+    double us = all / sms > longest ? all / sms : longest;
+    if (m.to > m.from) us += 4.0 + (rows / sms > row ? rows / sms : row);
+    else m.few = 0;
+    if (best_us < 0.0 || us < best_us) { best = m; best_us = us; }
+  }
+  if (best_us < 0.0) best.tiles = 0;
+  return best;
+}
+extern "C" void sx_attn_f32_mix(const int* cu, const int* past, int n_tokens, int n_seqs, int nh, int nkv, int sms, int* out4) {
+  const AttnF32Mix m = attn_f32_mix(cu, past, n_tokens, n_seqs, nh, nkv, attn_f32_rows(nh, nkv), sms);
+  out4[0] = m.tiles; out4[1] = m.few; out4[2] = m.from; out4[3] = m.to;
+}
+
 template <int HD>
 static int attn_f32_tile_launch(const float* q, const float* k, const float* v, float* out, const int* positions, const int* seq_of_token,
                                 const int* block_table, int maxp, int n_tokens, int nh, int nkv, float scale, int window, float softcap,
-                                const float* sinks, int chunk, int out_stride, float out_scale, cudaStream_t stream) {
+                                const float* sinks, int chunk, int out_stride, float out_scale, int few, cudaStream_t stream) {
   constexpr int KW = 4;
   const size_t smem = (size_t)2 * 16 * KW * (2 * HD + 20) * 4 + (size_t)2 * (HD / 16) * 3 * 32 * 16;
   cudaError_t e = cudaFuncSetAttribute(attn_f32_tile_kernel<HD, KW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   return sx_launch(attn_f32_tile_kernel<HD, KW>, dim3((unsigned)nh, (unsigned)((n_tokens + 31) / 32)), dim3(64 * KW), smem, stream, q, k, v, out, positions,
-                   seq_of_token, block_table, maxp, n_tokens, nh, nkv, scale, window, softcap, sinks, chunk, out_stride, out_scale);
+                   seq_of_token, block_table, maxp, n_tokens, nh, nkv, scale, window, softcap, sinks, chunk, out_stride, out_scale, few);
 }
 
 template <int HD, int R>
 static int attn_f32_launch(const float* q, const float* k, const float* v, float* out, const int* positions, const int* seq_of_token,
-                           const int* block_table, int maxp, int n_tokens, int nh, int nkv, float scale, int window, float softcap,
+                           const int* block_table, int maxp, int begin, int end, int few, int nh, int nkv, float scale, int window, float softcap,
                            const float* sinks, int chunk, int out_stride, float out_scale, cudaStream_t stream) {
   const int G = nh / nkv, hg = (G + R - 1) / R;
-  const AttnF32Plan plan = attn_f32_plan(R, n_tokens, nh, nkv, maxp, sx_sm_count());
+  const AttnF32Plan plan = attn_f32_plan(R, end - begin, nh, nkv, maxp, sx_sm_count());
   const int tpb = plan.tpb, cluster = plan.cluster;
-  const dim3 grid((unsigned)cluster, (unsigned)(nkv * hg), (unsigned)((n_tokens + tpb - 1) / tpb));
+  const dim3 grid((unsigned)cluster, (unsigned)(nkv * hg), (unsigned)((end - begin + tpb - 1) / tpb));
   if (cluster > 1)
     return sx_launch_cluster(attn_f32_kernel<HD, R>, grid, dim3(256), 0, stream, cluster, q, k, v, out, positions, seq_of_token, block_table,
-                             maxp, n_tokens, nh, nkv, scale, window, softcap, sinks, chunk, out_stride, out_scale, tpb, cluster);
+                             maxp, end, nh, nkv, scale, window, softcap, sinks, chunk, out_stride, out_scale, tpb, cluster, begin, few);
   return sx_launch(attn_f32_kernel<HD, R>, grid, dim3(256), 0, stream, q, k, v, out, positions, seq_of_token, block_table, maxp,
-                   n_tokens, nh, nkv, scale, window, softcap, sinks, chunk, out_stride, out_scale, tpb, 1);
+                   end, nh, nkv, scale, window, softcap, sinks, chunk, out_stride, out_scale, tpb, 1, begin, few);
 }
 
 static int attn_generic_any(const void* q, const void* k_pages, const void* v_pages, void* out,
                             const int* positions, const int* seq_of_token, const int* block_table,
                             int maxp, int n_tokens, int nh, int nkv, int hd, float scale, int window,
                             int dt, int vd, float softcap, const float* sinks, int chunk, int out_stride, float out_scale,
-                            int n_seqs, cudaStream_t stream) {
+                            int n_seqs, const int* cu, const int* past, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
   if (hd <= 0 || hd > 512 || vd <= 0 || vd > 512 || nkv <= 0 || nh % nkv != 0 || nh > 65535 || out_stride < nh * vd)
     return SX_ERR_SIZE;
   if (dt == SX_F32 && hd == vd && (hd == 64 || hd == 128) && n_tokens <= 65535 && nkv <= 8191 &&
       (((uintptr_t)q | (uintptr_t)k_pages | (uintptr_t)v_pages) & 15) == 0) {
+    const AttnF32Mix mix = attn_f32_mix(cu, past, n_tokens, n_seqs, nh, nkv, attn_f32_rows(nh, nkv), sx_sm_count());
+    int begin = 0, end = n_tokens;
+    if (mix.tiles) {
 #define ATTN_F32_TILES(HD) attn_f32_tile_launch<HD>((const float*)q, (const float*)k_pages, (const float*)v_pages, (float*)out, positions, \
                                                     seq_of_token, block_table, maxp, n_tokens, nh, nkv, scale, window, softcap, sinks,  \
-                                                    chunk, out_stride, out_scale, stream)
-    if (attn_f32_tiles(n_tokens, n_seqs, nh, sx_sm_count())) return hd == 64 ? ATTN_F32_TILES(64) : ATTN_F32_TILES(128);
+                                                    chunk, out_stride, out_scale, mix.few, stream)
+      const int rc = hd == 64 ? ATTN_F32_TILES(64) : ATTN_F32_TILES(128);
 #undef ATTN_F32_TILES
+      if (rc || mix.to <= mix.from) return rc;
+      begin = mix.from;
+      end = mix.to;
+    }
 #define ATTN_F32(HD, R) attn_f32_launch<HD, R>((const float*)q, (const float*)k_pages, (const float*)v_pages, (float*)out, positions, \
-                                               seq_of_token, block_table, maxp, n_tokens, nh, nkv, scale, window, softcap, sinks, chunk, \
-                                               out_stride, out_scale, stream)
+                                               seq_of_token, block_table, maxp, begin, end, mix.tiles ? mix.few : 0, nh, nkv, scale, window, softcap, \
+                                               sinks, chunk, out_stride, out_scale, stream)
     if (attn_f32_rows(nh, nkv) == 2) return hd == 64 ? ATTN_F32(64, 2) : ATTN_F32(128, 2);
     return hd == 64 ? ATTN_F32(64, 4) : ATTN_F32(128, 4);
 #undef ATTN_F32
@@ -1754,18 +1838,18 @@ extern "C" int sx_attn_generic(const void* q, const void* k_pages, const void* v
                                int maxp, int n_tokens, int nh, int nkv, int hd, float scale, int window,
                                int dt, cudaStream_t stream) {
   return attn_generic_any(q, k_pages, v_pages, out, positions, seq_of_token, block_table, maxp, n_tokens, nh, nkv, hd, scale,
-                          window, dt, hd, 0.f, nullptr, 0, nh * hd, 1.f, n_tokens, stream);
+                          window, dt, hd, 0.f, nullptr, 0, nh * hd, 1.f, n_tokens, nullptr, nullptr, stream);
 }
 
-// with the options the plain entry point leaves out (see the kernel's comment), and how many sequences the tokens are of
-// (at most: rows of the block table)
+// with the options the plain entry point leaves out (see the kernel's comment), how many sequences the tokens are of (at most: rows of
+// the block table), and in host memory, or null, the first token of each and the number of all, and the keys each had before
 extern "C" int sx_attn_generic_ex(const void* q, const void* k_pages, const void* v_pages, void* out,
                                   const int* positions, const int* seq_of_token, const int* block_table,
                                   int maxp, int n_tokens, int nh, int nkv, int hd, float scale, int window,
                                   int dt, int vd, float softcap, const float* sinks, int chunk, int out_stride,
-                                  float out_scale, int n_seqs, cudaStream_t stream) {
+                                  float out_scale, int n_seqs, const int* cu, const int* past, cudaStream_t stream) {
   return attn_generic_any(q, k_pages, v_pages, out, positions, seq_of_token, block_table, maxp, n_tokens, nh, nkv, hd, scale,
-                          window, dt, vd, softcap, sinks, chunk, out_stride, out_scale, n_seqs, stream);
+                          window, dt, vd, softcap, sinks, chunk, out_stride, out_scale, n_seqs, cu, past, stream);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -7,6 +7,7 @@ the kernels, every call raises ``KernelsUnavailable``.
 """
 from __future__ import annotations
 
+import ctypes
 from typing import Optional
 
 import torch
@@ -369,6 +370,17 @@ def attn_scored(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, c
                                  head_bias=head_bias, dist_bias=dist_bias, softmax=softmax, gate=gate, out=out)
 
 
+def _portions(ctx):
+    """What each sequence brings and had before, as ``attn_generic`` takes it, made once a step; ``None`` where the host does not
+    know."""
+    if ctx.host is None:
+        return None
+    both = ctx.scratch.get("portions")
+    if both is None:
+        both = ctx.scratch["portions"] = tuple((ctypes.c_int * len(x))(*x) for x in (ctx.host["cu_seqlens"], ctx.host["seq_past"]))
+    return both
+
+
 def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, ctx, block_table: torch.Tensor,
               nh: int, nkv: int, hd: int, scale: float, window: Optional[int], *, vd: Optional[int] = None,
               softcap: Optional[float] = None, sinks: Optional[torch.Tensor] = None, chunk: Optional[int] = None,
@@ -391,7 +403,7 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, ctx
                                        block_table, nh, nkv, hd, scale, window, softcap=softcap, sinks=sinks, chunk=chunk,
                                        out=out, out_col=out_col, out_scale=out_scale)
         return attn_generic(q, k_pages, v_pages, ctx.positions, ctx.seq_of_token, block_table, nh, nkv, hd, scale, window,
-                            out, vd=vd, softcap=softcap, sinks=sinks, chunk=chunk, out_scale=out_scale, out_col=out_col)
+                            out, vd=vd, softcap=softcap, sinks=sinks, chunk=chunk, out_scale=out_scale, out_col=out_col, portions=_portions(ctx))
     if fast_supported(q.dtype, nh, nkv, hd):
         if ctx.all_single:
             max_pages = (ctx.max_len + 63) // 64
@@ -408,4 +420,4 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, ctx
             return kernel(q, k_pages, v_pages, tiles[0], tiles[1], ctx.cu_seqlens, ctx.seq_past, ctx.seq_lens,
                           block_table, nh, nkv, hd, scale, window, sinks=sinks)
     return attn_generic(q, k_pages, v_pages, ctx.positions, ctx.seq_of_token, block_table, nh, nkv, hd,
-                        scale, window, sinks=sinks)
+                        scale, window, sinks=sinks, portions=_portions(ctx))

@@ -183,13 +183,15 @@ def attn_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, 
                  seq_of_token: torch.Tensor, block_table: torch.Tensor, nh: int, nkv: int, hd: int,
                  scale: float, window: Optional[int] = None, out: Optional[torch.Tensor] = None, *,
                  vd: Optional[int] = None, softcap: Optional[float] = None, sinks: Optional[torch.Tensor] = None,
-                 chunk: Optional[int] = None, out_scale: float = 1.0, out_col: int = 0) -> torch.Tensor:
+                 chunk: Optional[int] = None, out_scale: float = 1.0, out_col: int = 0, portions=None) -> torch.Tensor:
     """Causal (optionally windowed) attention of packed tokens over the paged cache, 32-bit math.
 
     Options: ``vd`` value head size (default ``hd``); ``softcap``: scores become ``softcap * tanh(score / softcap)``;
     ``sinks`` float32 ``[nh]``: ``exp(sink)`` joins each head's softmax denominator; ``chunk``: a query sees only
     keys of its own chunk of that many positions; ``out`` may be wider than ``nh * vd`` (the result fills its columns
-    from ``out_col`` on) and is multiplied by ``out_scale``."""
+    from ``out_col`` on) and is multiplied by ``out_scale``; ``portions`` (two arrays of ``ctypes``
+    integers on the host): each sequence's first token and the number of all, and the keys each had before; by these the float32
+    kernels are chosen (without them their numbers alone are known)."""
     require_cuda(q, k_pages, v_pages, positions, seq_of_token, block_table, out, sinks)
     T = q.shape[0]
     vd = hd if vd is None else vd
@@ -199,13 +201,16 @@ def attn_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, 
         raise KernelError("attn_generic: sinks are float32, one per query head")
     if out.dtype != q.dtype or out_col + nh * vd > out.shape[1]:
         raise KernelError("attn_generic: the output does not fit")
+    starts, past = portions if portions is not None else (None, None)
+    if portions is not None and (len(starts) != block_table.shape[0] + 1 or len(past) != block_table.shape[0]):
+        raise KernelError("attn_generic: one start a sequence and the number of tokens, one past a sequence")
     o = out if out_col == 0 else out.view(-1)[out_col:]
     check(fn("generic", "sx_attn_generic_ex")(
         ptr(q), ptr(k_pages), ptr(v_pages), ptr(o), ptr(positions), ptr(seq_of_token), ptr(block_table),
         c_int(block_table.shape[1]), c_int(T), c_int(nh), c_int(nkv), c_int(hd), c_float(scale),
         c_int(0 if window is None else int(window)), c_int(dt_code(q.dtype)), c_int(vd),
         c_float(0.0 if softcap is None else float(softcap)), ptr(sinks), c_int(0 if chunk is None else int(chunk)),
-        c_int(out.shape[1]), c_float(out_scale), c_int(block_table.shape[0]), stream()), "attn_generic")
+        c_int(out.shape[1]), c_float(out_scale), c_int(block_table.shape[0]), starts, past, stream()), "attn_generic")
     return out
 
 

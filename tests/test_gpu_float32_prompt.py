@@ -3,6 +3,8 @@ tiles, pages and groups of keys.  A sum of n products of pieces is off by less t
 n = 64 on (16 roundings of 2^-23 within a slice of 16, one of 2^-24 a slice, 2^-23 for the pieces left out), which is the
 bound on a score; a weight is off by twice that and a few roundings, and the weighted mean by the weights' relative error and
 (keys + 16) roundings times the largest value."""
+import ctypes
+import itertools
 import math
 
 import pytest
@@ -23,6 +25,10 @@ def setup(nh, nkv, hd, past, new, seed):
     pos = torch.cat([torch.arange(p, p + n) for p, n in zip(past, new)]).to(torch.int32)
     sot = torch.cat([torch.full((n,), i) for i, n in enumerate(new)]).to(torch.int32)
     return q, ks, vs, pos, sot
+
+
+def portions(past, new):
+    return (ctypes.c_int * (len(new) + 1))(*([0] + list(itertools.accumulate(new)))), (ctypes.c_int * len(past))(*past)
 
 
 def run(q, ks, vs, pos, sot, past, new, nkv, hd, scale, window=None, out=None, **options):
@@ -145,3 +151,43 @@ def test_time_of_rows_that_are_not_finite():
         assert y.isfinite().all()
         return start.elapsed_time(end)
     assert ms(big, far) <= 10 * ms(q, kp)
+
+
+# sequences of fewer than 6, 17 or 33 tokens (left to the other kernel) and of so many: ahead of others, behind them and between, next
+# to a tile's edge and across it
+@pytest.mark.parametrize("past,new", [([300, 0], [1, 70]), ([0, 90, 64], [62, 5, 6]), ([0, 9, 0, 70, 3], [30, 4, 90, 5, 1]), ([5, 0, 128, 0], [6, 57, 1, 65]),
+                                      ([0, 100, 20, 0], [64, 6, 7, 90]), ([0, 1500, 0], [81, 16, 90]), ([0, 0, 2000], [60, 100, 32])])
+@pytest.mark.parametrize("known", [False, True])
+@pytest.mark.parametrize("nh,nkv,hd", [(40, 8, 128), (37, 37, 64)])
+def test_steps_of_long_and_short_portions(nh, nkv, hd, known, past, new):
+    q, ks, vs, pos, sot = setup(nh, nkv, hd, past, new, sum(new))
+    out = run(q, ks, vs, pos, sot, past, new, nkv, hd, hd ** -0.5, out=torch.full((sum(new), nh * hd), 3.0, device="cuda"),
+              portions=portions(past, new) if known else None)
+    want = attention(q, ks, vs, pos, sot, hd ** -0.5, None, None, None, None).view(sum(new), -1)
+    off = (hd + 4) * ULP * float(q.norm(dim=-1).max()) * max(float(k.norm(dim=-1).max()) for k in ks) * hd ** -0.5
+    bound = (2 * off + (max(p + n for p, n in zip(past, new)) + 16) * ULP) * max(float(v.abs().max()) for v in vs)
+    assert (out.double().cpu() - want).abs().max() <= bound
+
+
+@pytest.mark.parametrize("known", [False, True])
+def test_time_of_steps_of_long_and_short_portions(known):
+    """A prompt of 500 tokens with twenty single tokens behind 1,000 others, or eight behind 6,000, costs about what either costs alone."""
+    from synaptix_b200 import ops
+    nh, nkv, hd = 16, 8, 128
+
+    def ms(past, new):
+        q, ks, vs, pos, sot = setup(nh, nkv, hd, past, new, 1)
+        kp, vp, bt = make_paged(ks, vs, nkv, hd, torch.float32, seed=2)
+        args = dev(q.view(sum(new), -1)), kp, vp, dev(pos), dev(sot), bt, nh, nkv, hd, hd ** -0.5
+        more = {"portions": portions(past, new)} if known else {}
+        ops.attn_generic(*args, **more)
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        for _ in range(20):
+            ops.attn_generic(*args, **more)
+        end.record()
+        end.synchronize()
+        return start.elapsed_time(end)
+    assert ms([0] + [1000] * 20, [500] + [1] * 20) <= 2.5 * (ms([0], [500]) + ms([1000] * 20, [1] * 20))
+    if known:
+        assert ms([0, 6000], [500, 8]) <= 2.0 * (ms([0], [500]) + ms([6000], [8]))

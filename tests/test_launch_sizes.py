@@ -51,3 +51,29 @@ def test_float32_launches_follow_the_sms(sms):
         assert cluster == 8 or blocks * cluster >= sms or pages < 2 * cluster
         assert cluster == 1 or (blocks * cluster // 2 < sms and tokens == 1)
         assert tokens == (rows // heads if cluster == 1 and heads < rows and blocks >= sms * (rows // heads) else 1)
+
+
+@pytest.mark.parametrize("lens", [[40], [500, 1, 1, 5], [1, 500], [3, 64, 2, 20, 5, 6], [6, 6, 6, 6, 6, 6, 6], [30, 70, 5, 8, 6, 200], [1] * 40, [200, 5, 7, 7, 7]])
+@pytest.mark.parametrize("past", [0, 300, 5000])
+def test_float32_attention_of_long_and_short_portions(lens, past):
+    """Sequences that bring less than the others' tiles are worth lie within the range that is handed on, and the rest has tiles."""
+    f = library("generic").sx_attn_f32_mix
+    f.restype = None
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    out = (ctypes.c_int * 4)()
+    array = lambda x: (ctypes.c_int * len(x))(*x)  # noqa: E731
+    f(array(cu), array([past if n < 40 else 0 for n in lens]), cu[-1], len(lens), 64, 8, 148, out)
+    tiles, few, first, last = out
+
+    def worth(rest):
+        per = sum(rest) // len(rest) if rest else 0
+        return per >= 16 and -(-sum(rest) // 32) * 64 * min(per, 32) >= 32 * 148 // 3
+    assert bool(tiles) == any(worth([n for n in lens if n >= k]) for k in ((0,) if len(lens) == 1 else (6, 17, 33)))
+    if tiles:
+        small = [(a, b) for a, b in zip(cu, cu[1:]) if b - a < few]
+        assert (first, last) == ((small[0][0], small[-1][1]) if small else (0, 0)) and worth([n for n in lens if n >= few])
+        assert few in ((6, 17, 33) if small else (0,)) and (past < 5000 or few > 8 or not any(6 <= n <= 8 for n in lens))
+    f(None, None, cu[-1], len(lens), 64, 8, 148, out)        # (where the lengths are not known, any may be short)
+    assert list(out) == [int(worth(lens))] + ([6, 0, cu[-1]] if len(lens) > 1 else [0, 0, 0])
