@@ -268,6 +268,9 @@ __global__ void __launch_bounds__(128) gemm_rows_kernel(const TA* __restrict__ A
 // two rows, 28 layers of a 0.6B model and its head 1.24 -> 1.13 ms a step): with NORM, A is the residual stream and the rows' RMS
 // norm is formed as they are read (the sum of squares beside the products, gain on the way, the factor on the results);
 // F32_ROWS_SILU reads a stacked [gate; up] and stores silu(gate) * up; F32_ROWS_ADD adds into C, the residual stream.
+// Each is a kernel of its own: told apart at run time they cost the plain product of 9 to 16 rows 10 % (4,096 x 1,024 11.0 -> 12.5 us,
+// 151,936 x 1,024 319 -> 357).  G rows of A are asked for together: four where K is short and the rows' latency counts (12 rows, 1,024 x
+// 252 6.6 -> 4.1 us), one where W streams (151,936 x 1,024 with 9 to 16 rows 318 us, 341 with four) and with a norm.
 enum { F32_ROWS_STORE = 0, F32_ROWS_SILU = 1, F32_ROWS_ADD = 2 };
 struct F32RowsEnd {
   const float* bias;     // [N] or null
@@ -276,20 +279,20 @@ struct F32RowsEnd {
   const float* gain;     // [K] (NORM)
   float eps;
 };
-template <int MR, int KS, bool NORM>
+template <int MR, int KS, bool NORM, int EPI>
 __global__ void __launch_bounds__(256, MR <= 2 ? 4 : (MR == 4 ? 3 : 2)) gemm_rows_f32_kernel(const float* __restrict__ A, const float* __restrict__ W,
                                                             float* __restrict__ C, int M, int N, int K, const F32RowsEnd end) {
-  constexpr int R = 4, GROUPS = 8 / KS, V = MR * R, FV = V < 32 ? V : 32;
+  constexpr bool SILU = EPI == F32_ROWS_SILU;
+  constexpr int R = 4, G = KS == 8 || MR < 4 || NORM ? 1 : 4, GROUPS = 8 / KS, V = MR * R, FV = V < 32 ? V : 32;
   __shared__ float part[8][V];
   __shared__ float squares[8][MR];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, group = warp / KS, ks = warp % KS;
-  const bool silu = end.epi == F32_ROWS_SILU;
-  const int n_out = silu ? N / 2 : N, cols = silu ? R / 2 : R;           // outputs in all, and of a warp's four rows
+  const int n_out = SILU ? N / 2 : N, cols = SILU ? R / 2 : R;           // outputs in all, and of a warp's four rows
   const int n0 = (blockIdx.x * GROUPS + group) * cols;
   const float* wr[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int row = silu ? min(n0 + (r & 1), n_out - 1) + (r >> 1) * n_out : min(n0 + r, N - 1);      // (two gate rows, two up rows)
+    const int row = SILU ? min(n0 + (r & 1), n_out - 1) + (r >> 1) * n_out : min(n0 + r, N - 1);      // (two gate rows, two up rows)
     wr[r] = W + (size_t)row * K;
   }
   float acc[MR][R], sq[MR];
@@ -314,15 +317,20 @@ __global__ void __launch_bounds__(256, MR <= 2 ? 4 : (MR == 4 ? 3 : 2)) gemm_row
     for (int r = 0; r < R; ++r) w[r] = __ldg(reinterpret_cast<const float4*>(wr[r] + k));
     if (NORM) gn = __ldg(reinterpret_cast<const float4*>(end.gain + k));
 #pragma unroll
-    for (int i = 0; i < MR; ++i) {
-      float4 a = *reinterpret_cast<const float4*>(A + (size_t)min(i, M - 1) * K + k);
-      if (NORM) {
-        sq[i] = fmaf(a.w, a.w, fmaf(a.z, a.z, fmaf(a.y, a.y, fmaf(a.x, a.x, sq[i]))));
-        a.x *= gn.x; a.y *= gn.y; a.z *= gn.z; a.w *= gn.w;
-      }
+    for (int i0 = 0; i0 < MR; i0 += G) {
+      float4 a[G];
 #pragma unroll
-      for (int r = 0; r < R; ++r)
-        acc[i][r] = fmaf(a.w, w[r].w, fmaf(a.z, w[r].z, fmaf(a.y, w[r].y, fmaf(a.x, w[r].x, acc[i][r]))));
+      for (int i = 0; i < G; ++i) a[i] = *reinterpret_cast<const float4*>(A + (size_t)min(i0 + i, M - 1) * K + k);
+#pragma unroll
+      for (int i = 0; i < G; ++i) {
+        if (NORM) {
+          sq[i0 + i] = fmaf(a[i].w, a[i].w, fmaf(a[i].z, a[i].z, fmaf(a[i].y, a[i].y, fmaf(a[i].x, a[i].x, sq[i0 + i]))));
+          a[i].x *= gn.x; a[i].y *= gn.y; a[i].z *= gn.z; a[i].w *= gn.w;
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          acc[i0 + i][r] = fmaf(a[i].w, w[r].w, fmaf(a[i].z, w[r].z, fmaf(a[i].y, w[r].y, fmaf(a[i].x, w[r].x, acc[i0 + i][r]))));
+      }
     }
   }
 #pragma unroll
@@ -346,7 +354,7 @@ __global__ void __launch_bounds__(256, MR <= 2 ? 4 : (MR == 4 ? 3 : 2)) gemm_row
     float s = 0.f, u = 0.f, f = 1.f;
 #pragma unroll
     for (int w = 0; w < KS; ++w) s += part[g * KS + w][i % V];
-    if (silu)
+    if (SILU)
 #pragma unroll
       for (int w = 0; w < KS; ++w) u += part[g * KS + w][i % V + 2];
     if (NORM) {
@@ -357,10 +365,10 @@ __global__ void __launch_bounds__(256, MR <= 2 ? 4 : (MR == 4 ? 3 : 2)) gemm_row
     }
     float* c = C + (size_t)m * n_out + n;
     s = s * f + (end.bias ? end.bias[n] : 0.f);
-    if (silu) {
+    if (SILU) {
       u = u * f + (end.bias ? end.bias[n_out + n] : 0.f);
       *c = s / (1.f + expf(-s)) * u;
-    } else if (end.epi == F32_ROWS_ADD) {
+    } else if (EPI == F32_ROWS_ADD) {
       *c += s;
     } else {
       *c = soft_limit(s, end.cap);
@@ -601,20 +609,26 @@ __global__ void __launch_bounds__(128, BM == 32 ? 4 : 3) gemm_tile_f32_kernel(co
   cluster_sync_all();                             // nobody's shared memory goes away while it is read
 }
 
-template <int MR, bool NORM>
+template <int MR, bool NORM, int EPI>
 static int gemm_rows_f32_launch(const float* A, const float* W, float* C, int M, int N, int K, const F32RowsEnd& end, cudaStream_t stream) {
-  const int n_out = end.epi == F32_ROWS_SILU ? N / 2 : N, cols = end.epi == F32_ROWS_SILU ? 2 : 4, tiles = (n_out + cols - 1) / cols;
-  if (K >= 1024) return sx_launch(gemm_rows_f32_kernel<MR, 8, NORM>, dim3(tiles), dim3(256), 0, stream, A, W, C, M, N, K, end);
-  if (K >= 256) return sx_launch(gemm_rows_f32_kernel<MR, 2, NORM>, dim3((tiles + 3) / 4), dim3(256), 0, stream, A, W, C, M, N, K, end);
-  return sx_launch(gemm_rows_f32_kernel<MR, 1, NORM>, dim3((tiles + 7) / 8), dim3(256), 0, stream, A, W, C, M, N, K, end);
+  const int n_out = EPI == F32_ROWS_SILU ? N / 2 : N, cols = EPI == F32_ROWS_SILU ? 2 : 4, tiles = (n_out + cols - 1) / cols;
+  if (K >= 1024) return sx_launch(gemm_rows_f32_kernel<MR, 8, NORM, EPI>, dim3(tiles), dim3(256), 0, stream, A, W, C, M, N, K, end);
+  if (K >= 256) return sx_launch(gemm_rows_f32_kernel<MR, 2, NORM, EPI>, dim3((tiles + 3) / 4), dim3(256), 0, stream, A, W, C, M, N, K, end);
+  return sx_launch(gemm_rows_f32_kernel<MR, 1, NORM, EPI>, dim3((tiles + 7) / 8), dim3(256), 0, stream, A, W, C, M, N, K, end);
+}
+template <bool NORM, int EPI>
+static int gemm_rows_f32_of(const float* A, const float* W, float* C, int M, int N, int K, const F32RowsEnd& end, cudaStream_t stream) {
+  if (M <= 1) return gemm_rows_f32_launch<1, NORM, EPI>(A, W, C, M, N, K, end, stream);
+  if (M <= 2) return gemm_rows_f32_launch<2, NORM, EPI>(A, W, C, M, N, K, end, stream);
+  if (M <= 4) return gemm_rows_f32_launch<4, NORM, EPI>(A, W, C, M, N, K, end, stream);
+  if (M <= 8) return gemm_rows_f32_launch<8, NORM, EPI>(A, W, C, M, N, K, end, stream);
+  return gemm_rows_f32_launch<16, NORM, EPI>(A, W, C, M, N, K, end, stream);
 }
 template <bool NORM>
 static int gemm_rows_f32(const float* A, const float* W, float* C, int M, int N, int K, const F32RowsEnd& end, cudaStream_t stream) {
-  if (M <= 1) return gemm_rows_f32_launch<1, NORM>(A, W, C, M, N, K, end, stream);
-  if (M <= 2) return gemm_rows_f32_launch<2, NORM>(A, W, C, M, N, K, end, stream);
-  if (M <= 4) return gemm_rows_f32_launch<4, NORM>(A, W, C, M, N, K, end, stream);
-  if (M <= 8) return gemm_rows_f32_launch<8, NORM>(A, W, C, M, N, K, end, stream);
-  return gemm_rows_f32_launch<16, NORM>(A, W, C, M, N, K, end, stream);
+  if (end.epi == F32_ROWS_SILU) return gemm_rows_f32_of<NORM, F32_ROWS_SILU>(A, W, C, M, N, K, end, stream);
+  if (end.epi == F32_ROWS_ADD) return gemm_rows_f32_of<NORM, F32_ROWS_ADD>(A, W, C, M, N, K, end, stream);
+  return gemm_rows_f32_of<NORM, F32_ROWS_STORE>(A, W, C, M, N, K, end, stream);
 }
 
 // The tiles of more rows: rows of a tile, and blocks that share a tile's K.
