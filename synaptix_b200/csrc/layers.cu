@@ -721,7 +721,7 @@ __global__ void __launch_bounds__(LY_THREADS, 1) decode_layers_kernel(const __gr
           }
           if (!stream) {
             if (g0 == 0) asm volatile("bar.sync 6, %0;\n" ::"n"(LY_EPI * 32) : "memory");      // (the factors, see below)
-            v *= sh->factor[p >> 1][n];
+            v *= sh->factor[p >> 1][tn];                // (columns without a token: results that nothing reads)
           } else if (ok) {
             v += sh->h[row][n];
             sh->h[row][n] = v;
