@@ -54,6 +54,7 @@
 #define LY_SPIN (1u << 21)                // looks at words of another block (half a microsecond each), at a barrier of this one
 #define LY_SPIN_BAR (1u << 20)             // (a look at a barrier suspends the warp for up to LY_NAP ns: spinning warps slow the others down)
 #define LY_NAP 2000
+#define SX_ERR_NO_ROOM 10006
 
 struct LyLayer {
   const bf16* w[4];                       // q/k/v, o, gate and up, down
@@ -877,6 +878,7 @@ extern "C" int sx_decode_layers_plan(int T, int W, int nh, int nkv, int hd, int 
 
 // layers: n_layers records on the device, 9 x 8 bytes each (`LyLayer`); h_in, h_out float32 [T, W] (one tensor may be both); the
 // cache's keys and values as rows of 128 values from k_base / v_base on, `kv_rows` of them; words: see sx_decode_layers_plan.
+// SX_ERR_NO_ROOM: the stream has a part of the device's SMs only, so that the blocks cannot run at once; nothing was launched.
 extern "C" int sx_decode_layers(const void* layers, int n_layers, void* words, const float* h_in, float* h_out, const int* seq_lens,
                                 const int* block_table, int maxp, int n_pages, void* k_base, void* v_base, long long kv_rows,
                                 const float* inv_freq, int T, int W, int nh, int nkv, int hd, int ff, float scale, float eps, float qk_eps,
@@ -907,7 +909,10 @@ extern "C" int sx_decode_layers(const void* layers, int n_layers, void* words, c
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, ly_kernel(T), mk, mv, (const LyArgs)a);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, ly_kernel(T), mk, mv, (const LyArgs)a);
+  if (e != cudaErrorCooperativeLaunchTooLarge) return (int)e;
+  (void)cudaGetLastError();                             // (nothing was launched, and nothing else is told of it)
+  return SX_ERR_NO_ROOM;
 }
 
 // as the other libraries' status words: which bounded wait ran out (0: none)

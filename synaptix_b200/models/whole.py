@@ -96,13 +96,17 @@ def run_layers(model, h: torch.Tensor, ctx, cache) -> bool:
     # The records and the workspace belong to the step's arrays: a captured step keeps them for its replays, any other one
     # makes them anew.
     kept = ctx.scratch.get("decode_layers")
+    if kept == "no room":
+        return False
     if kept is None or kept[0] != records or kept[2].numel() < need:
         if torch.cuda.is_current_stream_capturing():
             return False
         kept = ctx.scratch["decode_layers"] = (records, torch.tensor(records, dtype=torch.int64).to(h.device, non_blocking=True),
                                                torch.zeros(need, dtype=torch.int64, device=h.device))
     inv_freq, _ = a._rotation()
-    ops.decode_layers(kept[1], kept[2], h, ctx.seq_lens, ctx.block_tables[group], k_rows, v_rows,
-                      cache.view(model.steps[0].cache_entry).k.shape[0], inv_freq, a.nh, a.nkv, a.hd, ff, a.scale, first.norm1.eps,
-                      a.qk_norm_eps if a.qk_norm_eps is not None else 0.0)
-    return True
+    if ops.decode_layers(kept[1], kept[2], h, ctx.seq_lens, ctx.block_tables[group], k_rows, v_rows,
+                         cache.view(model.steps[0].cache_entry).k.shape[0], inv_freq, a.nh, a.nkv, a.hd, ff, a.scale, first.norm1.eps,
+                         a.qk_norm_eps if a.qk_norm_eps is not None else 0.0):
+        return True
+    ctx.scratch["decode_layers"] = "no room"       # (so that the step is walked when it is captured, too)
+    return False

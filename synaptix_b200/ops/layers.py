@@ -6,12 +6,13 @@ from typing import Optional
 
 import torch
 
-from ._lib import KernelError, c_int, check, fn, launch, launcher, raw_stream, require_cuda
+from ._lib import KernelError, c_int, check, fn, launcher, raw_stream, require_cuda
 
 # Rows a step: with more, every block's share of the activations (tagged words, twice their size) costs more than the kernel saves.
 # Measured with forms for four and eight rows, ms a step at 4B sizes and 1,100 keys: 4 rows 2.02 to 2.07 against 2.07 with five kernels
 # a layer, 8 rows 2.62 against 2.20 (0.6B: 0.72 to 0.80 against 0.76, 0.99 against 0.82).
 MAX_ROWS = 2
+NO_ROOM = 10006       # the library's code for a stream whose share of the SMs does not hold all blocks at once
 RECORD = 9            # 8-byte numbers a layer: q/k/v, o, gate and up, down; gains of norm1, norm2, q and k heads; first cache row
 
 _WORDS = {}
@@ -29,11 +30,12 @@ def decode_layers_words(T: int, W: int, nh: int, nkv: int, hd: int, ff: int, n_l
 
 def decode_layers(layers: torch.Tensor, words: torch.Tensor, h: torch.Tensor, seq_lens: torch.Tensor, block_table: torch.Tensor,
                   k_rows: torch.Tensor, v_rows: torch.Tensor, n_pages: int, inv_freq: Optional[torch.Tensor], nh: int, nkv: int, hd: int,
-                  ff: int, scale: float, eps: float, qk_eps: float) -> None:
+                  ff: int, scale: float, eps: float, qk_eps: float) -> bool:
     """``h [T, W]`` (float32, in place) through the layers of ``layers`` (int64 ``[n, RECORD]`` on the device).
 
     ``k_rows`` / ``v_rows [rows, hd]``: the cache of all layers as rows, a layer's from its record's last number on;
-    ``words``: ``decode_layers_words`` zeros (int64) that no launch running at the same time uses."""
+    ``words``: ``decode_layers_words`` zeros (int64) that no launch running at the same time uses.  ``False``: the blocks
+    cannot run at once on the current stream (it has a part of the SMs only), and nothing was launched."""
     require_cuda(layers, words, h, seq_lens, block_table, k_rows, v_rows, inv_freq)
     T, W = h.shape
     if h.dtype != torch.float32 or layers.dtype != torch.int64 or layers.dim() != 2 or layers.shape[1] != RECORD:
@@ -47,10 +49,14 @@ def decode_layers(layers: torch.Tensor, words: torch.Tensor, h: torch.Tensor, se
         raise KernelError("decode_layers: int32 lengths and block tables of every row")
     if inv_freq is not None and (inv_freq.dtype != torch.float32 or inv_freq.numel() != hd // 2):
         raise KernelError("decode_layers: float32 frequencies of the whole head")
-    launch(launcher("layers", "sx_decode_layers"), (
+    code = launcher("layers", "sx_decode_layers")(
         layers.data_ptr(), layers.shape[0], words.data_ptr(), h.data_ptr(), h.data_ptr(), seq_lens.data_ptr(), block_table.data_ptr(),
         block_table.shape[1], n_pages, k_rows.data_ptr(), v_rows.data_ptr(), k_rows.shape[0], None if inv_freq is None else inv_freq.data_ptr(),
-        T, W, nh, nkv, hd, ff, scale, eps, qk_eps, raw_stream()), "decode_layers")
+        T, W, nh, nkv, hd, ff, scale, eps, qk_eps, raw_stream())
+    if code == NO_ROOM:
+        return False
+    check(code, "decode_layers")
+    return True
 
 
 def decode_layers_status(reset: bool = False) -> int:

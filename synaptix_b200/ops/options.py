@@ -35,7 +35,11 @@ switches in its runtime options (crates/synaptix-config/src/runtime.rs, ``AttnBa
 ``repeat_layers``   prompt steps: the launches of layers of one form are recorded from one of them and made again with the
                     others' pointers (else every layer's parts are walked)
 ``decode_layers``   single-token steps of one or two rows of a dense decoder in bfloat16: all layers in one kernel (else five
-                    kernels a layer)
+                    kernels a layer).  It takes every SM, so it waits for what other streams run and lets nothing of theirs run
+                    beside it: a step alone is shorter (0.6B 0.67 -> 0.58 ms, 4B 1.90 -> 1.70), but the steps of two engines on
+                    streams of their own line up (both together 0.84 -> 1.12 ms, 3.08 -> 3.38), and another stream's products
+                    wait (3.4 times as long beside 4B steps).  A program that shares the device so turns it off before its steps
+                    are captured.  On a stream that has a part of the SMs only, the layers are walked
 """
 from __future__ import annotations
 

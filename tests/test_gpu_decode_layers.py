@@ -213,6 +213,36 @@ def test_other_layers_are_walked(change):
     assert _records(model, cache, h) is None
 
 
+def test_where_the_blocks_have_no_room(monkeypatch):
+    """A launch that the device refuses for want of SMs leaves the step to the walk, also when it is captured; any other error is raised."""
+    from synaptix_b200.models import whole
+    from synaptix_b200.ops import KernelError, layers
+    from synaptix_b200.parts import Runtime
+    from synaptix_b200.parts.base import StepContext
+    model, cache, h = _model()
+    codes, calls = [10006], []
+    monkeypatch.setattr(whole.ops, "decode_layers_words", lambda *a: 64)
+    monkeypatch.setattr(layers, "decode_layers_words", lambda *a: 64)
+    monkeypatch.setattr(layers, "require_cuda", lambda *a: None)
+    monkeypatch.setattr(layers, "raw_stream", lambda: 0)
+    monkeypatch.setattr(layers, "launcher", lambda *a: lambda *args: calls.append(args) or codes[0])
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+
+    def ctx():
+        i32 = lambda *x: torch.zeros(*x, dtype=torch.int32)  # noqa: E731
+        return StepContext(all_single=True, n_seqs=1, runtime=Runtime(torch.device("cpu"), torch.bfloat16), seq_lens=i32(1), block_tables=[i32(1, 4)])
+    c = ctx()
+    assert not whole.run_layers(model, h, c, cache) and len(calls) == 1
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    assert not whole.run_layers(model, h, c, cache) and len(calls) == 1
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    codes[0] = 0
+    assert whole.run_layers(model, h, ctx(), cache) and len(calls) == 2
+    codes[0] = 700
+    with pytest.raises(KernelError):
+        whole.run_layers(model, h, ctx(), cache)
+
+
 def test_other_models_are_walked():
     from synaptix_b200.models.whole import _records
     assert _records(*_model(use_sliding_window=True, sliding_window=64, max_window_layers=1)) is None
