@@ -266,7 +266,8 @@ __global__ void __launch_bounds__(128) gemm_rows_kernel(const TA* __restrict__ A
 //
 // What stands around a product of a few rows is done by the product (kernels of 3 to 4 us each, that did nothing but wait and copy;
 // two rows, 28 layers of a 0.6B model and its head 1.24 -> 1.13 ms a step): with NORM, A is the residual stream and the rows' RMS
-// norm is formed as they are read (the sum of squares beside the products, gain on the way, the factor on the results);
+// norm is formed as they are read (the sum of squares beside the products, gain on the way, the factor on the results, but for a
+// power of two of it that keeps small rows above the least number);
 // F32_ROWS_SILU reads a stacked [gate; up] and stores silu(gate) * up; F32_ROWS_ADD adds into C, the residual stream.
 // Each is a kernel of its own: told apart at run time they cost the plain product of 9 to 16 rows 10 % (4,096 x 1,024 11.0 -> 12.5 us,
 // 151,936 x 1,024 319 -> 357).  G rows of A are asked for together: four where K is short and the rows' latency counts (12 rows, 1,024 x
@@ -278,7 +279,14 @@ struct F32RowsEnd {
   int epi;
   const float* gain;     // [K] (NORM)
   float eps;
+  float up;              // a power of two at most as large as the rows' largest factor: see the kernel
 };
+// (1 / sqrt(eps) is what rows of next to nothing are multiplied by; without it ahead of the sums they would fall below the least number)
+static float f32_rows_up(float eps) {
+  float up = 1.f;
+  while (up < 0x1p20f && 4.f * up * up * eps <= 1.f) up *= 2.f;
+  return up;
+}
 template <int MR, int KS, bool NORM, int EPI>
 __global__ void __launch_bounds__(256, MR <= 2 ? 4 : (MR == 4 ? 3 : 2)) gemm_rows_f32_kernel(const float* __restrict__ A, const float* __restrict__ W,
                                                             float* __restrict__ C, int M, int N, int K, const F32RowsEnd end) {
@@ -315,7 +323,10 @@ __global__ void __launch_bounds__(256, MR <= 2 ? 4 : (MR == 4 ? 3 : 2)) gemm_row
     float4 w[R], gn;
 #pragma unroll
     for (int r = 0; r < R; ++r) w[r] = __ldg(reinterpret_cast<const float4*>(wr[r] + k));
-    if (NORM) gn = __ldg(reinterpret_cast<const float4*>(end.gain + k));
+    if (NORM) {
+      gn = __ldg(reinterpret_cast<const float4*>(end.gain + k));
+      gn.x *= end.up; gn.y *= end.up; gn.z *= end.up; gn.w *= end.up;
+    }
 #pragma unroll
     for (int i0 = 0; i0 < MR; i0 += G) {
       float4 a[G];
@@ -361,7 +372,13 @@ __global__ void __launch_bounds__(256, MR <= 2 ? 4 : (MR == 4 ? 3 : 2)) gemm_row
       float q = 0.f;
 #pragma unroll
       for (int w = 0; w < KS; ++w) q += squares[g * KS + w][m];
-      f = rsqrtf(q / (float)K + end.eps);
+      f = rsqrtf(q / (float)K + end.eps) / end.up;
+      if (f == 0.f) {                             // squares beyond the largest number: the rows are their elements times nothing
+        bool finite = true;
+        for (int k = 0; k < K; ++k) finite &= isfinite(A[(size_t)m * K + k]);
+        s = u = finite ? 0.f : NAN;
+        f = 1.f;
+      }
     }
     float* c = C + (size_t)m * n_out + n;
     s = s * f + (end.bias ? end.bias[n] : 0.f);
@@ -725,7 +742,7 @@ extern "C" int sx_gemm_rows_f32(const float* A, const float* W, float* C, int M,
   if (M <= 0 || N <= 0) return 0;
   if (M > 16 || K <= 0 || (K & 3) || epi < 0 || epi > 2 || (epi == F32_ROWS_SILU && (N & 1))) return SX_ERR_SIZE;
   if (((uintptr_t)A | (uintptr_t)W | (uintptr_t)gain) & 15) return SX_ERR_ALIGN;
-  F32RowsEnd end = {bias, 0.f, epi, gain, eps};
+  F32RowsEnd end = {bias, 0.f, epi, gain, eps, f32_rows_up(eps)};
   return gain ? gemm_rows_f32<true>(A, W, C, M, N, K, end, stream) : gemm_rows_f32<false>(A, W, C, M, N, K, end, stream);
 }
 

@@ -48,6 +48,28 @@ def test_rows(M, N, K, normed):
     assert ((y - z * u).abs() <= 1.1 * dg * (u.abs() + du) + z.abs() * du + 8 * ULP * (z * u).abs() + 1e-37).all()
 
 
+@pytest.mark.parametrize("M", [1, 3, 12])
+@pytest.mark.parametrize("N,K", [(30, 252), (30, 1020), (62, 2052)])
+@pytest.mark.parametrize("eps", [1e-6, 1e-12, 0.5])
+@pytest.mark.parametrize("size", [2.0 ** -140, 2.0 ** -132, 2.0 ** -100, 2.0 ** 50, 2.0 ** 125])
+def test_norm_at_the_ends_of_the_range(M, N, K, eps, size):
+    """Rows of next to nothing keep what a norm ahead of the product keeps of them (half of the least number, 2^-149, is lost of an
+    element, of it times the gain, and of a sum, and the factor behind the sums is below 2); rows whose squares overflow are nothing, as they are there."""
+    from synaptix_b200 import ops
+    x, w, _, gain = operands(M, N, K)
+    x, w = (x / 3).clamp(-4, 4) * size, w * K ** 0.5
+    gain = gain * 4
+    got = ops.gemm_rows_f32(x, w, gain=gain, eps=eps).double()
+    if size == 2.0 ** 125:
+        assert (got == 0).all() and (ops.gemm_generic(ops.add_rmsnorm(x, None, gain, eps, torch.float32), w) == 0).all()
+        x[0, 1] = float("inf")
+        got = ops.gemm_rows_f32(x, w, gain=gain, eps=eps)
+        assert got[0].isnan().all() and (got[1:] == 0).all()
+        return
+    want, bound = product(x, w, gain, eps)
+    assert ((got - want).abs() <= bound + 2.0 ** -149 * (w.double().abs() * (gain.double().abs() + 1) + 2).sum(1)).all()
+
+
 def test_what_it_refuses():
     from synaptix_b200 import ops
     x, w, bias, gain = operands(4, 16, 64)
