@@ -96,6 +96,32 @@ def test_against_the_plain_implementation_and_the_walked_step(engines, name, len
         assert err <= 1.3 * other + 1e-3 * ref.norm()
 
 
+# the page numbers that the producers hold, 32 at a time, change at every 2,048 keys, within a share and between shares; shares
+# of more pages than the ring has stages; two rows of unequal length.  Scores are made large, so that a few keys count and the others' pages tell
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens", [(2045,), (2047,), (2050,), (4100, 60), (2049, 5000), (7950,)])
+@pytest.mark.parametrize("name", ["g1", "g3"])
+def test_long_contexts_against_the_walked_step(name, lens):
+    from helpers import folder
+    from synaptix_b200 import ops
+    from synaptix_b200.engine import Engine
+    from synaptix_b200.models import load_model
+    model = load_model(folder(config(name)), dtype="bfloat16")
+    for layer in model.layers:
+        layer.mixer.scale *= 2
+    eng = Engine(model, max_tokens=8192)
+    poison_cache(eng)
+    toks = [random_tokens(SIZES[name]["vocab_size"], n + 4, 20 + i) for i, n in enumerate(lens)]
+    run = lambda: steps(eng, [t[:-4] for t in toks], [t[-4:] for t in toks])  # noqa: E731
+    got, n = run()
+    fresh(eng)
+    with ops.options(decode_layers=False):
+        want, m = run()
+    assert n <= 6 < m
+    for i in range(len(lens)):
+        assert_close(got[i], want[i], "bfloat16", f"{name} {lens} row {i}")
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("name,lens", [("g3", (100, 66)), ("g1", (20,))])
 def test_without_graphs(engines, name, lens):
