@@ -1,5 +1,6 @@
 // Plain kernels for every operation of a decoder step, for float32 and bfloat16 storage,
-// all arithmetic in 32-bit (FFMA only: no tensor cores, no TF32).  They take every size;
+// all numbers and sums in 32-bit (no TF32; float32 products of more than 16 rows and attention of prompt portions run on the tensor
+// cores, with operands in pieces that keep all 24 bits; everything else is FFMA).  They take every size;
 // they are the whole of the float32 path, and the fallback of the bfloat16 path for sizes
 // that the fast kernels refuse.
 //
@@ -254,8 +255,8 @@ __global__ void __launch_bounds__(128) gemm_rows_kernel(const TA* __restrict__ A
 }
 
 // ---------------------------------------------------------------------------------------
-// The float32 product, rows of whole 16-byte pieces (K % 4 == 0, aligned operands): the same FFMA arithmetic, every sum in
-// 32-bit, in an order fixed by the sizes.
+// The float32 product, rows of whole 16-byte pieces (K % 4 == 0, aligned operands): every sum in 32-bit, in an order fixed by the
+// sizes; FFMA up to 16 rows, the tensor cores on pieces beyond.
 //
 // Up to 16 rows: gemm_rows_f32_kernel streams W once.  A warp owns four rows of W and every KS-th 128-wide slice of K (the KS
 // warps of a group cover a row, so a narrow matrix still puts some 16 warps on every SM and a row's bytes are all on their way
@@ -649,10 +650,10 @@ static int gemm_rows_f32(const float* A, const float* W, float* C, int M, int N,
 }
 
 // The tiles of more rows: rows of a tile, and blocks that share a tile's K.
-// Tiles of 64 rows only where they come to two a SM (1,024 x 6,144 x 1,024: 350 us; 263 x 4,096 x 1,024: 98 us, 78 in tiles of
-// 32 rows, which waste less of the last tile and keep more warps an SM).  About a block an SM is enough (263 x 1,024 x 3,072 in tiles
-// of 32 rows on 148 SMs: 72 blocks 127 us, 144 in clusters of two 71, 288 in clusters of four 82); every block of a cluster keeps at
-// least 128 of K.
+// Tiles of 64 rows only where they come to two a SM (us, tiles of 32 and of 64: 263 x 4,096 x 1,024 49 and 95, 300 x 6,144 x 1,024 98
+// and 95, 512 x 6,144 143 and 135, 1,024 x 6,144 257 and 259).  About a block an SM is mostly enough (tiles of 32 by one, two, four and eight
+// blocks on 148 SMs: 200 x 1,024 x 2,048 67, 41, 30, 31; 263 x 1,024 x 3,072 99, 57, 62, 52; 263 x 4,096 x 1,024 49, 59, 64, 64; not so 600 x
+// 1,024 x 3,072, 140, 120, 98, 89); every block of a cluster keeps at least 128 of K.
 struct F32Plan { int rows, cluster; };
 static F32Plan gemm_f32_plan(int M, int N, int K, int sms) {
   const long long tiles_n = (N + 127LL) / 128;
@@ -1427,8 +1428,9 @@ __global__ void __launch_bounds__(256) attn_f32_kernel(
 // the 32 columns of four instructions (values) is the one in which a thread's numbers are neighbours in memory.  A row with a
 // score or result that is not finite is done again in 32 bits by a warp (attn_f32_row; two prompts of 150 tokens, all rows so, 32 -> 76 us,
 // 2,048 tokens 0.55 -> 3.07 ms, where the kernel above takes 2.5).  Two prompts of 150 tokens, 16 heads of 128: 70 -> 30 us, what is left is the latency of a page
-// (3.5 us: 192 products of pieces and 1,000 other instructions a warp); with four warps and 32 keys a turn 37 us (2,048 tokens 930
-// against 1,059), with the results scaled and divided by the threads that hold them, 64 divisions one after the other, 44.
+// (3.5 to 4.4 us: 192 products of pieces and 1,000 other instructions a warp); with four warps and 32 keys a turn 37 us (2,048 tokens of
+// 32 heads 930, where this took 1,059 and now takes 1,095), with the results scaled and divided by the threads that hold them, 64 divisions
+// one after the other, 44.
 // ---------------------------------------------------------------------------------------
 // one query row by one warp, 16 keys at a time: their keys and values are on the way together
 template <int HD>
@@ -1730,7 +1732,7 @@ extern "C" void sx_attn_f32_plan(int n_tokens, int nh, int nkv, int maxp, int sm
 // Tiles of 32 rows where a sequence brings 16 tokens and more on average and there are tiles for a third of the SMs, more where a tile
 // has several sequences, which it walks through one after the other (us, the kernel of eight lanes a key first; 16 heads of 128: 33
 // tokens 7.6 and 11.4, 65 14.9 and 14.5, 129 30.5 and 18.5, 300 95 and 29, 4 x 16 12.4 and 20.3, 16 x 16 41 and 21; 16 of 64: 65 8.5
-// and 9.1, 96 12.7 and 10.7; 32 of 64: 4 x 16 behind 500 47 and 54; 32 of 128: 64 23 and 12, 8 x 16 34 and 21, 2,048 4,246 and 1,059).
+// and 9.1, 96 12.7 and 10.7; 32 of 64: 4 x 16 behind 500 47 and 54; 32 of 128: 64 23 and 12, 8 x 16 34 and 21, 2,048 4,246 and 1,095).
 static bool attn_f32_tiles(int n_tokens, int n_seqs, int nh, int sms) {
   const long long per_seq = n_seqs > 0 ? n_tokens / n_seqs : 0, blocks = (n_tokens + 31LL) / 32 * nh;
   return per_seq >= 16 && blocks * (per_seq < 32 ? per_seq : 32) >= 32LL * sms / 3;

@@ -20,10 +20,11 @@
 //     results by the rows' factors;
 //   * attention: a block per (sequence, kv head, share of the pages); a warp takes 16 keys at a time, K and V come
 //     through the same ring (TMA, 128-byte swizzle); shares are merged by their blocks through the same tagged words.
-// Measured (one row, ms a step with head and sampling; five kernels a layer before): 0.6B, 28 layers, 200 keys 0.65 -> 0.54, 1,500
-// keys 0.67 -> 0.58; 4B, 36 layers, 200 keys 1.91 -> 1.62, 1,500 keys 1.95 -> 1.73 (4.9 TB/s; the weights alone take 1.24).  Two
-// rows 2.02 -> 1.85.  What is left at 4B: HBM idles while a layer's parts exchange (1 us from the last store to the last reader, six
-// times) and attention's few blocks work (8 us), beyond the 4 us that the ring holds.
+// Measured (ms a step with head and sampling, five kernels a layer -> this; one row): 0.6B, 28 layers, 200 keys 0.65 -> 0.56, 1,500
+// keys 0.67 -> 0.59; 1.7B 1.00 -> 0.83, 1.01 -> 0.85; 4B, 36 layers 1.90 -> 1.64, 1.94 -> 1.72 (7.5 GB in 1.58, 4.75 TB/s); 8B 3.18 ->
+// 2.60, 3.19 -> 2.69.  Two rows: 0.69 -> 0.59, 1.11 -> 0.90, 1.96 -> 1.76, 2.98 -> 2.74 at 200 keys; 7,000 keys 0.94 -> 0.82, 1.34 -> 1.16,
+// 2.26 -> 2.09, 3.30 -> 3.07.  Models of two or four layers 1 to 10 % shorter.  What is left: 11 to 12 us a layer beyond its bytes, at 0.6B
+// as at 4B: the parts' exchanges (1 us from the last store to the last reader, six times) and attention's few blocks, beyond what the ring holds.
 // What the warps of a block run is kept small (loops not unrolled, every part of the code in one place): a layer walks through all
 // of it once, and code that does not fit the instruction cache (32 KB) is fetched again in every layer:
 // the first form, 104 KB of code, took 0.78 ms a step where 52 KB took 0.64 (0.6B, 30 keys).  And warps wait suspended (mbarrier.try_wait, named barriers) where they can:

@@ -70,7 +70,7 @@ def residual_add(h: torch.Tensor, delta: torch.Tensor) -> None:
 def gemm_generic(a: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
                  out: Optional[torch.Tensor] = None, bias: Optional[torch.Tensor] = None, cap: float = 0.0) -> torch.Tensor:
     """``a[M, K] @ w[N, K].T`` (``+ bias``, float32 ``[N]``; then ``cap * tanh(. / cap)`` if ``cap > 0``) with 32-bit
-    accumulation on CUDA cores (no tensor cores)."""
+    sums; float32 operands keep all their bits (more than 16 rows: on the tensor cores, in pieces)."""
     require_cuda(a, w, out, bias)
     M, K = a.shape
     N, K2 = w.shape

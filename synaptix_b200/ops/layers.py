@@ -10,7 +10,8 @@ from ._lib import KernelError, c_int, check, fn, launcher, raw_stream, require_c
 
 # Rows a step: with more, every block's share of the activations (tagged words, twice their size) costs more than the kernel saves.
 # Measured with forms for four and eight rows, ms a step at 4B sizes and 1,100 keys: 4 rows 2.02 to 2.07 against 2.07 with five kernels
-# a layer, 8 rows 2.62 against 2.20 (0.6B: 0.72 to 0.80 against 0.76, 0.99 against 0.82).
+# a layer, 8 rows 2.62 against 2.20 (0.6B: 0.72 to 0.80 against 0.76, 0.99 against 0.82).  One and two rows are shorter at every size
+# measured: 0.6B, 1.7B, 4B, 8B and models of two layers, 30 to 7,000 keys (figures in the source).
 MAX_ROWS = 2
 NO_ROOM = 10006       # the library's code for a stream whose share of the SMs does not hold all blocks at once
 RECORD = 9            # 8-byte numbers a layer: q/k/v, o, gate and up, down; gains of norm1, norm2, q and k heads; first cache row
