@@ -1826,7 +1826,8 @@ static int attn_generic_any(const void* q, const void* k_pages, const void* v_pa
                             const int* positions, const int* seq_of_token, const int* block_table,
                             int maxp, int n_tokens, int nh, int nkv, int hd, float scale, int window,
                             int dt, int vd, float softcap, const float* sinks, int chunk, int out_stride, float out_scale,
-                            int n_seqs, const int* cu, const int* past, cudaStream_t stream) {
+                            int n_seqs, const int* cu, const int* past, int* launched, cudaStream_t stream) {
+  *launched = 1;
   if (n_tokens <= 0) return 0;
   if (hd <= 0 || hd > 512 || vd <= 0 || vd > 512 || nkv <= 0 || nh % nkv != 0 || nh > 65535 || out_stride < nh * vd)
     return SX_ERR_SIZE;
@@ -1843,6 +1844,7 @@ static int attn_generic_any(const void* q, const void* k_pages, const void* v_pa
       if (rc || mix.to <= mix.from) return rc;
       begin = mix.from;
       end = mix.to;
+      *launched = 2;
     }
 #define ATTN_F32(HD, R) attn_f32_launch<HD, R>((const float*)q, (const float*)k_pages, (const float*)v_pages, (float*)out, positions, \
                                                seq_of_token, block_table, maxp, begin, end, mix.tiles ? mix.few : 0, nh, nkv, scale, window, softcap, \
@@ -1870,19 +1872,21 @@ extern "C" int sx_attn_generic(const void* q, const void* k_pages, const void* v
                                const int* positions, const int* seq_of_token, const int* block_table,
                                int maxp, int n_tokens, int nh, int nkv, int hd, float scale, int window,
                                int dt, cudaStream_t stream) {
+  int launched;
   return attn_generic_any(q, k_pages, v_pages, out, positions, seq_of_token, block_table, maxp, n_tokens, nh, nkv, hd, scale,
-                          window, dt, hd, 0.f, nullptr, 0, nh * hd, 1.f, n_tokens, nullptr, nullptr, stream);
+                          window, dt, hd, 0.f, nullptr, 0, nh * hd, 1.f, n_tokens, nullptr, nullptr, &launched, stream);
 }
 
 // with the options the plain entry point leaves out (see the kernel's comment), how many sequences the tokens are of (at most: rows of
-// the block table), and in host memory, or null, the first token of each and the number of all, and the keys each had before
+// the block table), and in host memory, or null, the first token of each and the number of all, and the keys each had before; launched: how
+// many kernels it was
 extern "C" int sx_attn_generic_ex(const void* q, const void* k_pages, const void* v_pages, void* out,
                                   const int* positions, const int* seq_of_token, const int* block_table,
                                   int maxp, int n_tokens, int nh, int nkv, int hd, float scale, int window,
                                   int dt, int vd, float softcap, const float* sinks, int chunk, int out_stride,
-                                  float out_scale, int n_seqs, const int* cu, const int* past, cudaStream_t stream) {
+                                  float out_scale, int n_seqs, const int* cu, const int* past, int* launched, cudaStream_t stream) {
   return attn_generic_any(q, k_pages, v_pages, out, positions, seq_of_token, block_table, maxp, n_tokens, nh, nkv, hd, scale,
-                          window, dt, vd, softcap, sinks, chunk, out_stride, out_scale, n_seqs, cu, past, stream);
+                          window, dt, vd, softcap, sinks, chunk, out_stride, out_scale, n_seqs, cu, past, launched, stream);
 }
 
 // ---------------------------------------------------------------------------------------

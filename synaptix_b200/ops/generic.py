@@ -1,6 +1,7 @@
 """Python faces of the plain kernels in ``csrc/generic.cu`` (every size, float32 and bfloat16)."""
 from __future__ import annotations
 
+import ctypes
 from typing import Optional
 
 import torch
@@ -205,12 +206,14 @@ def attn_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, 
     if portions is not None and (len(starts) != block_table.shape[0] + 1 or len(past) != block_table.shape[0]):
         raise KernelError("attn_generic: one start a sequence and the number of tokens, one past a sequence")
     o = out if out_col == 0 else out.view(-1)[out_col:]
-    check(fn("generic", "sx_attn_generic_ex")(
+    launched = c_int(1)
+    code = fn("generic", "sx_attn_generic_ex")(
         ptr(q), ptr(k_pages), ptr(v_pages), ptr(o), ptr(positions), ptr(seq_of_token), ptr(block_table),
         c_int(block_table.shape[1]), c_int(T), c_int(nh), c_int(nkv), c_int(hd), c_float(scale),
         c_int(0 if window is None else int(window)), c_int(dt_code(q.dtype)), c_int(vd),
         c_float(0.0 if softcap is None else float(softcap)), ptr(sinks), c_int(0 if chunk is None else int(chunk)),
-        c_int(out.shape[1]), c_float(out_scale), c_int(block_table.shape[0]), starts, past, stream()), "attn_generic")
+        c_int(out.shape[1]), c_float(out_scale), c_int(block_table.shape[0]), starts, past, ctypes.byref(launched), stream())
+    check(code, "attn_generic", launches=launched.value)
     return out
 
 

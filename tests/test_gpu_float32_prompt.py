@@ -169,6 +169,22 @@ def test_steps_of_long_and_short_portions(nh, nkv, hd, known, past, new):
     assert (out.double().cpu() - want).abs().max() <= bound
 
 
+@pytest.mark.parametrize("past,new,kernels", [([0, 0], [70, 90], 1), ([0, 50], [90, 1], 2), ([9, 50], [1, 1], 1), ([0], [90], 1)])
+def test_kernels_of_a_step_are_counted(past, new, kernels):
+    from synaptix_b200 import ops
+
+    class Counter:
+        kernel_launches = 0
+    q, ks, vs, pos, sot = setup(40, 8, 64, past, new, 2)
+    run(q, ks, vs, pos, sot, past, new, 8, 64, 0.125, portions=portions(past, new))        # (loaded)
+    ops.set_launch_counter(Counter)
+    try:
+        run(q, ks, vs, pos, sot, past, new, 8, 64, 0.125, portions=portions(past, new))
+    finally:
+        ops.set_launch_counter(None)
+    assert Counter.kernel_launches == kernels
+
+
 @pytest.mark.parametrize("known", [False, True])
 def test_time_of_steps_of_long_and_short_portions(known):
     """A prompt of 500 tokens with twenty single tokens behind 1,000 others, or eight behind 6,000, costs about what either costs alone."""
